@@ -329,7 +329,6 @@ struct tg_mesh {
     cudaStream_t last_stream = nullptr;  // stream of the last call, used to free asynchronously
     int64_t V = 0, T = 0, E = -1, F = -1;
     int4 *tvs = nullptr;
-    int32_t *vt_win = nullptr;          // VT window table (window_count + 1 entries)
     // star processing order: vertices by first cell (see tg_star.cu)
     int32_t *vorder = nullptr;          // [V] vertex at each position (cell-less ones last)
     int64_t *pofs = nullptr;            // [V + 1] VT offsets in that order
@@ -827,7 +826,6 @@ tg_status tg_mesh_destroy(tg_mesh *m)
     cudaStream_t s = m->last_stream;
     for (auto &r : m->rel) free_rel(r, s, true);
     if (m->tvs) cudaFreeAsync(m->tvs, s);
-    if (m->vt_win) cudaFreeAsync(m->vt_win, s);
     if (m->vorder) cudaFreeAsync(m->vorder, s);
     if (m->pofs) cudaFreeAsync(m->pofs, s);
     if (m->vtp) cudaFreeAsync(m->vtp, s);
@@ -902,8 +900,6 @@ static tg_status mesh_create_impl(const int32_t *tv, int64_t T, int64_t V, int o
     scan_batch(&job, 1, m->scan, m->st, s);
     TRY(dalloc(&vt, 4 * T, s));
     launch_vt_fill(m->tvs, T, vt_off, occ, vt, s);
-    TRY(dalloc(&m->vt_win, window_count(4 * T, star_window()) + 1, s));
-    launch_window_starts(vt_off, V, 4 * T, star_window(), m->vt_win, s);
     // VT row sort, which also marks each vertex's star-order key; then the
     // star processing order: positions, row lengths, offsets, rows, windows
     uint2 *vrank;
@@ -912,7 +908,7 @@ static tg_status mesh_create_impl(const int32_t *tv, int64_t T, int64_t V, int o
     TRY(tmp.alloc(&vrank, nwk + 1));
     TRY(tmp.alloc(&vkey, V));
     TRY(tmp.alloc(&dcount, V));
-    launch_vt_sort(vt_off, m->vt_win, vt, V, 4 * T, m->tvs, vflag, vkey, heavy_cnt, s);
+    launch_vt_sort(vt_off, vt, V, m->tvs, vflag, vkey, heavy_cnt, s);
     {
         ScanJob jf{vflag, vrank, nwk, SCAN_POPC_RANK, 0};
         scan_batch(&jf, 1, m->scan, m->st, s);

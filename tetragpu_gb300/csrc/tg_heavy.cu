@@ -27,6 +27,7 @@
 #include <climits>
 
 #include "tg_internal.h"
+#include "tg_rowsort.h"
 
 namespace tg {
 namespace {
@@ -68,34 +69,6 @@ __device__ __forceinline__ void set_bit(uint32_t *bits, long long p)
 __device__ __forceinline__ bool pair_less(int2 a, int2 b)
 {
     return a.x < b.x || (a.x == b.x && a.y < b.y);
-}
-
-template <typename T, typename Less>
-__device__ void sift_down(T *a, int root, int n, Less less)
-{
-    while (true) {
-        int child = 2 * root + 1;
-        if (child >= n) return;
-        if (child + 1 < n && less(a[child], a[child + 1])) child++;
-        if (!less(a[root], a[child])) return;
-        const T t = a[root];
-        a[root] = a[child];
-        a[child] = t;
-        root = child;
-    }
-}
-
-// heapsort: O(n log n) whatever the input, no recursion, no extra memory
-template <typename T, typename Less>
-__device__ void heap_sort(T *a, int n, Less less)
-{
-    for (int start = n / 2 - 1; start >= 0; start--) sift_down(a, start, n, less);
-    for (int end = n - 1; end > 0; end--) {
-        const T t = a[0];
-        a[0] = a[end];
-        a[end] = t;
-        sift_down(a, 0, end, less);
-    }
 }
 
 // the run [lo, hi) of neighbour x in the sorted pairs (empty when absent)

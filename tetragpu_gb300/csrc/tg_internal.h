@@ -177,13 +177,11 @@ void launch_window_starts(const int64_t *off, int64_t rows, int64_t n_entries, i
                           int32_t *wbase2 = nullptr);
 int star_window();    // the window size of star pass A over VT
 int star_window_b();  // the window size of star pass B
-// sort every VT row (tg_star.cu): window-staged, coalesced.  Also marks each
-// vertex's star-order key 4 * (lowest cell) + (slot in it) in vflag (4T bits,
-// zeroed by the caller) and stores it in vkey[v]; rows with no cells are left
-// alone.
-void launch_vt_sort(const int64_t *vt_off, const int32_t *win, int32_t *vt, int64_t V,
-                    int64_t nvt, const int4 *tvs, uint32_t *vflag, int64_t *vkey, int32_t *heavy_cnt,
-                    cudaStream_t s);
+// sort every VT row (tg_star.cu).  Also marks each vertex's star-order key
+// 4 * (lowest cell) + (slot in it) in vflag (4T bits, zeroed by the caller)
+// and stores it in vkey[v]; rows with no cells are left alone.
+void launch_vt_sort(const int64_t *vt_off, int32_t *vt, int64_t V, const int4 *tvs,
+                    uint32_t *vflag, int64_t *vkey, int32_t *heavy_cnt, cudaStream_t s);
 // Star processing order (vertices by first cell): vorder[pos] = vertex and
 // dcount[pos] = its row length, pos = rank of its key; vtp = VT rows in that
 // order, pofs = its offsets (rows with no cells last, length 0)

@@ -36,6 +36,7 @@
 //   k_edge_offsets  the id-ordered pass over edge occurrence slots: ET / EF /
 //             EE offsets and EV (one pass with a look-back scan)
 #include "tg_internal.h"
+#include "tg_rowsort.h"
 
 namespace tg {
 namespace {
@@ -815,59 +816,47 @@ __device__ __forceinline__ void mark_first(const int4 *__restrict__ tvs, uint32_
     atomicOr(vflag + (key >> 5), 1u << (key & 31));
 }
 
-// Sort every VT row ascending.  Rows starting in a window are staged in
-// shared memory and each entry lands at its rank in its row (cells in a row
-// are distinct); windows holding more than kCap entries fall back to an
-// insertion sort per row in global memory.  A block's time is mostly a chain
-// of dependent loads (window, offsets, cells, first cells): small blocks put
-// more chains in flight per SM.
+// Sort every VT row ascending, a row to a thread (tg_rowsort.h).  A block's
+// kVtsThreads rows are contiguous: they pass through shared memory so that
+// global memory sees whole rows; rows that do not fit are sorted in place.
+// Bound by its memory accesses (the rows once each way and a gathered cell per
+// vertex); ranking every entry against its row by a loop over shared memory
+// instead was issue-bound: 362 -> 137 us at 128^3 (12.6M cells), 70 -> 22 us on the
+// 64^3 coned mesh.
 constexpr int kVtsThreads = TG_VTS_THREADS;
+constexpr int kVtsCap = 32 * kVtsThreads;
 __global__ void __launch_bounds__(kVtsThreads)
-k_vt_sort(const int64_t *__restrict__ vt_off, const int *__restrict__ win, int *__restrict__ vt,
+k_vt_sort(const int64_t *__restrict__ vt_off, int64_t V, int *__restrict__ vt,
           const int4 *__restrict__ tvs, uint32_t *__restrict__ vflag, int64_t *__restrict__ vkey,
           int *__restrict__ heavy_cnt)
 {
     griddep_wait();
-    __shared__ int cell[kCap], out[kCap], meta[kCap];
-    // every thread reads the window's bounds itself (the same words)
-    const int s_vlo = win[blockIdx.x], s_vhi = win[blockIdx.x + 1];
-    const long long base = vt_off[s_vlo];
-    const int n = (int)(vt_off[s_vhi] - base);
-    if (n > kCap) {
-        for (int v = s_vlo + threadIdx.x; v < s_vhi; v += blockDim.x) {
-            const int64_t b = vt_off[v], e = vt_off[v + 1];
-            for (int64_t i = b + 1; i < e; i++) {
-                const int x = vt[i];
-                int64_t j = i - 1;
-                while (j >= b && vt[j] > x) {
-                    vt[j + 1] = vt[j];
-                    j--;
-                }
-                vt[j + 1] = x;
-            }
-            if (e > b) mark_first(tvs, vflag, vkey, heavy_cnt, v, vt[b], e - b);
-        }
-        return;
-    }
-    for (int v = s_vlo + threadIdx.x; v < s_vhi; v += blockDim.x) {
-        const int rs = (int)(vt_off[v] - base);
-        const int D = (int)(vt_off[v + 1] - vt_off[v]);
-        for (int i = 0; i < D; i++) meta[rs + i] = rs | (D << 10);
-    }
-    for (int e = threadIdx.x; e < n; e += blockDim.x) cell[e] = vt[base + e];
-    __syncthreads();
-    for (int e = threadIdx.x; e < n; e += blockDim.x) {
-        const int m = meta[e], rs = m_rs(m), D = m_D(m), x = cell[e];
-        int r = 0;
-        for (int j = rs; j < rs + D; j++) r += cell[j] < x;
-        out[rs + r] = x;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < n; e += blockDim.x) vt[base + e] = out[e];
-    for (int v = s_vlo + threadIdx.x; v < s_vhi; v += blockDim.x) {
-        const int64_t b = vt_off[v];
-        if (vt_off[v + 1] > b)
-            mark_first(tvs, vflag, vkey, heavy_cnt, v, out[b - base], vt_off[v + 1] - b);
+    __shared__ __align__(16) int cell[kVtsCap + 4];
+    const int64_t v0 = (int64_t)blockIdx.x * kVtsThreads;
+    const int64_t v1 = min(v0 + kVtsThreads, V);
+    const int64_t v = v0 + threadIdx.x;
+    const int64_t base = vt_off[v0];
+    const int64_t n = vt_off[v1] - base;
+    const int64_t b = v < V ? vt_off[v] : 0;
+    const int D = v < V ? (int)(vt_off[v + 1] - b) : 0;
+    const bool staged = n <= kVtsCap;   // block-uniform
+    // whole 16-byte words from the one holding the first entry (4T entries in
+    // all: the last word is whole)
+    const int shift = (int)(base & 3);
+    int *own = cell + shift + (int)(b - base);
+    if (staged) {
+        int4 *src = reinterpret_cast<int4 *>(vt + (base - shift));
+        const int words = (int)((n + shift + 3) >> 2);
+        for (int i = threadIdx.x; i < words; i += kVtsThreads)
+            reinterpret_cast<int4 *>(cell)[i] = src[i];
+        __syncthreads();
+        sort_rows_warp(own, D);
+        if (D > 0) mark_first(tvs, vflag, vkey, heavy_cnt, (int)v, own[0], D);
+        __syncthreads();
+        for (int i = threadIdx.x; i < (int)n; i += kVtsThreads) vt[base + i] = cell[shift + i];
+    } else {
+        sort_rows_warp(vt + b, D);
+        if (D > 0) mark_first(tvs, vflag, vkey, heavy_cnt, (int)v, vt[b], D);
     }
 }
 
@@ -1231,16 +1220,14 @@ void launch_star_b(const StarB &b, cudaStream_t s)
         launch_pdl(k_star_b<uint64_t>, n_windows_b(b.nvt), kThreads, 0, s, b);
 }
 
-void launch_vt_sort(const int64_t *vt_off, const int32_t *win, int32_t *vt, int64_t V,
-                    int64_t nvt, const int4 *tvs, uint32_t *vflag, int64_t *vkey, int32_t *heavy_cnt,
-                    cudaStream_t s)
+void launch_vt_sort(const int64_t *vt_off, int32_t *vt, int64_t V, const int4 *tvs,
+                    uint32_t *vflag, int64_t *vkey, int32_t *heavy_cnt, cudaStream_t s)
 {
     if (V == 0) return;
     Launch L("k_vt_sort", s);
-    launch_pdl(k_vt_sort, n_windows(nvt), kVtsThreads, 0, s, vt_off, win, vt, tvs, vflag, vkey,
-               heavy_cnt);
+    launch_pdl(k_vt_sort, (unsigned)((V + kVtsThreads - 1) / kVtsThreads), kVtsThreads, 0, s, vt_off,
+               V, vt, tvs, vflag, vkey, heavy_cnt);
 }
-
 
 void launch_vorder_place(const int64_t *vt_off, int64_t V, const int64_t *vkey,
                          const uint2 *vrank, int64_t nwk, const int32_t *heavy_cnt, int32_t *vorder,

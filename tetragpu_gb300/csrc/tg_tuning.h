@@ -27,7 +27,7 @@
 #define TG_EFA_LANES 2   // lanes per owned edge for its EF count in pass A
 #endif
 #ifndef TG_VTS_THREADS
-#define TG_VTS_THREADS 64   // threads per VT-sort block
+#define TG_VTS_THREADS 128   // threads per VT-sort block
 #endif
 #ifndef TG_EDGE_ITEMS
 #define TG_EDGE_ITEMS 8   // edge slots per thread of the edge-offset pass
