@@ -15,7 +15,7 @@ sin(ax) sin(by) sin(cz) + N(0, 1e-4).
   roofline  the whole path against HBM bandwidth: compulsory bytes of a step
             (TV and field read once, every output written once) / step time /
             the measured copy peak; `kernel` inside it is the dominant kernel
-            (k_star_b) on the compulsory bytes it is responsible for, timed
+            (k_star) on the compulsory bytes it is responsible for, timed
             live with CUDA events on its stream.
   e2e       the same steps through the C ABI with HOST buffers: pinned TV in
             through tg_mesh_create(tv_on_device = 0), the pinned field through
@@ -71,7 +71,7 @@ def load_workload(key: str):
     from tetragpu_gb300 import meshgen
     return WORKLOADS[key], (meshgen.workload_irregular() if key == "irregular"
                             else meshgen.workload_large())
-ROOFLINE_KERNEL = "k_star_b"
+ROOFLINE_KERNEL = "k_star"
 # CPU sample for the baseline legs: cells [0, SAMPLE_CELLS) of the same mesh
 # (a valid mesh itself), run through the oracle.
 SAMPLE_CELLS = 262144
@@ -188,13 +188,12 @@ def union_sizes(tg, batch) -> dict:
 def kernel_bytes(name: str, c: dict, tot: dict) -> int:
     """Compulsory bytes one launch of a kernel is responsible for: the path's
     inputs it reads once and the final outputs it writes once.  Intermediates
-    (pass A's candidate masks, the id-sorted incident edges, rank words,
-    offsets read back) are overhead and not credited.  k_star_b reads the
-    sorted TV (16 B per cell) and writes TE, TF, the ET entries, the VV
-    entries and every face's FT row."""
+    (first-occurrence bitmaps, edge records, rank words, offsets read back)
+    are overhead and not credited.  k_star reads the sorted TV (16 B per cell)
+    and VT (16 B per cell, 8 B per vertex); all it writes are intermediates."""
     V, E, F, T = c["V"], c["E"], c["F"], c["T"]
-    if name == "k_star_b":
-        return 16 * T + 4 * 6 * T + 4 * 4 * T + 4 * tot["ET"] + 4 * tot["VV"] + 8 * F
+    if name == "k_star":
+        return 16 * T + 4 * tot["VT"] + 8 * V
     raise KeyError(name)
 
 

@@ -331,12 +331,7 @@ struct tg_mesh {
     int4 *tvs = nullptr;
     // star processing order: vertices by first cell (see tg_star.cu)
     int32_t *vorder = nullptr;          // [V] vertex at each position (cell-less ones last)
-    int64_t *pofs = nullptr;            // [V + 1] VT offsets in that order
-    int32_t *vtp = nullptr;             // [4T] VT rows in that order
-    int32_t *st_win = nullptr;          // window table over pofs (star pass A)
-    int32_t *st_win_b = nullptr;        // the same for star pass B's windows
-    int32_t *st_wbase = nullptr;        // first entry of each pass A window
-    int32_t *st_wbase_b = nullptr;      // first entry of each pass B window
+    int32_t *heavy_off = nullptr;       // where each heavy star's entries start among theirs
     ScanWorkspace scan;                 // every prefix scan of the mesh (tg_scan.cu)
     // segments of cells (the meshes of a batch): cell starts, and after each
     // extraction their first edge and face ids (device, n_seg + 1 each)
@@ -347,7 +342,7 @@ struct tg_mesh {
     // stars of more than kMaxStar cells (tg_heavy.cu): processing positions
     // n_light .. n_light + n_heavy - 1, heavy_entries VT entries in all
     int64_t n_light = 0, n_heavy = 0, heavy_entries = 0;
-    bool wide_stars = false;    // a light star holds more than 32 cells (64-bit star masks)
+    bool wide_stars = false;    // a light star holds more than 32 cells (64-bit masks)
     int max_deg = 0;            // largest degree above kMaxDeg seen by the extraction, else 0
     uint64_t *cadj = nullptr;   // link adjacency for critical points, aligned with VV
     DevStatus *st = nullptr;    // device
@@ -468,7 +463,7 @@ tg_status build_link_adjacency(tg_mesh *m, const int64_t *vv_off, const int32_t 
     TRY(tmp.alloc(&ostart, V));
     TRY(tmp.alloc(&win, window_count(nvv, crit_window()) + 1));
     launch_vv_lengths_in_order(vv_off, m->vorder, V, m->n_light + m->n_heavy, len, ostart, s);
-    ScanJob job{len, ooff, V, SCAN_COUNT_I32, 0};
+    ScanJob job{len, ooff, V, SCAN_COUNT_I32, nullptr};
     scan_batch(&job, 1, m->scan, m->st, s);
     launch_window_starts(ooff, V, nvv, crit_window(), win, s);
     launch_crit_adj(vv_off, vv, m->vorder, ooff, ostart, win, V, nvv, m->cadj, m->st,
@@ -478,7 +473,7 @@ tg_status build_link_adjacency(tg_mesh *m, const int64_t *vv_off, const int32_t 
 
 tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
 {
-    const int64_t V = m->V, T = m->T, NVT = 4 * T;
+    const int64_t V = m->V, T = m->T;
     const bool tt_vertex = (opts & TG_OPT_TT_VERTEX_SHARING) != 0;
     const bool want_tt_face = (mask & TG_TT) && !tt_vertex;
     const uint32_t star_rel = TG_TE | TG_EV | TG_ET | TG_TF | TG_FV | TG_FE | TG_FT | TG_EF |
@@ -491,75 +486,73 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
 
     if (want_star) {
         // the status is clean: the read-back that ended the last call reset it
-        // ---- pass A: first occurrences, neighbour counts, ET/EF row lengths ----
+        // ---- star pass: first occurrences, edge records, neighbour counts ----
         const int64_t nwe = (6 * T + 31) / 32, nwf = (4 * T + 31) / 32;
         uint32_t *eflag, *fflag, *fbnd;
         uint2 *erank, *frank, *brank;
-        uint32_t *ecnt = nullptr;
-        int32_t *deg;
         int64_t *vv_off;
-        const bool need_ecnt = mask & (TG_ET | TG_EF | TG_EE);
+        // FE is read off each face's first cell (k_face_fill), which the
+        // face's FT row and the cell's TF row tell; EF off TF
+        const bool need_tf = (mask & (TG_TF | TG_FE | TG_FF | TG_EF)) || want_tt_face;
+        const bool need_ft = (mask & (TG_FT | TG_FE | TG_FF)) || want_tt_face;
+        const bool need_te = mask & (TG_TE | TG_FE);
+        const bool need_ev = mask & (TG_EV | TG_EE);
+        // the edges by id: for everything per edge
+        const bool need_edge = need_te || need_ev || (mask & (TG_ET | TG_EF));
+        StarPass sp{};
         {
-            // the bitmaps pass A sets bits in and the neighbour counts: one
-            // zeroed allocation (the row lengths are read only where pass A
-            // wrote them: no zeroing)
+            // the bitmaps the star pass sets bits in, the neighbour counts
+            // and the record counter: one zeroed allocation
             Carve c;
             const size_t o_e = c.add<uint32_t>(nwe), o_f = c.add<uint32_t>(nwf),
-                         o_b = c.add<uint32_t>(nwf), o_d = c.add<int32_t>(V);
+                         o_b = c.add<uint32_t>(nwf), o_d = c.add<int32_t>(V),
+                         o_i = c.add<int32_t>(V),
+                         o_v = c.add<uint8_t>(V), o_n = c.add<uint32_t>(1);
             char *z;
             TRY(tmp.alloc(&z, (int64_t)c.bytes, true));
             eflag = (uint32_t *)(z + o_e);
             fflag = (uint32_t *)(z + o_f);
             fbnd = (uint32_t *)(z + o_b);
-            deg = (int32_t *)(z + o_d);
+            sp.deg_own = (int32_t *)(z + o_d);
+            sp.deg_in = (int32_t *)(z + o_i);
+            sp.vbnd = (uint8_t *)(z + o_v);
+            sp.n_rec = (uint32_t *)(z + o_n);
         }
         TRY(tmp.alloc(&erank, nwe + 1));
         TRY(tmp.alloc(&frank, nwf + 1));
         TRY(tmp.alloc(&brank, nwf + 1));
-        if (need_ecnt) TRY(tmp.alloc(&ecnt, 6 * T));
         TRY(dalloc(&vv_off, V + 1, s));
         tmp.track(vv_off);  // owned by the VV relation once it is ready
         int64_t *deg_sq;  // prefix of deg^2: its total sizes EE (sum deg^2 - 2E)
         TRY(tmp.alloc(&deg_sq, V + 1));
-        // pass A's candidate masks, pass B's input: their low 32 bits for
-        // every entry, the high 32 for the entries of stars of more than 32
-        // cells (an array only when the mesh has such stars; only their
-        // entries of it are touched)
-        const bool narrow = !m->wide_stars;
-        uint32_t *emask, *emask_hi = nullptr;
-        TRY(tmp.alloc(&emask, 3 * NVT));
-        if (!narrow) TRY(tmp.alloc(&emask_hi, 3 * NVT));
-        StarA a{m->pofs, m->st_win, m->st_wbase, m->vorder, m->vtp, m->tvs, V, NVT, deg, ecnt,
-                eflag, fflag, fbnd, m->st, emask, emask_hi, narrow, NVT - m->heavy_entries};
-        if (!ecnt) {
-            // pass A always records row lengths; give it a throwaway buffer
-            TRY(tmp.alloc(&ecnt, 6 * T));
-            a.ecnt = ecnt;
-        }
-        launch_star_a(a, s);
+        // at most six edges a cell (their number is read back below)
+        TRY(tmp.alloc(&sp.rec, 6 * T));
+        TRY(tmp.alloc(&sp.place, 6 * T));
+        if (m->wide_stars || m->n_heavy > 0) TRY(tmp.alloc(&sp.rec_hi, 6 * T));
+        if (need_tf || need_ft) TRY(tmp.alloc(&sp.fnext, 4 * T));
+        sp.n_light = m->n_light;
+        sp.vorder = m->vorder;
+        sp.vt_off = vt_off;
+        sp.vt = vt;
+        sp.tvs = m->tvs;
+        sp.eflag = eflag;
+        sp.fflag = fflag;
+        sp.fbnd = fbnd;
+        sp.st = m->st;
+        launch_star(sp, s);
         HeavyStars hv{};
         if (m->n_heavy > 0) {
-            hv.n_light = m->n_light;
+            hv.star = sp;
             hv.n_heavy = m->n_heavy;
-            hv.pofs = m->pofs;
-            hv.vorder = m->vorder;
-            hv.vtp = m->vtp;
-            hv.tvs = m->tvs;
-            hv.st = m->st;
+            hv.heavy_off = m->heavy_off;
             TRY(tmp.alloc(&hv.pairs, 3 * m->heavy_entries));
-            TRY(tmp.alloc(&hv.ids, 6 * m->heavy_entries));
-            hv.deg = deg;
-            hv.ecnt = a.ecnt;
-            hv.eflag = eflag;
-            hv.fflag = fflag;
-            hv.fbnd = fbnd;
-            launch_heavy_a(hv, s);
+            launch_heavy(hv, s);
         }
-        ScanJob jobs[5] = {{deg, vv_off, V, SCAN_COUNT_I32, 0},
-                           {eflag, erank, nwe, SCAN_POPC_RANK, 0},
-                           {fflag, frank, nwf, SCAN_POPC_RANK, 0},
-                           {fbnd, brank, nwf, SCAN_POPC_RANK, 0},
-                           {deg, deg_sq, V, SCAN_SQUARE_I32, 0}};
+        ScanJob jobs[5] = {{sp.deg_own, vv_off, V, SCAN_COUNT_I32, sp.deg_in},
+                           {eflag, erank, nwe, SCAN_POPC_RANK, nullptr},
+                           {fflag, frank, nwf, SCAN_POPC_RANK, nullptr},
+                           {fbnd, brank, nwf, SCAN_POPC_RANK, nullptr},
+                           {sp.deg_own, deg_sq, V, SCAN_DEG_SQUARE, sp.deg_in}};
         scan_batch(jobs, 5, m->scan, m->st, s);
 
         // ---- the one synchronisation: edge, face, neighbour and boundary
@@ -579,53 +572,55 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         m->E = E;
         m->F = F;
         if (m->seg_c) launch_seg_ranks(m->seg_c, m->n_seg, erank, frank, m->seg_ef, s);
-        int64_t *et_off = nullptr, *ef_off = nullptr, *ee_off = nullptr;
-        // EF rows are read off ET rows and TF (k_ef_fill): ET, TF and EV are
-        // made for EF too
-        const bool need_et = mask & (TG_ET | TG_EF);
-        if (need_et) TRY(dalloc(&et_off, E + 1, s));
-        if (mask & TG_EF) TRY(dalloc(&ef_off, E + 1, s));
-        if (mask & TG_EE) TRY(dalloc(&ee_off, E + 1, s));
-        if (et_off) tmp.track(et_off);
-        if (ef_off) tmp.track(ef_off);
-        if (ee_off) tmp.track(ee_off);
-        // ---- pass B: ids, VV, fixed-width relations, ET rows ----
-        const bool need_ev = mask & (TG_EV | TG_EE | TG_EF);
-        const bool need_te = mask & (TG_TE | TG_FE);
-        // FV and FE are read off each face's first cell (k_face_fill), which
-        // the face's FT row and the cell's TF row tell
-        const bool need_tf = (mask & (TG_TF | TG_FV | TG_FE | TG_FF | TG_EF)) || want_tt_face;
-        const bool need_ft = (mask & (TG_FT | TG_FV | TG_FE | TG_FF)) || want_tt_face;
+
+        // ---- ids: VV, EV, row lengths (per edge); TF, FT, FV (per cell).
+        // Each kernel goes out once its own buffers exist; the later
+        // allocations are made while it runs
         int32_t *vv, *eid_sorted = nullptr;
         int32_t *ev = nullptr, *te = nullptr, *tf = nullptr, *fv = nullptr, *ft = nullptr;
-        int64_t *ff_off = nullptr;
-        // each kernel goes out once its own buffers exist; the later
-        // allocations are made while it runs
-        if (need_ev) TRY(tmp.alloc(&ev, 2 * E));
-        if (et_off || ef_off || ee_off || ev) {
-            uint2 *len;
-            TRY(tmp.alloc(&len, E));
-            launch_edge_offsets(eflag, ecnt, m->tvs, deg, erank, 6 * T, E, et_off, ef_off, ee_off,
-                                ev, len, m->scan, m->st, s);
-        }
         TRY(dalloc(&vv, nvv, s));
         tmp.track(vv);
-        if (mask & TG_EE) TRY(tmp.alloc(&eid_sorted, nvv));
-        if (need_te) TRY(tmp.alloc(&te, 6 * T));
+        int2 *inc = nullptr;
+        if (mask & TG_EE) {
+            TRY(tmp.alloc(&eid_sorted, nvv));
+            TRY(tmp.alloc(&inc, nvv));
+        }
+        EdgePass ep{};
+        if (need_edge) TRY(tmp.alloc(&ep.edge, E));
+        if (need_edge && sp.rec_hi) TRY(tmp.alloc(&ep.edge_hi, E));
+        ep.E = E;
+        ep.rec = sp.rec; ep.place = sp.place; ep.rec_hi = sp.rec_hi; ep.pairs = hv.pairs;
+        ep.vt_off = vt_off; ep.vt = vt; ep.tvs = m->tvs;
+        ep.erank = need_edge ? erank : nullptr;
+        ep.fflag = fflag; ep.fbnd = fbnd; ep.vbnd = sp.vbnd;
+        ep.vv_off = vv_off; ep.inc = inc; ep.vv = vv;
+        ep.count_ef = (mask & TG_EF) != 0;
+        launch_edge_ids(ep, s);
         if (need_tf) TRY(tmp.alloc(&tf, 4 * T));
-        if (mask & TG_FV) TRY(tmp.alloc(&fv, 3 * F));
         if (need_ft) TRY(tmp.alloc(&ft, 2 * F));
-        if (mask & TG_FF) TRY(tmp.alloc(&ff_off, F + 1));
-        // CSR totals: ET = 6T, EF = 3F always; EE from the scan (read back
-        // only when EE is wanted); TT and FF from the boundary-face count
+        if (mask & TG_FV) TRY(tmp.alloc(&fv, 3 * F));
+        if (tf || ft || fv) launch_cell_faces(T, m->tvs, frank, sp.fnext, tf, ft, fv, s);
+        int64_t *et_off = nullptr, *ef_off = nullptr, *ee_off = nullptr, *ff_off = nullptr;
+        if (mask & TG_ET) TRY(dalloc(&et_off, E + 1, s));
+        if (et_off) tmp.track(et_off);
+        if (mask & TG_EF) TRY(dalloc(&ef_off, E + 1, s));
+        if (ef_off) tmp.track(ef_off);
+        if (mask & TG_EE) TRY(dalloc(&ee_off, E + 1, s));
+        if (ee_off) tmp.track(ee_off);
+        if (need_ev) TRY(tmp.alloc(&ev, 2 * E));
+        if (et_off || ef_off || ee_off || ev)
+            launch_edge_offsets(ep, et_off, ef_off, ee_off, ev, m->scan, m->st, s);
+        launch_vv_sort(vv_off, V, nvv, inc, vv, eid_sorted, s);
+        // CSR totals: ET = 6T, EF = 3F always; TT and FF from the
+        // boundary-face count
         int32_t *et = nullptr, *ef = nullptr, *ee = nullptr, *ff = nullptr, *tt = nullptr,
                 *fe = nullptr;
         int64_t *tt_off = nullptr;
         const int64_t n_et = 6 * T, n_ef = 3 * F;
         const int64_t n_tt = 4 * T - n_bnd, n_ff = 3 * (2 * F - n_bnd);
+        if (need_te) TRY(tmp.alloc(&te, 6 * T));
         if (et_off) TRY(dalloc(&et, n_et, s));
         if (ef_off) TRY(dalloc(&ef, n_ef, s));
-        if (et && !(mask & TG_ET)) tmp.track(et);   // a temporary for EF (et_off is tracked)
         if (mask & TG_FE) TRY(dalloc(&fe, 3 * F, s));
         if (want_tt_face) {
             TRY(dalloc(&tt_off, T + 1, s));
@@ -633,30 +628,9 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
             if (T == 0) CK(cudaMemsetAsync(tt_off, 0, 8, s));
         }
         if (mask & TG_FF) {
+            TRY(tmp.alloc(&ff_off, F + 1));
             TRY(dalloc(&ff, n_ff, s));
             if (T == 0) CK(cudaMemsetAsync(ff_off, 0, 8, s));
-        }
-        StarB b{};
-        b.pofs = m->pofs; b.win = m->st_win_b; b.wbase = m->st_wbase_b; b.vorder = m->vorder;
-        b.vtp = m->vtp;
-        b.tvs = m->tvs; b.V = V; b.nvt = NVT;
-        b.vv_off = vv_off; b.erank = erank; b.frank = frank; b.brank = brank;
-        b.emask = emask; b.emask_hi = emask_hi; b.narrow = narrow; b.vv = vv; b.eid_sorted = eid_sorted;
-        b.te = te; b.tf = tf; b.ft = ft;
-        b.et_off = et_off; b.et = et; b.st = m->st;
-        launch_star_b(b, s);
-        if (m->n_heavy > 0) {
-            hv.vv_off = vv_off;
-            hv.erank = erank;
-            hv.frank = frank;
-            hv.vv = vv;
-            hv.eid_sorted = eid_sorted;
-            hv.te = te;
-            hv.tf = tf;
-            hv.ft = ft;
-            hv.et = et;
-            hv.et_off = et_off;
-            launch_heavy_b(hv, s);
         }
         tmp.keep(vv);
         tmp.keep(vv_off);
@@ -666,19 +640,19 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
             m->cadj = nullptr;
         }
 
-        // EF, the per-cell TT rows, the per-face FV / FE / FF rows and on
+        // ET and EF rows, the per-cell TT rows, the per-face FE / FF rows and on
         // request the link adjacency of critical points, on a side stream
-        // beside EE (each reads only what pass B and the passes before it
-        // wrote)
+        // beside EE (each reads only what the passes before it wrote)
         const int64_t n_ee = sum_deg_sq - 2 * E;   // deg(a) + deg(b) - 2 per edge (a,b)
         if (ee_off) TRY(dalloc(&ee, n_ee, s));
         const bool prep_adj = (opts & TG_OPT_LINK_ADJACENCY) && (mask & TG_VV);
         if (prep_adj) TRY(dalloc(&m->cadj, nvv, s));
-        if (fv || fe || tt || ff_off || ff || ef || prep_adj) {
+        if (te || fe || tt || ff_off || ff || et || ef || prep_adj) {
             const cudaStream_t s2 = side.fork();
-            if (ef) launch_ef_fill(ev, E, et_off, et, m->tvs, tf, ef_off, ef, s2);
+            ep.te = te; ep.et_off = et_off; ep.ef_off = ef_off; ep.et = et; ep.ef = ef; ep.tf = tf;
+            if (te || et || ef) launch_edge_rows(ep, s2);
             if (tt || ff_off) launch_cell_tt(T, F, tf, ft, brank, tt_off, tt, ff_off, s2);
-            if (fv || fe || ff) launch_face_fill(ft, tf, m->tvs, te, brank, F, fv, fe, ff_off, ff, s2);
+            if (fe || ff) launch_face_fill(ft, tf, te, brank, F, fe, ff_off, ff, s2);
             if (prep_adj) TRY(build_link_adjacency(m, vv_off, vv, nvv, tmp, s2));
         }
         if (ee_off) {
@@ -698,9 +672,8 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         if (mask & TG_FV) give_fixed(TG_REL_FV, fv, F);
         if (mask & TG_FT) give_fixed(TG_REL_FT, ft, F);
         if (fe) set_fixed(m, TG_REL_FE, fe, F);
-        if (et && (mask & TG_ET)) {
+        if (et) {
             tmp.keep(et_off);
-            tmp.keep(et);
             set_csr(m, TG_REL_ET, et_off, et, E, n_et);
         }
         if (ef) {
@@ -724,7 +697,7 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         TRY(tmp.alloc(&cnt, T));
         TRY(dalloc(&tt_off, T + 1, s));
         launch_tt_vertex_count(m->tvs, T, vt_off, vt, cnt, s);
-        ScanJob job{cnt, tt_off, T, SCAN_COUNT_I32, 0};
+        ScanJob job{cnt, tt_off, T, SCAN_COUNT_I32, nullptr};
         scan_batch(&job, 1, m->scan, m->st, s);
         const void *src[1] = {tt_off + T};
         const bool w8[1] = {true};
@@ -750,7 +723,6 @@ tg_status tg::critical_points_rows(tg_mesh *m, int64_t v0, int64_t nv, const voi
     if (v0 < 0 || nv < 0 || v0 + nv > m->V) return fail(TG_ERR_INVALID_ARGUMENT, "bad vertex range");
     m->last_stream = s;
     if (!m->rel[TG_REL_VV].ready) TRY(tg_extract(m, TG_VV, 0, s));
-    const int64_t V = m->V;
     const Rel &vv = m->rel[TG_REL_VV];
     if (!m->cadj) {
         TRY(dalloc(&m->cadj, vv.entries, s));
@@ -801,11 +773,11 @@ const char *tg_tuning_info(void)
     std::call_once(once, [] {
         char buf[512];
         snprintf(buf, sizeof buf,
-                 "{\"TG_STAR_WIN\": %d, \"TG_STAR_WIN_B\": %d, \"TG_STAR_THREADS\": %d, "
-                 "\"TG_EFA_LANES\": %d, \"TG_VTS_THREADS\": %d, \"TG_EDGE_ITEMS\": %d, "
+                 "{\"TG_STAR_WIN\": %d, \"TG_STAR_THREADS\": %d, \"TG_STAR_PER\": %d, "
+                 "\"TG_VTS_THREADS\": %d, \"TG_EDGE_ITEMS\": %d, "
                  "\"TG_ADJ_WIN\": %d, \"TG_ADJ_THREADS\": %d, \"TG_EE_GROUP\": %d}",
-                 TG_STAR_WIN, TG_STAR_WIN_B, TG_STAR_THREADS, TG_EFA_LANES, TG_VTS_THREADS,
-                 TG_EDGE_ITEMS, TG_ADJ_WIN, TG_ADJ_THREADS, TG_EE_GROUP);
+                 TG_STAR_WIN, TG_STAR_THREADS, TG_STAR_PER, TG_VTS_THREADS, TG_EDGE_ITEMS,
+                 TG_ADJ_WIN, TG_ADJ_THREADS, TG_EE_GROUP);
         info = buf;
     });
     return info.c_str();
@@ -827,12 +799,7 @@ tg_status tg_mesh_destroy(tg_mesh *m)
     for (auto &r : m->rel) free_rel(r, s, true);
     if (m->tvs) cudaFreeAsync(m->tvs, s);
     if (m->vorder) cudaFreeAsync(m->vorder, s);
-    if (m->pofs) cudaFreeAsync(m->pofs, s);
-    if (m->vtp) cudaFreeAsync(m->vtp, s);
-    if (m->st_win) cudaFreeAsync(m->st_win, s);
-    if (m->st_win_b) cudaFreeAsync(m->st_win_b, s);
-    if (m->st_wbase) cudaFreeAsync(m->st_wbase, s);
-    if (m->st_wbase_b) cudaFreeAsync(m->st_wbase_b, s);
+    if (m->heavy_off) cudaFreeAsync(m->heavy_off, s);
     if (m->seg_c) cudaFreeAsync(m->seg_c, s);
     if (m->seg_ef) cudaFreeAsync(m->seg_ef, s);
     if (m->cadj) cudaFreeAsync(m->cadj, s);
@@ -896,36 +863,22 @@ static tg_status mesh_create_impl(const int32_t *tv, int64_t T, int64_t V, int o
     int64_t *vt_off;
     int32_t *vt;
     TRY(dalloc(&vt_off, V + 1, s));
-    ScanJob job{deg_t, vt_off, V, SCAN_COUNT_I32, 0};
+    ScanJob job{deg_t, vt_off, V, SCAN_COUNT_I32, nullptr};
     scan_batch(&job, 1, m->scan, m->st, s);
     TRY(dalloc(&vt, 4 * T, s));
     launch_vt_fill(m->tvs, T, vt_off, occ, vt, s);
     // VT row sort, which also marks each vertex's star-order key; then the
-    // star processing order: positions, row lengths, offsets, rows, windows
+    // star processing order
     uint2 *vrank;
     int64_t *vkey;
-    int32_t *dcount;
     TRY(tmp.alloc(&vrank, nwk + 1));
     TRY(tmp.alloc(&vkey, V));
-    TRY(tmp.alloc(&dcount, V));
-    launch_vt_sort(vt_off, vt, V, m->tvs, vflag, vkey, heavy_cnt, s);
-    {
-        ScanJob jf{vflag, vrank, nwk, SCAN_POPC_RANK, 0};
-        scan_batch(&jf, 1, m->scan, m->st, s);
-        TRY(dalloc(&m->vorder, V, s));
-        launch_vorder_place(vt_off, V, vkey, vrank, nwk, heavy_cnt, m->vorder, dcount, s);
-        TRY(dalloc(&m->pofs, V + 1, s));
-        ScanJob jd{dcount, m->pofs, V, SCAN_COUNT_I32, 0};
-        scan_batch(&jd, 1, m->scan, m->st, s);
-        TRY(dalloc(&m->vtp, 4 * T, s));
-        launch_vtp_fill(m->vorder, m->pofs, V, vt_off, vt, m->vtp, s);
-        TRY(dalloc(&m->st_win, window_count(4 * T, star_window()) + 1, s));
-        TRY(dalloc(&m->st_win_b, window_count(4 * T, star_window_b()) + 1, s));
-        TRY(dalloc(&m->st_wbase, window_count(4 * T, star_window()) + 1, s));
-        TRY(dalloc(&m->st_wbase_b, window_count(4 * T, star_window_b()) + 1, s));
-        launch_window_starts(m->pofs, V, 4 * T, star_window(), m->st_win, s, star_window_b(),
-                             m->st_win_b, m->st_wbase, m->st_wbase_b);
-    }
+    TRY(dalloc(&m->heavy_off, 4 * T / (kMaxStar + 1) + 1, s));
+    launch_vt_sort(vt_off, vt, V, 4 * T, m->tvs, vflag, vkey, heavy_cnt, m->heavy_off, s);
+    ScanJob jf{vflag, vrank, nwk, SCAN_POPC_RANK, nullptr};
+    scan_batch(&jf, 1, m->scan, m->st, s);
+    TRY(dalloc(&m->vorder, V, s));
+    launch_vorder_place(vt_off, V, vkey, vrank, nwk, heavy_cnt, m->vorder, s);
     CK(cudaGetLastError());
     set_csr(m, TG_REL_VT, vt_off, vt, V, 4 * T);
     // vertices with light stars, heavy ones, the heavy stars' entries and

@@ -1,21 +1,20 @@
-// tg_heavy.cu -- the slow path for vertices the star windows do not hold.
+// tg_heavy.cu -- the slow path for vertices the star pass does not hold.
 //
-// The star passes (tg_star.cu) keep a vertex's star positions as bits of a
-// 64-bit mask, so they take stars of at most kMaxStar = 64 cells.  A vertex
+// The star pass (tg_star.cu) keeps an edge's star positions as bits of a
+// 64-bit mask, so it takes stars of at most kMaxStar = 64 cells.  A vertex
 // in more cells ("heavy") is placed after every other vertex in the star
-// processing order, the windows stop where the heavy rows begin, and the
-// kernels here do that vertex's share of both passes, one thread per heavy
-// vertex, serially over its star.  They write exactly what the star passes
-// would: the reference CPU path has no bound on a star
-// (src/cpu_extraction.cpp:259-289), and neither has this one.
+// processing order, and k_heavy does that vertex's share of the pass, one
+// thread per heavy vertex, serially over its star: the reference CPU path has
+// no bound on a star (src/cpu_extraction.cpp:259-289), and neither has this.
 //
 // A heavy vertex v with star cells c_0 < c_1 < ... (its sorted VT row, star
 // positions j) lists every (neighbour u, position j) pair of its star and
 // sorts them by neighbour, then position.  A neighbour's run is the list of
 // positions holding it, ascending, so
 //   * the run's first position is the first occurrence of edge (v, u)
-//     (its cell and pair slot give the id, as in the star passes),
-//   * the run is the ET row of (v, u) when v is the low end,
+//     (its cell and pair slot give the id, as in the star pass),
+//   * the run is the ET row of (v, u) when v is the low end; the edge's record
+//     names the run's first pair and its length in place of a mask,
 //   * the first common position of the runs of x and y is the first
 //     occurrence of face (v, x, y), the second its other cell.
 //
@@ -47,18 +46,6 @@ __device__ __forceinline__ int pair_slot(int s, int t)  // s < t, reference TE o
 __device__ __forceinline__ bool holds(const int4 &w, int x)
 {
     return w.x == x || w.y == x || w.z == x || w.w == x;
-}
-__device__ __forceinline__ int omitted_slot(const int4 &w, int a, int b, int c)
-{
-    if (w.x != a && w.x != b && w.x != c) return 0;
-    if (w.y != a && w.y != b && w.y != c) return 1;
-    if (w.z != a && w.z != b && w.z != c) return 2;
-    return 3;
-}
-__device__ __forceinline__ int rank_of(const uint2 *__restrict__ rk, long long p)
-{
-    const uint2 w = rk[p >> 5];
-    return (int)w.y + __popc(w.x & ((1u << (p & 31)) - 1u));
 }
 __device__ __forceinline__ void set_bit(uint32_t *bits, long long p)
 {
@@ -128,50 +115,32 @@ __device__ __forceinline__ void face_others(const int4 &w, int sv, int o, int &x
 
 // Is position r of run [s0, ...) the first cell of face (v, u, x)?  True
 // when no earlier cell of the run holds x.
-__device__ __forceinline__ bool first_with(const HeavyStars &h, const int *cells, const int2 *a,
-                                           int s0, int r, int x)
+__device__ __forceinline__ bool first_with(const int4 *tvs, const int *cells, const int2 *a, int s0,
+                                           int r, int x)
 {
     for (int r2 = s0; r2 < r; r2++)
-        if (holds(h.tvs[cells[a[r2].y]], x)) return false;
+        if (holds(tvs[cells[a[r2].y]], x)) return false;
     return true;
 }
 
-struct Star {
-    int v, D;
-    const int *cells;
-    int2 *pairs;
-    int *ids;   // 6 per star entry: edge id at each run's first pair, then the ids sorted
-};
-
-__device__ Star heavy_star(const HeavyStars &h, int k)
-{
-    Star s;
-    const int64_t n_light = h.n_light;
-    const int64_t heavy_base = h.pofs[n_light];
-    const int64_t i = n_light + k;
-    const int64_t b0 = h.pofs[i];
-    s.v = h.vorder[i];
-    s.D = (int)(h.pofs[i + 1] - b0);
-    s.cells = h.vtp + b0;
-    s.pairs = h.pairs + 3 * (b0 - heavy_base);
-    s.ids = h.ids ? h.ids + 6 * (b0 - heavy_base) : nullptr;
-    return s;
-}
-
-// Pass A's share: neighbour count, first-occurrence flags and the ET / EF row
-// lengths of the edges v owns, the first-occurrence and boundary flags of the
-// faces whose lowest vertex is v.
-__global__ void __launch_bounds__(64) k_heavy_a(HeavyStars h)
+// The star pass's share: neighbour counts, first-occurrence flags and records
+// of the edges v owns, the first-occurrence and boundary flags and second
+// cells of the faces whose lowest vertex is v.
+__global__ void __launch_bounds__(64) k_heavy(HeavyStars h)
 {
     griddep_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= h.n_heavy) return;
-    const Star s = heavy_star(h, k);
-    const int v = s.v;
-    int2 *a = s.pairs;
+    const StarPass &p = h.star;
+    const int v = p.vorder[p.n_light + k];
+    const int64_t b0 = p.vt_off[v];
+    const int D = (int)(p.vt_off[v + 1] - b0);
+    const int *cells = p.vt + b0;
+    const int64_t pair0 = 3LL * h.heavy_off[k];
+    int2 *a = h.pairs + pair0;
     int n = 0;
-    for (int j = 0; j < s.D; j++) {
-        const int4 w = h.tvs[s.cells[j]];
+    for (int j = 0; j < D; j++) {
+        const int4 w = p.tvs[cells[j]];
 #pragma unroll
         for (int t = 0; t < 4; t++) {
             const int x = get4(w, t);
@@ -179,42 +148,45 @@ __global__ void __launch_bounds__(64) k_heavy_a(HeavyStars h)
         }
     }
     heap_sort(a, n, pair_less);
-    int deg = 0;
+    int n_own = 0;
     for (int s0 = 0; s0 < n;) {
         const int u = a[s0].x;
         int s1 = s0 + 1;
         while (s1 < n && a[s1].x == u) s1++;
-        deg++;
         if (u > v) {   // v owns the edge
-            const int c0 = s.cells[a[s0].y];
-            const int4 w0 = h.tvs[c0];
-            const long long p = 6LL * c0 + pair_slot(slot_of(w0, v), slot_of(w0, u));
+            const int c0 = cells[a[s0].y];
+            const int4 w0 = p.tvs[c0];
+            const long long slot = 6LL * c0 + pair_slot(slot_of(w0, v), slot_of(w0, u));
             const int n_et = s1 - s0;
+            // an edge has at most twice as many faces as cells
             int n_ef = 0;
-            for (int r = s0; r < s1; r++) {
-                const int4 w = h.tvs[s.cells[a[r].y]];
+            if (2LL * n_et > 0xffff && n_et <= 0xffff)
+                for (int r = s0; r < s1; r++) {
+                    const int4 w = p.tvs[cells[a[r].y]];
 #pragma unroll
-                for (int t = 0; t < 4; t++) {
-                    const int x = get4(w, t);
-                    if (x != v && x != u) n_ef += first_with(h, s.cells, a, s0, r, x);
+                    for (int t = 0; t < 4; t++) {
+                        const int x = get4(w, t);
+                        if (x != v && x != u) n_ef += first_with(p.tvs, cells, a, s0, r, x);
+                    }
                 }
-            }
             if (n_et > 0xffff || n_ef > 0xffff) {
-                atomicOr(&h.st->flags, ST_STAR_OVERFLOW);
-                atomicMin(&h.st->bad_vertex, v);
+                atomicOr(&p.st->flags, ST_STAR_OVERFLOW);
+                atomicMin(&p.st->bad_vertex, v);
             }
-            set_bit(h.eflag, p);
-            h.ecnt[p] = (uint32_t)n_et | ((uint32_t)n_ef << 16);
+            set_bit(p.eflag, slot);
+            const unsigned g = atomicAdd(p.n_rec, 1u);
+            p.rec[g] = make_uint2((unsigned)slot, (unsigned)(pair0 + s0));
+            p.place[g] = make_uint2((unsigned)n_own++, (unsigned)atomicAdd(p.deg_in + u, 1));
+            p.rec_hi[g] = (unsigned)n_et;
         }
         s0 = s1;
     }
-    h.deg[v] = deg;
-    if (deg > kMaxDeg) atomicMax(&h.st->max_deg, deg);
+    p.deg_own[v] = n_own;
     // faces whose lowest vertex is v: v in slot 0 (omit 1, 2 or 3) or in
     // slot 1 (omit 0)
-    for (int j = 0; j < s.D; j++) {
-        const int c = s.cells[j];
-        const int4 w = h.tvs[c];
+    for (int j = 0; j < D; j++) {
+        const int c = cells[j];
+        const int4 w = p.tvs[c];
         const int sv = slot_of(w, v);
         if (sv > 1) continue;
         const int o_lo = sv == 0 ? 1 : 0, o_hi = sv == 0 ? 3 : 0;
@@ -226,80 +198,16 @@ __global__ void __launch_bounds__(64) k_heavy_a(HeavyStars h)
             const int cnt = common_positions(a, x0, x1, y0, y1, f1, f2);
             if (f1 != j) continue;
             const long long q = 4LL * c + (3 - o);
-            set_bit(h.fflag, q);
-            if (cnt == 1) set_bit(h.fbnd, q);
+            set_bit(p.fflag, q);
+            if (p.fnext) p.fnext[q] = f2 < 0 ? -1 : cells[f2];
+            if (cnt == 1) {
+                set_bit(p.fbnd, q);
+                p.vbnd[v] = p.vbnd[x] = p.vbnd[y] = 1;
+            }
             if (cnt > 2) {
-                atomicOr(&h.st->flags, ST_NONMANIFOLD_FACE);
-                atomicMin(&h.st->bad_cell, c);
+                atomicOr(&p.st->flags, ST_NONMANIFOLD_FACE);
+                atomicMin(&p.st->bad_cell, c);
             }
-        }
-    }
-}
-
-// Pass B's share (the pairs stay sorted from pass A): VV row, edge ids and
-// the id-sorted incident edges, TE of the pairs v is the low end of, TF and
-// FT of the faces whose lowest vertex is v, ET rows of the edges v owns (EF
-// rows come from k_ef_fill, as for every edge).
-__global__ void __launch_bounds__(64) k_heavy_b(HeavyStars h)
-{
-    griddep_wait();
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= h.n_heavy) return;
-    const Star s = heavy_star(h, k);
-    const int v = s.v;
-    const int2 *a = s.pairs;
-    const int n = 3 * s.D;
-    int *id_at = s.ids;               // id at each run's first pair
-    int *id_sorted = s.ids + n;       // ids in run order, then sorted
-    const int64_t vb = h.vv_off[v];
-    int r = 0;
-    for (int s0 = 0; s0 < n;) {
-        const int u = a[s0].x;
-        int s1 = s0 + 1;
-        while (s1 < n && a[s1].x == u) s1++;
-        const int c0 = s.cells[a[s0].y];
-        const int4 w0 = h.tvs[c0];
-        const int sv = slot_of(w0, v), su = slot_of(w0, u);
-        const int id = rank_of(h.erank, 6LL * c0 + pair_slot(min(sv, su), max(sv, su)));
-        if (h.vv) h.vv[vb + r] = u;
-        id_at[s0] = id;
-        id_sorted[r] = id;
-        if (u > v && h.et) {
-            const int64_t o = h.et_off[id];
-            for (int q = s0; q < s1; q++) h.et[o + (q - s0)] = s.cells[a[q].y];
-        }
-        r++;
-        s0 = s1;
-    }
-    const int deg = r;
-    if (h.eid_sorted) {
-        heap_sort(id_sorted, deg, [](int x, int y) { return x < y; });
-        for (int q = 0; q < deg; q++) h.eid_sorted[vb + q] = id_sorted[q];
-    }
-    for (int j = 0; j < s.D; j++) {
-        const int c = s.cells[j];
-        const int4 w = h.tvs[c];
-        const int sv = slot_of(w, v);
-        if (h.te) {
-            for (int t = sv + 1; t < 4; t++) {
-                int lo, hi;
-                run_of(a, n, get4(w, t), lo, hi);
-                h.te[6LL * c + pair_slot(sv, t)] = id_at[lo];
-            }
-        }
-        if (sv > 1 || (!h.tf && !h.ft)) continue;
-        const int o_lo = sv == 0 ? 1 : 0, o_hi = sv == 0 ? 3 : 0;
-        for (int o = o_lo; o <= o_hi; o++) {
-            int x, y, x0, x1, y0, y1, f1, f2;
-            face_others(w, sv, o, x, y);
-            run_of(a, n, x, x0, x1);
-            run_of(a, n, y, y0, y1);
-            common_positions(a, x0, x1, y0, y1, f1, f2);
-            if (f1 != j) continue;
-            const long long q = 4LL * c + (3 - o);
-            const int c2 = f2 < 0 ? -1 : s.cells[f2];
-            const int fid = face_at_first(h.frank, h.tf, h.ft, q, c, c2);
-            if (c2 >= 0 && h.tf) h.tf[4LL * c2 + (3 - omitted_slot(h.tvs[c2], v, x, y))] = fid;
         }
     }
 }
@@ -412,18 +320,11 @@ k_crit_heavy(const int64_t *__restrict__ vv_off, const int *__restrict__ vv,
 
 }  // namespace
 
-void launch_heavy_a(const HeavyStars &h, cudaStream_t s)
+void launch_heavy(const HeavyStars &h, cudaStream_t s)
 {
     if (h.n_heavy == 0) return;
-    Launch L("k_heavy_a", s);
-    launch_pdl(k_heavy_a, (unsigned)((h.n_heavy + 63) / 64), 64, 0, s, h);
-}
-
-void launch_heavy_b(const HeavyStars &h, cudaStream_t s)
-{
-    if (h.n_heavy == 0) return;
-    Launch L("k_heavy_b", s);
-    launch_pdl(k_heavy_b, (unsigned)((h.n_heavy + 63) / 64), 64, 0, s, h);
+    Launch L("k_heavy", s);
+    launch_pdl(k_heavy, (unsigned)((h.n_heavy + 63) / 64), 64, 0, s, h);
 }
 
 void launch_ee_heavy(const int32_t *ev, int64_t E, const int64_t *vv_off, const int32_t *eid,

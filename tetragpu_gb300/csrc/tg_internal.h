@@ -45,17 +45,18 @@ static_assert(kAdjWin >= 64 && kAdjWin <= 4096, "link-adjacency window size");
 
 // ---- scans (tg_scan.cu) ----
 enum ScanKind : int {
-    SCAN_COUNT_I32 = 0,  // in: int32 counts, out: int64 offsets [n + 1]
+    SCAN_COUNT_I32 = 0,  // in: int32 counts (+ in2's when given), out: int64 offsets [n + 1]
     SCAN_POPC_RANK = 1,  // in: uint32 bit words, out: uint2 {word, popcount prefix} [n + 1],
                          //     out[n] = {0, total}: rank of bit p = one 8-byte load
-    SCAN_SQUARE_I32 = 2  // in: int32 x, out: int64 prefix of x*x [n + 1]
+    SCAN_DEG_SQUARE = 2  // in: int32 x (+ in2's), out: int64 prefix of x*x [n + 1]; the largest
+                         //     x above kMaxDeg goes to the status word's max_deg
 };
 struct ScanJob {
     const void *in;
     void *out;
     int64_t n;
     int kind;
-    int pad;
+    const int32_t *in2;
 };
 constexpr int kMaxScanJobs = 8;
 // Exclusive scans of up to kMaxScanJobs arrays in one launch, over a
@@ -166,124 +167,107 @@ void launch_canon(const int32_t *tv_in, int64_t T, int64_t V, int4 *tvs, int32_t
                   int4 *occ, DevStatus *st, cudaStream_t s);
 void launch_vt_fill(const int4 *tvs, int64_t T, const int64_t *vt_off, const int4 *occ,
                     int32_t *vt, cudaStream_t s);
-void launch_sort_rows(const int64_t *off, int32_t *ent, int64_t n_rows, cudaStream_t s);
 // Windows of win_size entries over a CSR: win[w] = first row starting at or
-// after entry win_size * w (w = 0 .. window_count), win[window_count] = rows;
-// wbase[w] (when given) = that row's first entry, off[win[w]] (below 2^31).
+// after entry win_size * w (w = 0 .. window_count), win[window_count] = rows.
 int64_t window_count(int64_t n_entries, int win_size);
 void launch_window_starts(const int64_t *off, int64_t rows, int64_t n_entries, int win_size,
-                          int32_t *win, cudaStream_t s, int win_size2 = 0,
-                          int32_t *win2 = nullptr, int32_t *wbase = nullptr,
-                          int32_t *wbase2 = nullptr);
-int star_window();    // the window size of star pass A over VT
-int star_window_b();  // the window size of star pass B
+                          int32_t *win, cudaStream_t s);
 // sort every VT row (tg_star.cu).  Also marks each vertex's star-order key
 // 4 * (lowest cell) + (slot in it) in vflag (4T bits, zeroed by the caller)
-// and stores it in vkey[v]; rows with no cells are left alone.
-void launch_vt_sort(const int64_t *vt_off, int32_t *vt, int64_t V, const int4 *tvs,
-                    uint32_t *vflag, int64_t *vkey, int32_t *heavy_cnt, cudaStream_t s);
-// Star processing order (vertices by first cell): vorder[pos] = vertex and
-// dcount[pos] = its row length, pos = rank of its key; vtp = VT rows in that
-// order, pofs = its offsets (rows with no cells last, length 0)
+// and stores it in vkey[v]; rows with no cells are left alone.  A vertex of
+// more than kMaxStar cells takes no key: it is counted in heavy_cnt[0] (vkey
+// -1 - index) with its entries in heavy_cnt[1], where they start in
+// heavy_off[index].
+void launch_vt_sort(const int64_t *vt_off, int32_t *vt, int64_t V, int64_t nvt, const int4 *tvs,
+                    uint32_t *vflag, int64_t *vkey, int32_t *heavy_cnt, int32_t *heavy_off,
+                    cudaStream_t s);
+// sort VV rows in place, or with inc (EdgePass) write them and the
+// incident-edge rows sorted
+void launch_vv_sort(const int64_t *vv_off, int64_t V, int64_t nvv, const int2 *inc, int32_t *vv,
+                    int32_t *eid, cudaStream_t s);
+// Star processing order (vertices by first cell): vorder[pos] = vertex, pos =
+// rank of its key
 void launch_vorder_place(const int64_t *vt_off, int64_t V, const int64_t *vkey,
                          const uint2 *vrank, int64_t nwk, const int32_t *heavy_cnt, int32_t *vorder,
-                         int32_t *dcount, cudaStream_t s);
-void launch_vtp_fill(const int32_t *vorder, const int64_t *pofs, int64_t V, const int64_t *vt_off,
-                     const int32_t *vt, int32_t *vtp, cudaStream_t s);
+                         cudaStream_t s);
 
-struct StarA {
-    const int64_t *pofs;       // VT offsets in star processing order (rows + 1)
-    const int32_t *win;        // window table over pofs
-    const int32_t *wbase;      // first entry of each window
-    const int32_t *vorder;     // vertex at each processing position
-    const int32_t *vtp;        // VT rows in processing order
+// Star pass (tg_star.cu): the edges and faces of the light vertices.
+struct StarPass {
+    int64_t n_light;           // the light vertices: vorder[0 .. n_light)
+    const int32_t *vorder;
+    const int64_t *vt_off;
+    const int32_t *vt;
     const int4 *tvs;
-    int64_t V;
-    int64_t nvt;               // VT entries (4 * cells)
-    int32_t *deg;              // [V] neighbour counts (zeroed by the caller)
-    uint32_t *ecnt;            // [6T] ET | EF << 16 row lengths at owned edges' first slots
     uint32_t *eflag;           // bit per edge occurrence 6c+j (first occurrences)
     uint32_t *fflag;           // bit per face occurrence 4c+k (first occurrences)
     uint32_t *fbnd;            // bit per face occurrence: first and only (boundary face)
+    uint8_t *vbnd;             // [V] whether a vertex lies on a boundary face (zeroed)
+    int32_t *fnext;            // [4T] a face's second cell (-1: none) at its first
+                               // occurrence, or null
+    int32_t *deg_own;          // [V] edges a vertex is the low end of (zeroed by the caller)
+    int32_t *deg_in;           // [V] edges it is the high end of (zeroed by the caller)
+    // a record per edge, in no particular order (capacity 6T):
+    uint2 *rec;                // {first occurrence slot, star positions of the low end's star
+                               // holding the edge (the low 32)}
+    uint2 *place;              // {place among the low end's own edges, among the high end's others}
+    uint32_t *rec_hi;          // the high 32 positions; null when no star is wider than 32
+    uint32_t *n_rec;           // the number of records (zeroed by the caller)
     DevStatus *st;
-    uint32_t *emask;           // [3][nvt] star positions holding each entry's candidates
-                               // (the low 32 of a star's up to 64 positions)
-    uint32_t *emask_hi;        // [3][nvt] the high 32, written only for stars of more
-                               // than 32 cells; null when the mesh has none
-    bool narrow;               // no star holds more than 32 cells (emask_hi is null)
-    int64_t light_end;         // entries of the light stars (they come first): 4T - heavy entries
 };
-void launch_star_a(const StarA &a, cudaStream_t s);
+void launch_star(const StarPass &p, cudaStream_t s);
 // seg_ef[i] = first edge id and seg_ef[n + 1 + i] = first face id of the
 // cells from seg_c[i] on (i = 0 .. n; seg_c[n] = T gives the totals)
 void launch_seg_ranks(const int64_t *seg_c, int64_t n, const uint2 *erank, const uint2 *frank,
                       int64_t *seg_ef, cudaStream_t s);
 
-// ET / EF / EE offsets in edge-id order from one scan over the 6T edge slots
-// ET/EF/EE offsets in edge-id order in one pass (also EV when ev is given;
-// len: E scratch words); edge_offsets_words = the tile words it needs in the
-// scan workspace
-int64_t edge_offsets_words(int64_t n_slots);
-void launch_edge_offsets(const uint32_t *eflag, const uint32_t *ecnt, const int4 *tvs,
-                         const int32_t *deg, const uint2 *erank, int64_t n_slots, int64_t E,
-                         int64_t *et_off, int64_t *ef_off, int64_t *ee_off, int32_t *ev,
-                         uint2 *len, ScanWorkspace &ws, DevStatus *st, cudaStream_t s);
+// TF, FT and FV (each may be null) from the faces' first occurrences; fnext
+// as StarPass leaves it (may be null when neither TF nor FT is wanted)
+void launch_cell_faces(int64_t T, const int4 *tvs, const uint2 *frank, const int32_t *fnext,
+                       int32_t *tf, int32_t *ft, int32_t *fv, cudaStream_t s);
 
-struct StarB {
-    const int64_t *pofs;       // as in StarA
-    const int32_t *win;        // window table over pofs with star_window_b()
-    const int32_t *wbase;      // first entry of each window
-    const int32_t *vorder;
-    const int32_t *vtp;
+// Per-edge passes over the star pass's records.
+struct EdgePass {
+    int64_t E;
+    const uint2 *rec;
+    const uint2 *place;
+    const uint32_t *rec_hi;    // null: no star of more than 32 cells
+    const int2 *pairs;         // the heavy stars' pairs (tg_heavy.cu), or null
+    const int64_t *vt_off;
+    const int32_t *vt;
     const int4 *tvs;
-    int64_t V;
-    int64_t nvt;
+    const uint2 *erank;        // {bits, prefix} per 32 edge occurrences; null when no ids are
+                               // wanted (neither inc nor edge)
+    const uint32_t *fflag, *fbnd;
+    const uint8_t *vbnd;
     const int64_t *vv_off;
-    const uint2 *erank;        // {bits, prefix} per 32 edge occurrences
-    const uint2 *frank;        // same for face occurrences
-    const uint2 *brank;        // same for boundary-face occurrences
-    const uint32_t *emask;     // [3][nvt] from pass A, as in StarA
-    const uint32_t *emask_hi;
-    bool narrow;               // as in StarA
-    int32_t *vv;               // [2E] VV rows
-    int32_t *eid_sorted;       // [2E] incident edge ids sorted by id, or null
-    int32_t *te;               // [6T] or null
-    int32_t *tf;               // [4T] or null
-    int32_t *ft;               // [2F] or null
-    const int64_t *et_off;
-    int32_t *et;               // or null
-    DevStatus *st;
+    // ids
+    int2 *inc;                 // [2E] each vertex's {neighbour, edge id}, unsorted, or null:
+    int32_t *vv;               // [2E] VV rows, unsorted
+    uint4 *edge;               // [E] by id: the record, {ET | EF << 16, EE} row lengths; or null
+    uint32_t *edge_hi;         // [E] rec_hi by id (with rec_hi)
+    int count_ef;              // whether the EF lengths are wanted
+    // rows (each or null), of the edges by id
+    int32_t *te;               // [6T]
+    const int64_t *et_off, *ef_off;
+    int32_t *et, *ef;
+    const int32_t *tf;         // read for ef
 };
-void launch_star_b(const StarB &b, cudaStream_t s);
-
-// A face at its first cell c (occurrence q = 4c + TF column), c2 its
-// second cell or -1: its id is the rank of q among first occurrences; its
-// FT row and its TF entry in c are written here, the caller writes TF in c2.
-// Pass B and the heavy-star pass call it, once per face (FV and FE follow
-// and the FF offset in k_face_fill).
-__device__ __forceinline__ int face_at_first(const uint2 *__restrict__ frank, int32_t *tf,
-                                             int32_t *ft, long long q, int c, int c2)
-{
-    const uint2 w = __ldg(frank + (q >> 5));
-    const int fid = (int)w.y + __popc(w.x & ((1u << (q & 31)) - 1u));
-    if (tf) tf[q] = fid;
-    if (ft) *reinterpret_cast<int2 *>(ft + 2LL * fid) = make_int2(c, c2);
-    return fid;
-}
+void launch_edge_ids(const EdgePass &p, cudaStream_t s);
+void launch_edge_rows(const EdgePass &p, cudaStream_t s);
+// ET / EF / EE offsets and EV (each may be null) from the edges by id;
+// edge_offsets_words = the tile words it needs in the scan workspace
+int64_t edge_offsets_words(int64_t max_edges);
+void launch_edge_offsets(const EdgePass &e, int64_t *et_off, int64_t *ef_off, int64_t *ee_off,
+                         int32_t *ev, ScanWorkspace &ws, DevStatus *st, cudaStream_t s);
 
 // TT offsets (4c - boundary faces before cell c), TT rows (or null), and the
 // closing TT and FF offsets.
 void launch_cell_tt(int64_t T, int64_t F, const int32_t *tf, const int32_t *ft, const uint2 *brank,
                     int64_t *tt_off, int32_t *tt, int64_t *ff_off, cudaStream_t s);
-// EF rows (one thread per edge) from ET, the sorted TV and TF
-void launch_ef_fill(const int32_t *ev, int64_t E, const int64_t *et_off, const int32_t *et,
-                    const int4 *tvs, const int32_t *tf, const int64_t *ef_off, int32_t *ef,
-                    cudaStream_t s);
-// per face (each may be null): FV, FE, FF offsets (but the closing one) and
-// FF rows (ff_off and ff together)
-void launch_face_fill(const int32_t *ft, const int32_t *tf, const int4 *tvs, const int32_t *te,
-                      const uint2 *brank, int64_t F, int32_t *fv, int32_t *fe, int64_t *ff_off,
-                      int32_t *ff, cudaStream_t s);
+// per face (each may be null): FE, FF offsets (but the closing one) and FF
+// rows (ff_off and ff together)
+void launch_face_fill(const int32_t *ft, const int32_t *tf, const int32_t *te, const uint2 *brank,
+                      int64_t F, int32_t *fe, int64_t *ff_off, int32_t *ff, cudaStream_t s);
 void launch_ee_fill(const int32_t *ev, int64_t E, const int64_t *vv_off, const int32_t *eid_sorted,
                     const int64_t *ee_off, int32_t *ee, cudaStream_t s);
 void launch_tt_vertex_count(const int4 *tvs, int64_t T, const int64_t *vt_off, const int32_t *vt,
@@ -294,27 +278,14 @@ void launch_tt_vertex_fill(const int4 *tvs, int64_t T, const int64_t *vt_off, co
 // ---- heavy vertices (tg_heavy.cu) ----
 // Stars of more than kMaxStar cells: they follow every other vertex with
 // cells in the star processing order (positions n_light .. n_light +
-// n_heavy - 1), and these kernels do their share of star passes A and B.
+// n_heavy - 1), and k_heavy does their share of the star pass.
 struct HeavyStars {
-    int64_t n_light, n_heavy;
-    const int64_t *pofs;
-    const int32_t *vorder;
-    const int32_t *vtp;
-    const int4 *tvs;
-    int2 *pairs;               // 3 per heavy star entry: (neighbour, position), sorted by pass A
-    int32_t *ids;              // 6 per heavy star entry (pass B scratch)
-    DevStatus *st;
-    // pass A
-    int32_t *deg;
-    uint32_t *ecnt, *eflag, *fflag, *fbnd;
-    // pass B
-    const int64_t *vv_off;
-    const uint2 *erank, *frank;
-    int32_t *vv, *eid_sorted, *te, *tf, *ft, *et;
-    const int64_t *et_off;
+    StarPass star;             // n_light, the mesh and the star pass's outputs (rec_hi not null)
+    int64_t n_heavy;
+    const int32_t *heavy_off;  // where each heavy star's entries start among the heavy entries
+    int2 *pairs;               // 3 per heavy star entry: (neighbour, position), sorted here
 };
-void launch_heavy_a(const HeavyStars &h, cudaStream_t s);
-void launch_heavy_b(const HeavyStars &h, cudaStream_t s);
+void launch_heavy(const HeavyStars &h, cudaStream_t s);
 // EE rows of edges with an endpoint of more than kMaxDeg neighbours
 void launch_ee_heavy(const int32_t *ev, int64_t E, const int64_t *vv_off, const int32_t *eid,
                      const int64_t *ee_off, int32_t *ee, cudaStream_t s);

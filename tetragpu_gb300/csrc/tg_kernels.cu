@@ -17,11 +17,11 @@
 // Kernels, in pipeline order (one thread per cell/face/edge unless noted):
 //   k_canon        sort TV rows, validate ids, count cells per vertex
 //   k_vt_fill      scatter cells into VT rows (atomic cursors)
-//   k_sort_rows    sort each CSR row in place (VT, incident-edge rows)
-//   k_star_a/b/c   the per-vertex star passes (tg_star.cu)
+//   k_vt_sort, k_star, k_cell_faces, k_edge_ids, k_edge_offsets, k_vv_sort,
+//   k_edge_rows    the star pass and what follows it (tg_star.cu)
 //   k_cell_tt      face-sharing TT
-//   k_face_fill    FV, FE (from TE of a face's first cell), FF
-//   k_ef_fill      EF from ET and TF;  k_ee_fill  EE;
+//   k_face_fill    FE (from TE of a face's first cell), FF
+//   k_ee_fill      EE
 //   k_tt_vertex_*  vertex-sharing TT
 #include <algorithm>
 #include <climits>
@@ -145,7 +145,7 @@ k_canon(const int32_t *tv, int64_t T, int V, int4 *tvs, int *deg_t, int4 *occ, D
 }
 
 // ---------------------------------------------------------------------------
-// k_vt_fill / k_sort_rows
+// k_vt_fill
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
 k_vt_fill(const int4 *__restrict__ tvs, int64_t T, const int64_t *__restrict__ vt_off,
@@ -161,25 +161,6 @@ k_vt_fill(const int4 *__restrict__ tvs, int64_t T, const int64_t *__restrict__ v
     vt[vt_off[w.y] + o.y] = (int)c;
     vt[vt_off[w.z] + o.z] = (int)c;
     vt[vt_off[w.w] + o.w] = (int)c;
-}
-
-__global__ void __launch_bounds__(256)
-k_sort_rows(const int64_t *__restrict__ off, int *__restrict__ ent, int64_t n_rows)
-{
-    griddep_wait();
-    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < n_rows) {
-        const int64_t b = off[r], e = off[r + 1];
-        for (int64_t i = b + 1; i < e; i++) {
-            const int x = ent[i];
-            int64_t j = i - 1;
-            while (j >= b && ent[j] > x) {
-                ent[j + 1] = ent[j];
-                j--;
-            }
-            ent[j + 1] = x;
-        }
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -233,61 +214,17 @@ k_cell_tt(int64_t T, int64_t F, const int *__restrict__ tf, const int *__restric
         if (i < n) row[i] = nbr[i];
 }
 
-// EF rows, a thread per edge e = (a, b): walk its ET row (cells ascending)
-// and take at each cell the two faces holding a and b (the columns omitting
-// one of the other two slots), smaller id first, keeping an id only when it
-// exceeds the last one kept.  A face's id is the rank of its first
-// occurrence (4 * cell + column), so a face first met at this cell has a
-// larger id than every face met before, and a face met again (its second
-// cell) has an id no larger than the last kept: the row comes out ascending
-// with each face once.
-__global__ void __launch_bounds__(256)
-k_ef_fill(const int2 *__restrict__ ev, int64_t E, const int64_t *__restrict__ et_off,
-          const int *__restrict__ et, const int4 *__restrict__ tvs, const int *__restrict__ tf,
-          const int64_t *__restrict__ ef_off, int *__restrict__ ef)
-{
-    griddep_wait();
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= E) return;
-    const int2 ab = __ldg(ev + e);
-    const int64_t r0 = __ldg(et_off + e), r1 = __ldg(et_off + e + 1);
-    int *out = ef + __ldg(ef_off + e);
-    int last = -1, n = 0;
-    for (int64_t r = r0; r < r1; r++) {
-        const int c = __ldg(et + r);
-        const int4 w = __ldg(tvs + c);
-        // the slots of a and b (rows sorted, a < b), the other two t1 < t2
-        const int sa = (w.x < ab.x) + (w.y < ab.x) + (w.z < ab.x) + (w.w < ab.x);
-        const int sb = (w.x < ab.y) + (w.y < ab.y) + (w.z < ab.y) + (w.w < ab.y);
-        const int t1 = sa == 0 ? (sb == 1 ? 2 : 1) : 0;
-        const int t2 = 6 - sa - sb - t1;
-        // face omitting t: column 3 - t (t1 < t2: column 3 - t2 first)
-        const int f2 = __ldg(tf + 4LL * c + (3 - t2)), f1 = __ldg(tf + 4LL * c + (3 - t1));
-        const int lo = min(f1, f2), hi = max(f1, f2);
-        if (lo > last) {
-            out[n++] = lo;
-            last = lo;
-        }
-        if (hi > last) {
-            out[n++] = hi;
-            last = hi;
-        }
-    }
-}
-
 // Thread per face f (consecutive threads write consecutive rows): its first
 // cell c (FT[f][0]) and its column in c's TF row give the face's occurrence
-// slot q = 4c + column and its vertices (c's sorted slots but 3 - column);
-// FV from c's vertices, FE from c's TE row, the FF offset 3 * (2f - boundary
-// faces before f, counted over occurrence slots up to q) and the FF row (the
-// faces of both cells, f itself (once in each row) and a missing second
-// cell as INT_MAX, sorted by a 19-comparator network: the first 6 (interior)
-// or 3 (boundary) are the row).
+// slot q = 4c + column and its slots in c (all but 3 - column); FE from c's TE
+// row, the FF offset 3 * (2f - boundary faces before f, counted over
+// occurrence slots up to q) and the FF row (the faces of both cells, f itself
+// (once in each row) and a missing second cell as INT_MAX, sorted by a
+// 19-comparator network: the first 6 (interior) or 3 (boundary) are the row).
 __global__ void __launch_bounds__(256)
-k_face_fill(const int *__restrict__ ft, const int *__restrict__ tf, const int4 *__restrict__ tvs,
-            const int *__restrict__ te, const uint2 *__restrict__ brank, int64_t F,
-            int *__restrict__ fv, int *__restrict__ fe, int64_t *__restrict__ ff_off,
-            int *__restrict__ ff)
+k_face_fill(const int *__restrict__ ft, const int *__restrict__ tf, const int *__restrict__ te,
+            const uint2 *__restrict__ brank, int64_t F, int *__restrict__ fe,
+            int64_t *__restrict__ ff_off, int *__restrict__ ff)
 {
     griddep_wait();
     const int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -295,22 +232,14 @@ k_face_fill(const int *__restrict__ ft, const int *__restrict__ tf, const int4 *
     const int2 cells = reinterpret_cast<const int2 *>(ft)[f];
     const int4 w0 = reinterpret_cast<const int4 *>(tf)[cells.x];
     const int col = w0.x == (int)f ? 0 : (w0.y == (int)f ? 1 : (w0.z == (int)f ? 2 : 3));
-    if (fv || fe) {
+    if (fe) {
         // the face's slots in its first cell: all but 3 - col
         const int omit = 3 - col;
         const int s0 = omit == 0 ? 1 : 0, s1 = omit <= 1 ? 2 : 1, s2 = omit <= 2 ? 3 : 2;
-        if (fv) {
-            const int4 w = tvs[cells.x];
-            fv[3 * f] = get4(w, s0);
-            fv[3 * f + 1] = get4(w, s1);
-            fv[3 * f + 2] = get4(w, s2);
-        }
-        if (fe) {
-            const int *row = te + 6LL * cells.x;
-            fe[3 * f] = row[pair_slot(s0, s1)];
-            fe[3 * f + 1] = row[pair_slot(s0, s2)];
-            fe[3 * f + 2] = row[pair_slot(s1, s2)];
-        }
+        const int *row = te + 6LL * cells.x;
+        fe[3 * f] = row[pair_slot(s0, s1)];
+        fe[3 * f + 1] = row[pair_slot(s0, s2)];
+        fe[3 * f + 2] = row[pair_slot(s1, s2)];
     }
     if (!ff) return;
     const int64_t off = 3 * (2 * f - rank_of(brank, 4LL * cells.x + col));
@@ -688,19 +617,6 @@ void launch_vt_fill(const int4 *tvs, int64_t T, const int64_t *vt_off, const int
     }
 }
 
-void launch_sort_rows(const int64_t *off, int32_t *ent, int64_t n_rows, cudaStream_t s)
-{
-    if (n_rows == 0) return;
-    {
-        Launch L("k_sort_rows", s);
-        launch_pdl(k_sort_rows, blocks_for(n_rows, 256), 256, 0, s, off, ent, n_rows);
-    }
-}
-
-
-
-
-
 void launch_cell_tt(int64_t T, int64_t F, const int32_t *tf, const int32_t *ft, const uint2 *brank,
                     int64_t *tt_off, int32_t *tt, int64_t *ff_off, cudaStream_t s)
 {
@@ -712,25 +628,13 @@ void launch_cell_tt(int64_t T, int64_t F, const int32_t *tf, const int32_t *ft, 
     }
 }
 
-void launch_ef_fill(const int32_t *ev, int64_t E, const int64_t *et_off, const int32_t *et,
-                    const int4 *tvs, const int32_t *tf, const int64_t *ef_off, int32_t *ef,
-                    cudaStream_t s)
-{
-    if (E == 0) return;
-    Launch L("k_ef_fill", s);
-    launch_pdl(k_ef_fill, blocks_for(E, 256), 256, 0, s, reinterpret_cast<const int2 *>(ev), E,
-               et_off, et, tvs, tf, ef_off, ef);
-}
-
-void launch_face_fill(const int32_t *ft, const int32_t *tf, const int4 *tvs, const int32_t *te,
-                      const uint2 *brank, int64_t F, int32_t *fv, int32_t *fe, int64_t *ff_off,
-                      int32_t *ff, cudaStream_t s)
+void launch_face_fill(const int32_t *ft, const int32_t *tf, const int32_t *te, const uint2 *brank,
+                      int64_t F, int32_t *fe, int64_t *ff_off, int32_t *ff, cudaStream_t s)
 {
     if (F == 0) return;
     {
         Launch L("k_face_fill", s);
-        launch_pdl(k_face_fill, blocks_for(F, 256), 256, 0, s, ft, tf, tvs, te, brank, F, fv, fe,
-                   ff_off, ff);
+        launch_pdl(k_face_fill, blocks_for(F, 256), 256, 0, s, ft, tf, te, brank, F, fe, ff_off, ff);
     }
 }
 

@@ -28,17 +28,17 @@ struct ScanParams {
     unsigned long long *next;   // the other buffer, zeroed here for the next scan
     int64_t next_words;
     unsigned *err;
+    int *max_deg;
     int n_jobs;
 };
 
-__device__ __forceinline__ int64_t load_value(const ScanJob &j, int64_t i)
+__device__ __forceinline__ int64_t load_value(const ScanJob &j, int64_t i, int *max_deg)
 {
-    if (j.kind == SCAN_COUNT_I32) return (int64_t)__ldg((const int32_t *)j.in + i);
-    if (j.kind == SCAN_SQUARE_I32) {
-        const int64_t x = __ldg((const int32_t *)j.in + i);
-        return x * x;
-    }
-    return (int64_t)__popc(__ldg((const uint32_t *)j.in + i));
+    if (j.kind == SCAN_POPC_RANK) return (int64_t)__popc(__ldg((const uint32_t *)j.in + i));
+    const int x = __ldg((const int32_t *)j.in + i) + (j.in2 ? __ldg(j.in2 + i) : 0);
+    if (j.kind == SCAN_COUNT_I32) return x;
+    if (x > kMaxDeg) atomicMax(max_deg, x);
+    return (int64_t)x * x;
 }
 
 __device__ __forceinline__ void store_value(const ScanJob &j, int64_t i, int64_t v)
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kThreads) k_scan(ScanParams p)
     int64_t s = 0;
 #pragma unroll
     for (int k = 0; k < kItems; k++) {
-        v[k] = (base + k < j.n) ? load_value(j, base + k) : 0;
+        v[k] = (base + k < j.n) ? load_value(j, base + k, p.max_deg) : 0;
         s += v[k];
     }
     int64_t excl;
@@ -139,6 +139,7 @@ void scan_batch(const ScanJob *jobs, int n_jobs, ScanWorkspace &ws, DevStatus *s
     ScanParams p{};
     p.n_jobs = n_jobs;
     p.err = &st->flags;
+    p.max_deg = &st->max_deg;
     int64_t max_tiles = 1;
     unsigned long long *cur;
     scan_ws_begin(ws, s, &cur, &p.next, &p.next_words);

@@ -1,4 +1,5 @@
-// tg_star.cu -- the per-vertex "star" passes of the relation pipeline.
+// tg_star.cu -- the per-vertex "star" pass of the relation pipeline and the
+// per-edge and per-cell passes that follow it.
 //
 // The star of a vertex v is its VT row: the cells around v, ascending.  Every
 // cell that holds an edge or a face at v is in it, so within the star
@@ -9,68 +10,39 @@
 // which is what the reference CPU ids are ranks of (src/cpu_extraction.cpp:
 // 28-62 edges, 122-174 faces).
 //
-// Work decomposition: the VT rows, in star processing order (vertices by
-// first cell, see k_vorder_place), are cut into windows of kWin entries (kWinB
-// for pass B).  A block owns the vertices whose rows START in its window (at
-// most kWin + kMaxStar - 1 entries), stages their cells and the cells' sorted
-// TV rows in shared memory (all gathers in flight at once), and gives one
-// thread to each (vertex, star cell) entry.  In pass A a shared-memory hash
-// keyed by (vertex, neighbour) holds, per neighbour, the mask of star
-// positions whose cell contains it (32-bit in a window whose stars have at
-// most 32 cells, else 64-bit); lanes holding the same key are merged by
-// __match_any_sync first, so one lane per group touches the table.  Pass A
-// leaves every entry's three candidate masks in global memory (their low 32
-// bits for every entry, the high 32 in a second array for the entries of
-// stars of more than 32 cells) and pass B stages them instead of rebuilding
-// the table.  With the masks, "first
-// position holding u" is a count-trailing-zeros and "first position holding
-// x and y" a ctz of an AND.
+// An edge and a face belong to their lowest vertex: only that vertex's star
+// looks at them, so every edge and every face is found once.
 //
-//   k_star_a  first-occurrence bitmaps (edges owned by v = v is the low end,
-//             faces owned by v = v is the lowest vertex, boundary faces), the
-//             ET / EF row lengths at each owned edge's first-occurrence slot,
-//             neighbour counts, the candidate masks
-//   k_star_b  ids (ranks of first occurrences), sorted VV rows, id-sorted
-//             incident edge ids, TE, TF, ET rows, and at each face's first
-//             cell its FT row
-//   k_edge_offsets  the id-ordered pass over edge occurrence slots: ET / EF /
-//             EE offsets and EV (one pass with a look-back scan)
+//   k_star          a warp per vertex, a lane per star cell: the vertex's own
+//                   edges (each with the mask of star positions holding it)
+//                   and faces; first-occurrence bitmaps, a record per edge, a
+//                   face's second cell at its first occurrence
+//   k_cell_faces    a thread per cell: TF, FT and FV of the faces first met in
+//                   it (the face ids are ranks in the bitmap)
+//   k_edge_ids      a thread per edge record: its id, its entries in its ends'
+//                   incident rows, its row lengths
+//   k_edge_offsets  EV and the ET / EF / EE offsets: three sums over the
+//                   lengths in id order (one pass with a look-back scan)
+//   k_inc_sort      VV rows and incident-edge rows sorted
+//   k_edge_rows     a lane per cell of an edge: TE, the ET and EF rows
+#include <type_traits>
+
 #include "tg_internal.h"
 #include "tg_rowsort.h"
 
 namespace tg {
 namespace {
 
-constexpr int kWin = TG_STAR_WIN;         // VT entries per block window
-constexpr int kCap = kWin + kMaxStar;     // staged entries (rows starting in the window)
-// pass B keeps more per entry (neighbour lists, ids, work lists; no table),
-// and its windows are sized so that eight of its blocks share an SM
-constexpr int kWinB = TG_STAR_WIN_B;
-constexpr int kEfLanesA = TG_EFA_LANES;   // lanes per owned edge for its EF count (pass A)
-constexpr int kCapB = kWinB + kMaxStar;
-constexpr int kThreads = TG_STAR_THREADS;
-constexpr int kHashBits = TG_STAR_HASH_BITS;
-constexpr int kHash = 1 << kHashBits;     // (vertex, neighbour) slots per block, >= 3 * kCap
-constexpr unsigned long long kEmpty = ~0ull;
+constexpr unsigned kAll = 0xffffffffu;
+constexpr int kNarrowStar = 31;   // the most cells a star may have for one lane a cell
 
 __device__ __forceinline__ int get4(const int4 &w, int i)
 {
     return i == 0 ? w.x : (i == 1 ? w.y : (i == 2 ? w.z : w.w));
 }
-__device__ __forceinline__ int slot_of(const int4 &w, int u)
-{
-    return (w.x < u) + (w.y < u) + (w.z < u) + (w.w < u);
-}
 __device__ __forceinline__ int pair_slot(int s, int t)  // s < t, reference TE order
 {
     return s == 0 ? t - 1 : (s == 1 ? t + 1 : 5);
-}
-__device__ __forceinline__ int omitted_slot(const int4 &w, int a, int b, int c)
-{
-    if (w.x != a && w.x != b && w.x != c) return 0;
-    if (w.y != a && w.y != b && w.y != c) return 1;
-    if (w.z != a && w.z != b && w.z != c) return 2;
-    return 3;
 }
 // id of occurrence p: the set bits of the first-occurrence bitmap below p
 __device__ __forceinline__ int rank_of(const uint2 *__restrict__ rk, long long p)
@@ -78,717 +50,560 @@ __device__ __forceinline__ int rank_of(const uint2 *__restrict__ rk, long long p
     const uint2 w = __ldg(rk + (p >> 5));
     return (int)w.y + __popc(w.x & ((1u << (p & 31)) - 1u));
 }
-// Star-position masks: bit j = position j of a vertex's star.  A block
-// whose window holds only stars of at most 32 cells works with 32-bit masks
-// (the GPU's integer operations are 32-bit: a 64-bit and, shift or
-// find-first-set costs several instructions), any other with 64-bit ones
-// (stars of at most kMaxStar = 64 cells).  Both run the same templated code;
-// the masks in global memory are 64-bit either way.
 __device__ __forceinline__ int mctz(unsigned m) { return __ffs((int)m) - 1; }
 __device__ __forceinline__ int mctz(unsigned long long m) { return __ffsll((long long)m) - 1; }
-__device__ __forceinline__ int mpopc(unsigned m) { return __popc(m); }
-__device__ __forceinline__ int mpopc(unsigned long long m) { return __popcll(m); }
-constexpr int kNarrowStar = 32;   // the most cells a star may have for 32-bit masks
-
-// pass A's row-start metadata word, above the row start, length and slot
-// fields: the row's neighbour count (bits 22-29; at most 3 * kMaxStar = 192)
-// and whether v has a boundary face (bit 30)
-constexpr int kRowCount = 1 << 22;
-constexpr int kRowBoundary = 1 << 30;
-static_assert(3 * kMaxStar < 256, "the neighbour count must fit its 8 bits");
-
-// Pass A's shared memory: the fields that do not depend on the mask width
-// first (staged before the width is chosen), the masks last.
-struct StageBaseA {
-    int cell[kCap];
-    int4 tv[kCap];
-    int vid[kCap];
-    int meta[kCap];                     // row start | D << 10 | slot of v << 20
-    unsigned long long hkey[kHash];     // (row start << 32) | neighbour, kEmpty if free
-    short cslot[kCap][3];               // hash slot of each entry's 3 candidates (other vertices)
-    int n, vlo, vhi, full;
-    long long base;
-};
-template <typename M>
-struct Stage : StageBaseA {
-    M hmask[kHash];                     // star positions whose cell holds the neighbour
-};
-
-// static shared memory is capped at 48 KiB per block
-static_assert(sizeof(Stage<unsigned long long>) <= 48 * 1024,
-              "star stage exceeds the static shared-memory limit");
-static_assert(offsetof(StageBaseA, tv) % 16 == 0, "staged rows must be 16-byte aligned for cp.async");
-
-// Pass B stages the same window without a hash: pass A leaves every VT
-// entry's three candidate masks in global memory.  It also lists each
-// vertex's neighbours (at 3 * row start, the most a row of D cells can have
-// is 3D) with their edge ids.
-struct StageBaseB {
-    int cell[kCapB];
-    int4 tv[kCapB];
-    int vid[kCapB];
-    int meta[kCapB];                     // row start | D << 10 | slot of v << 20
-    int hv[kCapB][3];                    // at first sightings: list index, then edge id
-    int cnt[kCapB];
-    int list_u[3 * kCapB];               // neighbours, then (after pass 2) their edge ids
-    int work[3 * kCapB];                 // first sightings (list index << 11 | entry << 2 |
-                                        // candidate): n_owned
-                                        // owned ones (u > v) from the front, n_work others
-                                        // from the back
-    unsigned head[kCapB / 32 + 1];      // bit rs: a row starts at entry rs
-    int n, vlo, vhi, n_work, n_owned, wide;
-    int n_pairs, n_faces;               // the last phase's work lists
-    long long base;
-};
-template <typename M>
-struct StageM : StageBaseB {
-    M cm[kCapB][3];                      // star positions holding each candidate
-    // with 32-bit masks, room for each listed neighbour's first occurrence
-    // (6 cell + pair slot): phase 2 then ranks a first sighting among the
-    // row's edge ids (the order of their first occurrences) together with
-    // its VV rank, with no pass rewriting the lists as ids
-    int lkey[sizeof(M) == 4 ? 3 * kCapB : 1];
-};
-static_assert(sizeof(StageM<unsigned long long>) <= 48 * 1024,
-              "star stage B exceeds the static shared-memory limit");
-static_assert(offsetof(StageBaseB, tv) % 16 == 0, "staged rows must be 16-byte aligned for cp.async");
-
-__device__ __forceinline__ int m_rs(int m) { return m & 1023; }
-__device__ __forceinline__ int m_D(int m) { return (m >> 10) & 1023; }
-__device__ __forceinline__ int m_sv(int m) { return (m >> 20) & 3; }
-
-__device__ __forceinline__ unsigned hslot(unsigned long long key)
-{
-    return (unsigned)((key * 0x9E3779B97F4A7C15ull) >> (64 - kHashBits));
-}
-
-template <typename M>
-__device__ __forceinline__ int h_insert(Stage<M> &S, unsigned long long key, M bits)
-{
-    unsigned h = hslot(key);
-    for (int probe = 0; probe < kHash; probe++) {
-        const unsigned long long old = atomicCAS(&S.hkey[h], kEmpty, key);
-        if (old == kEmpty || old == key) {
-            atomicOr(&S.hmask[h], bits);
-            return (int)h;
-        }
-        h = (h + 1) & (kHash - 1);
-    }
-    return -1;
-}
-
-__device__ __forceinline__ unsigned long long hk(int rs, int u)
-{
-    return ((unsigned long long)(unsigned)rs << 32) | (unsigned)u;
-}
-
-// Pass B's rows: the row starts are marked in a bitmap (head), and an
-// entry's row start is the nearest mark at or below it (rows hold at most
-// kMaxStar entries, so the search looks at most three words back).  Only
-// the row starts' vid / meta are written by the rows; the other entries copy
-// theirs, all threads at once.
-__device__ __forceinline__ void fill_rows(const unsigned *head, int *vid, int *meta, int n)
-{
-    for (int e = threadIdx.x; e < n; e += blockDim.x) {
-        int w = e >> 5;
-        unsigned bits = head[w] & (0xffffffffu >> (31 - (e & 31)));
-        for (int k = 0; k < 3 && !bits && w > 0; k++) bits = head[--w];
-        const int rs = 32 * w + 31 - __clz(bits | 1u);
-        if (rs != e) {
-            vid[e] = vid[rs];
-            meta[e] = meta[rs];
-        }
-    }
-}
-
-// The staging in one barrier: the window ends at the next window's first
-// entry or at the first heavy star's (light_end: heavy stars come after every
-// light one), each row's thread writes its entries' row metadata itself, the
-// table's keys and masks are cleared beside the row loads (as G, the widest
-// masks this launch uses: 64-bit ones cover the 32-bit layout too), and
-// whether a star of the window holds more than kNarrowStar cells (returned,
-// block-uniform) comes from the barrier itself.
-template <typename G>
-__device__ int stage_rows_a1(StageBaseA &S, const StarA &a)
-{
-    const int plo = __ldg(a.win + blockIdx.x), phi = __ldg(a.win + blockIdx.x + 1);
-    const int base = __ldg(a.wbase + blockIdx.x);
-    const int n = (int)(min((int64_t)__ldg(a.wbase + blockIdx.x + 1), a.light_end) - base);
-    for (int e = threadIdx.x; e < n; e += blockDim.x) cp_async<4>(&S.cell[e], a.vtp + base + e);
-    cp_async_commit();
-    if (threadIdx.x == 0) {
-        S.vlo = plo;
-        S.vhi = phi;
-        S.base = base;
-        S.n = n;
-        S.full = 0;
-    }
-    G *hm = reinterpret_cast<Stage<G> &>(S).hmask;
-    for (int h = threadIdx.x; h < kHash; h += blockDim.x) {
-        S.hkey[h] = kEmpty;
-        hm[h] = 0;
-    }
-    int wide = 0;
-    for (int i = plo + threadIdx.x; i < phi; i += blockDim.x) {
-        const int rs = (int)(a.pofs[i] - base);
-        const int D = (int)(a.pofs[i + 1] - a.pofs[i]);
-        if (D == 0 || rs >= n) continue;   // a heavy star's row: tg_heavy.cu's
-        wide |= D > kNarrowStar;
-        const int v = a.vorder[i];
-        for (int k = 0; k < D; k++) {
-            S.vid[rs + k] = v;
-            S.meta[rs + k] = rs | (D << 10);
-        }
-    }
-    cp_async_wait();
-    for (int e = threadIdx.x; e < n; e += blockDim.x) cp_async<16>(&S.tv[e], a.tvs + S.cell[e]);
-    cp_async_commit();
-    cp_async_wait();
-    return __syncthreads_or(wide);
-}
-
-// Fill the (vertex, neighbour) table from the staged cells.  Returns
-// false (block-uniformly) when the table overflows.
-// Z: the table's masks were cleared by the staging (stage_rows_a1)
-template <typename M, bool Z>
-__device__ bool stage_cells_and_hash(Stage<M> &S, const int *__restrict__ vorder, DevStatus *st)
-{
-    const int n = S.n;
-    if constexpr (!Z) {
-        for (int h = threadIdx.x; h < kHash; h += blockDim.x) S.hmask[h] = 0;
-        __syncthreads();
-    }
-    // insert the 3 other vertices of every staged cell, keyed by the row
-    for (int e0 = 0; e0 < n; e0 += blockDim.x) {
-        const int e = e0 + threadIdx.x;
-        const bool act = e < n;
-        const unsigned amask = __ballot_sync(0xffffffffu, act);
-        if (!act) continue;
-        const int v = S.vid[e];
-        const int m = S.meta[e];
-        const int rs = m_rs(m);
-        const int4 w = S.tv[e];
-        const int sv = slot_of(w, v);
-        S.meta[e] = m | (sv << 20);
-        const int ewarp = e - (threadIdx.x & 31);  // entry of lane 0 of this warp
-        const int shift = ewarp - rs;               // lane l sits at row position l + shift
-        // the lanes holding this row's entries are contiguous: match on the
-        // neighbour alone and keep those lanes
-        const int lo = max(-shift, 0), hi = min(-shift + m_D(m), 32);
-        const unsigned rowmask = (hi >= 32 ? 0xffffffffu : ((1u << hi) - 1u)) & ~((1u << lo) - 1u);
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const int t = k + (k >= sv);
-            const int u = get4(w, t);
-            const unsigned long long key = hk(rs, u);
-            const unsigned grp = __match_any_sync(amask, u) & rowmask;
-            const int leader = __ffs(grp) - 1;
-            int h = 0;
-            if ((int)(threadIdx.x & 31) == leader) {
-                // the group's row positions (below the star's size, so
-                // within the mask's width)
-                const M bits = shift >= 0 ? (M)grp << shift : (M)grp >> -shift;
-                h = h_insert(S, key, bits);
-                if (h < 0) {
-                    S.full = 1;
-                    h = 0;
-                }
-            }
-            S.cslot[e][k] = (short)__shfl_sync(amask, h, leader);
-        }
-    }
-    __syncthreads();
-    if (S.full) {
-        if (threadIdx.x == 0) {
-            atomicOr(&st->flags, ST_HASH_FULL);
-            atomicMin(&st->bad_vertex, vorder[S.vlo]);
-        }
-        return false;
-    }
-    return true;
-}
-
-// Occurrence indices (6 cell + pair, 4 cell + column) fit 31 bits (at most
-// kMaxCells cells): pass A computes them in 32-bit arithmetic (in pass B the
-// 64-bit forms keep its register allocation free of spills).
-__device__ __forceinline__ void set_bit(uint32_t *bits, int p)
-{
-    atomicOr(bits + (p >> 5), 1u << (p & 31));
-}
-
-// candidate index (0..2) of slot t in a cell where v sits in slot sv (t != sv)
-__device__ __forceinline__ int cand_of(int t, int sv) { return t - (t > sv); }
-
-// The two vertices of a face owned by the vertex in slot sv with slot o omitted.
-__device__ __forceinline__ void face_others(const int4 &w, int sv, int o, int &x, int &y)
-{
-    x = -1;
-    y = -1;
-#pragma unroll
-    for (int t = 0; t < 4; t++)
-        if (t != sv && t != o) {
-            if (x < 0) x = get4(w, t); else y = get4(w, t);
-        }
-}
 
 // ---------------------------------------------------------------------------
-template <typename M>
-__device__ __forceinline__ void star_a_body(Stage<M> &S, const StarA &a, int &n_work)
+// k_star.  Lane l of a vertex's warp holds star cell l (and l + 32 in a star
+// of 32 to 64 cells) and, of that cell's vertices, those above v: the
+// candidates.  The warp takes its smallest candidate u (one warp reduction);
+// a ballot of the lanes whose cell holds u is the edge's mask, and its lowest
+// bit the lane of the first occurrence.  A vertex costs one such round of a
+// dozen instructions per edge it owns (seven on average in a grid) and nothing
+// is shared between warps but the record buffer; the block-wide hash of
+// (vertex, neighbour) pairs this replaces spent 600 warp instructions a vertex
+// on table inserts, work lists and barriers, and a second pass over it 840
+// more, doing every edge from both of its ends.
+//
+// The edges of a block's vertices gather in shared memory; at its end the
+// block takes their places in the high ends' incident rows, flags their first
+// occurrences and writes the records, every lane busy.  What does not fit
+// there goes out at once.
+constexpr int kStarThreads = TG_STAR_THREADS;
+constexpr int kStarPer = TG_STAR_PER;                       // vertices per warp, in sequence
+constexpr int kStarBlock = (kStarThreads / 32) * kStarPer;  // vertices per block
+constexpr int kRecCap = TG_STAR_WIN;                        // edges kept per block
+static_assert(kStarPer <= 32, "a warp fetches its vertices' rows a lane each");
+
+template <bool W>
+struct RecBuf {
+    uint4 e[kRecCap];   // first occurrence, mask (low), place among its low end's edges, high end
+    uint32_t hi[W ? kRecCap : 1];
+    int n;       // edges asked for
+    int end;     // first of those that did not fit
+    unsigned base;
+};
+
+__device__ __forceinline__ int4 load_cell(const int4 *__restrict__ tvs, int c)
 {
-    // in the hash keys' space once the table is built (only its masks are
-    // read after that): the first sightings of owned edges (entry << 2 |
-    // candidate); each row's neighbour count and boundary flag live in the
-    // high bits of its row start's metadata word (kRowCount, kRowBoundary),
-    // zero since the staging wrote it
-    static_assert(sizeof(S.hkey) >= 3 * kCap * sizeof(int), "work list does not fit the keys");
-    int *work = reinterpret_cast<int *>(S.hkey);
-    if (!stage_cells_and_hash<M, true>(S, a.vorder, a.st)) return;
-    const int n = S.n;
-    for (int e = threadIdx.x; e < n; e += blockDim.x) {
-        const int v = S.vid[e], m = S.meta[e];
-        const int rs = m_rs(m), sv = m_sv(m), pos = e - rs;
-        const int4 w = S.tv[e];
-        const int c = S.cell[e];
-        M cm[3];
+    return c >= 0 ? __ldg(tvs + c) : make_int4(-1, -1, -1, -1);
+}
+
+template <bool W>
+__device__ __forceinline__ void put_edge(const StarPass &p, const uint4 &e, unsigned hi, int64_t g)
+{
+    const unsigned in = (unsigned)atomicAdd(p.deg_in + e.w, 1);
+    atomicOr(p.eflag + (e.x >> 5), 1u << (e.x & 31));
+    p.rec[g] = make_uint2(e.x, e.y);
+    p.place[g] = make_uint2(e.z, in);
+    if constexpr (W) p.rec_hi[g] = hi;
+}
+
+// One vertex; H: cells per lane.
+template <int H, bool W>
+__device__ __forceinline__ void star_vertex(const StarPass &p, RecBuf<W> &S, int v,
+                                            const int (&c)[H], const int4 (&w)[H])
+{
+    using M = typename std::conditional<H == 1, unsigned, unsigned long long>::type;
+    // d: the candidates in slots 1..3 (slot 0 is never above another vertex
+    // of its cell); one that has been looked at turns into its mask, marked by
+    // the top bit (a candidate is below 2^31, and so is a narrow star's mask:
+    // at most kNarrowStar cells); with two cells a lane the marks and the
+    // masks are apart
+    constexpr unsigned kDone = 0x80000000u;
+    const int lane = threadIdx.x & 31;
+    unsigned d[H][3];
+    M m[H][3];
 #pragma unroll
-        for (int k = 0; k < 3; k++) {
-            cm[k] = S.hmask[S.cslot[e][k]];
-            a.emask[k * a.nvt + S.base + e] = (uint32_t)cm[k];
-            if constexpr (sizeof(M) == 8)
-                if (m_D(m) > kNarrowStar) a.emask_hi[k * a.nvt + S.base + e] = (uint32_t)(cm[k] >> 32);
-        }
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            if (mctz(cm[k]) != pos) continue;                  // not the first sighting
-            atomicAdd(&S.meta[rs], kRowCount);
-            if (get4(w, k + (k >= sv)) > v) work[atomicAdd(&n_work, 1)] = (e << 2) | k;
-        }
-        // a face at v held by this cell alone (the AND of its two other
-        // vertices' masks is this position's bit): v is on the boundary
-        const M bit = (M)1 << pos;
-        if ((cm[0] & cm[1]) == bit || (cm[0] & cm[2]) == bit || (cm[1] & cm[2]) == bit)
-            atomicOr(&S.meta[rs], kRowBoundary);
-        if (sv <= 1) {
-            // faces whose lowest vertex is v: omit slot 1, 2, 3 when v is in
-            // slot 0; omit slot 0 when v is in slot 1.  The face's other two
-            // vertices are two of this entry's candidates.
-            const int o_lo = sv == 0 ? 1 : 0, o_hi = sv == 0 ? 3 : 0;
-            for (int o = o_lo; o <= o_hi; o++) {
-                const int ko = cand_of(o, sv);      // the omitted candidate
-                const M mf = ko == 0 ? cm[1] & cm[2] : (ko == 1 ? cm[0] & cm[2] : cm[0] & cm[1]);
-                if (mctz(mf) != pos) continue;
-                const int q = 4 * c + (3 - o);
-                set_bit(a.fflag, q);
-                const int ncell = mpopc(mf);
-                if (ncell == 1) set_bit(a.fbnd, q);
-                if (ncell > 2) {
-                    atomicOr(&a.st->flags, ST_NONMANIFOLD_FACE);
-                    atomicMin(&a.st->bad_cell, c);
-                }
-            }
-        }
+    for (int h = 0; h < H; h++) {
+        d[h][0] = w[h].y > v ? (unsigned)w[h].y : kDone;
+        d[h][1] = w[h].z > v ? (unsigned)w[h].z : kDone;
+        d[h][2] = w[h].w > v ? (unsigned)w[h].w : kDone;
+        m[h][0] = m[h][1] = m[h][2] = 0;
     }
-    __syncthreads();
-    // the edges v owns, kEfLanesA lanes to an edge: flag the first
-    // occurrence and record the ET and EF row lengths at that occurrence
-    // slot.  At a vertex with no boundary face every face (v,u,x) lies in
-    // two cells of the edge's star and every cell holds two of them, so an
-    // edge has as many faces as cells; at a boundary vertex each lane takes
-    // every kEfLanesA-th cell of the edge's star and counts the faces (v,u,x)
-    // whose first cell it is.
-    const int nw = n_work;
-    constexpr int L = kEfLanesA;
-    const int span = ((nw * L + (int)blockDim.x - 1) / (int)blockDim.x) * (int)blockDim.x;
-    for (int tt = threadIdx.x; tt < span; tt += blockDim.x) {   // block-uniform trip count
-        const int i = tt / L, sub = tt % L;
-        int n_ef = 0;
+    while (true) {
+        unsigned cn = min(d[0][0], min(d[0][1], d[0][2]));
+        if constexpr (H == 2) cn = min(cn, min(d[1][0], min(d[1][1], d[1][2])));
+        const unsigned u = __reduce_min_sync(kAll, cn);
+        if (u >= kDone) break;
         M mu = 0;
-        int p = 0;
-        if (i < nw) {
-            const int e = work[i] >> 2, k = work[i] & 3;
-            const int m = S.meta[e];
-            const int rs = m_rs(m), sv = m_sv(m);
-            const int t = k + (k >= sv);
-            const int u = get4(S.tv[e], t);
-            mu = S.hmask[S.cslot[e][k]];
-            p = 6 * S.cell[e] + pair_slot(sv, t);
-            M mm = (S.meta[rs] & kRowBoundary) ? mu : 0;
-            if (!mm && sub == 0) n_ef = mpopc(mu);
-            for (int q = 0; q < sub; q++) mm &= mm - 1;
-            while (mm) {
-                const int j = mctz(mm);
-                const int ej = rs + j;
-                const int ku = cand_of(slot_of(S.tv[ej], u), m_sv(S.meta[ej]));
+        bool hit[H][3];
 #pragma unroll
-                for (int kk = 0; kk < 3; kk++) {
-                    if (kk == ku) continue;
-                    n_ef += mctz(mu & S.hmask[S.cslot[ej][kk]]) == j;
+        for (int h = 0; h < H; h++) {
+            hit[h][0] = (unsigned)w[h].y == u;
+            hit[h][1] = (unsigned)w[h].z == u;
+            hit[h][2] = (unsigned)w[h].w == u;
+            const unsigned b = __ballot_sync(kAll, hit[h][0] || hit[h][1] || hit[h][2]);
+            mu |= (M)b << (32 * h);
+        }
+#pragma unroll
+        for (int h = 0; h < H; h++)
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                if constexpr (H == 1) {
+                    d[h][k] = hit[h][k] ? (unsigned)mu | kDone : d[h][k];
+                } else {
+                    d[h][k] = hit[h][k] ? kDone : d[h][k];
+                    m[h][k] = hit[h][k] ? mu : m[h][k];
                 }
+            }
+    }
+    if constexpr (H == 1) {
 #pragma unroll
-                for (int q = 0; q < L; q++) mm &= mm - 1;
+        for (int k = 0; k < 3; k++) m[0][k] = d[0][k] & ~kDone;
+    }
+
+    // the edges first met in this lane's cells
+    unsigned first[H][3];
+    int total = 0;
+#pragma unroll
+    for (int h = 0; h < H; h++)
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const M low = m[h][k] & (0 - m[h][k]);
+            first[h][k] = __ballot_sync(kAll, low == (M)1 << (lane + 32 * h));
+            total += __popc(first[h][k]);
+        }
+    if (total) {   // warp-uniform
+        int at = 0;
+        if (lane == 0) {
+            at = atomicAdd(&S.n, total);
+            p.deg_own[v] = total;
+        }
+        at = __shfl_sync(kAll, at, 0);
+        const bool fits = at + total <= kRecCap;
+        int64_t g = 0;
+        if (!fits) {
+            unsigned base = 0u;
+            if (lane == 0) {
+                atomicMin(&S.end, at);
+                base = atomicAdd(p.n_rec, (unsigned)total);
+            }
+            g = (int64_t)__shfl_sync(kAll, base, 0);
+        }
+        int i0 = 0;
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+            const int sv = (w[h].x < v) + (w[h].y < v) + (w[h].z < v);
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                if ((first[h][k] >> lane) & 1u) {
+                    const int i = i0 + __popc(first[h][k] & ((1u << lane) - 1u));
+                    const uint4 e = make_uint4((unsigned)(6 * c[h] + pair_slot(sv, k + 1)),
+                                               (unsigned)m[h][k], (unsigned)i,
+                                               (unsigned)get4(w[h], k + 1));
+                    unsigned hi = 0u;
+                    if constexpr (H == 2) hi = (unsigned)(m[h][k] >> 32);
+                    if (fits) {
+                        S.e[at + i] = e;
+                        if constexpr (W) S.hi[at + i] = hi;
+                    } else {
+                        put_edge<W>(p, e, hi, g + i);
+                    }
+                }
+                i0 += __popc(first[h][k]);
             }
         }
-#pragma unroll
-        for (int off = 1; off < L; off <<= 1) n_ef += __shfl_xor_sync(0xffffffffu, n_ef, off);
-        if (i < nw && sub == 0) {
-            set_bit(a.eflag, p);
-            a.ecnt[p] = (uint32_t)mpopc(mu) | ((uint32_t)n_ef << 16);
-        }
     }
-    for (int e = threadIdx.x; e < n; e += blockDim.x) {
-        const int m = S.meta[e];
-        if (m_rs(m) != e) continue;
-        const int d = (m >> 22) & 255;
-        a.deg[S.vid[e]] = d;
-        // vertices of more than kMaxDeg neighbours take the heavy paths of
-        // EE and critical points (tg_heavy.cu); the largest degree tells the
-        // host whether to launch them
-        if (d > kMaxDeg) atomicMax(&a.st->max_deg, d);
+
+    // faces whose lowest vertex is v: two of the candidates, the third left
+    // out (v in slot 0: slot 1, 2 or 3; v in slot 1: slot 0; the masks of
+    // slots at or below v's are zero)
+#pragma unroll
+    for (int h = 0; h < H; h++) {
+        const M bit = (M)1 << (lane + 32 * h);
+        const int sh = 4 * (c[h] & 7);
+        unsigned firsts = 0u, alone = 0u;
+        M more = 0;
+        int *next = p.fnext + 4LL * c[h];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const M f = k == 0 ? m[h][1] & m[h][2] : (k == 1 ? m[h][0] & m[h][2] : m[h][0] & m[h][1]);
+            const M rest = f & (f - 1);
+            // the column of the face omitting slot o is 3 - o
+            const int col = k == 0 ? ((w[h].x == v) ? 2 : 3) : 2 - k;
+            const int s2 = H == 1 ? 31 - __clz((int)(unsigned)rest) : 63 - __clzll((long long)rest);
+            int c2 = __shfl_sync(kAll, c[0], s2 & 31);
+            if constexpr (H == 2) {
+                const int c2b = __shfl_sync(kAll, c[1], s2 & 31);
+                if (s2 >= 32) c2 = c2b;
+            }
+            if ((f ^ rest) == bit) {
+                firsts |= 1u << col;
+                if (!rest) alone |= 1u << col;
+                more |= rest & (rest - 1);
+                if (p.fnext) next[col] = rest ? c2 : -1;
+            }
+        }
+        if (firsts) atomicOr(p.fflag + (c[h] >> 3), firsts << sh);
+        if (alone) {   // boundary faces
+            atomicOr(p.fbnd + (c[h] >> 3), alone << sh);
+#pragma unroll
+            for (int col = 0; col < 4; col++)
+                if ((alone >> col) & 1u) {
+                    p.vbnd[col == 3 ? w[h].y : w[h].x] = 1;
+                    p.vbnd[col >= 2 ? w[h].z : w[h].y] = 1;
+                    p.vbnd[col >= 1 ? w[h].w : w[h].z] = 1;
+                }
+        }
+        if (more) {
+            atomicOr(&p.st->flags, ST_NONMANIFOLD_FACE);
+            atomicMin(&p.st->bad_cell, c[h]);
+        }
     }
 }
 
-// G: the widest candidate masks the launch keeps in shared memory (32-bit
-// when no star of the mesh holds more than kNarrowStar cells, so that no
-// window is wide; else 64-bit for the windows holding such a star)
-template <typename G>
-__global__ void __launch_bounds__(kThreads, 8) k_star_a(StarA a)
+// W: the mesh has stars of more than kNarrowStar cells
+template <bool W>
+__global__ void __launch_bounds__(kStarThreads, W ? 8 : TG_STAR_MINB) k_star(StarPass p)
 {
     griddep_wait();
-    // sized for the widest masks this instantiation uses (32-bit ones leave
-    // room for larger windows at eight blocks per SM)
-    __shared__ __align__(16) unsigned char raw[sizeof(Stage<G>)];
-    __shared__ int n_work;
-    StageBaseA &S = *reinterpret_cast<StageBaseA *>(raw);
-    if (threadIdx.x == 0) n_work = 0;   // ordered before its use by the staging's barrier
-    const int wide = stage_rows_a1<G>(S, a);
-
-    if constexpr (sizeof(G) == 8) {
-        if (wide) {   // block-uniform
-            star_a_body(*reinterpret_cast<Stage<unsigned long long> *>(raw), a, n_work);
-            return;
-        }
+    __shared__ RecBuf<W> S;
+    if (threadIdx.x == 0) {
+        S.n = 0;
+        S.end = kRecCap;
     }
-    star_a_body(*reinterpret_cast<Stage<unsigned> *>(raw), a, n_work);
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const int64_t pos = (int64_t)blockIdx.x * kStarBlock + (threadIdx.x >> 5) * kStarPer;
+    // lane k < kStarPer: the warp's k-th vertex, its row's start and length
+    int lv = -1, lrs = 0, lD = 0;
+    if (lane < kStarPer && pos + lane < p.n_light) {
+        lv = p.vorder[pos + lane];
+        lrs = (int)p.vt_off[lv];
+        lD = (int)(p.vt_off[lv + 1] - lrs);
+    }
+    auto load_entry = [&](int k) {   // this lane's cell of the k-th vertex (the first 32)
+        const int rs = __shfl_sync(kAll, lrs, k), D = __shfl_sync(kAll, lD, k);
+        return lane < D ? __ldg(p.vt + rs + lane) : -1;
+    };
+    // the next vertex's cells and the one after's row are in flight while a
+    // vertex is worked on
+    int c0 = load_entry(0), c1 = load_entry(1);
+    int4 w0 = load_cell(p.tvs, c0);
+#pragma unroll 1
+    for (int k = 0; k < kStarPer; k++) {
+        const int v = __shfl_sync(kAll, lv, k);
+        if (v < 0) break;
+        const int4 w1 = load_cell(p.tvs, c1);
+        const int c2 = k + 2 < kStarPer ? load_entry(k + 2) : -1;
+        bool done = false;
+        if constexpr (W) {
+            const int rs = __shfl_sync(kAll, lrs, k), D = __shfl_sync(kAll, lD, k);
+            if (D > kNarrowStar) {
+                const int cb = lane + 32 < D ? __ldg(p.vt + rs + lane + 32) : -1;
+                const int c[2] = {c0, cb};
+                const int4 w[2] = {w0, load_cell(p.tvs, cb)};
+                star_vertex<2, W>(p, S, v, c, w);
+                done = true;
+            }
+        }
+        if (!done) {
+            const int c[1] = {c0};
+            const int4 w[1] = {w0};
+            star_vertex<1, W>(p, S, v, c, w);
+        }
+        c0 = c1;
+        w0 = w1;
+        c1 = c2;
+    }
+    __syncthreads();
+    const int kept = min(S.n, S.end);
+    if (threadIdx.x == 0 && kept) S.base = atomicAdd(p.n_rec, (unsigned)kept);
+    __syncthreads();
+    for (int i = threadIdx.x; i < kept; i += kStarThreads)
+        put_edge<W>(p, S.e[i], W ? S.hi[i] : 0u, (int64_t)S.base + i);
 }
 
 // ---------------------------------------------------------------------------
-// Stage pass B's window: cells (copied asynchronously, issued first), rows
-// (and whether a star has more than kNarrowStar cells), then the cells'
-// vertices and the candidate masks pass A computed, copied asynchronously
-// as soon as this thread's cells have landed.  Pass A has already rejected
-// every window this cannot hold, so nothing here fails.  Cells are staged up
-// to the window's end before heavy rows clip it (at most kCapB entries).
-// The candidate masks into shared memory: 32-bit in a window whose stars
-// hold at most kNarrowStar cells (the low halves), else 64-bit, the high
-// half copied for the entries of stars of more than kNarrowStar cells and
-// zero for the others (which is what their high half is).  The wide form
-// reads each entry's row length, so its rows must be filled in.
-__device__ __forceinline__ void copy_masks(StageM<unsigned> &S, const StarB &b, int base, int nst)
-{
-    for (int e = threadIdx.x; e < nst; e += blockDim.x)
-#pragma unroll
-        for (int k = 0; k < 3; k++) cp_async<4>(&S.cm[e][k], b.emask + k * b.nvt + base + e);
-}
-__device__ __forceinline__ void copy_masks(StageM<unsigned long long> &S, const StarB &b, int base,
-                                           int nst)
-{
-    for (int e = threadIdx.x; e < nst; e += blockDim.x) {
-        const bool hi = m_D(S.meta[e]) > kNarrowStar;
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            unsigned *half = reinterpret_cast<unsigned *>(&S.cm[e][k]);   // little-endian
-            cp_async<4>(half, b.emask + k * b.nvt + base + e);
-            if (hi)
-                cp_async<4>(half + 1, b.emask_hi + k * b.nvt + base + e);
-            else
-                half[1] = 0u;
-        }
-    }
-}
-
-template <typename G>
-__device__ void stage_rows_b(unsigned char *raw, const StarB &b)
-{
-    StageBaseB &S = *reinterpret_cast<StageBaseB *>(raw);
-    const int plo = __ldg(b.win + blockIdx.x), phi = __ldg(b.win + blockIdx.x + 1);
-    const int base = __ldg(b.wbase + blockIdx.x);
-    const int nst = min(__ldg(b.wbase + blockIdx.x + 1) - base, kCapB);
-    for (int e = threadIdx.x; e < nst; e += blockDim.x) cp_async<4>(&S.cell[e], b.vtp + base + e);
-    cp_async_commit();
-    if (threadIdx.x == 0) {
-        S.vlo = plo;
-        S.vhi = phi;
-        S.base = base;
-        S.n = __ldg(b.wbase + blockIdx.x + 1) - base;
-        S.n_work = 0;
-        S.n_owned = 0;
-        S.n_pairs = 0;
-        S.n_faces = 0;
-        S.wide = 0;
-    }
-    for (int w = threadIdx.x; w < kCapB / 32 + 1; w += blockDim.x) S.head[w] = 0u;
-    __syncthreads();
-    for (int i = plo + threadIdx.x; i < phi; i += blockDim.x) {
-        const int rs = (int)(b.pofs[i] - base);
-        const int D = (int)(b.pofs[i + 1] - b.pofs[i]);
-        if (D == 0) continue;
-        if (D > kMaxStar) {   // heavy rows (all after this one) are tg_heavy.cu's
-            atomicMin(&S.n, rs);
-            continue;
-        }
-        if (D > kNarrowStar) S.wide = 1;
-        S.vid[rs] = b.vorder[i];
-        S.meta[rs] = rs | (D << 10);
-        S.cnt[rs] = 0;
-        atomicOr(&S.head[rs >> 5], 1u << (rs & 31));
-    }
-    cp_async_wait();
-    for (int e = threadIdx.x; e < nst; e += blockDim.x) cp_async<16>(&S.tv[e], b.tvs + S.cell[e]);
-    // with 32-bit masks in global memory every window is narrow; else the
-    // width is known once the rows are in
-    if constexpr (sizeof(G) == 4)
-        copy_masks(*reinterpret_cast<StageM<unsigned> *>(raw), b, base, nst);
-    cp_async_commit();
-    __syncthreads();
-    fill_rows(S.head, S.vid, S.meta, S.n);
-    if constexpr (sizeof(G) == 8) {
-        // each thread's own entries: their rows were filled in just above
-        if (S.wide)
-            copy_masks(*reinterpret_cast<StageM<unsigned long long> *>(raw), b, base, nst);
-        else
-            copy_masks(*reinterpret_cast<StageM<unsigned> *>(raw), b, base, nst);
-        cp_async_commit();
-    }
-    cp_async_wait();
-    __syncthreads();
-}
-
-// flat index (entry * 3 + candidate) of candidate u of entry e's first sighting
-template <typename M>
-__device__ __forceinline__ int first_slot(const StageM<M> &S, int e, int k, int rs, int u)
-{
-    const int f = rs + mctz(S.cm[e][k]);
-    if (f == e) return 3 * e + k;
-    return 3 * f + cand_of(slot_of(S.tv[f], u), m_sv(S.meta[f]));
-}
-
-// hv entry of candidate u of entry e: the one at u's first sighting in e's row
-template <typename M>
-__device__ __forceinline__ int hv_of(const StageM<M> &S, int e, int k, int rs, int u)
-{
-    const int f = rs + mctz(S.cm[e][k]);
-    if (f == e) return S.hv[e][k];
-    return S.hv[f][cand_of(slot_of(S.tv[f], u), m_sv(S.meta[f]))];
-}
-
-template <typename M>
-__device__ __forceinline__ void star_b_body(StageM<M> &S, const StarB &b)
-{
-    const int n = S.n;
-
-    // 1. list every vertex's neighbours (each at its first sighting); the
-    //    first sightings form one work list, owned edges (u > v) from the
-    //    front, the others from the back
-    for (int e = threadIdx.x; e < n; e += blockDim.x) {
-        const int v = S.vid[e], m = S.meta[e];
-        const int rs = m_rs(m), pos = e - rs;
-        const int4 w = S.tv[e];
-        const int sv = slot_of(w, v);
-        S.meta[e] = m | (sv << 20);
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            if (mctz(S.cm[e][k]) != pos) continue;
-            const int t = k + (k >= sv);
-            const int u = get4(w, t);
-            const int li = atomicAdd(&S.cnt[rs], 1);
-            S.list_u[3 * rs + li] = u;
-            if constexpr (sizeof(M) == 4)
-                S.lkey[3 * rs + li] = 6 * S.cell[e] + pair_slot(min(sv, t), max(sv, t));
-            S.hv[e][k] = li;
-            const int item = (li << 11) | (e << 2) | k;
-            if (u > v)
-                S.work[atomicAdd(&S.n_owned, 1)] = item;
-            else
-                S.work[3 * kCapB - 1 - atomicAdd(&S.n_work, 1)] = item;
-        }
-    }
-    __syncthreads();
-    const int n_owned = S.n_owned, n_first = n_owned + S.n_work;
-    auto first_item = [&](int i) {
-        return i < n_owned ? S.work[i] : S.work[3 * kCapB - 1 - (i - n_owned)];
-    };
-
-    // 2. every first sighting: edge id and VV position (with 32-bit masks also
-    //    its place among v's incident edge ids, for EE)
-    if constexpr (sizeof(M) == 4) {
-        for (int i = threadIdx.x; i < n_first; i += blockDim.x) {
-            const int it = first_item(i);
-            const int e = (it >> 2) & 511, k = it & 3;
-            const int v = S.vid[e], rs = m_rs(S.meta[e]);
-            const int u = S.list_u[3 * rs + (it >> 11)], p = S.lkey[3 * rs + (it >> 11)];
-            const int deg = S.cnt[rs];
-            const int *lu = S.list_u + 3 * rs, *lk = S.lkey + 3 * rs;
-            int rank = 0, er = 0;
-            for (int j = 0; j < deg; j++) {
-                rank += lu[j] < u;
-                er += lk[j] < p;
-            }
-            const int id = rank_of(b.erank, p);
-            S.hv[e][k] = id;
-            const long long vb = b.vv_off[v];
-            if (b.vv) b.vv[vb + rank] = u;
-            if (b.eid_sorted) b.eid_sorted[vb + er] = id;
-        }
-        __syncthreads();
-    } else {
-    for (int i = threadIdx.x; i < n_first; i += blockDim.x) {
-        const int it = first_item(i);
-        const int e = (it >> 2) & 511, k = it & 3;
-        const int v = S.vid[e], m = S.meta[e];
-        const int rs = m_rs(m), sv = m_sv(m);
-        const int t = k + (k >= sv);
-        const int u = get4(S.tv[e], t);
-        const int deg = S.cnt[rs];
-        const int *lu = S.list_u + 3 * rs;
-        int rank = 0;
-        for (int j = 0; j < deg; j++) rank += lu[j] < u;
-        S.hv[e][k] = rank_of(b.erank, 6LL * S.cell[e] + pair_slot(min(sv, t), max(sv, t)));
-        if (b.vv) b.vv[b.vv_off[v] + rank] = u;
-    }
-    __syncthreads();
-    // the neighbour lists become edge-id lists (for the id order of EE)
-    if (b.eid_sorted) {
-        for (int i = threadIdx.x; i < n_first; i += blockDim.x) {
-            const int it = first_item(i);
-            const int e = (it >> 2) & 511, k = it & 3;
-            S.list_u[3 * m_rs(S.meta[e]) + (it >> 11)] = S.hv[e][k];
-        }
-        __syncthreads();
-    }
-
-    // 3a. each first sighting's place among v's incident edge ids (for EE)
-    if (b.eid_sorted) {
-        for (int i = threadIdx.x; i < n_first; i += blockDim.x) {
-            const int it = first_item(i);
-            const int e = (it >> 2) & 511, k = it & 3;
-            const int rs = m_rs(S.meta[e]);
-            const int id = S.hv[e][k];
-            const int deg = S.cnt[rs];
-            const int *li = S.list_u + 3 * rs;
-            int r = 0;
-            for (int j = 0; j < deg; j++) r += li[j] < id;
-            b.eid_sorted[b.vv_off[S.vid[e]] + r] = id;
-        }
-        __syncthreads();
-    }
-    }
-    // 3b. the ET offsets of the edges v owns, once per edge, at its first
-    //     sighting (in the neighbour lists' space, free from here on; ET
-    //     offsets are below 6T < 2^31)
-    int *eto = S.list_u;
-    if (b.et) {
-        for (int i = threadIdx.x; i < n_owned; i += blockDim.x) {
-            const int it = S.work[i];
-            const int e = (it >> 2) & 511, k = it & 3;
-            eto[3 * e + k] = (int)b.et_off[S.hv[e][k]];
-        }
-        // with 32-bit masks the pair list below goes to the spent first
-        // occurrences, not over the owned edges this loop reads: no barrier
-        // between the two (the ET offsets' loads stay in flight meanwhile)
-        if constexpr (sizeof(M) != 4) __syncthreads();
-    }
-    // 3c. TE of the pairs v is the low end of and the entry's cell in those
-    //     edges' ET rows (its place: the star positions below it holding the
-    //     other end); TF / FT's second cell of the faces v owns, handled at
-    //     their first cell.  An entry holds 3 - sv such pairs and, at sv <= 1,
-    //     up to three faces, so a loop over entries would leave most lanes
-    //     idle; the pairs (entry << 2 | other slot) and the faces (entry << 2
-    //     | omitted slot) are listed first, in the spent first occurrences (or
-    //     first-sighting list) and row counts, and the lists run with every
-    //     lane busy.  A window
-    //     with more first-cell faces than the face list holds handles its
-    //     faces entry by entry.
-    const bool do_pairs = b.te || b.et, do_faces = b.tf || b.ft;
-    int *pairs = sizeof(M) == 4 ? S.lkey : S.work;   // <= 3 per entry
-    int *faces = S.cnt;    // <= kCapB, else the fallback below
-    for (int e = threadIdx.x; e < n; e += blockDim.x) {
-        const int m = S.meta[e];
-        const int rs = m_rs(m), sv = m_sv(m), pos = e - rs;
-        if (do_pairs && sv < 3) {
-            const int p0 = atomicAdd(&S.n_pairs, 3 - sv);
-            for (int t = sv + 1; t < 4; t++) pairs[p0 + t - sv - 1] = (e << 2) | t;
-        }
-        if (do_faces && sv <= 1) {
-            const int o_lo = sv == 0 ? 1 : 0, o_hi = sv == 0 ? 3 : 0;
-            for (int o = o_lo; o <= o_hi; o++) {
-                const int ko = cand_of(o, sv);
-                const int ka = ko == 0 ? 1 : 0, kb = ko == 2 ? 1 : 2;
-                if (mctz(S.cm[e][ka] & S.cm[e][kb]) != pos) continue;
-                const int q = atomicAdd(&S.n_faces, 1);
-                if (q < kCapB) faces[q] = (e << 2) | o;
-            }
-        }
-    }
-    __syncthreads();
-    const int n_pairs = S.n_pairs, n_faces = S.n_faces;
-    for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) {
-        const int it = pairs[i];
-        const int e = it >> 2, t = it & 3, k = t - 1;   // cand_of(t, sv) for t > sv
-        const int m = S.meta[e];
-        const int rs = m_rs(m), sv = m_sv(m), pos = e - rs;
-        const int c = S.cell[e];
-        const int fs = first_slot(S, e, k, rs, get4(S.tv[e], t));
-        if (b.te) b.te[6LL * c + pair_slot(sv, t)] = (&S.hv[0][0])[fs];
-        if (b.et) b.et[(long long)eto[fs] + mpopc(S.cm[e][k] & (((M)1 << pos) - (M)1))] = c;
-    }
-    auto face = [&](int e, int o) {
-        const int m = S.meta[e];
-        const int rs = m_rs(m), sv = m_sv(m);
-        const int c = S.cell[e];
-        const int ko = cand_of(o, sv);
-        const int ka = ko == 0 ? 1 : 0, kb = ko == 2 ? 1 : 2;
-        const M mf = S.cm[e][ka] & S.cm[e][kb];
-        const M m2 = mf & (mf - 1);
-        const int j2 = m2 ? rs + mctz(m2) : -1;
-        const int c2 = m2 ? S.cell[j2] : -1;
-        const int fid = face_at_first(b.frank, b.tf, b.ft, 4LL * c + (3 - o), c, c2);
-        if (m2 && b.tf) {
-            int x, y;
-            face_others(S.tv[e], sv, o, x, y);
-            b.tf[4LL * c2 + (3 - omitted_slot(S.tv[j2], S.vid[e], x, y))] = fid;
-        }
-    };
-    if (n_faces <= kCapB) {
-        for (int i = threadIdx.x; i < n_faces; i += blockDim.x) face(faces[i] >> 2, faces[i] & 3);
-    } else {
-        for (int e = threadIdx.x; e < n; e += blockDim.x) {
-            const int m = S.meta[e];
-            const int rs = m_rs(m), sv = m_sv(m), pos = e - rs;
-            if (sv > 1) continue;
-            const int o_lo = sv == 0 ? 1 : 0, o_hi = sv == 0 ? 3 : 0;
-            for (int o = o_lo; o <= o_hi; o++) {
-                const int ko = cand_of(o, sv);
-                const int ka = ko == 0 ? 1 : 0, kb = ko == 2 ? 1 : 2;
-                if (mctz(S.cm[e][ka] & S.cm[e][kb]) == pos) face(e, o);
-            }
-        }
-    }
-}
-
-template <typename G>
-__global__ void __launch_bounds__(kThreads, 8) k_star_b(StarB b)
+// k_cell_faces.  The faces first met in cell c take the ids from c's rank on,
+// in column order: TF here and in the face's second cell, FT, FV.  A block's
+// faces have consecutive ids: their FT and FV rows pass through shared memory
+// and go out as whole lines.
+constexpr int kCellThreads = 256;
+__global__ void __launch_bounds__(kCellThreads)
+k_cell_faces(int64_t T, const int4 *__restrict__ tvs, const uint2 *__restrict__ frank,
+             const int4 *__restrict__ fnext, int *__restrict__ tf, int2 *__restrict__ ft,
+             int *__restrict__ fv)
 {
     griddep_wait();
-    __shared__ __align__(16) unsigned char raw[sizeof(StageM<G>)];
-    StageBaseB &S = *reinterpret_cast<StageBaseB *>(raw);
-    stage_rows_b<G>(raw, b);
-    if constexpr (sizeof(G) == 8) {
-        if (S.wide) {   // block-uniform
-            star_b_body(*reinterpret_cast<StageM<unsigned long long> *>(raw), b);
-            return;
+    __shared__ int2 s_ft[4 * kCellThreads];
+    __shared__ int s_fv[12 * kCellThreads];
+    const int64_t c0 = (int64_t)blockIdx.x * kCellThreads;   // a multiple of 8: a word's first cell
+    const int64_t c = c0 + threadIdx.x;
+    const int64_t f0 = (int64_t)__ldg(frank + (c0 >> 3)).y;
+    // the closing word counts every face: T is past the last word's first cell
+    // or on its boundary
+    const int64_t c1 = min(c0 + kCellThreads, T);
+    const uint2 r1 = __ldg(frank + (c1 >> 3));
+    const int nf = (int)((int64_t)r1.y + __popc(r1.x & ((1u << (4 * (int)(c1 & 7))) - 1u)) - f0);
+    unsigned first = 0u;
+    if (c < T) {
+        const uint2 rk = __ldg(frank + (c >> 3));
+        const int sh = 4 * (int)(c & 7);
+        first = (rk.x >> sh) & 15u;
+        if (first) {
+            int fid = (int)rk.y + __popc(rk.x & ((1u << sh) - 1u));
+            const int4 w = __ldg(tvs + c);
+            const int4 nx = fnext ? __ldg(fnext + c) : make_int4(-1, -1, -1, -1);
+            int4 w2[4];
+            if (tf) {
+#pragma unroll
+                for (int col = 0; col < 4; col++) {
+                    const int c2 = get4(nx, col);
+                    if (((first >> col) & 1u) && c2 >= 0) w2[col] = __ldg(tvs + c2);
+                }
+            }
+#pragma unroll
+            for (int col = 0; col < 4; col++) {
+                if (!((first >> col) & 1u)) continue;
+                // the face's vertices: all but slot 3 - col
+                const int a = col == 3 ? w.y : w.x, b = col >= 2 ? w.z : w.y;
+                const int d = col >= 1 ? w.w : w.z;
+                const int c2 = get4(nx, col);
+                const int k = fid - (int)f0;
+                if (ft) s_ft[k] = make_int2((int)c, c2);
+                if (fv) {
+                    s_fv[3 * k] = a;
+                    s_fv[3 * k + 1] = b;
+                    s_fv[3 * k + 2] = d;
+                }
+                if (tf) {
+                    tf[4 * c + col] = fid;
+                    if (c2 >= 0) {
+                        // sorted rows: the first slot that differs from (a, b, d)
+                        // is the one the face leaves out
+                        const int4 x = w2[col];
+                        const int o2 = x.x != a ? 0 : (x.y != b ? 1 : (x.z != d ? 2 : 3));
+                        tf[4LL * c2 + 3 - o2] = fid;
+                    }
+                }
+                fid++;
+            }
         }
     }
-    star_b_body(*reinterpret_cast<StageM<unsigned> *>(raw), b);
+    if (!ft && !fv) return;
+    __syncthreads();
+    if (ft)
+        for (int i = threadIdx.x; i < nf; i += kCellThreads) ft[f0 + i] = s_ft[i];
+    if (fv)
+        for (int i = threadIdx.x; i < 3 * nf; i += kCellThreads) fv[3 * f0 + i] = s_fv[i];
+}
+
+// ---------------------------------------------------------------------------
+struct EdgeEnds {
+    int c, j, v, u;   // first cell, pair slot there, low and high end
+};
+__device__ __forceinline__ EdgeEnds edge_ends(const int4 *__restrict__ tvs, unsigned slot)
+{
+    EdgeEnds e;
+    e.c = (int)(slot / 6u);
+    e.j = (int)(slot - 6u * (unsigned)e.c);
+    const int4 w = __ldg(tvs + e.c);
+    e.v = e.j < 3 ? w.x : (e.j < 5 ? w.y : w.z);
+    e.u = e.j == 0 ? w.y : (e.j == 1 || e.j == 3 ? w.z : w.w);
+    return e;
+}
+// the slots of v < u in w, which holds both
+__device__ __forceinline__ void slots_of(const int4 &w, int v, int u, int &s, int &t)
+{
+    s = (w.x < v) + (w.y < v);
+    t = 1 + (w.y < u) + (w.z < u);
+}
+
+// The cells of an edge record: the star positions of its owner v that its
+// mask holds, ascending.  W: masks of stars of more than kNarrowStar cells
+// have a high half in rec_hi; a star of more than 64 cells (tg_heavy.cu) keeps
+// its (neighbour, position) pairs instead: the mask is the run's first pair
+// and rec_hi its length.
+//
+// k_edge_ids, a thread per record: the edge's id (the rank of its first
+// occurrence), its entries in its ends' incident rows (unsorted: a row fills
+// from the front for the edges the vertex is the high end of, from the back
+// for its own), its row lengths; the record moves to its id's place, so that
+// the passes after this one write in id order.  Each cell of the edge holds
+// two of its faces and each face lies in two of its cells but for the boundary
+// faces, in one: faces = cells + boundary faces / 2.  A boundary face of the
+// edge makes both ends boundary vertices; only such edges look at their cells
+// (a boundary face is its only cell's first occurrence, so fbnd tells).
+template <bool W>
+__global__ void __launch_bounds__(256) k_edge_ids(EdgePass p)
+{
+    griddep_wait();
+    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= p.E) return;
+    const uint2 rec = __ldg(p.rec + r);
+    const uint2 place = __ldg(p.place + r);
+    const EdgeEnds e = edge_ends(p.tvs, rec.x);
+    const int64_t ru = __ldg(p.vv_off + e.u), rv1 = __ldg(p.vv_off + e.v + 1);
+    int id = 0;
+    if (p.erank) id = rank_of(p.erank, rec.x);
+    if (p.inc) {
+        p.inc[rv1 - 1 - place.x] = make_int2(e.u, id);
+        p.inc[ru + place.y] = make_int2(e.v, id);
+    } else {
+        p.vv[rv1 - 1 - place.x] = e.u;
+        p.vv[ru + place.y] = e.v;
+    }
+    if (!p.edge) return;
+    const bool walk = p.count_ef && __ldg(p.vbnd + e.v) && __ldg(p.vbnd + e.u);
+    const int64_t rs = W || walk ? __ldg(p.vt_off + e.v) : 0;
+    const int D = W ? (int)(__ldg(p.vt_off + e.v + 1) - rs) : 0;
+    const unsigned hi = W ? __ldg(p.rec_hi + r) : 0u;
+    int nb = 0, n_et;
+    auto look = [&](int pos) {
+        const int c = __ldg(p.vt + rs + pos);
+        int s, t;
+        slots_of(__ldg(p.tvs + c), e.v, e.u, s, t);
+        // its faces there leave out one of the other two slots
+        const unsigned out = 0xfu & ~((8u >> s) | (8u >> t));
+        nb += __popc((__ldg(p.fbnd + (c >> 3)) >> (4 * (c & 7))) & out);
+    };
+    if (W && D > kMaxStar) {
+        n_et = (int)hi;
+        if (walk)
+            for (int k = 0; k < n_et; k++) look(p.pairs[(int64_t)rec.y + k].y);
+    } else {
+        unsigned long long m = rec.y;
+        if (W && D > kNarrowStar) m |= (unsigned long long)hi << 32;
+        n_et = W ? __popcll(m) : __popc(rec.y);
+        if (walk)
+            for (; m; m &= m - 1) look(mctz(m));
+    }
+    const unsigned ee = (unsigned)((rv1 - __ldg(p.vv_off + e.v)) +
+                                   (__ldg(p.vv_off + e.u + 1) - ru) - 2);
+    p.edge[id] = make_uint4(rec.x, rec.y, (unsigned)n_et | (unsigned)(n_et + nb / 2) << 16, ee);
+    if constexpr (W) p.edge_hi[id] = hi;
+}
+
+// k_edge_rows: TE at each cell of an edge, ET and EF rows.  A warp takes 32
+// consecutive edges and spreads their cells over its lanes (a list in shared
+// memory), so that the cells gathered and the entries written by one
+// instruction belong to a few neighbouring edges and share cache lines: what
+// bounds the pass is the number of lines its instructions touch (about 0.8 a
+// clock and SM get through to L2).  A thread per edge touched 20 lines an
+// edge; records in the star pass's order 13, their ET and EF rows lying apart.
+//
+// EF: an edge's faces at a cell are the columns omitting one of the other two
+// slots.  A face's cells all hold the edge, so a row is the faces at the cells
+// where they are first met (fflag), ascending: ids are ranks of first
+// occurrences (4 * cell + column).
+constexpr int kRowsThreads = 128;
+constexpr int kRowsTake = 16;                // cells an edge lists at a time
+constexpr int kRowsCap = 32 * kRowsTake;
+template <bool W>
+__global__ void __launch_bounds__(kRowsThreads) k_edge_rows(EdgePass p)
+{
+    griddep_wait();
+    __shared__ unsigned s_at[kRowsThreads / 32][kRowsCap];          // the cell's place in VT
+    __shared__ unsigned char s_edge[kRowsThreads / 32][kRowsCap];   // the edge's lane
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int64_t id = (int64_t)blockIdx.x * kRowsThreads + threadIdx.x;
+    if ((id & ~(int64_t)31) >= p.E) return;   // warp-uniform
+    int v = 0, u = 0, rs = 0, et = 0, ef = 0;
+    unsigned long long m = 0ull;
+    if (id < p.E) {
+        const uint2 rec = __ldg(reinterpret_cast<const uint2 *>(p.edge + id));
+        const EdgeEnds e = edge_ends(p.tvs, rec.x);
+        v = e.v;
+        u = e.u;
+        rs = (int)__ldg(p.vt_off + v);
+        if (p.et) et = (int)__ldg(p.et_off + id);
+        if (p.ef) ef = (int)__ldg(p.ef_off + id);
+        m = rec.y;
+        if constexpr (W) {
+            const int D = (int)(__ldg(p.vt_off + v + 1) - rs);
+            if (D > kMaxStar) {   // alone, cell after cell
+                const int n = (int)p.edge_hi[id];
+                int k_ef = ef;
+                for (int k = 0; k < n; k++) {
+                    const int c = __ldg(p.vt + rs + p.pairs[(int64_t)rec.y + k].y);
+                    int s, t;
+                    slots_of(__ldg(p.tvs + c), v, u, s, t);
+                    if (p.te) p.te[6LL * c + pair_slot(s, t)] = (int)id;
+                    if (p.et) p.et[et + k] = c;
+                    if (p.ef) {
+                        const unsigned out = (__ldg(p.fflag + (c >> 3)) >> (4 * (c & 7))) & 0xfu &
+                                             ~((8u >> s) | (8u >> t));
+                        for (unsigned o = out; o; o &= o - 1)
+                            p.ef[k_ef++] = __ldg(p.tf + 4LL * c + mctz(o));
+                    }
+                }
+                m = 0ull;
+            } else if (D > kNarrowStar) {
+                m |= (unsigned long long)p.edge_hi[id] << 32;
+            }
+        }
+    }
+    unsigned *at = s_at[wp];
+    unsigned char *edge = s_edge[wp];
+    while (__any_sync(kAll, m != 0ull)) {
+        // this lane's cells (at most kRowsTake now) in the list
+        const int cnt = min(W ? __popcll(m) : __popc((unsigned)m), kRowsTake);
+        int end = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kAll, end, o);
+            if (lane >= o) end += y;
+        }
+        const int off = end - cnt, total = __shfl_sync(kAll, end, 31);
+        if constexpr (W) {
+            for (int k = off; k < end; k++, m &= m - 1) {
+                at[k] = (unsigned)(rs + mctz(m));
+                edge[k] = (unsigned char)lane;
+            }
+        } else {
+            unsigned mm = (unsigned)m;
+            for (int k = off; k < end; k++, mm &= mm - 1) {
+                at[k] = (unsigned)(rs + mctz(mm));
+                edge[k] = (unsigned char)lane;
+            }
+            m = mm;
+        }
+        __syncwarp();
+        const int etb = et - off;   // entry i of the list goes to etb + i
+        for (int i0 = 0; i0 < total; i0 += 32) {
+            const int i = i0 + lane;
+            const bool act = i < total;
+            const int l = act ? edge[i] : 0;
+            const int c = act ? __ldg(p.vt + at[i]) : 0;
+            const int xv = __shfl_sync(kAll, v, l), xu = __shfl_sync(kAll, u, l);
+            const int4 w = act ? __ldg(p.tvs + c) : make_int4(0, 0, 0, 0);
+            int s, t;
+            slots_of(w, xv, xu, s, t);
+            if (p.te && act) p.te[6LL * c + pair_slot(s, t)] = (int)(id - lane) + l;
+            if (p.et) {
+                const int b = __shfl_sync(kAll, etb, l);
+                if (act) p.et[b + i] = c;
+            }
+            if (p.ef) {
+                const int t1 = s == 0 ? (t == 1 ? 2 : 1) : 0, t2 = 6 - s - t - t1;
+                int4 f = make_int4(0, 0, 0, 0);
+                unsigned nib = 0u;
+                if (act) {
+                    f = __ldg(reinterpret_cast<const int4 *>(p.tf) + c);
+                    nib = __ldg(p.fflag + (c >> 3)) >> (4 * (c & 7));
+                }
+                // columns 3 - t2 < 3 - t1
+                const bool first_a = (nib >> (3 - t2)) & 1u, first_b = (nib >> (3 - t1)) & 1u;
+                const unsigned ba = __ballot_sync(kAll, first_a), bb = __ballot_sync(kAll, first_b);
+                // the entries of this edge before this one in the list's window
+                const int o = __shfl_sync(kAll, off, l) - i0;
+                const unsigned below = ((1u << lane) - 1u) & (o > 0 ? ~0u << o : ~0u);
+                int k = __shfl_sync(kAll, ef, l) + __popc(ba & below) + __popc(bb & below);
+                if (first_a) p.ef[k++] = get4(f, 3 - t2);
+                if (first_b) p.ef[k] = get4(f, 3 - t1);
+                // this lane's own edge: past the entries written for it now
+                const int lo = max(off - i0, 0), hi = min(end - i0, 32);
+                if (lo < hi) {
+                    const unsigned own = (hi == 32 ? ~0u : (1u << hi) - 1u) & (~0u << lo);
+                    ef += __popc(ba & own) + __popc(bb & own);
+                }
+            }
+        }
+        et += cnt;
+        __syncwarp();
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -797,18 +612,19 @@ __global__ void __launch_bounds__(kThreads, 8) k_star_b(StarB b)
 // A vertex whose star holds more than kMaxStar cells is heavy: it takes no
 // key and is numbered among the heavy vertices instead (vkey = -1 - index),
 // which follow every other vertex with cells in the processing order, so
-// the star passes' windows never mix them with the rest (tg_heavy.cu
-// processes them).
+// that the star pass stops where they begin (tg_heavy.cu processes them).
 __device__ __forceinline__ void mark_first(const int4 *__restrict__ tvs, uint32_t *vflag,
-                                           int64_t *vkey, int *heavy_cnt, int v, int c, int64_t D)
+                                           int64_t *vkey, int *heavy_cnt, int *heavy_off, int v,
+                                           int c, int D)
 {
     if (D > kMaxStar) {   // heavy_cnt[0]: heavy vertices, [1]: their star entries
-        vkey[v] = -1 - (long long)atomicAdd(heavy_cnt, 1);
-        atomicAdd(heavy_cnt + 1, (int)D);
+        const int k = atomicAdd(heavy_cnt, 1);
+        vkey[v] = -1 - (long long)k;
+        heavy_off[k] = atomicAdd(heavy_cnt + 1, D);   // its share of the heavy scratch
         return;
     }
     // heavy_cnt[2]: some light star holds more than kNarrowStar cells (the
-    // star passes then keep their candidate masks 64-bit in global memory)
+    // edge records then have a high half)
     if (D > kNarrowStar) heavy_cnt[2] = 1;
     const int4 w = __ldg(tvs + c);
     const long long key = 4LL * c + (w.x == v ? 0 : (w.y == v ? 1 : (w.z == v ? 2 : 3)));
@@ -816,79 +632,137 @@ __device__ __forceinline__ void mark_first(const int4 *__restrict__ tvs, uint32_
     atomicOr(vflag + (key >> 5), 1u << (key & 31));
 }
 
-// Sort every VT row ascending, a row to a thread (tg_rowsort.h).  A block's
+// ---------------------------------------------------------------------------
+// CSR rows sorted ascending, a row to a thread (tg_rowsort.h).  A block's
 // kVtsThreads rows are contiguous: they pass through shared memory so that
 // global memory sees whole rows; rows that do not fit are sorted in place.
-// Bound by its memory accesses (the rows once each way and a gathered cell per
-// vertex); ranking every entry against its row by a loop over shared memory
-// instead was issue-bound: 362 -> 137 us at 128^3 (12.6M cells), 70 -> 22 us on the
-// 64^3 coned mesh.
+// `first` is given each non-empty row's smallest entry.  Bound by its memory
+// accesses; ranking every entry against its row by a loop over shared memory
+// instead was issue-bound: VT 362 -> 137 us at 128^3 (12.6M cells), 70 -> 22
+// us on the 64^3 coned mesh.
 constexpr int kVtsThreads = TG_VTS_THREADS;
 constexpr int kVtsCap = 32 * kVtsThreads;
+struct RowStage {
+    int4 word[kVtsCap / 4 + 1];
+};
+// total: entries of the whole array
+template <typename Fn>
+__device__ __forceinline__ void sort_block_rows(RowStage &S, const int64_t *__restrict__ off, int64_t rows,
+                                                int64_t total, int *__restrict__ ent, Fn first)
+{
+    int *stage = reinterpret_cast<int *>(S.word);
+    const int64_t v0 = (int64_t)blockIdx.x * kVtsThreads;
+    const int64_t v1 = min(v0 + kVtsThreads, rows);
+    const int64_t v = v0 + threadIdx.x;
+    const int64_t base = off[v0];
+    const int64_t n = off[v1] - base;
+    const int64_t b = v < rows ? off[v] : 0;
+    const int D = v < rows ? (int)(off[v + 1] - b) : 0;
+    if (n > kVtsCap) {   // block-uniform
+        sort_rows_warp(ent + b, D);
+        if (D > 0) first((int)v, ent[b], D);
+        return;
+    }
+    // whole 16-byte words from the one holding the first entry
+    const int shift = (int)(base & 3);
+    const int words = (int)((n + shift + 3) >> 2);
+    for (int i = threadIdx.x; i < words; i += kVtsThreads) {
+        const int64_t g = base - shift + 4LL * i;
+        if (g + 4 <= total) {
+            S.word[i] = *reinterpret_cast<const int4 *>(ent + g);
+        } else {
+            for (int k = 0; g + k < total; k++) stage[4 * i + k] = ent[g + k];
+        }
+    }
+    __syncthreads();
+    int *row = stage + shift + (int)(b - base);
+    sort_rows_warp(row, D);
+    if (D > 0) first((int)v, row[0], D);
+    __syncthreads();
+    for (int i = threadIdx.x; i < (int)n; i += kVtsThreads) ent[base + i] = stage[shift + i];
+}
+
 __global__ void __launch_bounds__(kVtsThreads)
-k_vt_sort(const int64_t *__restrict__ vt_off, int64_t V, int *__restrict__ vt,
+k_vt_sort(const int64_t *__restrict__ vt_off, int64_t V, int64_t total, int *__restrict__ vt,
           const int4 *__restrict__ tvs, uint32_t *__restrict__ vflag, int64_t *__restrict__ vkey,
-          int *__restrict__ heavy_cnt)
+          int *__restrict__ heavy_cnt, int *__restrict__ heavy_off)
 {
     griddep_wait();
-    __shared__ __align__(16) int cell[kVtsCap + 4];
+    __shared__ RowStage S;
+    sort_block_rows(S, vt_off, V, total, vt, [&](int v, int c, int D) {
+        mark_first(tvs, vflag, vkey, heavy_cnt, heavy_off, v, c, D);
+    });
+}
+
+// VV rows in place
+__global__ void __launch_bounds__(kVtsThreads)
+k_vv_sort(const int64_t *__restrict__ off, int64_t V, int64_t total, int *__restrict__ vv)
+{
+    griddep_wait();
+    __shared__ RowStage S;
+    sort_block_rows(S, off, V, total, vv, [](int, int, int) {});
+}
+
+// VV and incident-edge rows from inc (the same rows, {neighbour, edge id}
+// pairs), each sorted by itself
+constexpr int kIncCap = 20 * kVtsThreads;
+__global__ void __launch_bounds__(kVtsThreads, 9)
+k_inc_sort(const int64_t *__restrict__ off, int64_t V, const int2 *__restrict__ inc,
+           int *__restrict__ vv, int *__restrict__ eid)
+{
+    griddep_wait();
+    __shared__ int s_row[2][kIncCap];
     const int64_t v0 = (int64_t)blockIdx.x * kVtsThreads;
-    const int64_t v1 = min(v0 + kVtsThreads, V);
     const int64_t v = v0 + threadIdx.x;
-    const int64_t base = vt_off[v0];
-    const int64_t n = vt_off[v1] - base;
-    const int64_t b = v < V ? vt_off[v] : 0;
-    const int D = v < V ? (int)(vt_off[v + 1] - b) : 0;
-    const bool staged = n <= kVtsCap;   // block-uniform
-    // whole 16-byte words from the one holding the first entry (4T entries in
-    // all: the last word is whole)
-    const int shift = (int)(base & 3);
-    int *own = cell + shift + (int)(b - base);
-    if (staged) {
-        int4 *src = reinterpret_cast<int4 *>(vt + (base - shift));
-        const int words = (int)((n + shift + 3) >> 2);
-        for (int i = threadIdx.x; i < words; i += kVtsThreads)
-            reinterpret_cast<int4 *>(cell)[i] = src[i];
-        __syncthreads();
-        sort_rows_warp(own, D);
-        if (D > 0) mark_first(tvs, vflag, vkey, heavy_cnt, (int)v, own[0], D);
-        __syncthreads();
-        for (int i = threadIdx.x; i < (int)n; i += kVtsThreads) vt[base + i] = cell[shift + i];
-    } else {
-        sort_rows_warp(vt + b, D);
-        if (D > 0) mark_first(tvs, vflag, vkey, heavy_cnt, (int)v, vt[b], D);
+    const int64_t base = off[v0];
+    const int64_t n = off[min(v0 + kVtsThreads, V)] - base;
+    const int64_t b = v < V ? off[v] : 0;
+    const int d = v < V ? (int)(off[v + 1] - b) : 0;
+    if (n > kIncCap) {   // block-uniform: in place
+        for (int k = 0; k < d; k++) {
+            const int2 x = inc[b + k];
+            vv[b + k] = x.x;
+            eid[b + k] = x.y;
+        }
+#pragma unroll 1
+        for (int q = 0; q < 2; q++) sort_rows_warp((q ? eid : vv) + b, d);
+        return;
+    }
+    for (int i = threadIdx.x; i < (int)n; i += kVtsThreads) {
+        const int2 x = __ldg(inc + base + i);
+        s_row[0][i] = x.x;
+        s_row[1][i] = x.y;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int q = 0; q < 2; q++) sort_rows_warp(s_row[q] + (int)(b - base), d);
+    __syncthreads();
+    for (int i = threadIdx.x; i < (int)n; i += kVtsThreads) {
+        vv[base + i] = s_row[0][i];
+        eid[base + i] = s_row[1][i];
     }
 }
 
 // ---------------------------------------------------------------------------
-// ET / EF / EE offsets in edge-id order.  Edge ids are ranks of first
-// occurrences, so scanning the 6T edge-occurrence slots in order visits the
-// edges in id order: a slot holding a first occurrence contributes the ET
-// and EF row lengths k_star_a left there and deg(a) + deg(b) - 2 for EE.
-// One pass: a block takes a tile of slots (in start order), gathers each of
-// its edges' row lengths (packed in one word by id) and EV, scans the three
-// sums with a look-back over the tiles before it, then writes the offsets of
-// its edges from the packed words it just wrote.
+// ET / EF / EE offsets: exclusive sums of the row lengths in edge-id order, in
+// one pass (a block takes the next tile in start order, sums it, adds the
+// tiles before it by look-back, and writes its offsets).  EV of the tile's
+// edges beside it.
 constexpr int kEdgeThreads = 256;
-constexpr int kEdgeItems = TG_EDGE_ITEMS;             // slots per thread: 8, 16 or 32
-constexpr int kEdgeTile = kEdgeItems * kEdgeThreads;  // slots per tile
-static_assert(kEdgeItems == 8 || kEdgeItems == 16 || kEdgeItems == 32, "slots per thread");
+constexpr int kEdgeItems = TG_EDGE_ITEMS;             // edges per thread
+constexpr int kEdgeTile = kEdgeItems * kEdgeThreads;  // edges per tile
+static_assert(kEdgeItems % 2 == 0, "edges per thread: whole 16-byte words");
 
 struct EdgeOffsets {
-    const uint32_t *eflag;
-    const uint32_t *ecnt;
+    const uint4 *edge;           // [E] as EdgePass
     const int4 *tvs;
-    const int32_t *deg;
-    const uint2 *erank;
-    int64_t n_slots, n_tiles;
+    int64_t E, n_tiles;
     unsigned long long *tiles;   // 3 * n_tiles tile words (ET, EF, EE), then the ticket
     unsigned long long *next;    // the workspace buffer zeroed for the next user
     int64_t next_words;
     unsigned *err;
-    uint2 *len;          // [E]: {ET | EF << 16, EE}
     int64_t *et_off, *ef_off, *ee_off;
-    int32_t *ev;         // [2E] or null: the edge's two vertices, ascending
-    int64_t E;
+    int2 *ev;
 };
 
 template <int NT>
@@ -932,18 +806,23 @@ __device__ __forceinline__ void block_scan3(long long x[3], long long excl[3], l
     __syncthreads();
 }
 
-__device__ __forceinline__ uint32_t slot_bits(const EdgeOffsets &p, long long s0)
+// len(k): the length of the thread's k-th row
+template <typename Fn>
+__device__ __forceinline__ void store_offsets(int64_t *out, int64_t k0, int64_t E, long long run, Fn len)
 {
-    // kEdgeItems consecutive slots starting at a multiple of kEdgeItems lie
-    // in one 32-bit word
-    if (s0 >= p.n_slots) return 0u;
-    const uint32_t w = p.eflag[s0 >> 5];
-    return kEdgeItems == 32 ? w : (w >> (s0 & 31)) & ((1u << kEdgeItems) - 1u);
+    if (!out) return;
+#pragma unroll
+    for (int k = 0; k < kEdgeItems; k += 2) {
+        const long long next = run + len(k);
+        if (k0 + k + 1 < E)   // two offsets, 16 bytes (k0 is even)
+            *reinterpret_cast<longlong2 *>(out + k0 + k) = make_longlong2(run, next);
+        else if (k0 + k < E)
+            out[k0 + k] = run;
+        run = next + len(k + 1);
+    }
 }
 
-// eight blocks per SM (32 registers): the extra resident blocks hide the
-// gathers' latency better than the few spilled registers cost
-__global__ void __launch_bounds__(kEdgeThreads, TG_EDGE_MINB) k_edge_offsets(EdgeOffsets p)
+__global__ void __launch_bounds__(kEdgeThreads) k_edge_offsets(EdgeOffsets p)
 {
     griddep_wait();
     {
@@ -956,38 +835,25 @@ __global__ void __launch_bounds__(kEdgeThreads, TG_EDGE_MINB) k_edge_offsets(Edg
     if (threadIdx.x == 0) s_tile = (long long)atomicAdd(p.tiles + 3 * p.n_tiles, 1ull);
     __syncthreads();
     const long long tile = s_tile;
-    if (p.n_tiles == 0) {   // no slots: the totals alone
+    if (p.n_tiles == 0) {   // no edges: the totals alone
         if (tile == 0 && threadIdx.x == 0) {
-            if (p.et_off) p.et_off[p.E] = 0;
-            if (p.ef_off) p.ef_off[p.E] = 0;
-            if (p.ee_off) p.ee_off[p.E] = 0;
+            if (p.et_off) p.et_off[0] = 0;
+            if (p.ef_off) p.ef_off[0] = 0;
+            if (p.ee_off) p.ee_off[0] = 0;
         }
         return;
     }
     if (tile >= p.n_tiles) return;
-    const long long s0 = tile * kEdgeTile + threadIdx.x * kEdgeItems;
+    const int64_t k0 = tile * kEdgeTile + (int64_t)threadIdx.x * kEdgeItems;
+    uint2 len[kEdgeItems];   // {ET | EF << 16, EE}
     long long x[3] = {0, 0, 0};
-    const uint32_t bits = slot_bits(p, s0);
-    const int id0 = bits ? rank_of(p.erank, s0) : 0;
-    int id = id0;
-    for (uint32_t m = bits; m; m &= m - 1) {
-        const int i = __ffs(m) - 1;
-        const long long s = s0 + i;
-        if (s >= p.n_slots) break;
-        const long long cell = s / 6;
-        const int j = (int)(s - 6 * cell);
-        const int4 w = __ldg(p.tvs + cell);
-        const int a = get4(w, j < 3 ? 0 : (j < 5 ? 1 : 2));
-        const int b = get4(w, j < 3 ? j + 1 : (j == 3 ? 2 : 3));
-        const uint32_t c = p.ecnt[s];
-        const int et = c & 0xffff, ef = c >> 16;
-        const int ee = p.ee_off ? __ldg(p.deg + a) + __ldg(p.deg + b) - 2 : 0;
-        x[0] += et;
-        x[1] += ef;
-        x[2] += ee;
-        p.len[id] = make_uint2(c, (uint32_t)ee);
-        if (p.ev) reinterpret_cast<int2 *>(p.ev)[id] = make_int2(a, b);
-        id++;
+#pragma unroll
+    for (int k = 0; k < kEdgeItems; k++) {
+        len[k] = k0 + k < p.E ? __ldg(reinterpret_cast<const uint2 *>(p.edge + k0 + k) + 1)
+                              : make_uint2(0u, 0u);
+        x[0] += len[k].x & 0xffffu;
+        x[1] += len[k].x >> 16;
+        x[2] += len[k].y;
     }
     long long excl[3], tot[3];
     block_scan3<kEdgeThreads>(x, excl, tot);
@@ -998,67 +864,50 @@ __global__ void __launch_bounds__(kEdgeThreads, TG_EDGE_MINB) k_edge_offsets(Edg
         if ((threadIdx.x & 31) == 0) s_pre[q] = pre;
     }
     __syncthreads();
-    long long run[3];
-#pragma unroll
-    for (int q = 0; q < 3; q++) run[q] = s_pre[q] + excl[q];
-    // this thread's packed words again (it wrote them: cache hits)
-    for (int k = id0; k < id; k++) {
-        const uint2 w = p.len[k];
-        if (p.et_off) p.et_off[k] = run[0];
-        if (p.ef_off) p.ef_off[k] = run[1];
-        if (p.ee_off) p.ee_off[k] = run[2];
-        run[0] += w.x & 0xffff;
-        run[1] += w.x >> 16;
-        run[2] += w.y;
-    }
+    store_offsets(p.et_off, k0, p.E, s_pre[0] + excl[0], [&](int k) { return len[k].x & 0xffffu; });
+    store_offsets(p.ef_off, k0, p.E, s_pre[1] + excl[1], [&](int k) { return len[k].x >> 16; });
+    store_offsets(p.ee_off, k0, p.E, s_pre[2] + excl[2], [&](int k) { return len[k].y; });
     if (tile == p.n_tiles - 1 && threadIdx.x == 0) {
         if (p.et_off) p.et_off[p.E] = s_pre[0] + tot[0];
         if (p.ef_off) p.ef_off[p.E] = s_pre[1] + tot[1];
         if (p.ee_off) p.ee_off[p.E] = s_pre[2] + tot[2];
     }
-}
-
-// win[w] = first vertex whose row starts at or after entry kWin * w, for
-// w in [0, n_win], with win[n_win] = V.  Vertex v owns the windows w with
-// off[v-1] < kWin * w <= off[v].  A second table over the same offsets with
-// another window size (win2, or null) comes from the same launch.
-__device__ __forceinline__ void window_owner(const long long lo, const long long hi, int64_t v,
-                                             int64_t n_win, int win_size, int *win, int *wbase,
-                                             long long base_v)
-{
-    long long w = lo < 0 ? 0 : lo / win_size + 1;
-    const long long w_hi = hi / win_size;
-    for (; w <= w_hi && w <= n_win; w++) {
-        win[w] = (int)v;
-        if (wbase) wbase[w] = (int)base_v;
+    if (!p.ev) return;
+#pragma unroll 4
+    for (int k = 0; k < kEdgeItems; k++) {
+        const int64_t id = tile * kEdgeTile + k * kEdgeThreads + threadIdx.x;
+        if (id < p.E) {
+            const EdgeEnds e = edge_ends(p.tvs, __ldg(reinterpret_cast<const unsigned *>(p.edge + id)));
+            p.ev[id] = make_int2(e.v, e.u);
+        }
     }
 }
 
+// win[w] = first vertex whose row starts at or after entry win_size * w, for
+// w in [0, n_win], with win[n_win] = V.  Vertex v owns the windows w with
+// off[v-1] < win_size * w <= off[v].
 __global__ void __launch_bounds__(256)
 k_window_starts(const int64_t *__restrict__ off, int64_t V, int64_t n_win, int win_size,
-                int *__restrict__ win, int64_t n_win2, int win_size2, int *__restrict__ win2,
-                int *__restrict__ wbase, int *__restrict__ wbase2)
+                int *__restrict__ win)
 {
     griddep_wait();
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (v > V) return;
     const long long lo = v == 0 ? -1 : off[v - 1];
-    const long long base_v = off[v];   // off[V] = the entry count
-    window_owner(lo, v == V ? (long long)win_size * n_win : off[v], v, n_win, win_size, win, wbase,
-                 base_v);
-    if (win2)
-        window_owner(lo, v == V ? (long long)win_size2 * n_win2 : off[v], v, n_win2, win_size2,
-                     win2, wbase2, base_v);
+    const long long hi = v == V ? (long long)win_size * n_win : off[v];
+    long long w = lo < 0 ? 0 : lo / win_size + 1;
+    for (const long long w_hi = hi / win_size; w <= w_hi && w <= n_win; w++) win[w] = (int)v;
 }
 
 // ---------------------------------------------------------------------------
 // Star processing order.  Vertex ids need not carry locality (meshes are
 // often renumbered; the workloads here permute them) while cell order usually
 // does (generators and partitioners emit cells in space-filling order).  The
-// star passes therefore visit vertices by first cell, the head of the sorted
+// star pass therefore visits vertices by first cell, the head of the sorted
 // VT row, ties by slot: consecutive vertices then share cells, so a block's
-// cell gathers hit L2 and the output sectors of cell- and id-ordered
-// relations it writes are completed by blocks running at the same time.
+// cell gathers hit L2, and so do those of the per-edge passes, whose records
+// come in that order; the output sectors of cell- and id-ordered relations
+// they write are completed by blocks running at the same time.
 // k_vt_sort marks each vertex's key 4 * first cell + slot in a bitmap over
 // the 4T cell slots; the key's rank is the vertex's position.  Heavy vertices
 // (vkey < 0) follow at n_light + their index; vertices without cells come
@@ -1066,19 +915,15 @@ k_window_starts(const int64_t *__restrict__ off, int64_t V, int64_t n_win, int w
 __global__ void __launch_bounds__(256)
 k_vorder_place(const int64_t *__restrict__ vt_off, int64_t V, const int64_t *__restrict__ vkey,
                const uint2 *__restrict__ vrank, int64_t nwk, const int *__restrict__ heavy_cnt,
-               int *__restrict__ vorder, int *__restrict__ dcount)
+               int *__restrict__ vorder)
 {
     griddep_wait();
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= V) return;
     const int64_t n_light = (int64_t)__ldg(&vrank[nwk].y);
     // the positions past the vertices with cells (their rows are empty)
-    if (v >= n_light + *heavy_cnt) {
-        vorder[v] = 0;
-        dcount[v] = 0;
-    }
-    const int D = (int)(vt_off[v + 1] - vt_off[v]);
-    if (D == 0) return;
+    if (v >= n_light + *heavy_cnt) vorder[v] = 0;
+    if (vt_off[v + 1] == vt_off[v]) return;
     const long long key = vkey[v];
     int64_t pos;
     if (key < 0) {
@@ -1088,48 +933,6 @@ k_vorder_place(const int64_t *__restrict__ vt_off, int64_t V, const int64_t *__r
         pos = (int64_t)r.y + __popc(r.x & ((1u << (key & 31)) - 1u));
     }
     vorder[pos] = (int)v;
-    dcount[pos] = D;
-}
-
-// VT rows copied into processing order: a warp fetches 32 rows' positions
-// and sources at once, then copies them one after another, lanes across the
-// row
-constexpr int kVtpRows = TG_VTP_ROWS;
-__global__ void __launch_bounds__(256, TG_VTP_MINB)
-k_vtp_fill(const int *__restrict__ vorder, const int64_t *__restrict__ pofs, int64_t V,
-           const int64_t *__restrict__ vt_off, const int *__restrict__ vt, int *__restrict__ vtp)
-{
-    griddep_wait();
-    const int64_t r0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32;
-    const int lane = threadIdx.x & 31;
-    if (r0 >= V) return;  // warp-uniform
-    const int64_t r = r0 + lane;
-    long long dst = 0, src = 0;
-    int D = 0;
-    if (r < V) {
-        dst = pofs[r];
-        D = (int)(pofs[r + 1] - dst);
-        if (D > 0) src = __ldg(vt_off + __ldg(vorder + r));
-    }
-    // kVtpRows rows at a time: their loads are in flight together (lane k
-    // takes entry k; entries past 32 of a longer row follow)
-    constexpr int R = kVtpRows;
-    for (int j = 0; j < 32; j += R) {
-        int x[R], Dj[R];
-        long long dj[R], sj[R];
-#pragma unroll
-        for (int t = 0; t < R; t++) {
-            Dj[t] = __shfl_sync(0xffffffffu, D, j + t);
-            dj[t] = __shfl_sync(0xffffffffu, dst, j + t);
-            sj[t] = __shfl_sync(0xffffffffu, src, j + t);
-            x[t] = lane < Dj[t] ? __ldg(vt + sj[t] + lane) : 0;
-        }
-#pragma unroll
-        for (int t = 0; t < R; t++) {
-            if (lane < Dj[t]) vtp[dj[t] + lane] = x[t];
-            for (int k = lane + 32; k < Dj[t]; k += 32) vtp[dj[t] + k] = __ldg(vt + sj[t] + k);
-        }
-    }
 }
 
 // First edge and face id of each segment of cells (a mesh of a batch):
@@ -1146,107 +949,119 @@ k_seg_ranks(const int64_t *__restrict__ seg_c, int64_t n, const uint2 *__restric
     seg_ef[n + 1 + i] = rank_of(frank, 4LL * seg_c[i]);
 }
 
-inline unsigned n_windows(int64_t nvt) { return (unsigned)(nvt / kWin + 1); }
-inline unsigned n_windows_b(int64_t nvt) { return (unsigned)(nvt / kWinB + 1); }
-
 }  // namespace
-
-int star_window() { return kWin; }
-int star_window_b() { return kWinB; }
 
 int64_t window_count(int64_t n_entries, int win_size) { return n_entries / win_size + 1; }
 
 void launch_window_starts(const int64_t *off, int64_t V, int64_t n_entries, int win_size,
-                          int32_t *win, cudaStream_t s, int win_size2, int32_t *win2,
-                          int32_t *wbase, int32_t *wbase2)
+                          int32_t *win, cudaStream_t s)
 {
     Launch L("k_window_starts", s);
     launch_pdl(k_window_starts, (unsigned)((V + 1 + 255) / 256), 256, 0, s,
-        off, V, window_count(n_entries, win_size), win_size, win,
-        win2 ? window_count(n_entries, win_size2) : 0, win_size2, win2, wbase, wbase2);
+        off, V, window_count(n_entries, win_size), win_size, win);
 }
 
-int64_t edge_offsets_words(int64_t n_slots)
+int64_t edge_offsets_words(int64_t max_edges)
 {
-    return 3 * ((n_slots + kEdgeTile - 1) / kEdgeTile) + 1;
+    return 3 * ((max_edges + kEdgeTile - 1) / kEdgeTile) + 1;
 }
 
-void launch_edge_offsets(const uint32_t *eflag, const uint32_t *ecnt, const int4 *tvs,
-                         const int32_t *deg, const uint2 *erank, int64_t n_slots, int64_t E,
-                         int64_t *et_off, int64_t *ef_off, int64_t *ee_off, int32_t *ev,
-                         uint2 *len, ScanWorkspace &ws, DevStatus *st, cudaStream_t s)
+void launch_edge_offsets(const EdgePass &e, int64_t *et_off, int64_t *ef_off, int64_t *ee_off,
+                         int32_t *ev, ScanWorkspace &ws, DevStatus *st, cudaStream_t s)
 {
-    const int64_t tiles = (n_slots + kEdgeTile - 1) / kEdgeTile;
     EdgeOffsets p{};
-    p.eflag = eflag;
-    p.ecnt = ecnt;
-    p.tvs = tvs;
-    p.deg = deg;
-    p.erank = erank;
-    p.n_slots = n_slots;
-    p.n_tiles = tiles;
+    p.edge = e.edge;
+    p.tvs = e.tvs;
+    p.E = e.E;
+    p.n_tiles = (e.E + kEdgeTile - 1) / kEdgeTile;
     p.err = &st->flags;
-    p.len = len;
     p.et_off = et_off;
     p.ef_off = ef_off;
     p.ee_off = ee_off;
-    p.ev = ev;
-    p.E = E;
+    p.ev = reinterpret_cast<int2 *>(ev);
     scan_ws_begin(ws, s, &p.tiles, &p.next, &p.next_words);
     {
         Launch L("k_edge_offsets", s);
-        launch_pdl(k_edge_offsets, (unsigned)std::max<int64_t>(tiles, 1), kEdgeThreads, 0, s, p);
+        launch_pdl(k_edge_offsets, (unsigned)std::max<int64_t>(p.n_tiles, 1), kEdgeThreads, 0, s, p);
     }
     scan_ws_end(ws, s);
 }
 
-void launch_star_a(const StarA &a, cudaStream_t s)
+void launch_star(const StarPass &p, cudaStream_t s)
 {
-    if (a.V == 0) return;
-    Launch L("k_star_a", s);
-    if (a.narrow)
-        launch_pdl(k_star_a<uint32_t>, n_windows(a.nvt), kThreads, 0, s, a);
+    if (p.n_light == 0) return;
+    Launch L("k_star", s);
+    const unsigned grid = (unsigned)((p.n_light + kStarBlock - 1) / kStarBlock);
+    if (p.rec_hi)
+        launch_pdl(k_star<true>, grid, kStarThreads, 0, s, p);
     else
-        launch_pdl(k_star_a<uint64_t>, n_windows(a.nvt), kThreads, 0, s, a);
+        launch_pdl(k_star<false>, grid, kStarThreads, 0, s, p);
 }
 
-void launch_star_b(const StarB &b, cudaStream_t s)
+void launch_cell_faces(int64_t T, const int4 *tvs, const uint2 *frank, const int32_t *fnext,
+                       int32_t *tf, int32_t *ft, int32_t *fv, cudaStream_t s)
 {
-    if (b.V == 0) return;
-    Launch L("k_star_b", s);
-    if (b.narrow)
-        launch_pdl(k_star_b<uint32_t>, n_windows_b(b.nvt), kThreads, 0, s, b);
-    else
-        launch_pdl(k_star_b<uint64_t>, n_windows_b(b.nvt), kThreads, 0, s, b);
+    if (T == 0) return;
+    Launch L("k_cell_faces", s);
+    launch_pdl(k_cell_faces, (unsigned)((T + kCellThreads - 1) / kCellThreads), kCellThreads, 0, s, T, tvs, frank,
+               reinterpret_cast<const int4 *>(fnext), tf, reinterpret_cast<int2 *>(ft), fv);
 }
 
-void launch_vt_sort(const int64_t *vt_off, int32_t *vt, int64_t V, const int4 *tvs,
-                    uint32_t *vflag, int64_t *vkey, int32_t *heavy_cnt, cudaStream_t s)
+void launch_edge_ids(const EdgePass &p, cudaStream_t s)
+{
+    if (p.E == 0) return;
+    Launch L("k_edge_ids", s);
+    const unsigned grid = (unsigned)((p.E + 255) / 256);
+    if (p.rec_hi)
+        launch_pdl(k_edge_ids<true>, grid, 256, 0, s, p);
+    else
+        launch_pdl(k_edge_ids<false>, grid, 256, 0, s, p);
+}
+
+void launch_edge_rows(const EdgePass &p, cudaStream_t s)
+{
+    if (p.E == 0) return;
+    Launch L("k_edge_rows", s);
+    const unsigned grid = (unsigned)((p.E + kRowsThreads - 1) / kRowsThreads);
+    if (p.rec_hi)
+        launch_pdl(k_edge_rows<true>, grid, kRowsThreads, 0, s, p);
+    else
+        launch_pdl(k_edge_rows<false>, grid, kRowsThreads, 0, s, p);
+}
+
+void launch_vt_sort(const int64_t *vt_off, int32_t *vt, int64_t V, int64_t nvt, const int4 *tvs,
+                    uint32_t *vflag, int64_t *vkey, int32_t *heavy_cnt, int32_t *heavy_off,
+                    cudaStream_t s)
 {
     if (V == 0) return;
     Launch L("k_vt_sort", s);
     launch_pdl(k_vt_sort, (unsigned)((V + kVtsThreads - 1) / kVtsThreads), kVtsThreads, 0, s, vt_off,
-               V, vt, tvs, vflag, vkey, heavy_cnt);
+               V, nvt, vt, tvs, vflag, vkey, heavy_cnt, heavy_off);
+}
+
+void launch_vv_sort(const int64_t *vv_off, int64_t V, int64_t nvv, const int2 *inc, int32_t *vv,
+                    int32_t *eid, cudaStream_t s)
+{
+    if (V == 0 || nvv == 0) return;
+    const unsigned grid = (unsigned)((V + kVtsThreads - 1) / kVtsThreads);
+    if (inc) {
+        Launch L("k_inc_sort", s);
+        launch_pdl(k_inc_sort, grid, kVtsThreads, 0, s, vv_off, V, inc, vv, eid);
+    } else {
+        Launch L("k_vv_sort", s);
+        launch_pdl(k_vv_sort, grid, kVtsThreads, 0, s, vv_off, V, nvv, vv);
+    }
 }
 
 void launch_vorder_place(const int64_t *vt_off, int64_t V, const int64_t *vkey,
                          const uint2 *vrank, int64_t nwk, const int32_t *heavy_cnt, int32_t *vorder,
-                         int32_t *dcount, cudaStream_t s)
+                         cudaStream_t s)
 {
     if (V == 0) return;
     Launch L("k_vorder_place", s);
     launch_pdl(k_vorder_place, (unsigned)((V + 255) / 256), 256, 0, s, vt_off, V, vkey, vrank, nwk,
-               heavy_cnt, vorder, dcount);
+               heavy_cnt, vorder);
 }
-
-void launch_vtp_fill(const int32_t *vorder, const int64_t *pofs, int64_t V, const int64_t *vt_off,
-                     const int32_t *vt, int32_t *vtp, cudaStream_t s)
-{
-    if (V == 0) return;
-    Launch L("k_vtp_fill", s);
-    launch_pdl(k_vtp_fill, (unsigned)((V + 255) / 256), 256, 0, s, vorder, pofs, V, vt_off, vt, vtp);
-}
-
 
 void launch_seg_ranks(const int64_t *seg_c, int64_t n, const uint2 *erank, const uint2 *frank,
                       int64_t *seg_ef, cudaStream_t s)

@@ -2,9 +2,9 @@
 
     python -m tetragpu_gb300.tune [--apply] [--steps K]
 
-The tile constants of the kernels (star-pass windows, block sizes of the
-VT sort and the link adjacency, EE lanes per edge, slots per thread of the
-edge-offset pass) are compile-time constants.  For every candidate setting
+The tile constants of the kernels (the star pass's block size and vertices
+per warp, block sizes of the row sorts and the link adjacency, EE lanes per
+edge, edges per thread of the edge-offset pass) are compile-time constants.  For every candidate setting
 (the default and one change at a time from it) this builds a variant of
 libtetragpu.so with -D overrides under tetragpu_gb300/_build/variants/, loads
 it, and times the batched pipeline (tg_batch create + all 13 relations with
@@ -41,16 +41,15 @@ TUNING_H = os.path.join(PKG, "csrc", "tg_tuning.h")
 # over the defaults there) and one change at a time from it
 CANDIDATES = [
     ("default", {}),
-    ("star_b_win_192", {"TG_STAR_WIN_B": 192}),
-    ("star_b_win_240", {"TG_STAR_WIN_B": 240}),
-    ("star_b_win_256", {"TG_STAR_WIN_B": 256}),
-    ("star_a_win_192", {"TG_STAR_WIN": 192}),
-    ("efa_lanes_1", {"TG_EFA_LANES": 1}),
+    ("star_per_2", {"TG_STAR_PER": 2}),
+    ("star_per_8", {"TG_STAR_PER": 8, "TG_STAR_WIN": 512}),
+    ("star_threads_256", {"TG_STAR_THREADS": 256, "TG_STAR_WIN": 512, "TG_STAR_MINB": 6}),
+    ("star_minb_10", {"TG_STAR_MINB": 10}),
     ("ee_group_8", {"TG_EE_GROUP": 8}),
     ("adj_threads_64", {"TG_ADJ_THREADS": 64}),
     ("adj_threads_256", {"TG_ADJ_THREADS": 256}),
-    ("vt_sort_threads_32", {"TG_VTS_THREADS": 32}),
-    ("vt_sort_threads_128", {"TG_VTS_THREADS": 128}),
+    ("vt_sort_threads_64", {"TG_VTS_THREADS": 64}),
+    ("vt_sort_threads_256", {"TG_VTS_THREADS": 256}),
     ("edge_items_16", {"TG_EDGE_ITEMS": 16}),
 ]
 # tet-count buckets of the batch's meshes: [lo, hi)
