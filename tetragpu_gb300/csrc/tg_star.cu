@@ -25,6 +25,7 @@
 //                   lengths in id order (one pass with a look-back scan)
 //   k_inc_sort      VV rows and incident-edge rows sorted
 //   k_edge_rows     a lane per cell of an edge: TE, the ET and EF rows
+#include <climits>
 #include <type_traits>
 
 #include "tg_internal.h"
@@ -65,44 +66,115 @@ __device__ __forceinline__ int mctz(unsigned long long m) { return __ffsll((long
 // on table inserts, work lists and barriers, and a second pass over it 840
 // more, doing every edge from both of its ends.
 //
-// The edges of a block's vertices gather in shared memory; at its end the
-// block takes their places in the high ends' incident rows, flags their first
-// occurrences and writes the records, every lane busy.  What does not fit
-// there goes out at once.
+// The edges of a warp's vertices gather in its own part of shared memory, and
+// go out with a lane each once the warp is through (or has no room for
+// another vertex): first-occurrence flags, places in the high ends' incident
+// rows, records.  No warp waits for another.
 constexpr int kStarThreads = TG_STAR_THREADS;
-constexpr int kStarPer = TG_STAR_PER;                       // vertices per warp, in sequence
-constexpr int kStarBlock = (kStarThreads / 32) * kStarPer;  // vertices per block
-constexpr int kRecCap = TG_STAR_WIN;                        // edges kept per block
+constexpr int kStarPer = TG_STAR_PER;     // most vertices per warp, in sequence
+constexpr int kRecCap = TG_STAR_WIN;      // edges a warp keeps
+constexpr int kStarWarps = kStarThreads / 32;
+constexpr int64_t kStarFill = 152 * 48;   // warps that fill the GPU once
 static_assert(kStarPer <= 32, "a warp fetches its vertices' rows a lane each");
+static_assert(kRecCap >= 3 * kMaxStar, "any one vertex's edges must fit");
 
 template <bool W>
 struct RecBuf {
-    uint4 e[kRecCap];   // first occurrence, mask (low), place among its low end's edges, high end
-    uint32_t hi[W ? kRecCap : 1];
-    int n;       // edges asked for
-    int end;     // first of those that did not fit
-    unsigned base;
+    uint2 e[kStarWarps][kRecCap];   // mask (low), high end
+    uint32_t hi[W ? kStarWarps : 1][W ? kRecCap : 1];
 };
 
 __device__ __forceinline__ int4 load_cell(const int4 *__restrict__ tvs, int c)
 {
     return c >= 0 ? __ldg(tvs + c) : make_int4(-1, -1, -1, -1);
 }
-
-template <bool W>
-__device__ __forceinline__ void put_edge(const StarPass &p, const uint4 &e, unsigned hi, int64_t g)
+// the slots of v < u in w, which holds both
+__device__ __forceinline__ void slots_of(const int4 &w, int v, int u, int &s, int &t)
 {
-    const unsigned in = (unsigned)atomicAdd(p.deg_in + e.w, 1);
-    atomicOr(p.eflag + (e.x >> 5), 1u << (e.x & 31));
-    p.rec[g] = make_uint2(e.x, e.y);
-    p.place[g] = make_uint2(e.z, in);
-    if constexpr (W) p.rec_hi[g] = hi;
+    s = (w.x < v) + (w.y < v);
+    t = 1 + (w.y < u) + (w.z < u);
 }
 
-// One vertex; H: cells per lane.
-template <int H, bool W>
+// the warp's n edges out; lane k holds its k-th vertex and where that vertex's
+// edges start among them (ascending; a vertex that comes later: past them all)
+template <bool W>
+__device__ __forceinline__ void put_edges(const StarPass &p, const RecBuf<W> &S, int n, int lv, int lrs,
+                                          int start)
+{
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    __syncwarp();
+    unsigned base = 0u;
+    if (lane == 0) base = atomicAdd(p.n_rec, (unsigned)n);
+    base = __shfl_sync(kAll, base, 0);
+    for (int i0 = 0; i0 < n; i0 += 32) {
+        const int i = i0 + lane;
+        int k = 0;   // the last vertex that starts at or before i
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1)
+            k += __shfl_sync(kAll, start, k + step) <= i ? step : 0;
+        const int v = __shfl_sync(kAll, lv, k), rs = __shfl_sync(kAll, lrs, k);
+        const unsigned place = (unsigned)(i - __shfl_sync(kAll, start, k));
+        if (i >= n) break;
+        const uint2 e = S.e[wp][i];
+        unsigned hi = 0u;
+        if constexpr (W) hi = S.hi[wp][i];
+        const unsigned in = (unsigned)atomicAdd(p.deg_in + e.y, 1);
+        // the first occurrence: the lowest position's cell
+        const int pos = e.x ? __ffs((int)e.x) - 1 : 31 + __ffs((int)hi);
+        const int c = __ldg(p.vt + rs + pos);
+        int sv, su;
+        slots_of(__ldg(p.tvs + c), v, (int)e.y, sv, su);
+        const unsigned slot = (unsigned)(6 * c + pair_slot(sv, su));
+        atomicOr(p.eflag + (slot >> 5), 1u << (slot & 31));
+        const int64_t g = (int64_t)base + i;
+        p.rec[g] = make_uint2(slot, e.x);
+        p.place[g] = make_uint2(place, in);
+        if constexpr (W) p.rec_hi[g] = hi;
+    }
+    __syncwarp();
+}
+
+// the highest set bit (-1: none; shuffles take their lane modulo 32)
+__device__ __forceinline__ int last_bit(unsigned m)
+{
+    int b;
+    asm("bfind.u32 %0, %1;" : "=r"(b) : "r"(m));
+    return b;
+}
+__device__ __forceinline__ int last_bit(unsigned long long m)
+{
+    int b;
+    asm("bfind.u64 %0, %1;" : "=r"(b) : "l"(m));
+    return b;
+}
+
+// predicated accesses: as branches the compiler splits and rejoins the warp
+// around each of them
+__device__ __forceinline__ void store_if(bool yes, int *at, int x)
+{
+    asm volatile("{ .reg .pred q; setp.ne.s32 q, %0, 0; @q st.global.s32 [%1], %2; }" ::"r"((int)yes),
+                 "l"(at), "r"(x)
+                 : "memory");
+}
+__device__ __forceinline__ void or_if(bool yes, uint32_t *at, unsigned x)
+{
+    asm volatile("{ .reg .pred q; setp.ne.s32 q, %0, 0; @q red.global.or.b32 [%1], %2; }" ::"r"((int)yes),
+                 "l"(at), "r"(x)
+                 : "memory");
+}
+__device__ __forceinline__ void store_shared_if(bool yes, unsigned at, const uint2 &x)
+{
+    asm volatile("{ .reg .pred q; setp.ne.s32 q, %0, 0; @q st.shared.v2.u32 [%1], {%2, %3}; }" ::"r"(
+                     (int)yes),
+                 "r"(at), "r"(x.x), "r"(x.y)
+                 : "memory");
+}
+
+// One vertex; H: cells per lane.  n: edges the warp holds, with room for any
+// vertex of such a star.  F: the faces' second cells are wanted (fnext).
+template <int H, bool W, bool F>
 __device__ __forceinline__ void star_vertex(const StarPass &p, RecBuf<W> &S, int v,
-                                            const int (&c)[H], const int4 (&w)[H])
+                                            const int (&c)[H], const int4 (&w)[H], int &n)
 {
     using M = typename std::conditional<H == 1, unsigned, unsigned long long>::type;
     // d: the candidates in slots 1..3 (slot 0 is never above another vertex
@@ -111,7 +183,7 @@ __device__ __forceinline__ void star_vertex(const StarPass &p, RecBuf<W> &S, int
     // at most kNarrowStar cells); with two cells a lane the marks and the
     // masks are apart
     constexpr unsigned kDone = 0x80000000u;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     unsigned d[H][3];
     M m[H][3];
 #pragma unroll
@@ -121,6 +193,8 @@ __device__ __forceinline__ void star_vertex(const StarPass &p, RecBuf<W> &S, int
         d[h][2] = w[h].w > v ? (unsigned)w[h].w : kDone;
         m[h][0] = m[h][1] = m[h][2] = 0;
     }
+    const int n0 = n;
+    unsigned out = (unsigned)__cvta_generic_to_shared(S.e[wp] + n);
     while (true) {
         unsigned cn = min(d[0][0], min(d[0][1], d[0][2]));
         if constexpr (H == 2) cn = min(cn, min(d[1][0], min(d[1][1], d[1][2])));
@@ -147,172 +221,142 @@ __device__ __forceinline__ void star_vertex(const StarPass &p, RecBuf<W> &S, int
                     m[h][k] = hit[h][k] ? mu : m[h][k];
                 }
             }
+        store_shared_if(lane == 0, out, make_uint2((unsigned)mu, u));
+        if constexpr (W)
+            if (lane == 0) S.hi[wp][n] = H == 2 ? (unsigned)((unsigned long long)mu >> 32) : 0u;
+        out += sizeof(uint2);
+        n++;
     }
-    if constexpr (H == 1) {
-#pragma unroll
-        for (int k = 0; k < 3; k++) m[0][k] = d[0][k] & ~kDone;
-    }
-
-    // the edges first met in this lane's cells
-    unsigned first[H][3];
-    int total = 0;
-#pragma unroll
-    for (int h = 0; h < H; h++)
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const M low = m[h][k] & (0 - m[h][k]);
-            first[h][k] = __ballot_sync(kAll, low == (M)1 << (lane + 32 * h));
-            total += __popc(first[h][k]);
-        }
-    if (total) {   // warp-uniform
-        int at = 0;
-        if (lane == 0) {
-            at = atomicAdd(&S.n, total);
-            p.deg_own[v] = total;
-        }
-        at = __shfl_sync(kAll, at, 0);
-        const bool fits = at + total <= kRecCap;
-        int64_t g = 0;
-        if (!fits) {
-            unsigned base = 0u;
-            if (lane == 0) {
-                atomicMin(&S.end, at);
-                base = atomicAdd(p.n_rec, (unsigned)total);
-            }
-            g = (int64_t)__shfl_sync(kAll, base, 0);
-        }
-        int i0 = 0;
-#pragma unroll
-        for (int h = 0; h < H; h++) {
-            const int sv = (w[h].x < v) + (w[h].y < v) + (w[h].z < v);
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                if ((first[h][k] >> lane) & 1u) {
-                    const int i = i0 + __popc(first[h][k] & ((1u << lane) - 1u));
-                    const uint4 e = make_uint4((unsigned)(6 * c[h] + pair_slot(sv, k + 1)),
-                                               (unsigned)m[h][k], (unsigned)i,
-                                               (unsigned)get4(w[h], k + 1));
-                    unsigned hi = 0u;
-                    if constexpr (H == 2) hi = (unsigned)(m[h][k] >> 32);
-                    if (fits) {
-                        S.e[at + i] = e;
-                        if constexpr (W) S.hi[at + i] = hi;
-                    } else {
-                        put_edge<W>(p, e, hi, g + i);
-                    }
-                }
-                i0 += __popc(first[h][k]);
-            }
-        }
-    }
+    store_if(lane == 0, p.deg_own + v, n - n0);
 
     // faces whose lowest vertex is v: two of the candidates, the third left
     // out (v in slot 0: slot 1, 2 or 3; v in slot 1: slot 0; the masks of
     // slots at or below v's are zero)
 #pragma unroll
     for (int h = 0; h < H; h++) {
+        if constexpr (H == 1) {
+#pragma unroll
+            for (int k = 0; k < 3; k++) m[0][k] = d[0][k] & ~kDone;
+        }
         const M bit = (M)1 << (lane + 32 * h);
         const int sh = 4 * (c[h] & 7);
+        // the column of the face omitting slot o is 3 - o
+        const int col0 = w[h].x == v ? 2 : 3;
         unsigned firsts = 0u, alone = 0u;
         M more = 0;
-        int *next = p.fnext + 4LL * c[h];
+        int *next = F ? p.fnext + 4LL * c[h] : nullptr;
+        int *next0 = F ? next + col0 : nullptr;
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             const M f = k == 0 ? m[h][1] & m[h][2] : (k == 1 ? m[h][0] & m[h][2] : m[h][0] & m[h][1]);
             const M rest = f & (f - 1);
-            // the column of the face omitting slot o is 3 - o
-            const int col = k == 0 ? ((w[h].x == v) ? 2 : 3) : 2 - k;
-            const int s2 = H == 1 ? 31 - __clz((int)(unsigned)rest) : 63 - __clzll((long long)rest);
-            int c2 = __shfl_sync(kAll, c[0], s2 & 31);
-            if constexpr (H == 2) {
-                const int c2b = __shfl_sync(kAll, c[1], s2 & 31);
-                if (s2 >= 32) c2 = c2b;
-            }
-            if ((f ^ rest) == bit) {
-                firsts |= 1u << col;
-                if (!rest) alone |= 1u << col;
-                more |= rest & (rest - 1);
-                if (p.fnext) next[col] = rest ? c2 : -1;
-            }
-        }
-        if (firsts) atomicOr(p.fflag + (c[h] >> 3), firsts << sh);
-        if (alone) {   // boundary faces
-            atomicOr(p.fbnd + (c[h] >> 3), alone << sh);
-#pragma unroll
-            for (int col = 0; col < 4; col++)
-                if ((alone >> col) & 1u) {
-                    p.vbnd[col == 3 ? w[h].y : w[h].x] = 1;
-                    p.vbnd[col >= 2 ? w[h].z : w[h].y] = 1;
-                    p.vbnd[col >= 1 ? w[h].w : w[h].z] = 1;
+            const bool is_first = (f ^ rest) == bit;
+            const unsigned mark = k == 0 ? 1u << col0 : 1u << (2 - k);
+            firsts |= is_first ? mark : 0u;
+            alone |= is_first && !rest ? mark : 0u;
+            more |= rest & (rest - 1);
+            if constexpr (F) {
+                const int s2 = last_bit(rest);
+                int c2 = __shfl_sync(kAll, c[0], s2);
+                if constexpr (H == 2) {
+                    const int c2b = __shfl_sync(kAll, c[1], s2);
+                    c2 = s2 >= 32 ? c2b : c2;
                 }
+                store_if(is_first, k == 0 ? next0 : next + (2 - k), rest ? c2 : -1);
+            }
         }
-        if (more) {
-            atomicOr(&p.st->flags, ST_NONMANIFOLD_FACE);
-            atomicMin(&p.st->bad_cell, c[h]);
+        or_if(firsts != 0u, p.fflag + (c[h] >> 3), firsts << sh);
+        if (__any_sync(kAll, alone || more)) {   // boundary faces, faces of too many cells
+            if (alone) {
+                atomicOr(p.fbnd + (c[h] >> 3), alone << sh);
+#pragma unroll
+                for (int col = 0; col < 4; col++)
+                    if ((alone >> col) & 1u) {
+                        p.vbnd[col == 3 ? w[h].y : w[h].x] = 1;
+                        p.vbnd[col >= 2 ? w[h].z : w[h].y] = 1;
+                        p.vbnd[col >= 1 ? w[h].w : w[h].z] = 1;
+                    }
+            }
+            if (more) {
+                // reported by the face's first cell
+                bool here = false;
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    const M f = k == 0 ? m[h][1] & m[h][2]
+                                       : (k == 1 ? m[h][0] & m[h][2] : m[h][0] & m[h][1]);
+                    const M rest = f & (f - 1);
+                    here |= (f ^ rest) == bit && (rest & (rest - 1)) != 0;
+                }
+                if (here) {
+                    atomicOr(&p.st->flags, ST_NONMANIFOLD_FACE);
+                    atomicMin(&p.st->bad_cell, c[h]);
+                }
+            }
         }
     }
 }
 
 // W: the mesh has stars of more than kNarrowStar cells
-template <bool W>
-__global__ void __launch_bounds__(kStarThreads, W ? 8 : TG_STAR_MINB) k_star(StarPass p)
+template <bool W, bool F>
+__global__ void __launch_bounds__(kStarThreads, W ? 8 : TG_STAR_MINB) k_star(StarPass p, int per)
 {
     griddep_wait();
     __shared__ RecBuf<W> S;
-    if (threadIdx.x == 0) {
-        S.n = 0;
-        S.end = kRecCap;
-    }
-    __syncthreads();
     const int lane = threadIdx.x & 31;
-    const int64_t pos = (int64_t)blockIdx.x * kStarBlock + (threadIdx.x >> 5) * kStarPer;
-    // lane k < kStarPer: the warp's k-th vertex, its row's start and length
+    const int64_t pos = ((int64_t)blockIdx.x * kStarWarps + (threadIdx.x >> 5)) * per;
+    // lane k < per: the warp's k-th vertex, its row's start and length
     int lv = -1, lrs = 0, lD = 0;
-    if (lane < kStarPer && pos + lane < p.n_light) {
+    if (lane < per && pos + lane < p.n_light) {
         lv = p.vorder[pos + lane];
         lrs = (int)p.vt_off[lv];
         lD = (int)(p.vt_off[lv + 1] - lrs);
     }
     auto load_entry = [&](int k) {   // this lane's cell of the k-th vertex (the first 32)
-        const int rs = __shfl_sync(kAll, lrs, k), D = __shfl_sync(kAll, lD, k);
+        const int rs = __shfl_sync(kAll, lrs, k & 31), D = __shfl_sync(kAll, lD, k & 31);
         return lane < D ? __ldg(p.vt + rs + lane) : -1;
     };
     // the next vertex's cells and the one after's row are in flight while a
-    // vertex is worked on
+    // vertex is worked on (past the warp's last vertex the rows are empty but
+    // for a wrap to its first, which is not looked at)
     int c0 = load_entry(0), c1 = load_entry(1);
     int4 w0 = load_cell(p.tvs, c0);
+    int n = 0, start = INT_MAX;
+    auto flush = [&](int k) {   // the edges of the vertices before the k-th
+        put_edges<W>(p, S, n, lv, lrs, start);
+        n = 0;
+        if (lane < k) start = -1;
+    };
 #pragma unroll 1
-    for (int k = 0; k < kStarPer; k++) {
+    for (int k = 0; k < per; k++) {
         const int v = __shfl_sync(kAll, lv, k);
         if (v < 0) break;
         const int4 w1 = load_cell(p.tvs, c1);
-        const int c2 = k + 2 < kStarPer ? load_entry(k + 2) : -1;
+        const int c2 = load_entry(k + 2);
         bool done = false;
         if constexpr (W) {
             const int rs = __shfl_sync(kAll, lrs, k), D = __shfl_sync(kAll, lD, k);
             if (D > kNarrowStar) {
+                if (n + 3 * D > kRecCap) flush(k);
+                if (lane == k) start = n;
                 const int cb = lane + 32 < D ? __ldg(p.vt + rs + lane + 32) : -1;
                 const int c[2] = {c0, cb};
                 const int4 w[2] = {w0, load_cell(p.tvs, cb)};
-                star_vertex<2, W>(p, S, v, c, w);
+                star_vertex<2, W, F>(p, S, v, c, w, n);
                 done = true;
             }
         }
         if (!done) {
+            if (n > kRecCap - 3 * kNarrowStar) flush(k);
+            if (lane == k) start = n;
             const int c[1] = {c0};
             const int4 w[1] = {w0};
-            star_vertex<1, W>(p, S, v, c, w);
+            star_vertex<1, W, F>(p, S, v, c, w, n);
         }
         c0 = c1;
         w0 = w1;
         c1 = c2;
     }
-    __syncthreads();
-    const int kept = min(S.n, S.end);
-    if (threadIdx.x == 0 && kept) S.base = atomicAdd(p.n_rec, (unsigned)kept);
-    __syncthreads();
-    for (int i = threadIdx.x; i < kept; i += kStarThreads)
-        put_edge<W>(p, S.e[i], W ? S.hi[i] : 0u, (int64_t)S.base + i);
+    if (n) put_edges<W>(p, S, n, lv, lrs, start);
 }
 
 // ---------------------------------------------------------------------------
@@ -404,13 +448,6 @@ __device__ __forceinline__ EdgeEnds edge_ends(const int4 *__restrict__ tvs, unsi
     e.u = e.j == 0 ? w.y : (e.j == 1 || e.j == 3 ? w.z : w.w);
     return e;
 }
-// the slots of v < u in w, which holds both
-__device__ __forceinline__ void slots_of(const int4 &w, int v, int u, int &s, int &t)
-{
-    s = (w.x < v) + (w.y < v);
-    t = 1 + (w.y < u) + (w.z < u);
-}
-
 // The cells of an edge record: the star positions of its owner v that its
 // mask holds, ascending.  W: masks of stars of more than kNarrowStar cells
 // have a high half in rec_hi; a star of more than 64 cells (tg_heavy.cu) keeps
@@ -991,11 +1028,13 @@ void launch_star(const StarPass &p, cudaStream_t s)
 {
     if (p.n_light == 0) return;
     Launch L("k_star", s);
-    const unsigned grid = (unsigned)((p.n_light + kStarBlock - 1) / kStarBlock);
-    if (p.rec_hi)
-        launch_pdl(k_star<true>, grid, kStarThreads, 0, s, p);
-    else
-        launch_pdl(k_star<false>, grid, kStarThreads, 0, s, p);
+    // vertices per warp: enough warps for every SM before long sequences
+    const int per = (int)std::min<int64_t>(std::max<int64_t>(p.n_light / kStarFill, 1), kStarPer);
+    const int64_t warps = (p.n_light + per - 1) / per;
+    const unsigned grid = (unsigned)((warps + kStarWarps - 1) / kStarWarps);
+    auto *k = p.rec_hi ? (p.fnext ? k_star<true, true> : k_star<true, false>)
+                       : (p.fnext ? k_star<false, true> : k_star<false, false>);
+    launch_pdl(k, grid, kStarThreads, 0, s, p, per);
 }
 
 void launch_cell_faces(int64_t T, const int4 *tvs, const uint2 *frank, const int32_t *fnext,

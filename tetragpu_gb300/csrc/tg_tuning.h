@@ -9,16 +9,16 @@
 
 // defaults of the rest
 #ifndef TG_STAR_WIN
-#define TG_STAR_WIN 256   // edge records a star-pass block keeps in shared memory
+#define TG_STAR_WIN 256   // edges a star-pass warp keeps in shared memory
 #endif
 #ifndef TG_STAR_THREADS
 #define TG_STAR_THREADS 128   // threads per star-pass block
 #endif
 #ifndef TG_STAR_PER
-#define TG_STAR_PER 4   // vertices per warp of the star pass
+#define TG_STAR_PER 16   // most vertices per warp of the star pass
 #endif
 #ifndef TG_STAR_MINB
-#define TG_STAR_MINB 12   // resident blocks per SM asked of the star pass
+#define TG_STAR_MINB 10   // resident blocks per SM asked of the star pass
 #endif
 #ifndef TG_VTS_THREADS
 #define TG_VTS_THREADS 128   // threads per VT-sort block
