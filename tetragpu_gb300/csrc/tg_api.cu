@@ -342,7 +342,7 @@ struct tg_mesh {
     // stars of more than kMaxStar cells (tg_heavy.cu): processing positions
     // n_light .. n_light + n_heavy - 1, heavy_entries VT entries in all
     int64_t n_light = 0, n_heavy = 0, heavy_entries = 0;
-    bool wide_stars = false;    // a light star holds more than 32 cells (64-bit masks)
+    int64_t n_wide = 0;         // light stars of more than 31 cells (64-bit masks)
     int max_deg = 0;            // largest degree above kMaxDeg seen by the extraction, else 0
     uint64_t *cadj = nullptr;   // link adjacency for critical points, aligned with VV
     DevStatus *st = nullptr;    // device
@@ -507,7 +507,7 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
             const size_t o_e = c.add<uint32_t>(nwe), o_f = c.add<uint32_t>(nwf),
                          o_b = c.add<uint32_t>(nwf), o_d = c.add<int32_t>(V),
                          o_i = c.add<int32_t>(V),
-                         o_v = c.add<uint8_t>(V), o_n = c.add<uint32_t>(1);
+                         o_v = c.add<uint8_t>(V), o_n = c.add<uint32_t>(2);
             char *z;
             TRY(tmp.alloc(&z, (int64_t)c.bytes, true));
             eflag = (uint32_t *)(z + o_e);
@@ -517,6 +517,7 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
             sp.deg_in = (int32_t *)(z + o_i);
             sp.vbnd = (uint8_t *)(z + o_v);
             sp.n_rec = (uint32_t *)(z + o_n);
+            sp.n_wide = sp.n_rec + 1;
         }
         TRY(tmp.alloc(&erank, nwe + 1));
         TRY(tmp.alloc(&frank, nwf + 1));
@@ -528,7 +529,8 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         // at most six edges a cell (their number is read back below)
         TRY(tmp.alloc(&sp.rec, 6 * T));
         TRY(tmp.alloc(&sp.place, 6 * T));
-        if (m->wide_stars || m->n_heavy > 0) TRY(tmp.alloc(&sp.rec_hi, 6 * T));
+        if (m->n_wide > 0 || m->n_heavy > 0) TRY(tmp.alloc(&sp.rec_hi, 6 * T));
+        if (m->n_wide > 0) TRY(tmp.alloc(&sp.wide, m->n_wide));
         if (need_tf || need_ft) TRY(tmp.alloc(&sp.fnext, 4 * T));
         sp.n_light = m->n_light;
         sp.vorder = m->vorder;
@@ -540,6 +542,7 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         sp.fbnd = fbnd;
         sp.st = m->st;
         launch_star(sp, s);
+        launch_star_wide(sp, m->n_wide, s);
         HeavyStars hv{};
         if (m->n_heavy > 0) {
             hv.star = sp;
@@ -882,14 +885,14 @@ static tg_status mesh_create_impl(const int32_t *tv, int64_t T, int64_t V, int o
     CK(cudaGetLastError());
     set_csr(m, TG_REL_VT, vt_off, vt, V, 4 * T);
     // vertices with light stars, heavy ones, the heavy stars' entries and
-    // whether a light star holds more than 32 cells
+    // the light stars of more than 31 cells
     const void *rd[4] = {&vrank[nwk].y, heavy_cnt, heavy_cnt + 1, heavy_cnt + 2};
     const bool w8[4] = {false, false, false, false};
     TRY(sync_read(m, s, 4, rd, w8));
     m->n_light = T ? m->sz_host[0] : 0;
     m->n_heavy = T ? m->sz_host[1] : 0;
     m->heavy_entries = T ? m->sz_host[2] : 0;
-    m->wide_stars = T ? m->sz_host[3] != 0 : false;
+    m->n_wide = T ? m->sz_host[3] : 0;
     return check_flags(m);
 }
 

@@ -177,7 +177,7 @@ void launch_window_starts(const int64_t *off, int64_t rows, int64_t n_entries, i
 // and stores it in vkey[v]; rows with no cells are left alone.  A vertex of
 // more than kMaxStar cells takes no key: it is counted in heavy_cnt[0] (vkey
 // -1 - index) with its entries in heavy_cnt[1], where they start in
-// heavy_off[index].
+// heavy_off[index].  heavy_cnt[2] counts the wide light stars.
 void launch_vt_sort(const int64_t *vt_off, int32_t *vt, int64_t V, int64_t nvt, const int4 *tvs,
                     uint32_t *vflag, int64_t *vkey, int32_t *heavy_cnt, int32_t *heavy_off,
                     cudaStream_t s);
@@ -210,11 +210,17 @@ struct StarPass {
     uint2 *rec;                // {first occurrence slot, star positions of the low end's star
                                // holding the edge (the low 32)}
     uint2 *place;              // {place among the low end's own edges, among the high end's others}
-    uint32_t *rec_hi;          // the high 32 positions; null when no star is wider than 32
+    uint32_t *rec_hi;          // the high 32 positions, of edges of wide stars only; null when
+                               // there are none
     uint32_t *n_rec;           // the number of records (zeroed by the caller)
+    int32_t *wide;             // [V] light vertices of wide stars (more than 31 cells), or null
+    uint32_t *n_wide;          // their number (zeroed by the caller)
     DevStatus *st;
 };
+// launch_star lists the wide stars for launch_star_wide (n_wide: at least
+// their number)
 void launch_star(const StarPass &p, cudaStream_t s);
+void launch_star_wide(const StarPass &p, int64_t n_wide, cudaStream_t s);
 // seg_ef[i] = first edge id and seg_ef[n + 1 + i] = first face id of the
 // cells from seg_c[i] on (i = 0 .. n; seg_c[n] = T gives the totals)
 void launch_seg_ranks(const int64_t *seg_c, int64_t n, const uint2 *erank, const uint2 *frank,

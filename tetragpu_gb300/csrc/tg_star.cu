@@ -13,7 +13,8 @@
 // An edge and a face belong to their lowest vertex: only that vertex's star
 // looks at them, so every edge and every face is found once.
 //
-//   k_star          a warp per vertex, a lane per star cell: the vertex's own
+//   k_star, k_star_wide
+//                   a warp per vertex, a lane per star cell: the vertex's own
 //                   edges (each with the mask of star positions holding it)
 //                   and faces; first-occurrence bitmaps, a record per edge, a
 //                   face's second cell at its first occurrence
@@ -78,10 +79,11 @@ constexpr int64_t kStarFill = 152 * 48;   // warps that fill the GPU once
 static_assert(kStarPer <= 32, "a warp fetches its vertices' rows a lane each");
 static_assert(kRecCap >= 3 * kMaxStar, "any one vertex's edges must fit");
 
-template <bool W>
+// H: cells per lane (2: stars of more than kNarrowStar cells)
+template <int H>
 struct RecBuf {
     uint2 e[kStarWarps][kRecCap];   // mask (low), high end
-    uint32_t hi[W ? kStarWarps : 1][W ? kRecCap : 1];
+    uint32_t hi[H == 2 ? kStarWarps : 1][H == 2 ? kRecCap : 1];
 };
 
 __device__ __forceinline__ int4 load_cell(const int4 *__restrict__ tvs, int c)
@@ -97,8 +99,8 @@ __device__ __forceinline__ void slots_of(const int4 &w, int v, int u, int &s, in
 
 // the warp's n edges out; lane k holds its k-th vertex and where that vertex's
 // edges start among them (ascending; a vertex that comes later: past them all)
-template <bool W>
-__device__ __forceinline__ void put_edges(const StarPass &p, const RecBuf<W> &S, int n, int lv, int lrs,
+template <int H>
+__device__ __forceinline__ void put_edges(const StarPass &p, const RecBuf<H> &S, int n, int lv, int lrs,
                                           int start)
 {
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
@@ -117,7 +119,7 @@ __device__ __forceinline__ void put_edges(const StarPass &p, const RecBuf<W> &S,
         if (i >= n) break;
         const uint2 e = S.e[wp][i];
         unsigned hi = 0u;
-        if constexpr (W) hi = S.hi[wp][i];
+        if constexpr (H == 2) hi = S.hi[wp][i];
         const unsigned in = (unsigned)atomicAdd(p.deg_in + e.y, 1);
         // the first occurrence: the lowest position's cell
         const int pos = e.x ? __ffs((int)e.x) - 1 : 31 + __ffs((int)hi);
@@ -129,7 +131,7 @@ __device__ __forceinline__ void put_edges(const StarPass &p, const RecBuf<W> &S,
         const int64_t g = (int64_t)base + i;
         p.rec[g] = make_uint2(slot, e.x);
         p.place[g] = make_uint2(place, in);
-        if constexpr (W) p.rec_hi[g] = hi;
+        if constexpr (H == 2) p.rec_hi[g] = hi;
     }
     __syncwarp();
 }
@@ -172,8 +174,8 @@ __device__ __forceinline__ void store_shared_if(bool yes, unsigned at, const uin
 
 // One vertex; H: cells per lane.  n: edges the warp holds, with room for any
 // vertex of such a star.  F: the faces' second cells are wanted (fnext).
-template <int H, bool W, bool F>
-__device__ __forceinline__ void star_vertex(const StarPass &p, RecBuf<W> &S, int v,
+template <int H, bool F>
+__device__ __forceinline__ void star_vertex(const StarPass &p, RecBuf<H> &S, int v,
                                             const int (&c)[H], const int4 (&w)[H], int &n)
 {
     using M = typename std::conditional<H == 1, unsigned, unsigned long long>::type;
@@ -222,8 +224,8 @@ __device__ __forceinline__ void star_vertex(const StarPass &p, RecBuf<W> &S, int
                 }
             }
         store_shared_if(lane == 0, out, make_uint2((unsigned)mu, u));
-        if constexpr (W)
-            if (lane == 0) S.hi[wp][n] = H == 2 ? (unsigned)((unsigned long long)mu >> 32) : 0u;
+        if constexpr (H == 2)
+            if (lane == 0) S.hi[wp][n] = (unsigned)(mu >> 32);
         out += sizeof(uint2);
         n++;
     }
@@ -296,12 +298,13 @@ __device__ __forceinline__ void star_vertex(const StarPass &p, RecBuf<W> &S, int
     }
 }
 
-// W: the mesh has stars of more than kNarrowStar cells
-template <bool W, bool F>
-__global__ void __launch_bounds__(kStarThreads, W ? 8 : TG_STAR_MINB) k_star(StarPass p, int per)
+// The light vertices of at most kNarrowStar cells; the others go on a list
+// (about in processing order) that k_star_wide takes.
+template <bool F>
+__global__ void __launch_bounds__(kStarThreads, TG_STAR_MINB) k_star(StarPass p, int per)
 {
     griddep_wait();
-    __shared__ RecBuf<W> S;
+    __shared__ RecBuf<1> S;
     const int lane = threadIdx.x & 31;
     const int64_t pos = ((int64_t)blockIdx.x * kStarWarps + (threadIdx.x >> 5)) * per;
     // lane k < per: the warp's k-th vertex, its row's start and length
@@ -310,6 +313,7 @@ __global__ void __launch_bounds__(kStarThreads, W ? 8 : TG_STAR_MINB) k_star(Sta
         lv = p.vorder[pos + lane];
         lrs = (int)p.vt_off[lv];
         lD = (int)(p.vt_off[lv + 1] - lrs);
+        if (lD > kNarrowStar) p.wide[atomicAdd(p.n_wide, 1u)] = lv;
     }
     auto load_entry = [&](int k) {   // this lane's cell of the k-th vertex (the first 32)
         const int rs = __shfl_sync(kAll, lrs, k & 31), D = __shfl_sync(kAll, lD, k & 31);
@@ -321,42 +325,49 @@ __global__ void __launch_bounds__(kStarThreads, W ? 8 : TG_STAR_MINB) k_star(Sta
     int c0 = load_entry(0), c1 = load_entry(1);
     int4 w0 = load_cell(p.tvs, c0);
     int n = 0, start = INT_MAX;
-    auto flush = [&](int k) {   // the edges of the vertices before the k-th
-        put_edges<W>(p, S, n, lv, lrs, start);
-        n = 0;
-        if (lane < k) start = -1;
-    };
 #pragma unroll 1
     for (int k = 0; k < per; k++) {
         const int v = __shfl_sync(kAll, lv, k);
         if (v < 0) break;
         const int4 w1 = load_cell(p.tvs, c1);
         const int c2 = load_entry(k + 2);
-        bool done = false;
-        if constexpr (W) {
-            const int rs = __shfl_sync(kAll, lrs, k), D = __shfl_sync(kAll, lD, k);
-            if (D > kNarrowStar) {
-                if (n + 3 * D > kRecCap) flush(k);
-                if (lane == k) start = n;
-                const int cb = lane + 32 < D ? __ldg(p.vt + rs + lane + 32) : -1;
-                const int c[2] = {c0, cb};
-                const int4 w[2] = {w0, load_cell(p.tvs, cb)};
-                star_vertex<2, W, F>(p, S, v, c, w, n);
-                done = true;
+        if (__shfl_sync(kAll, lD, k) <= kNarrowStar) {
+            if (n > kRecCap - 3 * kNarrowStar) {   // out with the edges of the vertices before this
+                put_edges<1>(p, S, n, lv, lrs, start);
+                n = 0;
+                if (lane < k) start = -1;
             }
-        }
-        if (!done) {
-            if (n > kRecCap - 3 * kNarrowStar) flush(k);
             if (lane == k) start = n;
             const int c[1] = {c0};
             const int4 w[1] = {w0};
-            star_vertex<1, W, F>(p, S, v, c, w, n);
+            star_vertex<1, F>(p, S, v, c, w, n);
+        } else if (lane == k) {
+            start = n;   // no edges here
         }
         c0 = c1;
         w0 = w1;
         c1 = c2;
     }
-    if (n) put_edges<W>(p, S, n, lv, lrs, start);
+    if (n) put_edges<1>(p, S, n, lv, lrs, start);
+}
+
+// a vertex of kNarrowStar + 1 to kMaxStar cells per warp
+template <bool F>
+__global__ void __launch_bounds__(kStarThreads) k_star_wide(StarPass p)
+{
+    griddep_wait();
+    __shared__ RecBuf<2> S;
+    const int lane = threadIdx.x & 31;
+    const unsigned i = blockIdx.x * kStarWarps + (threadIdx.x >> 5);
+    if (i >= *p.n_wide) return;
+    const int v = p.wide[i];
+    const int rs = (int)p.vt_off[v], D = (int)(p.vt_off[v + 1] - rs);
+    const int c[2] = {lane < D ? __ldg(p.vt + rs + lane) : -1,
+                      lane + 32 < D ? __ldg(p.vt + rs + lane + 32) : -1};
+    const int4 w[2] = {load_cell(p.tvs, c[0]), load_cell(p.tvs, c[1])};
+    int n = 0;
+    star_vertex<2, F>(p, S, v, c, w, n);
+    if (n) put_edges<2>(p, S, n, v, rs, lane == 0 ? 0 : INT_MAX);
 }
 
 // ---------------------------------------------------------------------------
@@ -486,7 +497,7 @@ __global__ void __launch_bounds__(256) k_edge_ids(EdgePass p)
     const bool walk = p.count_ef && __ldg(p.vbnd + e.v) && __ldg(p.vbnd + e.u);
     const int64_t rs = W || walk ? __ldg(p.vt_off + e.v) : 0;
     const int D = W ? (int)(__ldg(p.vt_off + e.v + 1) - rs) : 0;
-    const unsigned hi = W ? __ldg(p.rec_hi + r) : 0u;
+    const unsigned hi = W && D > kNarrowStar ? __ldg(p.rec_hi + r) : 0u;
     int nb = 0, n_et;
     auto look = [&](int pos) {
         const int c = __ldg(p.vt + rs + pos);
@@ -502,7 +513,7 @@ __global__ void __launch_bounds__(256) k_edge_ids(EdgePass p)
             for (int k = 0; k < n_et; k++) look(p.pairs[(int64_t)rec.y + k].y);
     } else {
         unsigned long long m = rec.y;
-        if (W && D > kNarrowStar) m |= (unsigned long long)hi << 32;
+        if (W) m |= (unsigned long long)hi << 32;
         n_et = W ? __popcll(m) : __popc(rec.y);
         if (walk)
             for (; m; m &= m - 1) look(mctz(m));
@@ -510,7 +521,7 @@ __global__ void __launch_bounds__(256) k_edge_ids(EdgePass p)
     const unsigned ee = (unsigned)((rv1 - __ldg(p.vv_off + e.v)) +
                                    (__ldg(p.vv_off + e.u + 1) - ru) - 2);
     p.edge[id] = make_uint4(rec.x, rec.y, (unsigned)n_et | (unsigned)(n_et + nb / 2) << 16, ee);
-    if constexpr (W) p.edge_hi[id] = hi;
+    if (W && D > kNarrowStar) p.edge_hi[id] = hi;
 }
 
 // k_edge_rows: TE at each cell of an edge, ET and EF rows.  A warp takes 32
@@ -660,9 +671,6 @@ __device__ __forceinline__ void mark_first(const int4 *__restrict__ tvs, uint32_
         heavy_off[k] = atomicAdd(heavy_cnt + 1, D);   // its share of the heavy scratch
         return;
     }
-    // heavy_cnt[2]: some light star holds more than kNarrowStar cells (the
-    // edge records then have a high half)
-    if (D > kNarrowStar) heavy_cnt[2] = 1;
     const int4 w = __ldg(tvs + c);
     const long long key = 4LL * c + (w.x == v ? 0 : (w.y == v ? 1 : (w.z == v ? 2 : 3)));
     vkey[v] = key;
@@ -726,9 +734,14 @@ k_vt_sort(const int64_t *__restrict__ vt_off, int64_t V, int64_t total, int *__r
 {
     griddep_wait();
     __shared__ RowStage S;
+    int wide = 0;
     sort_block_rows(S, vt_off, V, total, vt, [&](int v, int c, int D) {
+        wide = D > kNarrowStar && D <= kMaxStar;
         mark_first(tvs, vflag, vkey, heavy_cnt, heavy_off, v, c, D);
     });
+    // heavy_cnt[2]: light stars of more than kNarrowStar cells
+    wide = __syncthreads_count(wide);
+    if (wide && threadIdx.x == 0) atomicAdd(heavy_cnt + 2, wide);
 }
 
 // VV rows in place
@@ -1032,9 +1045,15 @@ void launch_star(const StarPass &p, cudaStream_t s)
     const int per = (int)std::min<int64_t>(std::max<int64_t>(p.n_light / kStarFill, 1), kStarPer);
     const int64_t warps = (p.n_light + per - 1) / per;
     const unsigned grid = (unsigned)((warps + kStarWarps - 1) / kStarWarps);
-    auto *k = p.rec_hi ? (p.fnext ? k_star<true, true> : k_star<true, false>)
-                       : (p.fnext ? k_star<false, true> : k_star<false, false>);
-    launch_pdl(k, grid, kStarThreads, 0, s, p, per);
+    launch_pdl(p.fnext ? k_star<true> : k_star<false>, grid, kStarThreads, 0, s, p, per);
+}
+
+void launch_star_wide(const StarPass &p, int64_t n_wide, cudaStream_t s)
+{
+    if (n_wide == 0) return;
+    Launch L("k_star_wide", s);
+    launch_pdl(p.fnext ? k_star_wide<true> : k_star_wide<false>,
+               (unsigned)((n_wide + kStarWarps - 1) / kStarWarps), kStarThreads, 0, s, p);
 }
 
 void launch_cell_faces(int64_t T, const int4 *tvs, const uint2 *frank, const int32_t *fnext,
