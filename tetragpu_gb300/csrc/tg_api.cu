@@ -331,6 +331,7 @@ struct tg_mesh {
     int4 *tvs = nullptr;
     // star processing order: vertices by first cell (see tg_star.cu)
     int32_t *vorder = nullptr;          // [V] vertex at each position (cell-less ones last)
+    int32_t *vpos = nullptr;            // [V] position of each vertex
     int32_t *heavy_off = nullptr;       // where each heavy star's entries start among theirs
     ScanWorkspace scan;                 // every prefix scan of the mesh (tg_scan.cu)
     // segments of cells (the meshes of a batch): cell starts, and after each
@@ -344,7 +345,11 @@ struct tg_mesh {
     int64_t n_light = 0, n_heavy = 0, heavy_entries = 0;
     int64_t n_wide = 0;         // light stars of more than 31 cells (64-bit masks)
     int max_deg = 0;            // largest degree above kMaxDeg seen by the extraction, else 0
-    uint64_t *cadj = nullptr;   // link adjacency for critical points, aligned with VV
+    bool wide_deg = false;      // a vertex has more than kNarrowDeg neighbours
+    // the link adjacency of critical points (LinkGraph; adj null: not built)
+    int64_t *lg_off = nullptr;
+    int32_t *lg_ent = nullptr;
+    void *lg_adj = nullptr;
     DevStatus *st = nullptr;    // device
     DevStatus *st_host = nullptr;
     int64_t *sz_host = nullptr; // pinned slots for sizes read back at sync points
@@ -447,29 +452,57 @@ void set_csr(tg_mesh *m, int r, int64_t *off, int32_t *ent, int64_t rows, int64_
     x.opts = opts;
 }
 
-// The link adjacency of critical points into m->cadj (allocated by the
-// caller), on stream s: VV's rows visited in the star processing order, so
-// that the neighbours' rows a window reads were read by the windows just
-// before it (in L2); the order's row lengths, their prefix and its window
-// table are temporaries of tmp.
-tg_status build_link_adjacency(tg_mesh *m, const int64_t *vv_off, const int32_t *vv, int64_t nvv,
-                               Temps &tmp, cudaStream_t s)
+void free_link_graph(tg_mesh *m, cudaStream_t s)
 {
-    const int64_t V = m->V;
-    int32_t *len, *win;
-    int64_t *ooff, *ostart;
-    TRY(tmp.alloc(&len, V));
-    TRY(tmp.alloc(&ooff, V + 1));
-    TRY(tmp.alloc(&ostart, V));
-    TRY(tmp.alloc(&win, window_count(nvv, crit_window()) + 1));
-    launch_vv_lengths_in_order(vv_off, m->vorder, V, m->n_light + m->n_heavy, len, ostart, s);
-    ScanJob job{len, ooff, V, SCAN_COUNT_I32, nullptr};
-    scan_batch(&job, 1, m->scan, m->st, s);
-    launch_window_starts(ooff, V, nvv, crit_window(), win, s);
-    launch_crit_adj(vv_off, vv, m->vorder, ooff, ostart, win, V, nvv, m->cadj, m->st,
-                    m->max_deg ? 1 : 0, s);
-    return TG_OK;
+    if (m->lg_off) cudaFreeAsync(m->lg_off, s);
+    if (m->lg_ent) cudaFreeAsync(m->lg_ent, s);
+    if (m->lg_adj) cudaFreeAsync(m->lg_adj, s);
+    m->lg_off = nullptr;
+    m->lg_ent = nullptr;
+    m->lg_adj = nullptr;
 }
+
+// entries of the link graph, at most: its rows are padded to multiples of eight
+int64_t link_entries(const tg_mesh *m, int64_t nvv) { return nvv + 7 * m->V; }
+
+LinkGraph link_graph(const tg_mesh *m, int64_t nvv)
+{
+    return {m->V, link_entries(m, nvv), m->lg_off, m->lg_ent, m->vorder, m->vpos, m->lg_adj, m->wide_deg};
+}
+
+// The link adjacency of critical points: VV renumbered into the star
+// processing order and its masks, kept on the mesh.  alloc makes every buffer,
+// the temporaries too, on the extraction's own stream (before a fork, so that
+// a side stream may use them); build launches.
+struct LinkBuild {
+    int32_t *len, *win;
+    tg_status alloc(tg_mesh *m, int64_t nvv, Temps &tmp, cudaStream_t s)
+    {
+        TRY(tmp.alloc(&len, m->V));
+        const int64_t n = link_entries(m, nvv);
+        TRY(tmp.alloc(&win, window_count(n, crit_window()) + 1));
+        int64_t *off;
+        int32_t *ent;
+        char *adj;
+        TRY(dalloc(&off, m->V + 1, s));
+        m->lg_off = off;
+        TRY(dalloc(&ent, n, s));
+        m->lg_ent = ent;
+        TRY(dalloc(&adj, n * (m->wide_deg ? 8 : 4), s));
+        m->lg_adj = adj;
+        return TG_OK;
+    }
+    void build(tg_mesh *m, const int64_t *vv_off, const int32_t *vv, int64_t nvv, cudaStream_t s)
+    {
+        const LinkGraph g = link_graph(m, nvv);
+        launch_vv_lengths_in_order(vv_off, m->vorder, m->V, len, s);
+        ScanJob job{len, m->lg_off, m->V, SCAN_COUNT_PAD8, nullptr};
+        scan_batch(&job, 1, m->scan, m->st, s);
+        launch_window_starts(m->lg_off, m->V, g.n_ent, crit_window(), win, s);
+        launch_rows_in_order(vv_off, vv, m->vorder, m->vpos, m->V, m->lg_off, m->lg_ent, s);
+        launch_crit_adj(g, win, m->st, m->max_deg ? 1 : 0, s);
+    }
+};
 
 tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
 {
@@ -568,6 +601,7 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         }
         if (m->st_host->flags) return check_flags(m);
         m->max_deg = m->st_host->max_deg > kMaxDeg ? m->st_host->max_deg : 0;
+        m->wide_deg = m->st_host->max_deg > kNarrowDeg;
         const int64_t nvv = m->sz_host[0];
         const int64_t E = m->sz_host[1], F = m->sz_host[2];
         const int64_t n_bnd = m->sz_host[3];  // boundary faces
@@ -638,10 +672,7 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         tmp.keep(vv);
         tmp.keep(vv_off);
         set_csr(m, TG_REL_VV, vv_off, vv, V, nvv);
-        if (m->cadj) {
-            cudaFreeAsync(m->cadj, s);
-            m->cadj = nullptr;
-        }
+        free_link_graph(m, s);
 
         // ET and EF rows, the per-cell TT rows, the per-face FE / FF rows and on
         // request the link adjacency of critical points, on a side stream
@@ -649,14 +680,15 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         const int64_t n_ee = sum_deg_sq - 2 * E;   // deg(a) + deg(b) - 2 per edge (a,b)
         if (ee_off) TRY(dalloc(&ee, n_ee, s));
         const bool prep_adj = (opts & TG_OPT_LINK_ADJACENCY) && (mask & TG_VV);
-        if (prep_adj) TRY(dalloc(&m->cadj, nvv, s));
+        LinkBuild lb;
+        if (prep_adj) TRY(lb.alloc(m, nvv, tmp, s));
         if (te || fe || tt || ff_off || ff || et || ef || prep_adj) {
             const cudaStream_t s2 = side.fork();
             ep.te = te; ep.et_off = et_off; ep.ef_off = ef_off; ep.et = et; ep.ef = ef; ep.tf = tf;
             if (te || et || ef) launch_edge_rows(ep, s2);
             if (tt || ff_off) launch_cell_tt(T, F, tf, ft, brank, tt_off, tt, ff_off, s2);
             if (fe || ff) launch_face_fill(ft, tf, te, brank, F, fe, ff_off, ff, s2);
-            if (prep_adj) TRY(build_link_adjacency(m, vv_off, vv, nvv, tmp, s2));
+            if (prep_adj) lb.build(m, vv_off, vv, nvv, s2);
         }
         if (ee_off) {
             launch_ee_fill(ev, E, vv_off, eid_sorted, ee_off, ee, s);
@@ -727,12 +759,14 @@ tg_status tg::critical_points_rows(tg_mesh *m, int64_t v0, int64_t nv, const voi
     m->last_stream = s;
     if (!m->rel[TG_REL_VV].ready) TRY(tg_extract(m, TG_VV, 0, s));
     const Rel &vv = m->rel[TG_REL_VV];
-    if (!m->cadj) {
-        TRY(dalloc(&m->cadj, vv.entries, s));
+    if (!m->lg_adj) {
         // VV rows longer than the adjacency masks take the heavy path of the
         // classification, so no status read-back here
+        free_link_graph(m, s);
         Temps adj_tmp(s);
-        TRY(build_link_adjacency(m, vv.off, vv.ent, vv.entries, adj_tmp, s));
+        LinkBuild lb;
+        TRY(lb.alloc(m, vv.entries, adj_tmp, s));
+        lb.build(m, vv.off, vv.ent, vv.entries, s);
     }
     Temps tmp(s);
     const size_t esz = field_type == TG_FIELD_F64 ? 8 : 4;
@@ -745,7 +779,9 @@ tg_status tg::critical_points_rows(tg_mesh *m, int64_t v0, int64_t nv, const voi
     }
     uint32_t *out = classes_out;
     if (!out_on_device) TRY(tmp.alloc(&out, 3 * nv));
-    launch_crit_classify(vv.off, vv.ent, m->cadj, f, field_type, v0, nv, out, s);
+    char *ordered = nullptr;
+    if (classify_orders_field(nv)) TRY(tmp.alloc(&ordered, m->V * (int64_t)esz));
+    launch_crit_classify(link_graph(m, vv.entries), f, field_type, ordered, v0, nv, out, s);
     if (m->max_deg) {
         // vertices of more than kMaxDeg neighbours: at most one per
         // kMaxDeg + 1 VV entries
@@ -805,7 +841,8 @@ tg_status tg_mesh_destroy(tg_mesh *m)
     if (m->heavy_off) cudaFreeAsync(m->heavy_off, s);
     if (m->seg_c) cudaFreeAsync(m->seg_c, s);
     if (m->seg_ef) cudaFreeAsync(m->seg_ef, s);
-    if (m->cadj) cudaFreeAsync(m->cadj, s);
+    if (m->vpos) cudaFreeAsync(m->vpos, s);
+    free_link_graph(m, s);
     if (m->st) cudaFreeAsync(m->st, s);
     if (m->scan.buf) {
         // after the last scan, whichever stream it ran on
@@ -853,7 +890,7 @@ static tg_status mesh_create_impl(const int32_t *tv, int64_t T, int64_t V, int o
     uint32_t *vflag;
     {
         Carve c;
-        const size_t o_d = c.add<int32_t>(V), o_f = c.add<uint32_t>(nwk), o_h = c.add<int32_t>(3);
+        const size_t o_d = c.add<int32_t>(V), o_f = c.add<uint32_t>(nwk), o_h = c.add<int32_t>(4);
         char *z;
         TRY(tmp.alloc(&z, (int64_t)c.bytes, true));
         deg_t = (int32_t *)(z + o_d);
@@ -881,7 +918,8 @@ static tg_status mesh_create_impl(const int32_t *tv, int64_t T, int64_t V, int o
     ScanJob jf{vflag, vrank, nwk, SCAN_POPC_RANK, nullptr};
     scan_batch(&jf, 1, m->scan, m->st, s);
     TRY(dalloc(&m->vorder, V, s));
-    launch_vorder_place(vt_off, V, vkey, vrank, nwk, heavy_cnt, m->vorder, s);
+    TRY(dalloc(&m->vpos, V, s));
+    launch_vorder_place(vt_off, V, vkey, vrank, nwk, heavy_cnt, m->vorder, m->vpos, s);
     CK(cudaGetLastError());
     set_csr(m, TG_REL_VT, vt_off, vt, V, 4 * T);
     // vertices with light stars, heavy ones, the heavy stars' entries and
@@ -1195,7 +1233,9 @@ int64_t tg_mesh_device_bytes(const tg_mesh *m)
         b += x.entries * 4;
         if (x.off) b += (x.rows + 1) * 8;
     }
-    if (m->cadj) b += m->rel[TG_REL_VV].entries * 8;
+    b += m->V * 8;
+    if (m->lg_adj)
+        b += link_entries(m, m->rel[TG_REL_VV].entries) * (m->wide_deg ? 12 : 8) + (m->V + 1) * 8;
     return b;
 }
 

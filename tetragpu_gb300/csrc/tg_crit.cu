@@ -10,78 +10,232 @@
 //     classes[3v+1] (:275-284) and the code to classes[3v+2]: (>=1, 0) -> 2,
 //     (0, >=1) -> 1, (1, 1) -> 3, anything else -> 4 (:303-330).
 //
-// Two kernels, so that a second field on the same mesh reuses the first:
-//   k_crit_adj       field-independent: for every VV entry (v, u), the bitmask
+// The graph both kernels work on is VV renumbered into the star processing
+// order (vertices by first cell): rows of neighbour positions, ascending, row
+// after row in that order.  Vertex ids need not carry locality; positions do,
+// so the neighbours' rows and field values a block gathers lie together.  (The
+// no-allocation entry point has no such order: there positions are ids.)
+//
+//   k_rows_in_order  VV -> the renumbered rows
+//   k_crit_adj       field-independent: for every entry (v, u), the bitmask
 //                    of v's neighbours adjacent to u.  Thread per edge (both
-//                    of its entries), v's row staged in shared memory.
+//                    of its entries), v's row in a shared-memory hash table.
 //   k_crit_classify  field-dependent: lower/upper split, then the components
 //                    of each kind counted by a bitmask search over the
 //                    adjacency masks of same-kind neighbours.
+// A second field on the same mesh reuses the first two.
+#include <climits>
+
 #include "tg_internal.h"
+#include "tg_rowsort.h"
 
 namespace tg {
 namespace {
 
-// Link adjacency: for every VV entry (v, u), bit j of the mask is set when
-// v's j-th neighbour is also a neighbour of u.  The common neighbours of v
-// and u give both entries (v, u) and (u, v), so one thread takes each edge
-// once, from its lower end v: it scans u's row from global memory, finds each
-// w in v's row (staged in shared memory) by binary search, and sets bit j in
-// (v, u)'s mask and bit i (w's place in u's row) in (u, v)'s, which sits at
-// v's place in u's row.  A block takes the vertices whose VV rows start in a
-// 256-entry window (win); the entries it owns (u > v) form a work list.
+__device__ __forceinline__ int pad8(int d) { return (d + 7) & ~7; }
+
+// eight entries from a 32-byte boundary in one load
+__device__ __forceinline__ void load8(const int *p, int (&x)[8])
+{
+    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]),
+                   "=r"(x[7])
+                 : "l"(p));
+}
+
+// ---------------------------------------------------------------------------
+// Rows into processing order, each padded with -1 to whole 32-byte sectors (so
+// that a thread loads eight entries at once): sixteen lanes copy a row, four rows' loads in flight; a thread sorts it (a
+// word between the rows in shared memory: 16-word rows would all begin in two
+// banks).
+constexpr int kOrderThreads = 128;
+constexpr int kOrderCap = 24 * kOrderThreads;
+constexpr int kOrderRows = 4;
+__global__ void __launch_bounds__(kOrderThreads, 9)
+k_rows_in_order(const int64_t *__restrict__ vv_off, const int *__restrict__ vv,
+                const int *__restrict__ order, const int *__restrict__ vpos, int64_t V,
+                const int64_t *__restrict__ off, int *__restrict__ ent)
+{
+    griddep_wait();
+    __shared__ int row[kOrderCap + kOrderThreads];
+    __shared__ long long s_src[kOrderThreads];
+    __shared__ int s_at[kOrderThreads], s_len[kOrderThreads];
+    const int64_t i0 = (int64_t)blockIdx.x * kOrderThreads;
+    const int64_t i1 = min(i0 + kOrderThreads, V);
+    const int64_t i = i0 + threadIdx.x;
+    const int64_t base = off[i0];
+    const int64_t n = off[i1] - base;
+    const int64_t b = off[min(i, i1)];
+    long long src = 0;
+    int d = 0;
+    if (i < V) {
+        const int v = __ldg(order + i);
+        src = __ldg(vv_off + v);
+        d = (int)(__ldg(vv_off + v + 1) - src);
+    }
+    if (n > kOrderCap) {   // block-uniform: in place
+        for (int k = 0; k < d; k++) ent[b + k] = __ldg(vpos + __ldg(vv + src + k));
+        for (int k = d; k < pad8(d); k++) ent[b + k] = -1;
+        sort_rows_warp(ent + b, d);
+        return;
+    }
+    s_src[threadIdx.x] = src;
+    s_at[threadIdx.x] = (int)(b - base);
+    s_len[threadIdx.x] = d;
+    __syncthreads();
+    constexpr int kStep = kOrderThreads / 16;
+    const int lane = threadIdx.x & 15;
+    for (int r = threadIdx.x >> 4; r < kOrderThreads; r += kStep * kOrderRows) {
+        int u[kOrderRows];
+#pragma unroll
+        for (int t = 0; t < kOrderRows; t++) {
+            const int q = r + kStep * t;
+            u[t] = lane < s_len[q] ? __ldg(vv + s_src[q] + lane) : -1;
+        }
+#pragma unroll
+        for (int t = 0; t < kOrderRows; t++)
+            if (u[t] >= 0) u[t] = __ldg(vpos + u[t]);
+#pragma unroll
+        for (int t = 0; t < kOrderRows; t++) {
+            const int q = r + kStep * t, at = s_at[q] + q, len = s_len[q], full = pad8(len);
+            if (lane < full) row[at + lane] = u[t];
+            for (int k = lane + 16; k < full; k += 16)
+                row[at + k] = k < len ? __ldg(vpos + __ldg(vv + s_src[q] + k)) : -1;
+        }
+    }
+    __syncthreads();
+    sort_rows_warp(row + (int)(b - base) + threadIdx.x, d);
+    __syncthreads();
+    for (int q = threadIdx.x >> 4; q < kOrderThreads; q += kStep) {
+        const int at = s_at[q], full = pad8(s_len[q]);
+        for (int k = lane; k < full; k += 16) ent[base + at + k] = row[at + q + k];
+    }
+}
+
+// row lengths of VV in that order
+__global__ void __launch_bounds__(256)
+k_vv_lengths_in_order(const int64_t *__restrict__ vv_off, const int *__restrict__ order, int64_t V,
+                      int *__restrict__ len)
+{
+    griddep_wait();
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= V) return;
+    const int v = order[i];
+    len[i] = (int)(vv_off[v + 1] - vv_off[v]);
+}
+
+// ---------------------------------------------------------------------------
+// Link adjacency: for every entry (v, u), bit j of the mask is set when v's
+// j-th neighbour is also a neighbour of u.  The common neighbours of v and u
+// give both entries (v, u) and (u, v), so one thread takes each edge once, from
+// its lower end v: it scans u's row from global memory, looks each w up in v's
+// row, and sets bit j in (v, u)'s mask and bit i (w's place in u's row) in
+// (u, v)'s, which sits at v's place in u's row.  A block takes the vertices
+// whose rows start in a 256-entry window (win); the entries it owns (u > v)
+// form a work list.
+//
+// The look-up is what the pass consists of (14 entries an edge), so a row gets
+// a hash table in shared memory: 2^k buckets of two words (64 buckets for 14
+// neighbours).  x = w * multiplier (odd) is a bijection of 32-bit words: its
+// top k bits are the bucket, and a neighbour's word holds the other bits above
+// its place in the row (k bits; a free word all ones, a place that no
+// neighbour has), so one 8-byte load and one compare decide.  The row's first
+// neighbour that finds its bucket full (one row of 12 has one) is kept apart,
+// where every look-up compares with it; a row with a second one is hashed
+// again with the next multiplier, and one that no multiplier was found for
+// keeps its sorted entries padded with INT_MAX for a binary search.  Bound by
+// the shared-memory pipe (86%) and issue (64%).  A binary search over VV in id
+// order (four dependent loads and 35 instructions an entry, neighbours' rows
+// scattered: 5.2 requests to L2 an edge against 2): 709 -> 488 us at 128^3,
+// 127 -> 88 us on the 64^3 coned mesh, the renumbering included 890 -> 780 us.
 constexpr int kAdjCap = kAdjWin + kMaxDeg;
 constexpr int kAdjThreads = TG_ADJ_THREADS;
+constexpr int kAdjWords = 8;       // table words per entry
+constexpr int kHashTries = 8;
 
-// u's row (urow, un entries; read four at a time from 16-byte boundaries
-// when the array is aligned: i from i0 = -(ub mod 4), one load instruction
-// per four entries; else one entry at a time) against v's row (row, d
-// entries, shared memory, padded with INT_MAX to top = the power of two at or
-// above d): each w found at position lo of v's row sets bit lo of bits_v and
-// bit i of bits_u; pv = v's place in u's row.  The search takes the steps
-// top / 2, .. 1 (those above top / 2 skipped by a per-thread predicate, so
-// the lanes of a warp stay together) and needs no bound: every probe lies in
-// the padded row.
-template <typename M, int TOP>
-__device__ __forceinline__ void adj_scan(const int *row, int d, int top,
-                                         const int *__restrict__ urow, int i0, int un, int lim,
-                                         bool vec, int v, M &bits_v, M &bits_u, int &pv)
+// buckets of a row of d entries, log2: two words each in the row's share
+__device__ __forceinline__ int hash_bits(int d) { return min(30 - __clz(kAdjWords * d), 8); }
+
+__device__ __forceinline__ unsigned multiplier(unsigned i)   // some odd word per i
 {
-    // the next four entries are loaded while the current four are searched
-    auto load4 = [&](int j) -> int4 {
-        if (vec && j + 4 <= lim) return __ldg(reinterpret_cast<const int4 *>(urow + j));
-        int4 x;
-        x.x = j < lim && j < un ? __ldg(urow + j) : 0;
-        x.y = j + 1 < lim && j + 1 < un ? __ldg(urow + j + 1) : 0;
-        x.z = j + 2 < lim && j + 2 < un ? __ldg(urow + j + 2) : 0;
-        x.w = j + 3 < lim && j + 3 < un ? __ldg(urow + j + 3) : 0;
-        return x;
-    };
-    int4 nxt = i0 < un ? load4(i0) : make_int4(0, 0, 0, 0);
-    for (; i0 < un; i0 += 4) {
-        const int4 cur = nxt;
-        if (i0 + 4 < un) nxt = load4(i0 + 4);
-        const int q[4] = {cur.x, cur.y, cur.z, cur.w};
-        // four searches in lock step (independent shared-memory loads in
-        // flight together); entries outside [0, un) search harmlessly and
-        // set nothing
-        int lo[4] = {0, 0, 0, 0};
+    unsigned x = (i + 1u) * 0x9E3779B1u;
+    x ^= x >> 15;
+    x *= 0x85EBCA77u;
+    x ^= x >> 13;
+    return x | 1u;
+}
+
+// v's row as u's row is matched against it: a hash table (mul not 0) or the
+// padded row
+struct AdjRow {
+    const unsigned *tab;
+    unsigned mul;
+    int apart, apart_at;   // the neighbour kept apart (-2: none) and its place
+    int k, d, top;         // top: the power of two at or above d
+};
+
+// u's row (urow, un entries) against v's: each w found at place j of v's row
+// sets bit j of bits_v and bit i of bits_u; pv = v's place in u's row.  PAD:
+// rows are padded with -1 (which no row holds) to whole sectors.  HASH: v's
+// row has a table; else a binary search of the steps top / 2, .. 1 (those
+// above top / 2 skipped by a per-thread predicate, so the lanes of a warp stay
+// together; every probe lies in the padded row).
+template <typename M, bool PAD, bool HASH>
+__device__ __forceinline__ void adj_scan(const AdjRow &R, const int *__restrict__ urow, int un, int v,
+                                         M &bits_v, M &bits_u, int &pv)
+{
+    const int *row = reinterpret_cast<const int *>(R.tab);
+    const int up = 32 - R.k;
+    for (int i0 = 0; i0 < un; i0 += 8) {
+        int q[8];
+        if constexpr (PAD) {
+            load8(urow + i0, q);
+        } else {
 #pragma unroll
-        for (int step = TOP / 2; step > 0; step >>= 1) {
-            if (2 * step > top) continue;
-#pragma unroll
-            for (int t = 0; t < 4; t++)
-                lo[t] += row[lo[t] + step - 1] < q[t] ? step : 0;
+            for (int t = 0; t < 8; t++) q[t] = i0 + t < un ? __ldg(urow + i0 + t) : -1;
         }
+        // look-ups in lock step (independent shared-memory loads in flight
+        // together)
+        unsigned hits = 0u;
 #pragma unroll
-        for (int t = 0; t < 4; t++) {
-            const int i = i0 + t;
-            const bool valid = i >= 0 && i < un;
-            if (valid && q[t] == v) pv = i;
-            const bool hit = valid && q[t] != v && row[lo[t]] == q[t];
-            bits_v |= (M)hit << lo[t];
-            bits_u |= (M)hit << (i & (8 * (int)sizeof(M) - 1));
+        for (int t0 = 0; t0 < 8; t0 += 4) {
+            unsigned at[4];
+            if constexpr (HASH) {
+                uint2 w[4];
+                unsigned x[4];
+#pragma unroll
+                for (int t = 0; t < 4; t++) {
+                    x[t] = (unsigned)q[t0 + t] * R.mul;
+                    w[t] = reinterpret_cast<const uint2 *>(R.tab)[x[t] >> up];
+                }
+                // the place, if below d (at most one of the two words is w's)
+#pragma unroll
+                for (int t = 0; t < 4; t++) {
+                    at[t] = min(w[t].x ^ (x[t] << R.k), w[t].y ^ (x[t] << R.k));
+                    at[t] = q[t0 + t] == R.apart ? (unsigned)R.apart_at : at[t];
+                }
+            } else {
+                int lo[4] = {0, 0, 0, 0};
+#pragma unroll
+                for (int step = kMaxDeg / 2; step > 0; step >>= 1) {
+                    if (2 * step > R.top) continue;
+#pragma unroll
+                    for (int t = 0; t < 4; t++)
+                        lo[t] += row[lo[t] + step - 1] < q[t0 + t] ? step : 0;
+                }
+#pragma unroll
+                for (int t = 0; t < 4; t++)
+                    at[t] = row[lo[t]] == q[t0 + t] ? (unsigned)lo[t] : ~0u;
+            }
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                pv = q[t0 + t] == v ? i0 + t0 + t : pv;
+                const bool hit = at[t] < (unsigned)R.d;
+                bits_v |= hit ? (M)1 << (at[t] & (8 * sizeof(M) - 1)) : (M)0;
+                hits |= hit ? 1u << (t0 + t) : 0u;
+            }
         }
+        bits_u |= (M)hits << (i0 & (8 * (int)sizeof(M) - 1));
     }
 }
 
@@ -91,162 +245,257 @@ __device__ __forceinline__ void adj_scan(const int *row, int d, int top,
 // is lower (u computes nothing); heavy = 2 reports them instead
 // (ST_HEAVY_DEG) for callers without the heavy path.  Light rows start
 // below kAdjWin in their window and end below kAdjCap, so they always fit.
-//
-// Windows run over the rows in `order` (the star processing order: vertices
-// by first cell, so consecutive windows share neighbours and the neighbours'
-// rows stay in L2; ooff = the row lengths' prefix in that order, ostart =
-// each row's start in VV, read beside ooff instead of after the vertex), or
-// in id order when order is null (ooff = vv_off).  A staged row keeps its
-// global start in gst[row start].
+// M: the masks (32-bit when no row holds more than 32 entries).  PAD: as in
+// adj_scan (row lengths include the padding).
+template <typename M, bool PAD>
 __global__ void __launch_bounds__(kAdjThreads)
-k_crit_adj(const int64_t *__restrict__ vv_off, const int *__restrict__ vv, int64_t n_vv,
-           const int *__restrict__ order, const int64_t *__restrict__ ooff,
-           const int64_t *__restrict__ ostart, const int *__restrict__ win,
-           unsigned long long *__restrict__ adj, DevStatus *st, int heavy)
+k_crit_adj(const int64_t *__restrict__ off, const int *__restrict__ ent, const int *__restrict__ win,
+           M *__restrict__ adj, DevStatus *st, int heavy)
 {
     griddep_wait();
-    __shared__ int nb[kAdjCap];
-    __shared__ int prow[2 * kAdjCap];   // the row starting at rs at 2 rs, INT_MAX to 2 rs + 2 d
-    __shared__ int meta[kAdjCap];   // row start | row length << 16; -1: no light row there
-    __shared__ int vid[kAdjCap];
-    __shared__ int own[kAdjCap];
-    __shared__ long long gst[kAdjCap];   // at a row start: the row's first entry in VV
+    __shared__ __align__(16) int nb[kAdjCap];
+    __shared__ __align__(16) unsigned tab[kAdjWords * kAdjCap];   // tables (or padded rows)
+    // an entry's row by its first entry here; kNoRow: no light row there
+    __shared__ __align__(16) unsigned short meta[kAdjCap];
+    __shared__ unsigned short own[kAdjCap];
+    // at a row's first entry: its vertex, its length, its multiplier (0 without
+    // a table), the neighbour kept apart and its place
+    __shared__ int vid[kAdjCap], apart[kAdjCap];
+    __shared__ unsigned mul[kAdjCap];
+    __shared__ unsigned char len[kAdjCap], apart_at[kAdjCap];
     __shared__ int n_own;
+    constexpr unsigned kNoRow = 0xffffu;
+    const int lane = threadIdx.x & 31;
     // every thread reads the window's bounds itself (the same words: one
     // transaction each), so the block needs no barrier before the rows
-    // unless the heavy modes mark the slots of rows they leave out
+    // unless the heavy modes leave rows out
     const int s_vlo = win[blockIdx.x], s_vhi = win[blockIdx.x + 1];
-    const long long s_base = ooff[s_vlo];
-    const int s_n = (int)(ooff[s_vhi] - s_base);
+    const long long base = off[s_vlo];
+    const int s_n = (int)(off[s_vhi] - base);
+    if (s_n == 0) return;
+    const int n = min(s_n, kAdjCap);
     if (threadIdx.x == 0) n_own = 0;
     if (heavy) {
-        for (int e = threadIdx.x; e < kAdjCap; e += blockDim.x) meta[e] = -1;
+        for (int e = threadIdx.x; e < kAdjCap; e += kAdjThreads) meta[e] = kNoRow;
         __syncthreads();
     }
-    const int n = min(s_n, kAdjCap);
-    const long long base = s_base;
     if (heavy == 2 && s_n > kAdjCap) {  // a row longer than kMaxDeg lies in this window
         if (threadIdx.x == 0) {
             atomicOr(&st->flags, ST_HEAVY_DEG);
-            atomicMin(&st->bad_vertex, order ? order[s_vlo] : s_vlo);
+            atomicMin(&st->bad_vertex, s_vlo);
         }
         return;
     }
-    for (int i = s_vlo + threadIdx.x; i < s_vhi; i += blockDim.x) {
-        const int rs = (int)(ooff[i] - base);
-        const int d = (int)(ooff[i + 1] - ooff[i]);
+    if constexpr (PAD) {
+        for (int e = 4 * threadIdx.x; e < n; e += 4 * kAdjThreads) cp_async<16>(&nb[e], ent + base + e);
+    } else {
+        for (int e = threadIdx.x; e < n; e += kAdjThreads) cp_async<4>(&nb[e], ent + base + e);
+    }
+    cp_async_commit();
+    for (int j = threadIdx.x; j < kAdjWords * kAdjCap / 4; j += kAdjThreads)   // free words
+        if (4 * j < kAdjWords * n)
+            reinterpret_cast<uint4 *>(tab)[j] = make_uint4(~0u, ~0u, ~0u, ~0u);
+    for (int i = s_vlo + threadIdx.x; i < s_vhi; i += kAdjThreads) {
+        const int rs = (int)(off[i] - base);
+        const int d = (int)(off[i + 1] - off[i]);
         if (d == 0) continue;
-        const int v = order ? order[i] : i;
         if (d > kMaxDeg) {
             if (heavy == 2) {
                 atomicOr(&st->flags, ST_HEAVY_DEG);
-                atomicMin(&st->bad_vertex, v);
+                atomicMin(&st->bad_vertex, i);
             }
             continue;
         }
-        const long long g0 = order ? ostart[i] : base + rs;
-        gst[rs] = g0;
-        // the row's entries are copied asynchronously as soon as its start
-        // is known
-        for (int k = 0; k < d; k++) {
-            meta[rs + k] = rs | (d << 16);
-            vid[rs + k] = v;
-            cp_async<4>(&nb[rs + k], vv + g0 + k);
+        vid[rs] = i;
+        len[rs] = (unsigned char)d;
+        mul[rs] = multiplier(0u);
+        apart[rs] = -2;
+        if constexpr (PAD) {
+            const unsigned two = (unsigned)rs * 0x10001u;
+            for (int k = 0; k < d; k += 8)
+                *reinterpret_cast<uint4 *>(meta + rs + k) = make_uint4(two, two, two, two);
+        } else {
+            for (int k = 0; k < d; k++) meta[rs + k] = (unsigned short)rs;
         }
     }
-    cp_async_commit();
     cp_async_wait();
     __syncthreads();
-    for (int e = threadIdx.x; e < n; e += blockDim.x) {
-        const int m = meta[e];
-        if (m < 0) continue;
-        const int rs = m & 0xffff, d = m >> 16;
-        prow[rs + e] = nb[e];            // 2 rs + (e - rs)
-        prow[rs + e + d] = INT_MAX;
-        bool mine = nb[e] > vid[e];
-        if (!mine && heavy == 1) {       // a heavy lower end computes nothing
-            const int u = nb[e];
-            mine = __ldg(vv_off + u + 1) - __ldg(vv_off + u) > kMaxDeg;
+    // the entries into their rows' tables; those of a row that did not fit
+    // again under the next multiplier.  The owned entries on the first way.
+    for (int trial = 0; trial < kHashTries; trial++) {
+        const unsigned c = multiplier((unsigned)trial);
+        bool failed = false;
+        for (int e0 = threadIdx.x - lane; e0 < n; e0 += kAdjThreads) {
+            const int e = e0 + lane;
+            const unsigned rs = e < n ? meta[e] : kNoRow;
+            const int u = rs != kNoRow ? nb[e] : -1;
+            if (u >= 0 && mul[rs] == c) {
+                const int k = hash_bits(len[rs]);
+                const unsigned x = (unsigned)u * c;
+                const unsigned word = x << k | (unsigned)(e - rs);
+                unsigned *bucket = tab + kAdjWords * rs + 2 * (x >> (32 - k));
+                if (atomicCAS(bucket, ~0u, word) != ~0u && atomicCAS(bucket + 1, ~0u, word) != ~0u) {
+                    if (atomicCAS(&apart[rs], -2, u) == -2) {
+                        apart_at[rs] = (unsigned char)(e - rs);
+                    } else {
+                        failed = true;
+                        mul[rs] = 0u;   // this row again
+                    }
+                }
+            }
+            if (trial == 0) {
+                bool mine = u >= 0 && u > vid[rs];
+                if (heavy == 1 && u >= 0 && !mine)   // a heavy lower end computes nothing
+                    mine = __ldg(off + u + 1) - __ldg(off + u) > kMaxDeg;
+                const unsigned b = __ballot_sync(0xffffffffu, mine);
+                int o = 0;
+                if (lane == 0 && b) o = atomicAdd(&n_own, __popc(b));
+                o = __shfl_sync(0xffffffffu, o, 0) + __popc(b & ((1u << lane) - 1u));
+                if (mine) own[o] = (unsigned short)e;
+            }
         }
-        if (mine) own[atomicAdd(&n_own, 1)] = e;
+        if (!__syncthreads_or(failed)) break;
+        for (int e = threadIdx.x; e < n; e += kAdjThreads) {
+            const unsigned rs = meta[e];
+            if (rs == kNoRow || mul[rs]) continue;
+            // this entry's part of the row's share of the tables: free words,
+            // or out of multipliers the row itself
+            unsigned *t = tab + kAdjWords * rs;
+            if (trial + 1 < kHashTries) {
+                for (int j = 0; j < kAdjWords; j++) t[kAdjWords * (e - rs) + j] = ~0u;
+                if (e == rs) apart[rs] = -2;
+            } else {
+                t[e - rs] = nb[e] >= 0 ? (unsigned)nb[e] : (unsigned)INT_MAX;
+                t[e - rs + len[rs]] = (unsigned)INT_MAX;
+            }
+        }
+        __syncthreads();
+        if (trial + 1 < kHashTries) {
+            for (int e = threadIdx.x; e < n; e += kAdjThreads)
+                if (meta[e] == e && !mul[e]) mul[e] = multiplier((unsigned)trial + 1u);
+            __syncthreads();
+        }
     }
-    __syncthreads();
     const int no = n_own;
-    const bool vec = (reinterpret_cast<uintptr_t>(vv) & 15) == 0;
-    for (int k = threadIdx.x; k < no; k += blockDim.x) {
-        const int e = own[k];
-        const int m = meta[e], rs = m & 0xffff, d = m >> 16;
-        const int v = vid[e], u = nb[e];
-        const int64_t ub = vv_off[u];
-        const int un = (int)(vv_off[u + 1] - ub);
+    for (int k = threadIdx.x; k < no; k += kAdjThreads) {
+        const int e = own[k], rs = meta[e], d = len[rs];
+        const int v = vid[rs], u = nb[e];
+        const int64_t ub = off[u];
+        const int un = (int)(off[u + 1] - ub);
         if (un > kMaxDeg && heavy != 1) continue;  // reported by u's own block
-        // entries of u's row at or past the array's end are not loaded
-        const int lim = (int)min(n_vv - ub, (int64_t)INT_MAX);
         int pv = -1;
-        unsigned long long bv, bu;
-        const int top = d <= 1 ? 1 : 1 << (32 - __clz(d - 1));
-        if (d <= 32 && un <= 32) {   // both masks fit 32 bits (the common case)
+        M bv, bu;
+        AdjRow R;
+        R.tab = tab + kAdjWords * rs;
+        R.mul = mul[rs];
+        R.apart = apart[rs];
+        R.apart_at = apart_at[rs];
+        R.k = hash_bits(d);
+        R.d = d;
+        R.top = d <= 1 ? 1 : 1 << (32 - __clz(d - 1));
+        if (sizeof(M) == 4 || (d <= 32 && un <= 32)) {   // both masks fit 32 bits
             unsigned bv32 = 0u, bu32 = 0u;
-            adj_scan<unsigned, 32>(prow + 2 * rs, d, top, vv + ub, vec ? -(int)(ub & 3) : 0, un,
-                                   lim, vec, v, bv32, bu32, pv);
+            if (R.mul) adj_scan<unsigned, PAD, true>(R, ent + ub, un, v, bv32, bu32, pv);
+            else adj_scan<unsigned, PAD, false>(R, ent + ub, un, v, bv32, bu32, pv);
             bv = bv32;
             bu = bu32;
         } else {
-            bv = bu = 0ull;
-            adj_scan<unsigned long long, 64>(prow + 2 * rs, d, top, vv + ub,
-                                             vec ? -(int)(ub & 3) : 0, un, lim, vec, v, bv, bu,
-                                             pv);
+            bv = bu = 0;
+            if (R.mul) adj_scan<M, PAD, true>(R, ent + ub, un, v, bv, bu, pv);
+            else adj_scan<M, PAD, false>(R, ent + ub, un, v, bv, bu, pv);
         }
-        adj[gst[rs] + (e - rs)] = bv;
+        adj[base + e] = bv;
         // u's mask is u's to keep only when u's row is light (else it has none)
         if (pv >= 0 && un <= kMaxDeg) adj[ub + pv] = bu;
     }
 }
 
+// ---------------------------------------------------------------------------
 constexpr int kClassifyThreads = 128;
+// From this many vertices on the field is put in processing order first (a
+// launch and a buffer: 3 us), so that a block's field gathers lie together;
+// below, they hit L1 and L2 anyway.  A call by id and in order: 9.3 and 11.4 us
+// at 4,913 vertices, 11.2 and 11.4 us at 118k, 15.0 and 13.0 us at 185k, 180
+// and 105 us at 2.1M.
+constexpr int64_t kOrderField = 1 << 17;
+
+// a field's values by position: of every vertex (vpos null: a thread per
+// position), or of the vertices from v0 on (a thread per vertex)
+template <typename F>
+__global__ void __launch_bounds__(256)
+k_field_in_order(const F *__restrict__ field_v0, const int *__restrict__ order,
+                 const int *__restrict__ vpos, int64_t v0, int64_t nv, F *__restrict__ out)
+{
+    griddep_wait();
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nv) return;
+    if (vpos) out[vpos[v0 + i]] = field_v0[i];
+    else out[i] = __ldg(field_v0 + order[i]);
+}
 
 // Components of the lower and upper link subgraphs by bitmask search: a
 // component grows from its lowest unvisited member, each member reached
 // once adding its same-kind neighbours (its adjacency mask) to the frontier.
 // Every neighbour is visited exactly once, so a vertex costs deg iterations
 // whatever the link's shape (no data-dependent find loops).
-template <typename F>
+//
+// A thread per vertex: positions 0 .. nv - 1 (vpos null), or the positions of
+// the vertices v0 .. v0 + nv - 1 (a vertex range that holds every neighbour of
+// its vertices: a whole mesh of a batch).  order: the vertex at each position
+// (null: positions are ids), for ties and output.  field: values by position,
+// or (BY_ID) by vertex from v0.
+template <typename F, typename M, bool PAD, bool BY_ID>
 __global__ void __launch_bounds__(kClassifyThreads)
-k_crit_classify(const int64_t *__restrict__ vv_off, const int *__restrict__ vv,
-                const unsigned long long *__restrict__ adj, const F *__restrict__ field_v0,
-                int64_t v0, int64_t nv, unsigned *__restrict__ classes3_v0)
+k_crit_classify(const int64_t *__restrict__ off, const int *__restrict__ ent,
+                const M *__restrict__ adj, const F *__restrict__ field,
+                const int *__restrict__ order, const int *__restrict__ vpos, int64_t v0, int64_t nv,
+                unsigned *__restrict__ classes3_v0)
 {
     griddep_wait();
-    // rows [v0, v0 + nv); field and classes indexed from v0 (a vertex range
-    // holds every neighbour of its vertices when it is a whole mesh of a batch)
-    const int64_t v = v0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= v0 + nv) return;
-    const F *field = field_v0 - v0;
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nv) return;
+    const int64_t i = vpos ? vpos[v0 + t] : t;
+    const int64_t v = vpos ? v0 + t : (order ? order[t] : t);
     unsigned *classes3 = classes3_v0 - 3 * v0;
-    const int64_t b = vv_off[v];
-    const int n = (int)(vv_off[v + 1] - b);
+    const int64_t b = off[i];
+    const int n = (int)(off[i + 1] - b);
     if (n > kMaxDeg) return;   // tg_heavy.cu classifies it
+    auto first = [](M m) {
+        return sizeof(M) == 8 ? __ffsll((long long)m) - 1 : __ffs((int)(unsigned)m) - 1;
+    };
     unsigned lo = 0, up = 0;
     {
-        const F fv = field[v];
-        unsigned long long lower = 0ull;
-        for (int k = 0; k < n; k++) {
-            const int u = __ldg(vv + b + k);
-            const F fu = __ldg(field + u);
-            const bool is_lower = (fu == fv) ? (u < (int)v) : (fu < fv);
-            lower |= (unsigned long long)is_lower << k;
+        if constexpr (BY_ID) field -= v0;
+        const F fv = field[BY_ID ? v : i];
+        M lower = 0, all = 0;
+        auto look = [&](int k, int u) {
+            if (u < 0) return;   // padding
+            all |= (M)1 << k;
+            const F fu = __ldg(field + (BY_ID && order ? __ldg(order + u) : u));
+            bool is_lower = fu < fv;
+            if (fu == fv) is_lower = (order ? __ldg(order + u) : u) < (int)v;
+            lower |= (M)is_lower << k;
+        };
+        if constexpr (PAD) {
+            for (int k = 0; k < n; k += 8) {
+                int u[8];
+                load8(ent + b + k, u);
+#pragma unroll
+                for (int t = 0; t < 8; t++) look(k + t, u[t]);
+            }
+        } else {
+            for (int k = 0; k < n; k++) look(k, __ldg(ent + b + k));
         }
-        const unsigned long long all = n == 64 ? ~0ull : (1ull << n) - 1ull;
-        unsigned long long rem = all;
+        M rem = all;
         while (rem) {
-            const int s = __ffsll((long long)rem) - 1;
-            const bool is_lo = (lower >> s) & 1ull;
-            const unsigned long long kind = is_lo ? lower : (all & ~lower);
-            unsigned long long comp = 1ull << s, frontier = comp;
+            const int s = first(rem);
+            const bool is_lo = (lower >> s) & 1;
+            const M kind = is_lo ? lower : (all & ~lower);
+            M comp = (M)1 << s, frontier = comp;
             while (frontier) {
-                const int j = __ffsll((long long)frontier) - 1;
+                const int j = first(frontier);
                 frontier &= frontier - 1;
-                const unsigned long long nb = __ldg(adj + b + j) & kind & ~comp;
+                const M nb = __ldg(adj + b + j) & kind & ~comp;
                 comp |= nb;
                 frontier |= nb;
             }
@@ -268,64 +517,88 @@ k_crit_classify(const int64_t *__restrict__ vv_off, const int *__restrict__ vv,
 
 int crit_window() { return kAdjWin; }
 
-void launch_crit_adj(const int64_t *vv_off, const int32_t *vv, const int32_t *order,
-                     const int64_t *ooff, const int64_t *ostart, const int32_t *vv_win,
-                     int64_t V, int64_t n_vv, uint64_t *adj, DevStatus *st, int heavy,
-                     cudaStream_t s)
+void launch_rows_in_order(const int64_t *vv_off, const int32_t *vv, const int32_t *order,
+                          const int32_t *vpos, int64_t V, const int64_t *off, int32_t *ent,
+                          cudaStream_t s)
 {
     if (V == 0) return;
-    Launch L("k_crit_adj", s);
-    launch_pdl(k_crit_adj, (unsigned)window_count(n_vv, kAdjWin), kAdjThreads, 0, s,
-        vv_off, vv, n_vv, order, order ? ooff : vv_off, ostart, vv_win,
-        reinterpret_cast<unsigned long long *>(adj), st, heavy);
+    Launch L("k_rows_in_order", s);
+    launch_pdl(k_rows_in_order, (unsigned)((V + kOrderThreads - 1) / kOrderThreads), kOrderThreads, 0, s,
+               vv_off, vv, order, vpos, V, off, ent);
 }
 
-namespace {
-// row lengths and row starts of VV in the star processing order (positions
-// past the vertices with cells hold placeholders: length 0)
-__global__ void __launch_bounds__(256)
-k_vv_lengths_in_order(const int64_t *__restrict__ vv_off, const int *__restrict__ order,
-                      int64_t V, int64_t n_with_cells, int *__restrict__ len,
-                      int64_t *__restrict__ start)
-{
-    griddep_wait();
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= V) return;
-    int d = 0;
-    int64_t b = 0;
-    if (i < n_with_cells) {
-        const int v = order[i];
-        b = vv_off[v];
-        d = (int)(vv_off[v + 1] - b);
-    }
-    len[i] = d;
-    start[i] = b;
-}
-}  // namespace
-
-void launch_vv_lengths_in_order(const int64_t *vv_off, const int32_t *order, int64_t V,
-                                int64_t n_with_cells, int32_t *len, int64_t *start, cudaStream_t s)
+void launch_vv_lengths_in_order(const int64_t *vv_off, const int32_t *order, int64_t V, int32_t *len,
+                                cudaStream_t s)
 {
     if (V == 0) return;
     Launch L("k_vv_lengths_in_order", s);
-    launch_pdl(k_vv_lengths_in_order, (unsigned)((V + 255) / 256), 256, 0, s, vv_off, order, V,
-               n_with_cells, len, start);
+    launch_pdl(k_vv_lengths_in_order, (unsigned)((V + 255) / 256), 256, 0, s, vv_off, order, V, len);
 }
 
-void launch_crit_classify(const int64_t *vv_off, const int32_t *vv, const uint64_t *adj,
-                          const void *field, int field_type, int64_t v0, int64_t nv,
-                          uint32_t *classes3, cudaStream_t s)
+void launch_crit_adj(const LinkGraph &g, const int32_t *win, DevStatus *st, int heavy, cudaStream_t s)
+{
+    if (g.V == 0) return;
+    Launch L("k_crit_adj", s);
+    const unsigned grid = (unsigned)window_count(g.n_ent, kAdjWin);
+    if (!g.order)   // plain VV: 64-bit masks
+        launch_pdl(k_crit_adj<unsigned long long, false>, grid, kAdjThreads, 0, s, g.off, g.ent, win,
+                   (unsigned long long *)g.adj, st, heavy);
+    else if (g.wide)
+        launch_pdl(k_crit_adj<unsigned long long, true>, grid, kAdjThreads, 0, s, g.off, g.ent, win,
+                   (unsigned long long *)g.adj, st, heavy);
+    else
+        launch_pdl(k_crit_adj<unsigned, true>, grid, kAdjThreads, 0, s, g.off, g.ent, win,
+                   (unsigned *)g.adj, st, heavy);
+}
+
+namespace {
+template <typename F, bool BY_ID>
+void classify(const LinkGraph &g, const F *field, const int32_t *vpos, int64_t v0, int64_t nv,
+              uint32_t *classes3, cudaStream_t s)
+{
+    const unsigned grid = (unsigned)((nv + kClassifyThreads - 1) / kClassifyThreads);
+    Launch L("k_crit_classify", s);
+    if (!g.order)
+        launch_pdl(k_crit_classify<F, unsigned long long, false, BY_ID>, grid, kClassifyThreads, 0, s,
+                   g.off, g.ent, (const unsigned long long *)g.adj, field, g.order, vpos, v0, nv,
+                   classes3);
+    else if (g.wide)
+        launch_pdl(k_crit_classify<F, unsigned long long, true, BY_ID>, grid, kClassifyThreads, 0, s,
+                   g.off, g.ent, (const unsigned long long *)g.adj, field, g.order, vpos, v0, nv,
+                   classes3);
+    else
+        launch_pdl(k_crit_classify<F, unsigned, true, BY_ID>, grid, kClassifyThreads, 0, s, g.off, g.ent,
+                   (const unsigned *)g.adj, field, g.order, vpos, v0, nv, classes3);
+}
+
+template <typename F>
+void classify(const LinkGraph &g, const F *field, F *ordered, int64_t v0, int64_t nv,
+              uint32_t *classes3, cudaStream_t s)
+{
+    const int32_t *vpos = nv < g.V ? g.vpos : nullptr;
+    if (!ordered) {
+        classify<F, true>(g, field, vpos, v0, nv, classes3, s);
+        return;
+    }
+    {
+        Launch L("k_field_in_order", s);
+        launch_pdl(k_field_in_order<F>, (unsigned)((nv + 255) / 256), 256, 0, s, field, g.order, vpos, v0,
+                   nv, ordered);
+    }
+    classify<F, false>(g, ordered, vpos, v0, nv, classes3, s);
+}
+}  // namespace
+
+bool classify_orders_field(int64_t nv) { return nv >= kOrderField; }
+
+void launch_crit_classify(const LinkGraph &g, const void *field, int field_type, void *ordered,
+                          int64_t v0, int64_t nv, uint32_t *classes3, cudaStream_t s)
 {
     if (nv == 0) return;
-    const unsigned grid = (unsigned)((nv + kClassifyThreads - 1) / kClassifyThreads);
-    const auto *a = reinterpret_cast<const unsigned long long *>(adj);
-    Launch L("k_crit_classify", s);
     if (field_type == 1)
-        launch_pdl(k_crit_classify<double>, grid, kClassifyThreads, 0, s,
-            vv_off, vv, a, (const double *)field, v0, nv, classes3);
+        classify(g, (const double *)field, (double *)ordered, v0, nv, classes3, s);
     else
-        launch_pdl(k_crit_classify<float>, grid, kClassifyThreads, 0, s,
-            vv_off, vv, a, (const float *)field, v0, nv, classes3);
+        classify(g, (const float *)field, (float *)ordered, v0, nv, classes3, s);
 }
 
 }  // namespace tg

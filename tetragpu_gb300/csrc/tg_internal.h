@@ -37,6 +37,7 @@ enum StatusFlag : unsigned int {
 // fast path: star positions and neighbours are bits of a 64-bit mask.
 constexpr int kMaxStar = 64;
 constexpr int kMaxDeg = 64;
+constexpr int kNarrowDeg = 32;   // the most neighbours of a 32-bit link mask
 
 // VV entries per window of the link-adjacency kernel (tg_crit.cu): its
 // window table has n_vv / kAdjWin + 2 entries
@@ -48,8 +49,9 @@ enum ScanKind : int {
     SCAN_COUNT_I32 = 0,  // in: int32 counts (+ in2's when given), out: int64 offsets [n + 1]
     SCAN_POPC_RANK = 1,  // in: uint32 bit words, out: uint2 {word, popcount prefix} [n + 1],
                          //     out[n] = {0, total}: rank of bit p = one 8-byte load
+    SCAN_COUNT_PAD8 = 3, // SCAN_COUNT_I32 of the counts rounded up to multiples of eight
     SCAN_DEG_SQUARE = 2  // in: int32 x (+ in2's), out: int64 prefix of x*x [n + 1]; the largest
-                         //     x above kMaxDeg goes to the status word's max_deg
+                         //     x above kNarrowDeg goes to the status word's max_deg
 };
 struct ScanJob {
     const void *in;
@@ -186,10 +188,11 @@ void launch_vt_sort(const int64_t *vt_off, int32_t *vt, int64_t V, int64_t nvt, 
 void launch_vv_sort(const int64_t *vv_off, int64_t V, int64_t nvv, const int2 *inc, int32_t *vv,
                     int32_t *eid, cudaStream_t s);
 // Star processing order (vertices by first cell): vorder[pos] = vertex, pos =
-// rank of its key
+// rank of its key; vpos the way back (heavy vertices after the light ones,
+// vertices without cells last, counted in heavy_cnt[3])
 void launch_vorder_place(const int64_t *vt_off, int64_t V, const int64_t *vkey,
-                         const uint2 *vrank, int64_t nwk, const int32_t *heavy_cnt, int32_t *vorder,
-                         cudaStream_t s);
+                         const uint2 *vrank, int64_t nwk, int32_t *heavy_cnt, int32_t *vorder,
+                         int32_t *vpos, cudaStream_t s);
 
 // Star pass (tg_star.cu): the edges and faces of the light vertices.
 struct StarPass {
@@ -303,27 +306,36 @@ void launch_crit_heavy(const int64_t *vv_off, const int32_t *vv, int64_t v0, int
                        int32_t *list, int32_t *n_list, int32_t *scratch, cudaStream_t s);
 
 // critical points (tg_crit.cu)
-// vv_win: window table of VV (launch_window_starts over vv_off, crit_window())
+// The graph of the link adjacency: VV's rows by position, each vertex named by
+// its position in `order`, entries ascending and padded with -1 to a multiple
+// of eight; or (order null) VV itself, unpadded, positions being ids
+struct LinkGraph {
+    int64_t V, n_ent;              // n_ent: at least the entries, padding included
+    const int64_t *off;
+    const int32_t *ent;
+    const int32_t *order, *vpos;   // vertex at each position, and back; both null or neither
+    void *adj;                     // a mask per entry: 64-bit when wide, else 32-bit
+    bool wide;                     // a row holds more than 32 entries (always so without order)
+};
+// VV's row lengths by position, and (off their prefix) its rows
+void launch_vv_lengths_in_order(const int64_t *vv_off, const int32_t *order, int64_t V, int32_t *len,
+                                cudaStream_t s);
+void launch_rows_in_order(const int64_t *vv_off, const int32_t *vv, const int32_t *order,
+                          const int32_t *vpos, int64_t V, const int64_t *off, int32_t *ent,
+                          cudaStream_t s);
+// the masks; win: window table of off (launch_window_starts, crit_window())
 int crit_window();
 // heavy: 0 no row longer than kMaxDeg, 1 such rows get the heavy path
 // (masks of their light neighbours computed from the light side), 2 report
-// them with ST_HEAVY_DEG
-// order / ooff / ostart: visit the rows in this vertex order (ooff: the row
-// lengths' prefix in it, V + 1 entries; ostart: each row's start in VV;
-// vv_win a window table over ooff), or null for id order (vv_win over vv_off)
-void launch_crit_adj(const int64_t *vv_off, const int32_t *vv, const int32_t *order,
-                     const int64_t *ooff, const int64_t *ostart, const int32_t *vv_win,
-                     int64_t V, int64_t n_vv, uint64_t *adj, DevStatus *st, int heavy,
-                     cudaStream_t s);
-// len[i] = length and start[i] = first entry of VV row order[i] (0 from
-// n_with_cells on)
-void launch_vv_lengths_in_order(const int64_t *vv_off, const int32_t *order, int64_t V,
-                                int64_t n_with_cells, int32_t *len, int64_t *start,
-                                cudaStream_t s);
-// classify rows [v0, v0 + nv): field and classes3 hold nv values / rows from v0
-void launch_crit_classify(const int64_t *vv_off, const int32_t *vv, const uint64_t *adj,
-                          const void *field, int field_type, int64_t v0, int64_t nv,
-                          uint32_t *classes3, cudaStream_t s);
+// them with ST_HEAVY_DEG (positions are ids)
+void launch_crit_adj(const LinkGraph &g, const int32_t *win, DevStatus *st, int heavy, cudaStream_t s);
+// classify the vertices [v0, v0 + nv) (all of them, or a range that holds
+// every neighbour of its vertices): field and classes3 hold nv values / rows
+// from v0; ordered: scratch for V field values if classify_orders_field(nv)
+// (never without an order), else null
+bool classify_orders_field(int64_t nv);
+void launch_crit_classify(const LinkGraph &g, const void *field, int field_type, void *ordered,
+                          int64_t v0, int64_t nv, uint32_t *classes3, cudaStream_t s);
 
 // the message tg_last_error_string returns on this thread
 void set_last_error(const char *msg);

@@ -37,7 +37,8 @@ __device__ __forceinline__ int64_t load_value(const ScanJob &j, int64_t i, int *
     if (j.kind == SCAN_POPC_RANK) return (int64_t)__popc(__ldg((const uint32_t *)j.in + i));
     const int x = __ldg((const int32_t *)j.in + i) + (j.in2 ? __ldg(j.in2 + i) : 0);
     if (j.kind == SCAN_COUNT_I32) return x;
-    if (x > kMaxDeg) atomicMax(max_deg, x);
+    if (j.kind == SCAN_COUNT_PAD8) return (x + 7) & ~7;
+    if (x > kNarrowDeg) atomicMax(max_deg, x);
     return (int64_t)x * x;
 }
 

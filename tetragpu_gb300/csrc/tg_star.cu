@@ -964,25 +964,32 @@ k_window_starts(const int64_t *__restrict__ off, int64_t V, int64_t n_win, int w
 // last.
 __global__ void __launch_bounds__(256)
 k_vorder_place(const int64_t *__restrict__ vt_off, int64_t V, const int64_t *__restrict__ vkey,
-               const uint2 *__restrict__ vrank, int64_t nwk, const int *__restrict__ heavy_cnt,
-               int *__restrict__ vorder)
+               const uint2 *__restrict__ vrank, int64_t nwk, int *__restrict__ heavy_cnt,
+               int *__restrict__ vorder, int *__restrict__ vpos)
 {
     griddep_wait();
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= V) return;
     const int64_t n_light = (int64_t)__ldg(&vrank[nwk].y);
-    // the positions past the vertices with cells (their rows are empty)
-    if (v >= n_light + *heavy_cnt) vorder[v] = 0;
-    if (vt_off[v + 1] == vt_off[v]) return;
-    const long long key = vkey[v];
     int64_t pos;
-    if (key < 0) {
-        pos = n_light + (-1 - key);
+    if (vt_off[v + 1] == vt_off[v]) {
+        const unsigned together = __activemask();
+        const int lane = threadIdx.x & 31, leader = __ffs((int)together) - 1;
+        int at = 0;
+        if (lane == leader) at = atomicAdd(heavy_cnt + 3, __popc(together));
+        at = __shfl_sync(together, at, leader) + __popc(together & ((1u << lane) - 1u));
+        pos = n_light + heavy_cnt[0] + at;
     } else {
-        const uint2 r = __ldg(vrank + (key >> 5));
-        pos = (int64_t)r.y + __popc(r.x & ((1u << (key & 31)) - 1u));
+        const long long key = vkey[v];
+        if (key < 0) {
+            pos = n_light + (-1 - key);
+        } else {
+            const uint2 r = __ldg(vrank + (key >> 5));
+            pos = (int64_t)r.y + __popc(r.x & ((1u << (key & 31)) - 1u));
+        }
     }
     vorder[pos] = (int)v;
+    vpos[v] = (int)pos;
 }
 
 // First edge and face id of each segment of cells (a mesh of a batch):
@@ -1112,13 +1119,13 @@ void launch_vv_sort(const int64_t *vv_off, int64_t V, int64_t nvv, const int2 *i
 }
 
 void launch_vorder_place(const int64_t *vt_off, int64_t V, const int64_t *vkey,
-                         const uint2 *vrank, int64_t nwk, const int32_t *heavy_cnt, int32_t *vorder,
-                         cudaStream_t s)
+                         const uint2 *vrank, int64_t nwk, int32_t *heavy_cnt, int32_t *vorder,
+                         int32_t *vpos, cudaStream_t s)
 {
     if (V == 0) return;
     Launch L("k_vorder_place", s);
     launch_pdl(k_vorder_place, (unsigned)((V + 255) / 256), 256, 0, s, vt_off, V, vkey, vrank, nwk,
-               heavy_cnt, vorder);
+               heavy_cnt, vorder, vpos);
 }
 
 void launch_seg_ranks(const int64_t *seg_c, int64_t n, const uint2 *erank, const uint2 *frank,
