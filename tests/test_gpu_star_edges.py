@@ -59,3 +59,15 @@ def test_cells_given_twice(gpu_lib, oracle):
     m = meshgen.kuhn_mesh((2, 1, 1), seed=6)
     one = m.tv[::4]
     _check(gpu_lib, oracle, np.concatenate([one, one[:, ::-1]]), m.n_verts)
+
+
+@pytest.mark.parametrize("k", [13, 14, 15, 16, 21, 22, 23, 24, 30, 31, 61, 62, 63, 64])
+def test_edge_rows_of_given_lengths(gpu_lib, oracle, k):
+    # EE at the edges of its tiers (rows of fewer than 16, 24, at most 32, 64):
+    # the axis vertices of the rings have k + 1 edges, some edges only in the
+    # last warp of a block, the totals not multiples of four
+    rng = np.random.default_rng(100 + k)
+    ring = np.array([[0, 1, 2 + i, 2 + (i + 1) % k] for i in range(k)])
+    tv = np.concatenate([ring + j * (k + 2) for j in range(5)])
+    n = 5 * (k + 2)
+    _check(gpu_lib, oracle, rng.permutation(n)[tv].astype(np.int32), n)

@@ -584,12 +584,17 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
             TRY(tmp.alloc(&hv.pairs, 3 * m->heavy_entries));
             launch_heavy(hv, s);
         }
-        ScanJob jobs[5] = {{sp.deg_own, vv_off, V, SCAN_COUNT_I32, sp.deg_in},
+        // (the incident-edge rows of EE are padded)
+        const bool want_ee = mask & TG_EE;
+        int64_t *eid_off = nullptr;
+        if (want_ee) TRY(tmp.alloc(&eid_off, V + 1));
+        ScanJob jobs[6] = {{sp.deg_own, vv_off, V, SCAN_COUNT_I32, sp.deg_in},
                            {eflag, erank, nwe, SCAN_POPC_RANK, nullptr},
                            {fflag, frank, nwf, SCAN_POPC_RANK, nullptr},
                            {fbnd, brank, nwf, SCAN_POPC_RANK, nullptr},
-                           {sp.deg_own, deg_sq, V, SCAN_DEG_SQUARE, sp.deg_in}};
-        scan_batch(jobs, 5, m->scan, m->st, s);
+                           {sp.deg_own, deg_sq, V, SCAN_DEG_SQUARE, sp.deg_in},
+                           {sp.deg_own, eid_off, V, SCAN_EID_WORDS, sp.deg_in}};
+        scan_batch(jobs, want_ee ? 6 : 5, m->scan, m->st, s);
 
         // ---- the one synchronisation: edge, face, neighbour and boundary
         // counts size every output from here on ----
@@ -602,6 +607,7 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         if (m->st_host->flags) return check_flags(m);
         m->max_deg = m->st_host->max_deg > kMaxDeg ? m->st_host->max_deg : 0;
         m->wide_deg = m->st_host->max_deg > kNarrowDeg;
+        const int largest_deg = m->st_host->max_deg;
         const int64_t nvv = m->sz_host[0];
         const int64_t E = m->sz_host[1], F = m->sz_host[2];
         const int64_t n_bnd = m->sz_host[3];  // boundary faces
@@ -613,13 +619,14 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         // ---- ids: VV, EV, row lengths (per edge); TF, FT, FV (per cell).
         // Each kernel goes out once its own buffers exist; the later
         // allocations are made while it runs
-        int32_t *vv, *eid_sorted = nullptr;
+        int32_t *vv;
+        uint32_t *eid = nullptr;
         int32_t *ev = nullptr, *te = nullptr, *tf = nullptr, *fv = nullptr, *ft = nullptr;
         TRY(dalloc(&vv, nvv, s));
         tmp.track(vv);
         int2 *inc = nullptr;
         if (mask & TG_EE) {
-            TRY(tmp.alloc(&eid_sorted, nvv));
+            TRY(tmp.alloc(&eid, nvv + 16 * V));   // eid_words of each row at most
             TRY(tmp.alloc(&inc, nvv));
         }
         EdgePass ep{};
@@ -647,7 +654,8 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         if (need_ev) TRY(tmp.alloc(&ev, 2 * E));
         if (et_off || ef_off || ee_off || ev)
             launch_edge_offsets(ep, et_off, ef_off, ee_off, ev, m->scan, m->st, s);
-        launch_vv_sort(vv_off, V, nvv, inc, vv, eid_sorted, s);
+        if (inc) launch_inc_sort(vv_off, V, inc, vv, eid_off, eid, s);
+        else launch_vv_sort(vv_off, V, nvv, vv, s);
         // CSR totals: ET = 6T, EF = 3F always; TT and FF from the
         // boundary-face count
         int32_t *et = nullptr, *ef = nullptr, *ee = nullptr, *ff = nullptr, *tt = nullptr,
@@ -691,8 +699,8 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
             if (prep_adj) lb.build(m, vv_off, vv, nvv, s2);
         }
         if (ee_off) {
-            launch_ee_fill(ev, E, vv_off, eid_sorted, ee_off, ee, s);
-            if (m->max_deg) launch_ee_heavy(ev, E, vv_off, eid_sorted, ee_off, ee, s);
+            launch_ee_fill(ev, E, eid_off, eid, ee_off, ee, largest_deg, s);
+            if (m->max_deg) launch_ee_heavy(ev, E, vv_off, eid_off, eid, ee_off, ee, s);
         }
         side.join();
         CK(cudaGetLastError());
@@ -814,9 +822,9 @@ const char *tg_tuning_info(void)
         snprintf(buf, sizeof buf,
                  "{\"TG_STAR_WIN\": %d, \"TG_STAR_THREADS\": %d, \"TG_STAR_PER\": %d, "
                  "\"TG_VTS_THREADS\": %d, \"TG_EDGE_ITEMS\": %d, "
-                 "\"TG_ADJ_WIN\": %d, \"TG_ADJ_THREADS\": %d, \"TG_EE_GROUP\": %d}",
+                 "\"TG_ADJ_WIN\": %d, \"TG_ADJ_THREADS\": %d}",
                  TG_STAR_WIN, TG_STAR_THREADS, TG_STAR_PER, TG_VTS_THREADS, TG_EDGE_ITEMS,
-                 TG_ADJ_WIN, TG_ADJ_THREADS, TG_EE_GROUP);
+                 TG_ADJ_WIN, TG_ADJ_THREADS);
         info = buf;
     });
     return info.c_str();

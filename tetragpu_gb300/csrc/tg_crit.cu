@@ -32,17 +32,6 @@
 namespace tg {
 namespace {
 
-__device__ __forceinline__ int pad8(int d) { return (d + 7) & ~7; }
-
-// eight entries from a 32-byte boundary in one load
-__device__ __forceinline__ void load8(const int *p, int (&x)[8])
-{
-    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]),
-                   "=r"(x[7])
-                 : "l"(p));
-}
-
 // ---------------------------------------------------------------------------
 // Rows into processing order, each padded with -1 to whole 32-byte sectors (so
 // that a thread loads eight entries at once): sixteen lanes copy a row, four rows' loads in flight; a thread sorts it (a
@@ -189,7 +178,10 @@ __device__ __forceinline__ void adj_scan(const AdjRow &R, const int *__restrict_
     for (int i0 = 0; i0 < un; i0 += 8) {
         int q[8];
         if constexpr (PAD) {
-            load8(urow + i0, q);
+            unsigned w8[8];
+            load8(reinterpret_cast<const unsigned *>(urow + i0), w8);
+#pragma unroll
+            for (int t = 0; t < 8; t++) q[t] = (int)w8[t];
         } else {
 #pragma unroll
             for (int t = 0; t < 8; t++) q[t] = i0 + t < un ? __ldg(urow + i0 + t) : -1;
@@ -478,10 +470,10 @@ k_crit_classify(const int64_t *__restrict__ off, const int *__restrict__ ent,
         };
         if constexpr (PAD) {
             for (int k = 0; k < n; k += 8) {
-                int u[8];
-                load8(ent + b + k, u);
+                unsigned u[8];
+                load8(reinterpret_cast<const unsigned *>(ent + b + k), u);
 #pragma unroll
-                for (int t = 0; t < 8; t++) look(k + t, u[t]);
+                for (int t = 0; t < 8; t++) look(k + t, (int)u[t]);
             }
         } else {
             for (int k = 0; k < n; k++) look(k, __ldg(ent + b + k));

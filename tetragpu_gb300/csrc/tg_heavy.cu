@@ -217,22 +217,25 @@ __global__ void __launch_bounds__(64) k_heavy(HeavyStars h)
 // itself (in both) dropped.
 __global__ void __launch_bounds__(256)
 k_ee_heavy(const int *__restrict__ ev, int64_t E, const int64_t *__restrict__ vv_off,
-           const int *__restrict__ eid, const int64_t *__restrict__ ee_off, int *__restrict__ ee)
+           const int64_t *__restrict__ eid_off, const unsigned *__restrict__ eid,
+           const int64_t *__restrict__ ee_off, int *__restrict__ ee)
 {
     griddep_wait();
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < E;
          e += (int64_t)gridDim.x * blockDim.x) {
         const int2 ab = reinterpret_cast<const int2 *>(ev)[e];
-        const int64_t ra = vv_off[ab.x], rb = vv_off[ab.y];
-        const int na = (int)(vv_off[ab.x + 1] - ra), nb = (int)(vv_off[ab.y + 1] - rb);
+        const int na = (int)(vv_off[ab.x + 1] - vv_off[ab.x]);
+        const int nb = (int)(vv_off[ab.y + 1] - vv_off[ab.y]);
+        const int64_t ra = eid_off[ab.x], rb = eid_off[ab.y];
+        // k_ee_fill's: rows of at most kMaxDeg words, padding included
         if (max(na, nb) <= kMaxDeg) continue;
         int64_t o = ee_off[e];
         int i = 0, j = 0;
         while (i < na || j < nb) {
-            int x;
+            unsigned x;
             if (j >= nb || (i < na && eid[ra + i] < eid[rb + j])) x = eid[ra + i++];
             else x = eid[rb + j++];
-            if (x != (int)e) ee[o++] = x;
+            if (x != (unsigned)e) ee[o++] = (int)x;
         }
     }
 }
@@ -327,13 +330,13 @@ void launch_heavy(const HeavyStars &h, cudaStream_t s)
     launch_pdl(k_heavy, (unsigned)((h.n_heavy + 63) / 64), 64, 0, s, h);
 }
 
-void launch_ee_heavy(const int32_t *ev, int64_t E, const int64_t *vv_off, const int32_t *eid,
-                     const int64_t *ee_off, int32_t *ee, cudaStream_t s)
+void launch_ee_heavy(const int32_t *ev, int64_t E, const int64_t *vv_off, const int64_t *eid_off,
+                     const uint32_t *eid, const int64_t *ee_off, int32_t *ee, cudaStream_t s)
 {
     if (E == 0) return;
     Launch L("k_ee_heavy", s);
     const int64_t blocks = std::min<int64_t>((E + 255) / 256, 152 * 16);
-    launch_pdl(k_ee_heavy, (unsigned)blocks, 256, 0, s, ev, E, vv_off, eid, ee_off, ee);
+    launch_pdl(k_ee_heavy, (unsigned)blocks, 256, 0, s, ev, E, vv_off, eid_off, eid, ee_off, ee);
 }
 
 void launch_crit_heavy(const int64_t *vv_off, const int32_t *vv, int64_t v0, int64_t nv,

@@ -50,8 +50,9 @@ enum ScanKind : int {
     SCAN_POPC_RANK = 1,  // in: uint32 bit words, out: uint2 {word, popcount prefix} [n + 1],
                          //     out[n] = {0, total}: rank of bit p = one 8-byte load
     SCAN_COUNT_PAD8 = 3, // SCAN_COUNT_I32 of the counts rounded up to multiples of eight
+    SCAN_EID_WORDS = 4,  // SCAN_COUNT_I32 of eid_words of the counts
     SCAN_DEG_SQUARE = 2  // in: int32 x (+ in2's), out: int64 prefix of x*x [n + 1]; the largest
-                         //     x above kNarrowDeg goes to the status word's max_deg
+                         //     x goes to the status word's max_deg
 };
 struct ScanJob {
     const void *in;
@@ -183,10 +184,12 @@ void launch_window_starts(const int64_t *off, int64_t rows, int64_t n_entries, i
 void launch_vt_sort(const int64_t *vt_off, int32_t *vt, int64_t V, int64_t nvt, const int4 *tvs,
                     uint32_t *vflag, int64_t *vkey, int32_t *heavy_cnt, int32_t *heavy_off,
                     cudaStream_t s);
-// sort VV rows in place, or with inc (EdgePass) write them and the
-// incident-edge rows sorted
-void launch_vv_sort(const int64_t *vv_off, int64_t V, int64_t nvv, const int2 *inc, int32_t *vv,
-                    int32_t *eid, cudaStream_t s);
+// sort VV rows in place
+void launch_vv_sort(const int64_t *vv_off, int64_t V, int64_t nvv, int32_t *vv, cudaStream_t s);
+// VV rows and incident-edge rows from inc (EdgePass), sorted; the latter at
+// eid_off (SCAN_EID_WORDS), padded with ~0 to eid_words
+void launch_inc_sort(const int64_t *vv_off, int64_t V, const int2 *inc, int32_t *vv,
+                     const int64_t *eid_off, uint32_t *eid, cudaStream_t s);
 // Star processing order (vertices by first cell): vorder[pos] = vertex, pos =
 // rank of its key; vpos the way back (heavy vertices after the light ones,
 // vertices without cells last, counted in heavy_cnt[3])
@@ -277,8 +280,10 @@ void launch_cell_tt(int64_t T, int64_t F, const int32_t *tf, const int32_t *ft, 
 // rows (ff_off and ff together)
 void launch_face_fill(const int32_t *ft, const int32_t *tf, const int32_t *te, const uint2 *brank,
                       int64_t F, int32_t *fe, int64_t *ff_off, int32_t *ff, cudaStream_t s);
-void launch_ee_fill(const int32_t *ev, int64_t E, const int64_t *vv_off, const int32_t *eid_sorted,
-                    const int64_t *ee_off, int32_t *ee, cudaStream_t s);
+// EE rows; eid / eid_off: incident-edge rows as launch_inc_sort leaves them,
+// max_deg the longest
+void launch_ee_fill(const int32_t *ev, int64_t E, const int64_t *eid_off, const uint32_t *eid,
+                    const int64_t *ee_off, int32_t *ee, int max_deg, cudaStream_t s);
 void launch_tt_vertex_count(const int4 *tvs, int64_t T, const int64_t *vt_off, const int32_t *vt,
                             int32_t *cnt, cudaStream_t s);
 void launch_tt_vertex_fill(const int4 *tvs, int64_t T, const int64_t *vt_off, const int32_t *vt,
@@ -296,8 +301,8 @@ struct HeavyStars {
 };
 void launch_heavy(const HeavyStars &h, cudaStream_t s);
 // EE rows of edges with an endpoint of more than kMaxDeg neighbours
-void launch_ee_heavy(const int32_t *ev, int64_t E, const int64_t *vv_off, const int32_t *eid,
-                     const int64_t *ee_off, int32_t *ee, cudaStream_t s);
+void launch_ee_heavy(const int32_t *ev, int64_t E, const int64_t *vv_off, const int64_t *eid_off,
+                     const uint32_t *eid, const int64_t *ee_off, int32_t *ee, cudaStream_t s);
 // classes of the vertices in [v0, v0 + nv) with more than kMaxDeg neighbours
 // (at most max_listed of them): list (capacity max_listed) and n_list (one
 // int, zeroed by the caller) are scratch, scratch holds one int per VV entry
@@ -372,6 +377,19 @@ __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wa
 // data in flight, so a kernel can put many dependent-load chains' loads in
 // flight at once.  A thread sees its own copies after cp_async_wait(); other
 // threads' after that and a barrier.
+// eight words from a 32-byte boundary (a sector) in one load
+__device__ __forceinline__ void load8(const unsigned *p, unsigned (&x)[8])
+{
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]),
+                   "=r"(x[7])
+                 : "l"(p));
+}
+__device__ __forceinline__ int pad8(int d) { return (d + 7) & ~7; }
+// words of an incident-edge row of d edges: 16, or with a free word at the end
+// a multiple of eight
+__device__ __forceinline__ int eid_words(int d) { return d < 16 ? 16 : pad8(d + 1); }
+
 template <int B>
 __device__ __forceinline__ void cp_async(void *smem, const void *gmem)
 {

@@ -263,33 +263,107 @@ k_face_fill(const int *__restrict__ ft, const int *__restrict__ tf, const int *_
         if (i < n) row[i] = r[i];
 }
 
-// EE: a warp takes 32 consecutive edges (each lane fetches one edge's
-// endpoints and offsets), then merges them one at a time.  For e = (a, b) the
-// sorted incident-edge rows of a and b (at most kMaxDeg = 64 each) form one
-// bitonic sequence over 32 * R positions (lane l holds positions l + 32 r):
-// a's row ascending in the first half, b's row descending in the second, both
-// padded with INT_MAX towards the middle.  One bitonic merge sorts it; e sits
-// twice at adjacent positions (it is in both rows, and the rows share nothing
-// else), so dropping both copies leaves e's EE row.  R = 1, 2 or 4 by the
-// longer row (16, 32, 64 entries).
-constexpr int kEeWarps = 8;
+// EE: an edge (a, b)'s row is the merge of the sorted incident-edge rows of a
+// and b without the edge itself, which is in both (they share nothing else).
+// A warp takes 32 consecutive edges, a lane each: both rows are loaded into
+// registers eight entries at a time (padded to whole sectors with ~0), a's
+// ascending and b's descending around ~0s form one bitonic sequence, and one bitonic merge in registers sorts it.  The warp's
+// rows are contiguous in EE: they pass through shared memory and go out as
+// whole lines.  Bound by the load / store pipe (80%; a lane's two rows are lines
+// of their own, the entries reach shared memory a word at a time).  Four lanes
+// to an edge instead, whose entries went out in 16-byte pieces, sent 11
+// requests to L2 an edge (0.8 a clock and SM, what gets through; now 4) and 33
+// warp instructions (19): 92 -> 64 us at 64^3, 135 -> 93 us beside other kernels
+// on the 64^3 coned mesh, whose rows pass 16.
+constexpr int kEeThreads = 128;
+constexpr int kEeWarps = kEeThreads / 32;
+// words that a warp's rows come to, of ends of at most N edges
+constexpr int ee_stage(int n) { return 32 * (2 * n - 2) + 4; }
 
-template <int R>
-__device__ __forceinline__ void ee_merge_one(const int *__restrict__ eid, int64_t ra, int na,
-                                             int64_t rb, int nb, int ei, int *__restrict__ out,
-                                             int lane)
+template <int P>
+__device__ __forceinline__ void bitonic_merge(unsigned (&x)[P])
 {
-    constexpr int N = 32 * R, H = N / 2;
-    int x[R];
+#pragma unroll
+    for (int stride = P / 2; stride >= 1; stride >>= 1) {
+#pragma unroll
+        for (int i = 0; i < P; i++) {
+            if (i & stride) continue;
+            const unsigned lo = min(x[i], x[i + stride]);
+            x[i + stride] = max(x[i], x[i + stride]);
+            x[i] = lo;
+        }
+    }
+}
+
+// One edge a lane, rows of at most N entries; a lane's n words of EE (from o;
+// the lanes' rows follow one another) through `stage`.  P: the power of two at
+// or above 2 N; a, b: the rows' first 16 words.
+template <int N, int P>
+__device__ __forceinline__ void ee_merge_lanes(const unsigned (&a)[16], const unsigned (&b)[16],
+                                               const unsigned *__restrict__ ra,
+                                               const unsigned *__restrict__ rb, unsigned e, int64_t o,
+                                               int n, unsigned *stage, int *__restrict__ ee)
+{
+    unsigned x[P];
+#pragma unroll
+    for (int i = N; i < P - N; i++) x[i] = ~0u;
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+        x[i] = a[i];
+        x[P - 1 - i] = b[i];
+    }
+#pragma unroll
+    for (int k = 16; k < N; k += 8) {
+        unsigned t[8], u[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) t[i] = u[i] = ~0u;
+        if (a[15] != ~0u) load8(ra + k, t);
+        if (b[15] != ~0u) load8(rb + k, u);
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            x[k + i] = t[i];
+            x[P - 1 - (k + i)] = u[i];
+        }
+    }
+    bitonic_merge<P>(x);
+    const int lane = threadIdx.x & 31;
+    const int64_t o0 = __shfl_sync(kFull, o, 0);
+    const int shift = (int)(o0 & 3);   // word i of the stage is word i of the line o0 is in
+    const int at = shift + (int)(o - o0);
+    // sorted: an entry above e follows both copies of e
+#pragma unroll
+    for (int i = 0; i < 2 * N; i++)
+        if (i < n + 2 && x[i] != e) stage[at + (x[i] > e ? i - 2 : i)] = x[i];
+    __syncwarp();
+    const int end = __reduce_max_sync(kFull, n >= 0 ? at + n : 0);
+    int *line = ee + (o0 - shift);
+    for (int i = 4 * lane; i < end; i += 128) {
+        const uint4 w = *reinterpret_cast<const uint4 *>(stage + i);
+        if (i >= shift && i + 4 <= end) {
+            *reinterpret_cast<uint4 *>(line + i) = w;
+        } else {
+            const unsigned q[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+            for (int t = 0; t < 4; t++)
+                if (i + t >= shift && i + t < end) line[i + t] = (int)q[t];
+        }
+    }
+}
+
+// An edge by the whole warp: the same merge over 32 * R positions (lane l holds
+// positions l + 32 r), for rows of at most 16 R entries.
+template <int R>
+__device__ __forceinline__ void ee_merge_warp_r(const unsigned *__restrict__ ra, int na,
+                                                const unsigned *__restrict__ rb, int nb, unsigned e,
+                                                int *__restrict__ out, int lane)
+{
+    constexpr int P = 32 * R;
+    unsigned x[R];
 #pragma unroll
     for (int r = 0; r < R; r++) {
         const int p = lane + 32 * r;
-        if (p < H) {
-            x[r] = p < na ? __ldg(eid + ra + p) : INT_MAX;
-        } else {
-            const int j = N - 1 - p;
-            x[r] = j < nb ? __ldg(eid + rb + j) : INT_MAX;
-        }
+        const int j = P - 1 - p;
+        x[r] = p < P / 2 ? (p < na ? __ldg(ra + p) : ~0u) : (j < nb ? __ldg(rb + j) : ~0u);
     }
     // strides >= 32: between registers
 #pragma unroll
@@ -297,7 +371,7 @@ __device__ __forceinline__ void ee_merge_one(const int *__restrict__ eid, int64_
 #pragma unroll
         for (int r = 0; r < R; r++) {
             if (r & sr) continue;
-            const int lo = min(x[r], x[r + sr]), hi = max(x[r], x[r + sr]);
+            const unsigned lo = min(x[r], x[r + sr]), hi = max(x[r], x[r + sr]);
             x[r] = lo;
             x[r + sr] = hi;
         }
@@ -308,121 +382,94 @@ __device__ __forceinline__ void ee_merge_one(const int *__restrict__ eid, int64_
         const bool upper = lane & sl;
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            const int y = __shfl_xor_sync(kFull, x[r], sl);
+            const unsigned y = __shfl_xor_sync(kFull, x[r], sl);
             x[r] = upper ? max(x[r], y) : min(x[r], y);
         }
     }
-    // the row is sorted: an entry above e follows both copies of e
-    const int n = na + nb;
+    // (the two copies of e are at adjacent positions)
 #pragma unroll
     for (int r = 0; r < R; r++) {
         const int p = lane + 32 * r;
-        if (p < n && x[r] != ei) out[p - (x[r] > ei ? 2 : 0)] = x[r];
+        if (p < na + nb && x[r] != e) out[p - (x[r] > e ? 2 : 0)] = (int)x[r];
     }
 }
-
-// Rows of at most 16 entries each (the common case: 14 neighbours inside a
-// Kuhn grid) go 32 / G edges at a time, G lanes to an edge, 32 / G registers
-// to a lane (position gl + G r): the same bitonic merge over 32 positions,
-// the strides of G and more between registers, the smaller ones between the
-// group's lanes.
-constexpr int kEeGroup = TG_EE_GROUP;
-static_assert(kEeGroup == 4 || kEeGroup == 8, "lanes per edge: 4 or 8");
-
-template <int G>
-__device__ __forceinline__ void ee_merge_group(const int *__restrict__ eid, int64_t ra, int na,
-                                               int64_t rb, int nb, int ei, int *__restrict__ out,
-                                               int gl)
+// entries of a row (at most kMaxDeg; kMaxDeg + 1: more, the heavy path's)
+__device__ __forceinline__ int ee_row_length(const unsigned *__restrict__ row, int lane)
 {
-    constexpr int R = 32 / G;
-    int x[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-        const int p = gl + G * r;
-        if (p < 16) {
-            x[r] = p < na ? __ldg(eid + ra + p) : INT_MAX;
-        } else {
-            const int j = 31 - p;
-            x[r] = j < nb ? __ldg(eid + rb + j) : INT_MAX;
-        }
+    int n = 0;
+    while (n <= kMaxDeg) {
+        // words n .. n + 15, then eight at a time: the row goes on while the
+        // last word is an entry
+        const int w = n == 0 ? 16 : 8;
+        const unsigned ends = __ballot_sync(kFull, lane < w && __ldg(row + n + (lane < w ? lane : 0)) == ~0u);
+        if (ends) return min(n + __ffs((int)ends) - 1, kMaxDeg + 1);
+        n += w;
     }
-    // strides 16 .. G: between registers (register stride sr = stride / G)
-#pragma unroll
-    for (int sr = 16 / G; sr >= 1; sr >>= 1) {
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-            if (r & sr) continue;
-            const int lo = min(x[r], x[r + sr]), hi = max(x[r], x[r + sr]);
-            x[r] = lo;
-            x[r + sr] = hi;
-        }
-    }
-    // strides G / 2 .. 1: lanes of the group
-#pragma unroll
-    for (int sl = G / 2; sl >= 1; sl >>= 1) {
-        const bool upper = gl & sl;
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-            const int y = __shfl_xor_sync(kFull, x[r], sl);
-            x[r] = upper ? max(x[r], y) : min(x[r], y);
-        }
-    }
-    // the row is sorted: an entry above e follows both copies of e
-    const int n = na + nb;
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-        const int p = gl + G * r;
-        if (p < n && x[r] != ei) out[p - (x[r] > ei ? 2 : 0)] = x[r];
-    }
+    return kMaxDeg + 1;
+}
+__device__ __noinline__ void ee_merge_warp(const unsigned *__restrict__ ra, const unsigned *__restrict__ rb,
+                                           unsigned e, int *__restrict__ out, int lane)
+{
+    const int na = ee_row_length(ra, lane), nb = ee_row_length(rb, lane), m = max(na, nb);
+    if (m > kMaxDeg) return;   // k_ee_heavy's
+    if (m <= 32) ee_merge_warp_r<2>(ra, na, rb, nb, e, out, lane);
+    else ee_merge_warp_r<4>(ra, na, rb, nb, e, out, lane);
 }
 
-__global__ void __launch_bounds__(kEeWarps * 32)
-k_ee_fill(const int *__restrict__ ev, int64_t E, const int64_t *__restrict__ vv_off,
-          const int *__restrict__ eid, const int64_t *__restrict__ ee_off, int *__restrict__ ee)
+// eid: each vertex's incident edges, ascending, from word eid_off[v] on, padded
+// with ~0 to 16 words, or beyond those to a multiple of eight that leaves a
+// ~0 at the end (so that a row's sixteenth word tells whether it goes on).
+// ROWS: 16 or 24 when every row is shorter than that (fewer registers), else 0.
+template <int ROWS>
+__global__ void __launch_bounds__(kEeThreads, ROWS == 16 ? 9 : 5)
+k_ee_fill(const int2 *__restrict__ ev, int64_t E, const int64_t *__restrict__ eid_off,
+          const unsigned *__restrict__ eid, const int64_t *__restrict__ ee_off, int *__restrict__ ee)
 {
     griddep_wait();
+    __shared__ __align__(16) unsigned s_stage[kEeWarps][ee_stage(ROWS == 16 ? 16 : 24)];
     const int lane = threadIdx.x & 31;
     const int64_t e0 = ((int64_t)blockIdx.x * kEeWarps + (threadIdx.x >> 5)) * 32;
     if (e0 >= E) return;  // warp-uniform
+    const int64_t e = e0 + lane;
+    int64_t o = 0;
+    const unsigned *ra = eid, *rb = eid;
+    int n = -2;   // no edge
+    unsigned a[16], b[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) a[i] = b[i] = ~0u;
+    if (e < E) {
+        const int2 ab = __ldg(ev + e);
+        o = __ldg(ee_off + e);
+        n = (int)(__ldg(ee_off + e + 1) - o);
+        ra += __ldg(eid_off + ab.x);
+        rb += __ldg(eid_off + ab.y);
+        load8(ra, reinterpret_cast<unsigned(&)[8]>(a[0]));
+        load8(ra + 8, reinterpret_cast<unsigned(&)[8]>(a[8]));
+        load8(rb, reinterpret_cast<unsigned(&)[8]>(b[0]));
+        load8(rb + 8, reinterpret_cast<unsigned(&)[8]>(b[8]));
+    }
+    unsigned *stage = s_stage[threadIdx.x >> 5];
+    // a row of 16 or more
+    const bool more = ROWS != 16 && (a[15] != ~0u || b[15] != ~0u);
+    if (ROWS == 16 || !__any_sync(kFull, more)) {
+        ee_merge_lanes<16, 32>(a, b, ra, rb, (unsigned)e, o, n, stage, ee);
+        return;
+    }
+    if constexpr (ROWS == 16) return;
+    bool longer = false;   // of 24 or more
+    if (ROWS == 0 && a[15] != ~0u) longer |= __ldg(ra + 23) != ~0u;
+    if (ROWS == 0 && b[15] != ~0u) longer |= __ldg(rb + 23) != ~0u;
+    if (ROWS == 24 || !__any_sync(kFull, longer)) {
+        ee_merge_lanes<24, 64>(a, b, ra, rb, (unsigned)e, o, n, stage, ee);
+        return;
+    }
+    if constexpr (ROWS != 0) return;
+    // by the whole warp
     const int cnt = E - e0 < 32 ? (int)(E - e0) : 32;
-    int64_t my_ra = 0, my_rb = 0, my_out = 0;
-    int my_na = 0, my_nb = 0;
-    if (lane < cnt) {
-        const int2 ab = __ldg(reinterpret_cast<const int2 *>(ev) + e0 + lane);
-        my_ra = __ldg(vv_off + ab.x);
-        my_rb = __ldg(vv_off + ab.y);
-        my_na = (int)(__ldg(vv_off + ab.x + 1) - my_ra);
-        my_nb = (int)(__ldg(vv_off + ab.y + 1) - my_rb);
-        my_out = __ldg(ee_off + e0 + lane);
-    }
-    const unsigned small = __ballot_sync(kFull, lane < cnt && max(my_na, my_nb) <= 16);
-    // rows longer than kMaxDeg: the heavy path's (k_ee_heavy)
-    const unsigned big = __ballot_sync(kFull, lane < cnt && max(my_na, my_nb) <= kMaxDeg) & ~small;
-    // small edges, 32 / G per round (group g takes the (k + g)-th one)
-    constexpr int G = kEeGroup;
-    const int g = lane / G, gl = lane % G;
-    const int n_small = __popc(small);
-    const bool all_small = small == 0xffffffffu;   // no lanes to skip (the common case)
-    for (int k = 0; k < n_small; k += 32 / G) {
-        const int which = k + g;
-        const int src = all_small ? which : (which < n_small ? (int)__fns(small, 0, which + 1) : 0);
-        const int64_t ra = __shfl_sync(kFull, my_ra, src), rb = __shfl_sync(kFull, my_rb, src);
-        int na = __shfl_sync(kFull, my_na, src), nb = __shfl_sync(kFull, my_nb, src);
-        const int64_t o = __shfl_sync(kFull, my_out, src);
-        if (which >= n_small) na = nb = 0;  // an idle group: nothing to write
-        ee_merge_group<G>(eid, ra, na, rb, nb, (int)(e0 + src), ee + o, gl);
-    }
-    // longer rows one edge at a time over the whole warp
-    for (unsigned rest = big; rest; rest &= rest - 1) {
-        const int j = __ffs(rest) - 1;
-        const int64_t ra = __shfl_sync(kFull, my_ra, j), rb = __shfl_sync(kFull, my_rb, j);
-        const int na = __shfl_sync(kFull, my_na, j), nb = __shfl_sync(kFull, my_nb, j);
-        int *out = ee + __shfl_sync(kFull, my_out, j);
-        const int ei = (int)(e0 + j);
-        if (max(na, nb) <= 32)
-            ee_merge_one<2>(eid, ra, na, rb, nb, ei, out, lane);
-        else
-            ee_merge_one<4>(eid, ra, na, rb, nb, ei, out, lane);
+    for (int j = 0; j < cnt; j++) {
+        const unsigned *pa = (const unsigned *)__shfl_sync(kFull, (unsigned long long)ra, j);
+        const unsigned *pb = (const unsigned *)__shfl_sync(kFull, (unsigned long long)rb, j);
+        ee_merge_warp(pa, pb, (unsigned)(e0 + j), ee + __shfl_sync(kFull, o, j), lane);
     }
 }
 
@@ -638,15 +685,14 @@ void launch_face_fill(const int32_t *ft, const int32_t *tf, const int32_t *te, c
     }
 }
 
-void launch_ee_fill(const int32_t *ev, int64_t E, const int64_t *vv_off, const int32_t *eid_sorted,
-                    const int64_t *ee_off, int32_t *ee, cudaStream_t s)
+void launch_ee_fill(const int32_t *ev, int64_t E, const int64_t *eid_off, const uint32_t *eid,
+                    const int64_t *ee_off, int32_t *ee, int max_deg, cudaStream_t s)
 {
     if (E == 0) return;
-    {
-        Launch L("k_ee_fill", s);
-        launch_pdl(k_ee_fill, blocks_for((E + 31) / 32, kEeWarps), kEeWarps * 32, 0, s, ev, E, vv_off, eid_sorted,
-                                                                   ee_off, ee);
-    }
+    Launch L("k_ee_fill", s);
+    launch_pdl(max_deg < 16 ? k_ee_fill<16> : (max_deg < 24 ? k_ee_fill<24> : k_ee_fill<0>),
+               blocks_for(E, kEeThreads), kEeThreads, 0, s, reinterpret_cast<const int2 *>(ev), E, eid_off,
+               eid, ee_off, ee);
 }
 
 void launch_tt_vertex_count(const int4 *tvs, int64_t T, const int64_t *vt_off, const int32_t *vt,

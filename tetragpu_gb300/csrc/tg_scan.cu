@@ -32,13 +32,14 @@ struct ScanParams {
     int n_jobs;
 };
 
-__device__ __forceinline__ int64_t load_value(const ScanJob &j, int64_t i, int *max_deg)
+__device__ __forceinline__ int64_t load_value(const ScanJob &j, int64_t i, int &largest)
 {
     if (j.kind == SCAN_POPC_RANK) return (int64_t)__popc(__ldg((const uint32_t *)j.in + i));
     const int x = __ldg((const int32_t *)j.in + i) + (j.in2 ? __ldg(j.in2 + i) : 0);
     if (j.kind == SCAN_COUNT_I32) return x;
-    if (j.kind == SCAN_COUNT_PAD8) return (x + 7) & ~7;
-    if (x > kNarrowDeg) atomicMax(max_deg, x);
+    if (j.kind == SCAN_COUNT_PAD8) return pad8(x);
+    if (j.kind == SCAN_EID_WORDS) return eid_words(x);
+    largest = max(largest, x);
     return (int64_t)x * x;
 }
 
@@ -106,10 +107,16 @@ __global__ void __launch_bounds__(kThreads) k_scan(ScanParams p)
     const int64_t base = tile * kTile + (int64_t)threadIdx.x * kItems;
     int64_t v[kItems];
     int64_t s = 0;
+    int largest = 0;
 #pragma unroll
     for (int k = 0; k < kItems; k++) {
-        v[k] = (base + k < j.n) ? load_value(j, base + k, p.max_deg) : 0;
+        v[k] = (base + k < j.n) ? load_value(j, base + k, largest) : 0;
         s += v[k];
+    }
+    if (j.kind == SCAN_DEG_SQUARE) {   // block-uniform
+        largest = __reduce_max_sync(0xffffffffu, largest);
+        if ((threadIdx.x & 31) == 0 && largest > *(volatile int *)p.max_deg)
+            atomicMax(p.max_deg, largest);
     }
     int64_t excl;
     const int64_t total = block_exclusive_scan<kThreads>(s, excl, sm);

@@ -754,30 +754,38 @@ k_vv_sort(const int64_t *__restrict__ off, int64_t V, int64_t total, int *__rest
 }
 
 // VV and incident-edge rows from inc (the same rows, {neighbour, edge id}
-// pairs), each sorted by itself
+// pairs), each sorted by itself; the incident-edge rows padded with ~0 to
+// eid_words at eid_off
 constexpr int kIncCap = 20 * kVtsThreads;
 __global__ void __launch_bounds__(kVtsThreads, 9)
 k_inc_sort(const int64_t *__restrict__ off, int64_t V, const int2 *__restrict__ inc,
-           int *__restrict__ vv, int *__restrict__ eid)
+           int *__restrict__ vv, const int64_t *__restrict__ eid_off, int *__restrict__ eid)
 {
     griddep_wait();
     __shared__ int s_row[2][kIncCap];
+    __shared__ int s_at[kVtsThreads], s_len[kVtsThreads];
+    __shared__ long long s_out[kVtsThreads];
     const int64_t v0 = (int64_t)blockIdx.x * kVtsThreads;
     const int64_t v = v0 + threadIdx.x;
     const int64_t base = off[v0];
     const int64_t n = off[min(v0 + kVtsThreads, V)] - base;
     const int64_t b = v < V ? off[v] : 0;
     const int d = v < V ? (int)(off[v + 1] - b) : 0;
+    const int64_t out = v < V ? eid_off[v] : 0;
     if (n > kIncCap) {   // block-uniform: in place
         for (int k = 0; k < d; k++) {
             const int2 x = inc[b + k];
             vv[b + k] = x.x;
-            eid[b + k] = x.y;
+            eid[out + k] = x.y;
         }
+        for (int k = d; k < (v < V ? eid_words(d) : 0); k++) eid[out + k] = -1;
 #pragma unroll 1
-        for (int q = 0; q < 2; q++) sort_rows_warp((q ? eid : vv) + b, d);
+        for (int q = 0; q < 2; q++) sort_rows_warp(q ? eid + out : vv + b, d);
         return;
     }
+    s_at[threadIdx.x] = (int)(b - base);
+    s_len[threadIdx.x] = d;
+    s_out[threadIdx.x] = out;
     for (int i = threadIdx.x; i < (int)n; i += kVtsThreads) {
         const int2 x = __ldg(inc + base + i);
         s_row[0][i] = x.x;
@@ -787,9 +795,13 @@ k_inc_sort(const int64_t *__restrict__ off, int64_t V, const int2 *__restrict__ 
 #pragma unroll 1
     for (int q = 0; q < 2; q++) sort_rows_warp(s_row[q] + (int)(b - base), d);
     __syncthreads();
-    for (int i = threadIdx.x; i < (int)n; i += kVtsThreads) {
-        vv[base + i] = s_row[0][i];
-        eid[base + i] = s_row[1][i];
+    for (int i = threadIdx.x; i < (int)n; i += kVtsThreads) vv[base + i] = s_row[0][i];
+    const int rows = (int)min((int64_t)kVtsThreads, V - v0);
+    for (int r = threadIdx.x >> 4; r < rows; r += kVtsThreads / 16) {
+        const int at = s_at[r], len = s_len[r], words = eid_words(len);
+        int *row = eid + s_out[r];
+        for (int k = threadIdx.x & 15; k < words; k += 16)
+            row[k] = k < len ? s_row[1][at + k] : -1;
     }
 }
 
@@ -1104,18 +1116,21 @@ void launch_vt_sort(const int64_t *vt_off, int32_t *vt, int64_t V, int64_t nvt, 
                V, nvt, vt, tvs, vflag, vkey, heavy_cnt, heavy_off);
 }
 
-void launch_vv_sort(const int64_t *vv_off, int64_t V, int64_t nvv, const int2 *inc, int32_t *vv,
-                    int32_t *eid, cudaStream_t s)
+void launch_vv_sort(const int64_t *vv_off, int64_t V, int64_t nvv, int32_t *vv, cudaStream_t s)
 {
     if (V == 0 || nvv == 0) return;
-    const unsigned grid = (unsigned)((V + kVtsThreads - 1) / kVtsThreads);
-    if (inc) {
-        Launch L("k_inc_sort", s);
-        launch_pdl(k_inc_sort, grid, kVtsThreads, 0, s, vv_off, V, inc, vv, eid);
-    } else {
-        Launch L("k_vv_sort", s);
-        launch_pdl(k_vv_sort, grid, kVtsThreads, 0, s, vv_off, V, nvv, vv);
-    }
+    Launch L("k_vv_sort", s);
+    launch_pdl(k_vv_sort, (unsigned)((V + kVtsThreads - 1) / kVtsThreads), kVtsThreads, 0, s, vv_off, V,
+               nvv, vv);
+}
+
+void launch_inc_sort(const int64_t *vv_off, int64_t V, const int2 *inc, int32_t *vv,
+                     const int64_t *eid_off, uint32_t *eid, cudaStream_t s)
+{
+    if (V == 0) return;
+    Launch L("k_inc_sort", s);
+    launch_pdl(k_inc_sort, (unsigned)((V + kVtsThreads - 1) / kVtsThreads), kVtsThreads, 0, s, vv_off, V,
+               inc, vv, eid_off, reinterpret_cast<int *>(eid));
 }
 
 void launch_vorder_place(const int64_t *vt_off, int64_t V, const int64_t *vkey,

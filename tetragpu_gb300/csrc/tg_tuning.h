@@ -32,6 +32,3 @@
 #ifndef TG_ADJ_THREADS
 #define TG_ADJ_THREADS 128   // threads per link-adjacency block
 #endif
-#ifndef TG_EE_GROUP
-#define TG_EE_GROUP 4   // lanes per edge for EE rows of at most 16 + 16 entries
-#endif

@@ -3,8 +3,7 @@
     python -m tetragpu_gb300.tune [--apply] [--steps K]
 
 The tile constants of the kernels (the star pass's block size and vertices
-per warp, block sizes of the row sorts and the link adjacency, EE lanes per
-edge, edges per thread of the edge-offset pass) are compile-time constants.  For every candidate setting
+per warp, block sizes of the row sorts and the link adjacency, edges per thread of the edge-offset pass) are compile-time constants.  For every candidate setting
 (the default and one change at a time from it) this builds a variant of
 libtetragpu.so with -D overrides under tetragpu_gb300/_build/variants/, loads
 it, and times the batched pipeline (tg_batch create + all 13 relations with
@@ -45,7 +44,6 @@ CANDIDATES = [
     ("star_per_8", {"TG_STAR_PER": 8, "TG_STAR_WIN": 512}),
     ("star_threads_256", {"TG_STAR_THREADS": 256, "TG_STAR_WIN": 512, "TG_STAR_MINB": 6}),
     ("star_minb_10", {"TG_STAR_MINB": 10}),
-    ("ee_group_8", {"TG_EE_GROUP": 8}),
     ("adj_threads_64", {"TG_ADJ_THREADS": 64}),
     ("adj_threads_256", {"TG_ADJ_THREADS": 256}),
     ("vt_sort_threads_64", {"TG_VTS_THREADS": 64}),
