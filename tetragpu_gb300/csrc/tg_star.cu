@@ -947,18 +947,20 @@ __global__ void __launch_bounds__(kEdgeThreads) k_edge_offsets(EdgeOffsets p)
 
 // win[w] = first vertex whose row starts at or after entry win_size * w, for
 // w in [0, n_win], with win[n_win] = V.  Vertex v owns the windows w with
-// off[v-1] < win_size * w <= off[v].
+// off[v-1] < win_size * w <= off[v]; the windows past the last entry (n_win may
+// be sized for more) are all threads' work.
 __global__ void __launch_bounds__(256)
 k_window_starts(const int64_t *__restrict__ off, int64_t V, int64_t n_win, int win_size,
                 int *__restrict__ win)
 {
     griddep_wait();
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t past = off[V] / win_size + 1;
+    for (int64_t w = past + v; w <= n_win; w += (int64_t)gridDim.x * blockDim.x) win[w] = (int)V;
     if (v > V) return;
-    const long long lo = v == 0 ? -1 : off[v - 1];
-    const long long hi = v == V ? (long long)win_size * n_win : off[v];
-    long long w = lo < 0 ? 0 : lo / win_size + 1;
-    for (const long long w_hi = hi / win_size; w <= w_hi && w <= n_win; w++) win[w] = (int)v;
+    const long long lo = v == 0 ? -1 : off[v - 1], hi = off[v];
+    for (long long w = lo < 0 ? 0 : lo / win_size + 1; w <= hi / win_size && w <= n_win; w++)
+        win[w] = (int)v;
 }
 
 // ---------------------------------------------------------------------------
