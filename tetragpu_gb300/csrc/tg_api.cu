@@ -1,10 +1,12 @@
 // tg_api.cu -- host orchestration of the relation pipeline behind the C ABI
 // declared in include/tetragpu.h.
 //
-// One tg_mesh owns its device buffers.  Memory comes from the device's
-// stream-ordered pool (cudaMallocAsync) with an unlimited release threshold,
-// so repeated extractions reuse blocks instead of returning them to the
-// driver.  tg_extract synchronises the stream at two points, to learn the
+// One tg_mesh owns its device buffers.  Memory comes from stream-ordered pools
+// with an unlimited release threshold, so repeated extractions reuse blocks
+// instead of returning them to the driver; a stage's arrays come out of one
+// allocation each for what stays and what does not (some forty calls a step
+// before: 357 -> 308 us at 24,576 cells, 24 requests to the server 5.6 -> 3.2
+// ms).  tg_extract synchronises the stream at two points, to learn the
 // edge/face/neighbour counts and then the CSR totals that size the outputs;
 // everything between those points is asynchronous on the caller's stream.
 #include <algorithm>
@@ -13,6 +15,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -110,20 +113,42 @@ tg_status cuda_fail(cudaError_t e, const char *what, int line)
 
 constexpr int64_t kMaxCells = 357913941LL;  // 6 * cells must fit in 31 bits
 
+// Where memory comes from: the device's default stream-ordered pool for what a
+// mesh keeps, a pool of the library's own for temporaries.  Out of one pool, a
+// stage's temporaries took the place of the relations of the mesh destroyed
+// before, and relations of 5 GB found no room in one piece: the driver then
+// remaps memory, 2.7 ms of a 128^3 step in a loop that keeps the previous mesh
+// until the next is made.  Both pools keep what is freed for the next call (the
+// temporaries' up to an eighth of the device's memory); when one cannot grow,
+// the other gives back what it does not use.
+struct Pools {
+    cudaMemPool_t keep = nullptr, temp = nullptr;
+    bool ready = false;
+};
 std::mutex g_pool_mu;
-bool g_pool_ready[64];
+Pools g_pools[64];
 
-void setup_pool(int dev)
+const Pools *device_pools(int dev)
 {
+    if (dev < 0 || dev >= 64) return nullptr;
     std::lock_guard<std::mutex> lk(g_pool_mu);
-    if (dev < 0 || dev >= 64 || g_pool_ready[dev]) return;
-    cudaMemPool_t pool;
-    if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
+    Pools &p = g_pools[dev];
+    if (!p.ready) {
         uint64_t thr = UINT64_MAX;
-        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
+        if (cudaDeviceGetDefaultMemPool(&p.keep, dev) != cudaSuccess) p.keep = nullptr;
+        else cudaMemPoolSetAttribute(p.keep, cudaMemPoolAttrReleaseThreshold, &thr);
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        if (cudaMemPoolCreate(&p.temp, &props) != cudaSuccess) p.temp = nullptr;
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) thr = total_b / 8;
+        if (p.temp) cudaMemPoolSetAttribute(p.temp, cudaMemPoolAttrReleaseThreshold, &thr);
+        (void)cudaGetLastError();
+        p.ready = true;
     }
-    (void)cudaGetLastError();
-    g_pool_ready[dev] = true;
+    return p.keep && p.temp ? &p : nullptr;
 }
 
 // Pinned, device-mapped host slots for the status word and the sizes read
@@ -246,11 +271,23 @@ struct Fork {
     }
 };
 
+// Device memory of a mesh: one allocation that several arrays share, given
+// back (in the order of the mesh's last stream) when nothing refers to it.
+struct Block {
+    void *p = nullptr;
+    const tg_mesh *m = nullptr;
+    Block(void *q, const tg_mesh *mesh) : p(q), m(mesh) {}
+    Block(const Block &) = delete;
+    ~Block();
+};
+using BlockRef = std::shared_ptr<Block>;
+
 struct Rel {
     int64_t rows = 0, entries = 0;
     int width = 0;
     int64_t *off = nullptr;
     int32_t *ent = nullptr;
+    BlockRef hold_off, hold_ent;   // null for VT, which lies in the mesh's own block
     bool ready = false;
     uint32_t opts = 0;
 };
@@ -259,64 +296,81 @@ const int kWidth[14] = {0, 6, 2, 0, 4, 3, 3, 2, 0, 0, 0, 0, 0, 0};
 const char *kName[14] = {"validate", "TE", "EV", "ET", "TF", "FV", "FE",
                          "FT",       "EF", "VT", "TT", "FF", "EE", "VV"};
 
-// Scoped list of stream-ordered temporaries, freed when the stage ends.
+// Arrays that come out of one allocation, each on a 256-byte boundary: a call
+// to the allocator costs a microsecond or more, and a stage has up to twenty
+// arrays.  add() names the pointer to set.
+struct Plan {
+    void **at[32];
+    size_t off[32];
+    int n = 0;
+    size_t bytes = 0;
+    template <class T>
+    void add(T **out, int64_t count)
+    {
+        at[n] = (void **)out;
+        off[n++] = bytes;
+        bytes += ((size_t)std::max<int64_t>(count, 1) * sizeof(T) + 255) & ~size_t(255);
+    }
+    void place(void *base) const
+    {
+        for (int i = 0; i < n; i++) *at[i] = (char *)base + off[i];
+    }
+};
+
+// from the pool of kept memory (temp false) or of temporaries
+tg_status take(size_t bytes, cudaStream_t s, void **out, bool temp = false)
+{
+    bytes = std::max<size_t>(bytes, 256);
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    const Pools *p = device_pools(dev);
+    cudaError_t e = p ? cudaMallocFromPoolAsync(out, bytes, temp ? p->temp : p->keep, s)
+                      : cudaMallocAsync(out, bytes, s);
+    if (e == cudaErrorMemoryAllocation && p) {
+        (void)cudaGetLastError();
+        // what was freed on this stream counts once the stream is through
+        cudaStreamSynchronize(s);
+        cudaMemPoolTrimTo(temp ? p->keep : p->temp, 0);
+        e = cudaMallocFromPoolAsync(out, bytes, temp ? p->temp : p->keep, s);
+    }
+    return e == cudaSuccess ? TG_OK : cuda_fail(e, "cudaMallocFromPoolAsync", __LINE__);
+}
+
+// a plan's arrays in a block
+tg_status take_block(const Plan &plan, const tg_mesh *m, cudaStream_t s, BlockRef *out)
+{
+    if (plan.n == 0) return TG_OK;
+    void *q = nullptr;
+    TRY(take(plan.bytes, s, &q));
+    *out = std::make_shared<Block>(q, m);
+    plan.place(q);
+    return TG_OK;
+}
+
+// Stream-ordered temporaries, freed when the stage ends.
 struct Temps {
     cudaStream_t s;
-    void *p[64];
+    void *p[8];
     int n = 0;
     explicit Temps(cudaStream_t st) : s(st) {}
     ~Temps()
     {
-        for (int i = 0; i < n; i++)
-            if (p[i]) cudaFreeAsync(p[i], s);
+        for (int i = 0; i < n; i++) cudaFreeAsync(p[i], s);
     }
-    template <class T>
-    tg_status alloc(T **out, int64_t count, bool zero = false)
+    // a plan's arrays; the first zero_bytes zeroed
+    tg_status add(const Plan &plan, size_t zero_bytes = 0)
     {
-        size_t b = (size_t)std::max<int64_t>(count, 1) * sizeof(T);
-        if (n >= 64) return fail(TG_ERR_UNSUPPORTED, "too many temporaries in one stage");
+        if (plan.n == 0) return TG_OK;
+        if (n >= 8) return fail(TG_ERR_UNSUPPORTED, "too many temporaries in one stage");
         void *q = nullptr;
-        cudaError_t e = cudaMallocAsync(&q, b, s);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaMallocAsync (temporary)", __LINE__);
-        if (zero) {
-            e = cudaMemsetAsync(q, 0, b, s);
+        TRY(take(plan.bytes, s, &q, true));
+        p[n++] = q;
+        if (zero_bytes) {
+            const cudaError_t e = cudaMemsetAsync(q, 0, zero_bytes, s);
             if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync", __LINE__);
         }
-        p[n++] = q;
-        *out = (T *)q;
+        plan.place(q);
         return TG_OK;
-    }
-    // free q with the others if the stage fails (list sized for every path)
-    void track(void *q) { p[n++] = q; }
-    // hand a temporary over to the caller (it is not freed here)
-    void keep(void *q)
-    {
-        for (int i = 0; i < n; i++)
-            if (p[i] == q) p[i] = nullptr;
-    }
-};
-
-template <class T>
-tg_status dalloc(T **out, int64_t count, cudaStream_t s)
-{
-    size_t b = (size_t)std::max<int64_t>(count, 1) * sizeof(T);
-    void *q = nullptr;
-    cudaError_t e = cudaMallocAsync(&q, b, s);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMallocAsync", __LINE__);
-    *out = (T *)q;
-    return TG_OK;
-}
-
-// Offsets of several arrays in one allocation (each on a 256-byte boundary),
-// so that arrays zeroed together cost one memset.
-struct Carve {
-    size_t bytes = 0;
-    template <class T>
-    size_t add(int64_t n)
-    {
-        const size_t off = bytes;
-        bytes += ((size_t)std::max<int64_t>(n, 1) * sizeof(T) + 255) & ~size_t(255);
-        return off;
     }
 };
 
@@ -328,6 +382,8 @@ struct tg_mesh {
     int device = 0;
     cudaStream_t last_stream = nullptr;  // stream of the last call, used to free asynchronously
     int64_t V = 0, T = 0, E = -1, F = -1;
+    void *base = nullptr;       // one allocation: everything from here to VT, the scan workspace
+                                // and the status word
     int4 *tvs = nullptr;
     // star processing order: vertices by first cell (see tg_star.cu)
     int32_t *vorder = nullptr;          // [V] vertex at each position (cell-less ones last)
@@ -347,6 +403,7 @@ struct tg_mesh {
     int max_deg = 0;            // largest degree above kMaxDeg seen by the extraction, else 0
     bool wide_deg = false;      // a vertex has more than kNarrowDeg neighbours
     // the link adjacency of critical points (LinkGraph; adj null: not built)
+    BlockRef lg;
     int64_t *lg_off = nullptr;
     int32_t *lg_ent = nullptr;
     void *lg_adj = nullptr;
@@ -357,22 +414,9 @@ struct tg_mesh {
 
 namespace {
 
-void free_rel(Rel &r, cudaStream_t s = nullptr, bool async = false)
+Block::~Block()
 {
-    if (async) {
-        if (r.off) cudaFreeAsync(r.off, s);
-        if (r.ent) cudaFreeAsync(r.ent, s);
-    } else {
-        if (r.off) cudaFree(r.off);
-        if (r.ent) cudaFree(r.ent);
-    }
-    r = Rel();
-}
-
-tg_status reset_status(tg_mesh *m, cudaStream_t s)
-{
-    launch_reset_status(m->st, s);
-    return TG_OK;
+    if (p) cudaFreeAsync(p, m->last_stream);
 }
 
 // Read the status word plus up to 8 device scalars (int64 if `wide[i]`,
@@ -399,26 +443,27 @@ tg_status check_flags(const tg_mesh *m, unsigned mask_ok = 0)
     const DevStatus &h = *m->st_host;
     const unsigned f = h.flags & ~mask_ok;
     if (!f) return TG_OK;
+    auto lowest = [](int noted) { return INT_MAX - noted; };
     if (f & ST_BAD_ID)
-        return fail(TG_ERR_INVALID_MESH, "cell %d has a vertex id outside [0, %lld)", h.bad_cell,
+        return fail(TG_ERR_INVALID_MESH, "cell %d has a vertex id outside [0, %lld)", lowest(h.bad_cell),
                     (long long)m->V);
     if (f & ST_DUP_VERTEX)
-        return fail(TG_ERR_INVALID_MESH, "cell %d repeats a vertex", h.bad_cell);
+        return fail(TG_ERR_INVALID_MESH, "cell %d repeats a vertex", lowest(h.bad_cell));
     if (f & ST_NONMANIFOLD_FACE)
         return fail(TG_ERR_INVALID_MESH, "a face of cell %d lies in more than two cells",
-                    h.bad_cell);
+                    lowest(h.bad_cell));
     if (f & ST_HEAVY_STAR)
         return fail(TG_ERR_UNSUPPORTED,
                     "vertex %d lies in more than %d cells (largest star this build handles)",
-                    h.bad_vertex, kMaxStar);
+                    lowest(h.bad_vertex), kMaxStar);
     if (f & ST_HEAVY_DEG)
         return fail(TG_ERR_UNSUPPORTED,
                     "a vertex has %d neighbours (more than %d, the largest this build handles)",
                     h.max_deg, kMaxDeg);
     if (f & ST_HASH_FULL)
-        return fail(TG_ERR_UNSUPPORTED, "vertex %d: neighbour table overflow", h.bad_vertex);
+        return fail(TG_ERR_UNSUPPORTED, "vertex %d: neighbour table overflow", lowest(h.bad_vertex));
     if (f & ST_STAR_OVERFLOW)
-        return fail(TG_ERR_UNSUPPORTED, "vertex %d: neighbour summary overflow", h.bad_vertex);
+        return fail(TG_ERR_UNSUPPORTED, "vertex %d: neighbour summary overflow", lowest(h.bad_vertex));
     if (f & ST_SCAN_STALLED)
         return fail(TG_ERR_CUDA, "a prefix scan gave up waiting for a preceding tile");
     return fail(TG_ERR_CUDA, "unexpected device status 0x%x", f);
@@ -426,37 +471,37 @@ tg_status check_flags(const tg_mesh *m, unsigned mask_ok = 0)
 
 inline uint32_t bit(int r) { return 1u << r; }
 
-tg_status set_fixed(tg_mesh *m, int r, int32_t *ent, int64_t rows)
+void set_fixed(tg_mesh *m, int r, int32_t *ent, int64_t rows, const BlockRef &hold)
 {
-    free_rel(m->rel[r]);
+    m->rel[r] = Rel();
     Rel &x = m->rel[r];
     x.rows = rows;
     x.width = kWidth[r];
     x.entries = rows * kWidth[r];
     x.ent = ent;
+    x.hold_ent = hold;
     x.ready = true;
-    return TG_OK;
 }
 
 void set_csr(tg_mesh *m, int r, int64_t *off, int32_t *ent, int64_t rows, int64_t entries,
-             uint32_t opts = 0)
+             const BlockRef &hold_off, const BlockRef &hold_ent, uint32_t opts = 0)
 {
-    free_rel(m->rel[r]);
+    m->rel[r] = Rel();
     Rel &x = m->rel[r];
     x.rows = rows;
     x.entries = entries;
     x.width = 0;
     x.off = off;
     x.ent = ent;
+    x.hold_off = hold_off;
+    x.hold_ent = hold_ent;
     x.ready = true;
     x.opts = opts;
 }
 
-void free_link_graph(tg_mesh *m, cudaStream_t s)
+void free_link_graph(tg_mesh *m)
 {
-    if (m->lg_off) cudaFreeAsync(m->lg_off, s);
-    if (m->lg_ent) cudaFreeAsync(m->lg_ent, s);
-    if (m->lg_adj) cudaFreeAsync(m->lg_adj, s);
+    m->lg.reset();
     m->lg_off = nullptr;
     m->lg_ent = nullptr;
     m->lg_adj = nullptr;
@@ -478,17 +523,16 @@ struct LinkBuild {
     int32_t *len, *win;
     tg_status alloc(tg_mesh *m, int64_t nvv, Temps &tmp, cudaStream_t s)
     {
-        TRY(tmp.alloc(&len, m->V));
         const int64_t n = link_entries(m, nvv);
-        TRY(tmp.alloc(&win, window_count(n, crit_window()) + 1));
-        int64_t *off;
-        int32_t *ent;
+        Plan t, g;
+        t.add(&len, m->V);
+        t.add(&win, window_count(n, crit_window()) + 1);
+        TRY(tmp.add(t));
         char *adj;
-        TRY(dalloc(&off, m->V + 1, s));
-        m->lg_off = off;
-        TRY(dalloc(&ent, n, s));
-        m->lg_ent = ent;
-        TRY(dalloc(&adj, n * (m->wide_deg ? 8 : 4), s));
+        g.add(&m->lg_off, m->V + 1);
+        g.add(&m->lg_ent, n);
+        g.add(&adj, n * (m->wide_deg ? 8 : 4));
+        TRY(take_block(g, m, s, &m->lg));
         m->lg_adj = adj;
         return TG_OK;
     }
@@ -532,39 +576,43 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         const bool need_ev = mask & (TG_EV | TG_EE);
         // the edges by id: for everything per edge
         const bool need_edge = need_te || need_ev || (mask & (TG_ET | TG_EF));
+        const bool want_ee = mask & TG_EE;
         StarPass sp{};
+        HeavyStars hv{};
+        int64_t *deg_sq, *eid_off = nullptr;
         {
             // the bitmaps the star pass sets bits in, the neighbour counts
-            // and the record counter: one zeroed allocation
-            Carve c;
-            const size_t o_e = c.add<uint32_t>(nwe), o_f = c.add<uint32_t>(nwf),
-                         o_b = c.add<uint32_t>(nwf), o_d = c.add<int32_t>(V),
-                         o_i = c.add<int32_t>(V),
-                         o_v = c.add<uint8_t>(V), o_n = c.add<uint32_t>(2);
-            char *z;
-            TRY(tmp.alloc(&z, (int64_t)c.bytes, true));
-            eflag = (uint32_t *)(z + o_e);
-            fflag = (uint32_t *)(z + o_f);
-            fbnd = (uint32_t *)(z + o_b);
-            sp.deg_own = (int32_t *)(z + o_d);
-            sp.deg_in = (int32_t *)(z + o_i);
-            sp.vbnd = (uint8_t *)(z + o_v);
-            sp.n_rec = (uint32_t *)(z + o_n);
+            // and the record counter are zeroed
+            Plan t;
+            t.add(&eflag, nwe);
+            t.add(&fflag, nwf);
+            t.add(&fbnd, nwf);
+            t.add(&sp.deg_own, V);
+            t.add(&sp.deg_in, V);
+            t.add(&sp.vbnd, V);
+            t.add(&sp.n_rec, 2);
+            const size_t zero = t.bytes;
+            t.add(&erank, nwe + 1);
+            t.add(&frank, nwf + 1);
+            t.add(&brank, nwf + 1);
+            t.add(&deg_sq, V + 1);   // prefix of deg^2: its total sizes EE (sum deg^2 - 2E)
+            if (want_ee) t.add(&eid_off, V + 1);   // EE's incident-edge rows are padded
+            // at most six edges a cell (their number is read back below)
+            t.add(&sp.rec, 6 * T);
+            t.add(&sp.place, 6 * T);
+            if (m->n_wide > 0 || m->n_heavy > 0) t.add(&sp.rec_hi, 6 * T);
+            if (m->n_wide > 0) t.add(&sp.wide, m->n_wide);
+            if (m->n_heavy > 0) t.add(&hv.pairs, 3 * m->heavy_entries);
+            if (need_tf || need_ft) t.add(&sp.fnext, 4 * T);
+            TRY(tmp.add(t, zero));
             sp.n_wide = sp.n_rec + 1;
         }
-        TRY(tmp.alloc(&erank, nwe + 1));
-        TRY(tmp.alloc(&frank, nwf + 1));
-        TRY(tmp.alloc(&brank, nwf + 1));
-        TRY(dalloc(&vv_off, V + 1, s));
-        tmp.track(vv_off);  // owned by the VV relation once it is ready
-        int64_t *deg_sq;  // prefix of deg^2: its total sizes EE (sum deg^2 - 2E)
-        TRY(tmp.alloc(&deg_sq, V + 1));
-        // at most six edges a cell (their number is read back below)
-        TRY(tmp.alloc(&sp.rec, 6 * T));
-        TRY(tmp.alloc(&sp.place, 6 * T));
-        if (m->n_wide > 0 || m->n_heavy > 0) TRY(tmp.alloc(&sp.rec_hi, 6 * T));
-        if (m->n_wide > 0) TRY(tmp.alloc(&sp.wide, m->n_wide));
-        if (need_tf || need_ft) TRY(tmp.alloc(&sp.fnext, 4 * T));
+        BlockRef hold_vv_off, hold_vv, hold_tt, hold;
+        {
+            Plan o;
+            o.add(&vv_off, V + 1);
+            TRY(take_block(o, m, s, &hold_vv_off));
+        }
         sp.n_light = m->n_light;
         sp.vorder = m->vorder;
         sp.vt_off = vt_off;
@@ -576,18 +624,12 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         sp.st = m->st;
         launch_star(sp, s);
         launch_star_wide(sp, m->n_wide, s);
-        HeavyStars hv{};
         if (m->n_heavy > 0) {
             hv.star = sp;
             hv.n_heavy = m->n_heavy;
             hv.heavy_off = m->heavy_off;
-            TRY(tmp.alloc(&hv.pairs, 3 * m->heavy_entries));
             launch_heavy(hv, s);
         }
-        // (the incident-edge rows of EE are padded)
-        const bool want_ee = mask & TG_EE;
-        int64_t *eid_off = nullptr;
-        if (want_ee) TRY(tmp.alloc(&eid_off, V + 1));
         ScanJob jobs[6] = {{sp.deg_own, vv_off, V, SCAN_COUNT_I32, sp.deg_in},
                            {eflag, erank, nwe, SCAN_POPC_RANK, nullptr},
                            {fflag, frank, nwf, SCAN_POPC_RANK, nullptr},
@@ -616,22 +658,64 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         m->F = F;
         if (m->seg_c) launch_seg_ranks(m->seg_c, m->n_seg, erank, frank, m->seg_ef, s);
 
-        // ---- ids: VV, EV, row lengths (per edge); TF, FT, FV (per cell).
-        // Each kernel goes out once its own buffers exist; the later
-        // allocations are made while it runs
-        int32_t *vv;
+        // ---- every other array: relations that were asked for in one block (TT,
+        // which may be made again in its other form, and VV, which every
+        // extraction makes, in their own), the rest temporary
+        int32_t *vv, *ev = nullptr, *te = nullptr, *tf = nullptr, *fv = nullptr, *ft = nullptr;
+        int32_t *et = nullptr, *ef = nullptr, *ee = nullptr, *ff = nullptr, *tt = nullptr, *fe = nullptr;
+        int64_t *et_off = nullptr, *ef_off = nullptr, *ee_off = nullptr, *ff_off = nullptr;
+        int64_t *tt_off = nullptr;
         uint32_t *eid = nullptr;
-        int32_t *ev = nullptr, *te = nullptr, *tf = nullptr, *fv = nullptr, *ft = nullptr;
-        TRY(dalloc(&vv, nvv, s));
-        tmp.track(vv);
         int2 *inc = nullptr;
-        if (mask & TG_EE) {
-            TRY(tmp.alloc(&eid, nvv + 16 * V));   // eid_words of each row at most
-            TRY(tmp.alloc(&inc, nvv));
-        }
         EdgePass ep{};
-        if (need_edge) TRY(tmp.alloc(&ep.edge, E));
-        if (need_edge && sp.rec_hi) TRY(tmp.alloc(&ep.edge_hi, E));
+        // CSR totals: ET = 6T, EF = 3F always; TT and FF from the
+        // boundary-face count; EE deg(a) + deg(b) - 2 per edge (a,b)
+        const int64_t n_et = 6 * T, n_ef = 3 * F, n_ee = sum_deg_sq - 2 * E;
+        const int64_t n_tt = 4 * T - n_bnd, n_ff = 3 * (2 * F - n_bnd);
+        {
+            Plan t, o, ovv, ott;
+            ovv.add(&vv, nvv);
+            if (want_ee) {
+                t.add(&eid, nvv + 16 * V);   // eid_words of each row at most
+                t.add(&inc, nvv);
+            }
+            if (need_edge) t.add(&ep.edge, E);
+            if (need_edge && sp.rec_hi) t.add(&ep.edge_hi, E);
+            if (need_ev) (mask & TG_EV ? o : t).add(&ev, 2 * E);
+            if (need_te) (mask & TG_TE ? o : t).add(&te, 6 * T);
+            if (need_tf) (mask & TG_TF ? o : t).add(&tf, 4 * T);
+            if (need_ft) (mask & TG_FT ? o : t).add(&ft, 2 * F);
+            if (mask & TG_FV) o.add(&fv, 3 * F);
+            if (mask & TG_FE) o.add(&fe, 3 * F);
+            if (mask & TG_ET) {
+                o.add(&et_off, E + 1);
+                o.add(&et, n_et);
+            }
+            if (mask & TG_EF) {
+                o.add(&ef_off, E + 1);
+                o.add(&ef, n_ef);
+            }
+            if (want_ee) {
+                o.add(&ee_off, E + 1);
+                o.add(&ee, n_ee);
+            }
+            if (mask & TG_FF) {
+                o.add(&ff_off, F + 1);
+                o.add(&ff, n_ff);
+            }
+            if (want_tt_face) {
+                ott.add(&tt_off, T + 1);
+                ott.add(&tt, n_tt);
+            }
+            TRY(take_block(ovv, m, s, &hold_vv));
+            TRY(tmp.add(t));
+            TRY(take_block(o, m, s, &hold));
+            TRY(take_block(ott, m, s, &hold_tt));
+        }
+        if (T == 0 && tt_off) CK(cudaMemsetAsync(tt_off, 0, 8, s));
+        if (T == 0 && ff_off) CK(cudaMemsetAsync(ff_off, 0, 8, s));
+
+        // ---- ids: VV, EV, row lengths (per edge); TF, FT, FV (per cell)
         ep.E = E;
         ep.rec = sp.rec; ep.place = sp.place; ep.rec_hi = sp.rec_hi; ep.pairs = hv.pairs;
         ep.vt_off = vt_off; ep.vt = vt; ep.tvs = m->tvs;
@@ -640,53 +724,17 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         ep.vv_off = vv_off; ep.inc = inc; ep.vv = vv;
         ep.count_ef = (mask & TG_EF) != 0;
         launch_edge_ids(ep, s);
-        if (need_tf) TRY(tmp.alloc(&tf, 4 * T));
-        if (need_ft) TRY(tmp.alloc(&ft, 2 * F));
-        if (mask & TG_FV) TRY(tmp.alloc(&fv, 3 * F));
         if (tf || ft || fv) launch_cell_faces(T, m->tvs, frank, sp.fnext, tf, ft, fv, s);
-        int64_t *et_off = nullptr, *ef_off = nullptr, *ee_off = nullptr, *ff_off = nullptr;
-        if (mask & TG_ET) TRY(dalloc(&et_off, E + 1, s));
-        if (et_off) tmp.track(et_off);
-        if (mask & TG_EF) TRY(dalloc(&ef_off, E + 1, s));
-        if (ef_off) tmp.track(ef_off);
-        if (mask & TG_EE) TRY(dalloc(&ee_off, E + 1, s));
-        if (ee_off) tmp.track(ee_off);
-        if (need_ev) TRY(tmp.alloc(&ev, 2 * E));
         if (et_off || ef_off || ee_off || ev)
             launch_edge_offsets(ep, et_off, ef_off, ee_off, ev, m->scan, m->st, s);
         if (inc) launch_inc_sort(vv_off, V, inc, vv, eid_off, eid, s);
         else launch_vv_sort(vv_off, V, nvv, vv, s);
-        // CSR totals: ET = 6T, EF = 3F always; TT and FF from the
-        // boundary-face count
-        int32_t *et = nullptr, *ef = nullptr, *ee = nullptr, *ff = nullptr, *tt = nullptr,
-                *fe = nullptr;
-        int64_t *tt_off = nullptr;
-        const int64_t n_et = 6 * T, n_ef = 3 * F;
-        const int64_t n_tt = 4 * T - n_bnd, n_ff = 3 * (2 * F - n_bnd);
-        if (need_te) TRY(tmp.alloc(&te, 6 * T));
-        if (et_off) TRY(dalloc(&et, n_et, s));
-        if (ef_off) TRY(dalloc(&ef, n_ef, s));
-        if (mask & TG_FE) TRY(dalloc(&fe, 3 * F, s));
-        if (want_tt_face) {
-            TRY(dalloc(&tt_off, T + 1, s));
-            TRY(dalloc(&tt, n_tt, s));
-            if (T == 0) CK(cudaMemsetAsync(tt_off, 0, 8, s));
-        }
-        if (mask & TG_FF) {
-            TRY(tmp.alloc(&ff_off, F + 1));
-            TRY(dalloc(&ff, n_ff, s));
-            if (T == 0) CK(cudaMemsetAsync(ff_off, 0, 8, s));
-        }
-        tmp.keep(vv);
-        tmp.keep(vv_off);
-        set_csr(m, TG_REL_VV, vv_off, vv, V, nvv);
-        free_link_graph(m, s);
+        set_csr(m, TG_REL_VV, vv_off, vv, V, nvv, hold_vv_off, hold_vv);
+        free_link_graph(m);
 
         // ET and EF rows, the per-cell TT rows, the per-face FE / FF rows and on
         // request the link adjacency of critical points, on a side stream
         // beside EE (each reads only what the passes before it wrote)
-        const int64_t n_ee = sum_deg_sq - 2 * E;   // deg(a) + deg(b) - 2 per edge (a,b)
-        if (ee_off) TRY(dalloc(&ee, n_ee, s));
         const bool prep_adj = (opts & TG_OPT_LINK_ADJACENCY) && (mask & TG_VV);
         LinkBuild lb;
         if (prep_adj) TRY(lb.alloc(m, nvv, tmp, s));
@@ -705,50 +753,40 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         side.join();
         CK(cudaGetLastError());
 
-        auto give_fixed = [&](int r, int32_t *p, int64_t rows) {
-            tmp.keep(p);
-            set_fixed(m, r, p, rows);
-        };
-        if (mask & TG_EV) give_fixed(TG_REL_EV, ev, E);
-        if (mask & TG_TE) give_fixed(TG_REL_TE, te, T);
-        if (mask & TG_TF) give_fixed(TG_REL_TF, tf, T);
-        if (mask & TG_FV) give_fixed(TG_REL_FV, fv, F);
-        if (mask & TG_FT) give_fixed(TG_REL_FT, ft, F);
-        if (fe) set_fixed(m, TG_REL_FE, fe, F);
-        if (et) {
-            tmp.keep(et_off);
-            set_csr(m, TG_REL_ET, et_off, et, E, n_et);
-        }
-        if (ef) {
-            tmp.keep(ef_off);
-            set_csr(m, TG_REL_EF, ef_off, ef, E, n_ef);
-        }
-        if (ee) {
-            tmp.keep(ee_off);
-            set_csr(m, TG_REL_EE, ee_off, ee, E, n_ee);
-        }
-        if (ff) {
-            tmp.keep(ff_off);
-            set_csr(m, TG_REL_FF, ff_off, ff, F, n_ff);
-        }
-        if (tt) set_csr(m, TG_REL_TT, tt_off, tt, T, n_tt, 0);
+        if (mask & TG_EV) set_fixed(m, TG_REL_EV, ev, E, hold);
+        if (mask & TG_TE) set_fixed(m, TG_REL_TE, te, T, hold);
+        if (mask & TG_TF) set_fixed(m, TG_REL_TF, tf, T, hold);
+        if (mask & TG_FV) set_fixed(m, TG_REL_FV, fv, F, hold);
+        if (mask & TG_FT) set_fixed(m, TG_REL_FT, ft, F, hold);
+        if (fe) set_fixed(m, TG_REL_FE, fe, F, hold);
+        if (et) set_csr(m, TG_REL_ET, et_off, et, E, n_et, hold, hold);
+        if (ef) set_csr(m, TG_REL_EF, ef_off, ef, E, n_ef, hold, hold);
+        if (ee) set_csr(m, TG_REL_EE, ee_off, ee, E, n_ee, hold, hold);
+        if (ff) set_csr(m, TG_REL_FF, ff_off, ff, F, n_ff, hold, hold);
+        if (tt) set_csr(m, TG_REL_TT, tt_off, tt, T, n_tt, hold_tt, hold_tt, 0);
     }
 
     if ((mask & TG_TT) && tt_vertex) {
-        int32_t *cnt;
+        int32_t *cnt, *tt;
         int64_t *tt_off;
-        TRY(tmp.alloc(&cnt, T));
-        TRY(dalloc(&tt_off, T + 1, s));
+        BlockRef hold_off, hold_ent;
+        Plan t, o;
+        t.add(&cnt, T);
+        o.add(&tt_off, T + 1);
+        TRY(tmp.add(t));
+        TRY(take_block(o, m, s, &hold_off));
         launch_tt_vertex_count(m->tvs, T, vt_off, vt, cnt, s);
         ScanJob job{cnt, tt_off, T, SCAN_COUNT_I32, nullptr};
         scan_batch(&job, 1, m->scan, m->st, s);
         const void *src[1] = {tt_off + T};
         const bool w8[1] = {true};
         TRY(sync_read(m, s, 1, src, w8));
-        int32_t *tt;
-        TRY(dalloc(&tt, m->sz_host[0], s));
+        Plan e;
+        e.add(&tt, m->sz_host[0]);
+        TRY(take_block(e, m, s, &hold_ent));
         launch_tt_vertex_fill(m->tvs, T, vt_off, vt, tt_off, tt, s);
-        set_csr(m, TG_REL_TT, tt_off, tt, T, m->sz_host[0], TG_OPT_TT_VERTEX_SHARING);
+        set_csr(m, TG_REL_TT, tt_off, tt, T, m->sz_host[0], hold_off, hold_ent,
+                TG_OPT_TT_VERTEX_SHARING);
     }
     CK(cudaGetLastError());
     return TG_OK;
@@ -770,7 +808,7 @@ tg_status tg::critical_points_rows(tg_mesh *m, int64_t v0, int64_t nv, const voi
     if (!m->lg_adj) {
         // VV rows longer than the adjacency masks take the heavy path of the
         // classification, so no status read-back here
-        free_link_graph(m, s);
+        free_link_graph(m);
         Temps adj_tmp(s);
         LinkBuild lb;
         TRY(lb.alloc(m, vv.entries, adj_tmp, s));
@@ -779,28 +817,34 @@ tg_status tg::critical_points_rows(tg_mesh *m, int64_t v0, int64_t nv, const voi
     Temps tmp(s);
     const size_t esz = field_type == TG_FIELD_F64 ? 8 : 4;
     const void *f = field;
-    if (!field_on_device) {
-        char *d;
-        TRY(tmp.alloc(&d, (int64_t)(nv * esz)));
-        CK(cudaMemcpyAsync(d, field, nv * esz, cudaMemcpyHostToDevice, s));
-        f = d;
-    }
     uint32_t *out = classes_out;
-    if (!out_on_device) TRY(tmp.alloc(&out, 3 * nv));
-    char *ordered = nullptr;
-    if (classify_orders_field(nv)) TRY(tmp.alloc(&ordered, m->V * (int64_t)esz));
+    char *d_field, *ordered = nullptr;
+    int32_t *list, *n_list, *scratch;
+    // vertices of more than kMaxDeg neighbours: at most one per kMaxDeg + 1 VV
+    // entries
+    const int64_t max_listed = std::min<int64_t>(nv, vv.entries / (kMaxDeg + 1) + 1);
+    {
+        Plan t;
+        size_t zero = 0;
+        if (m->max_deg) {
+            t.add(&n_list, 1);
+            zero = t.bytes;
+            t.add(&list, max_listed);
+            t.add(&scratch, vv.entries);
+        }
+        if (!field_on_device) t.add(&d_field, nv * (int64_t)esz);
+        if (!out_on_device) t.add(&out, 3 * nv);
+        if (classify_orders_field(nv)) t.add(&ordered, m->V * (int64_t)esz);
+        TRY(tmp.add(t, zero));
+    }
+    if (!field_on_device) {
+        CK(cudaMemcpyAsync(d_field, field, nv * esz, cudaMemcpyHostToDevice, s));
+        f = d_field;
+    }
     launch_crit_classify(link_graph(m, vv.entries), f, field_type, ordered, v0, nv, out, s);
-    if (m->max_deg) {
-        // vertices of more than kMaxDeg neighbours: at most one per
-        // kMaxDeg + 1 VV entries
-        const int64_t max_listed = std::min<int64_t>(nv, vv.entries / (kMaxDeg + 1) + 1);
-        int32_t *list, *n_list, *scratch;
-        TRY(tmp.alloc(&list, max_listed));
-        TRY(tmp.alloc(&n_list, 1, true));
-        TRY(tmp.alloc(&scratch, vv.entries));
+    if (m->max_deg)
         launch_crit_heavy(vv.off, vv.ent, v0, nv, max_listed, f, field_type, out, list, n_list,
                           scratch, s);
-    }
     CK(cudaGetLastError());
     if (!out_on_device) {
         CK(cudaMemcpyAsync(classes_out, out, (size_t)nv * 12, cudaMemcpyDeviceToHost, s));
@@ -843,19 +887,14 @@ tg_status tg_mesh_destroy(tg_mesh *m)
     // stream-ordered frees on the stream the mesh was last used on, then one
     // wait for that stream (no device-wide synchronisation)
     cudaStream_t s = m->last_stream;
-    for (auto &r : m->rel) free_rel(r, s, true);
-    if (m->tvs) cudaFreeAsync(m->tvs, s);
-    if (m->vorder) cudaFreeAsync(m->vorder, s);
-    if (m->heavy_off) cudaFreeAsync(m->heavy_off, s);
+    for (auto &r : m->rel) r = Rel();
+    free_link_graph(m);
     if (m->seg_c) cudaFreeAsync(m->seg_c, s);
     if (m->seg_ef) cudaFreeAsync(m->seg_ef, s);
-    if (m->vpos) cudaFreeAsync(m->vpos, s);
-    free_link_graph(m, s);
-    if (m->st) cudaFreeAsync(m->st, s);
-    if (m->scan.buf) {
+    if (m->base) {
         // after the last scan, whichever stream it ran on
         if (m->scan.used && m->scan.last != s) cudaStreamWaitEvent(s, m->scan.done, 0);
-        cudaFreeAsync(m->scan.buf, s);
+        cudaFreeAsync(m->base, s);
     }
     cudaStreamSynchronize(s);  // no copy into the pinned slots is still in flight
     if (m->scan.done) cudaEventDestroy(m->scan.done);
@@ -871,65 +910,66 @@ static tg_status mesh_create_impl(const int32_t *tv, int64_t T, int64_t V, int o
                                   cudaStream_t s, tg_mesh *m)
 {
     CK(cudaGetDevice(&m->device));
-    setup_pool(m->device);
     m->st_host = (DevStatus *)g_pinned.get();
     m->sz_host = (int64_t *)g_pinned.get();
     if (!m->st_host || !m->sz_host) return fail(TG_ERR_OUT_OF_MEMORY, "pinned host memory");
-    TRY(dalloc(&m->st, 1, s));
-    TRY(reset_status(m, s));
-    TRY(dalloc(&m->tvs, T, s));
+    // the scan workspace of every later scan on the mesh, zeroed once
+    m->scan.job_words = std::max(scan_job_words(std::max(std::max(V, T), (6 * T + 31) / 32)),
+                                 (edge_offsets_words(6 * T) + kMaxScanJobs - 1) / kMaxScanJobs);
+    int64_t *vt_off;
+    int32_t *vt;
+    {
+        Plan b;
+        b.add(&m->st, 1);
+        b.add(&m->scan.buf, 2 * kMaxScanJobs * m->scan.job_words);
+        const size_t zero = b.bytes;
+        b.add(&m->tvs, T);
+        b.add(&vt_off, V + 1);
+        b.add(&vt, 4 * T);
+        b.add(&m->vorder, V);
+        b.add(&m->vpos, V);
+        b.add(&m->heavy_off, 4 * T / (kMaxStar + 1) + 1);
+        TRY(take(b.bytes, s, &m->base));
+        b.place(m->base);
+        CK(cudaMemsetAsync(m->base, 0, zero, s));
+    }
     const int32_t *src = tv;
     if (!on_device && T > 0) {
         CK(cudaMemcpyAsync(m->tvs, tv, (size_t)T * 16, cudaMemcpyHostToDevice, s));
         src = reinterpret_cast<const int32_t *>(m->tvs);
     }
-    // the scan workspace of every later scan on the mesh, zeroed once
-    m->scan.job_words = std::max(scan_job_words(std::max(std::max(V, T), (6 * T + 31) / 32)),
-                                 (edge_offsets_words(6 * T) + kMaxScanJobs - 1) / kMaxScanJobs);
-    const size_t ws_bytes = (size_t)2 * kMaxScanJobs * m->scan.job_words * 8;
-    CK(cudaMallocAsync((void **)&m->scan.buf, ws_bytes, s));
-    CK(cudaMemsetAsync(m->scan.buf, 0, ws_bytes, s));
     CK(cudaEventCreateWithFlags(&m->scan.done, cudaEventDisableTiming));
     Temps tmp(s);
-    // the per-vertex cell counts and the first-cell bitmap: one zeroed
-    // allocation
     const int64_t nwk = (4 * T + 31) / 32;
     int32_t *deg_t, *heavy_cnt;
     uint32_t *vflag;
-    {
-        Carve c;
-        const size_t o_d = c.add<int32_t>(V), o_f = c.add<uint32_t>(nwk), o_h = c.add<int32_t>(4);
-        char *z;
-        TRY(tmp.alloc(&z, (int64_t)c.bytes, true));
-        deg_t = (int32_t *)(z + o_d);
-        vflag = (uint32_t *)(z + o_f);
-        heavy_cnt = (int32_t *)(z + o_h);
-    }
     int4 *occ;
-    TRY(tmp.alloc(&occ, T));
+    uint2 *vrank;
+    int64_t *vkey;
+    {
+        // the per-vertex cell counts and the first-cell bitmap are zeroed
+        Plan t;
+        t.add(&deg_t, V);
+        t.add(&vflag, nwk);
+        t.add(&heavy_cnt, 4);
+        const size_t zero = t.bytes;
+        t.add(&occ, T);
+        t.add(&vrank, nwk + 1);
+        t.add(&vkey, V);
+        TRY(tmp.add(t, zero));
+    }
     launch_canon(src, T, V, m->tvs, deg_t, occ, m->st, s);
-    int64_t *vt_off;
-    int32_t *vt;
-    TRY(dalloc(&vt_off, V + 1, s));
     ScanJob job{deg_t, vt_off, V, SCAN_COUNT_I32, nullptr};
     scan_batch(&job, 1, m->scan, m->st, s);
-    TRY(dalloc(&vt, 4 * T, s));
     launch_vt_fill(m->tvs, T, vt_off, occ, vt, s);
     // VT row sort, which also marks each vertex's star-order key; then the
     // star processing order
-    uint2 *vrank;
-    int64_t *vkey;
-    TRY(tmp.alloc(&vrank, nwk + 1));
-    TRY(tmp.alloc(&vkey, V));
-    TRY(dalloc(&m->heavy_off, 4 * T / (kMaxStar + 1) + 1, s));
     launch_vt_sort(vt_off, vt, V, 4 * T, m->tvs, vflag, vkey, heavy_cnt, m->heavy_off, s);
     ScanJob jf{vflag, vrank, nwk, SCAN_POPC_RANK, nullptr};
     scan_batch(&jf, 1, m->scan, m->st, s);
-    TRY(dalloc(&m->vorder, V, s));
-    TRY(dalloc(&m->vpos, V, s));
     launch_vorder_place(vt_off, V, vkey, vrank, nwk, heavy_cnt, m->vorder, m->vpos, s);
     CK(cudaGetLastError());
-    set_csr(m, TG_REL_VT, vt_off, vt, V, 4 * T);
+    set_csr(m, TG_REL_VT, vt_off, vt, V, 4 * T, nullptr, nullptr);
     // vertices with light stars, heavy ones, the heavy stars' entries and
     // the light stars of more than 31 cells
     const void *rd[4] = {&vrank[nwk].y, heavy_cnt, heavy_cnt + 1, heavy_cnt + 2};
@@ -1085,7 +1125,7 @@ tg_status tg_copy_relation_async_i32(tg_mesh *m, int r, int32_t *off_host, int32
                         kName[r], (long long)x.entries);
         int32_t *d = nullptr;
         const size_t b = (size_t)(x.rows + 1) * 4;
-        CK(cudaMallocAsync(&d, b, s));
+        TRY(take(b, s, (void **)&d, true));
         launch_narrow(x.off, d, x.rows + 1, s);
         const cudaError_t e = cudaMemcpyAsync(off_host, d, b, cudaMemcpyDeviceToHost, s);
         cudaFreeAsync(d, s);   // stream-ordered: after the copy
@@ -1121,7 +1161,7 @@ tg_status tg_copy_relations_async_i32(tg_mesh *m, uint32_t mask, int32_t *const 
     }
     int32_t *d = nullptr;
     if (j.n > 0) {
-        CK(cudaMallocAsync(&d, (size_t)j.start[j.n] * 4, s));
+        TRY(take((size_t)j.start[j.n] * 4, s, (void **)&d, true));
         j.dst = d;
         launch_narrow_multi(j, s);
     }
@@ -1159,7 +1199,11 @@ tg_status tg_export_relation_i64(const tg_mesh *m, int r, int64_t *entries_out,
     if (entries_out && x.entries) {
         int64_t *dst = entries_out;
         Temps tmp(s);
-        if (!out_on_device) TRY(tmp.alloc(&dst, x.entries));
+        if (!out_on_device) {
+            Plan t;
+            t.add(&dst, x.entries);
+            TRY(tmp.add(t));
+        }
         launch_widen(x.ent, dst, x.entries, s);
         if (!out_on_device)
             CK(cudaMemcpyAsync(entries_out, dst, (size_t)x.entries * 8, cudaMemcpyDeviceToHost, s));
@@ -1250,15 +1294,17 @@ int64_t tg_mesh_device_bytes(const tg_mesh *m)
 }  // extern "C"
 
 // ---------------------------------------------------------------------------
-// internal: segments (tg_batch.cu)
+// internal: temporaries and segments (tg_batch.cu)
+tg_status tg::take_temp(size_t bytes, cudaStream_t s, void **out) { return take(bytes, s, out, true); }
+
 tg_status tg::mesh_set_segments(tg_mesh *m, const int64_t *seg_c_host, int64_t n, cudaStream_t s)
 {
     if (m->seg_c) cudaFreeAsync(m->seg_c, s);
     if (m->seg_ef) cudaFreeAsync(m->seg_ef, s);
     m->seg_c = m->seg_ef = nullptr;
     m->n_seg = n;
-    TRY(dalloc(&m->seg_c, n + 1, s));
-    TRY(dalloc(&m->seg_ef, 2 * (n + 1), s));
+    TRY(take((size_t)(n + 1) * 8, s, (void **)&m->seg_c));
+    TRY(take((size_t)(n + 1) * 16, s, (void **)&m->seg_ef));
     CK(cudaMemcpyAsync(m->seg_c, seg_c_host, (size_t)(n + 1) * 8, cudaMemcpyHostToDevice, s));
     CK(cudaStreamSynchronize(s));  // the host array may go away
     return TG_OK;

@@ -88,6 +88,12 @@ tg_status bfail(tg_status code, const char *msg)
     return code;
 }
 
+template <class T>
+cudaError_t temp(size_t bytes, cudaStream_t s, T **out)
+{
+    return take_temp(bytes, s, (void **)out) == TG_OK ? cudaSuccess : cudaErrorMemoryAllocation;
+}
+
 #define TRY_B(call)                                                                 \
     do {                                                                            \
         tg_status t_ = (call);                                                      \
@@ -182,12 +188,12 @@ tg_status tg_batch_create(const int32_t *tv, const int64_t *n_cells, const int64
         if (tv_on_device) {
             d_in = const_cast<int4 *>(reinterpret_cast<const int4 *>(tv));
         } else {
-            e = cudaMallocAsync(&d_in, (size_t)T * 16, s);
+            e = temp((size_t)T * 16, s, &d_in);
             if (e == cudaSuccess)
                 e = cudaMemcpyAsync(d_in, tv, (size_t)T * 16, cudaMemcpyHostToDevice, s);
         }
-        if (e == cudaSuccess) e = cudaMallocAsync(&d_tv, (size_t)T * 16, s);
-        if (e == cudaSuccess) e = cudaMallocAsync(&d_seg, (size_t)(n_meshes + 1) * 16, s);
+        if (e == cudaSuccess) e = temp((size_t)T * 16, s, &d_tv);
+        if (e == cudaSuccess) e = temp((size_t)(n_meshes + 1) * 16, s, &d_seg);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(d_seg, b->c0.data(), (size_t)(n_meshes + 1) * 8,
                                 cudaMemcpyHostToDevice, s);
@@ -339,7 +345,7 @@ tg_status tg_batch_copy_relation(tg_batch *b, int64_t i, int r, int64_t *off_hos
     int64_t *d_off = nullptr;
     cudaError_t e = cudaSuccess;
     if (n_ent > 0 && ent_host) {
-        e = cudaMallocAsync(&d_ent, (size_t)n_ent * 4, s);
+        e = temp((size_t)n_ent * 4, s, &d_ent);
         if (e == cudaSuccess) {
             Launch L("k_rebase32", s);
             launch_pdl(k_rebase32, blocks(n_ent), 256, 0, s, ent + e_lo, n_ent, (int)shift, d_ent);
@@ -347,7 +353,7 @@ tg_status tg_batch_copy_relation(tg_batch *b, int64_t i, int r, int64_t *off_hos
         }
     }
     if (e == cudaSuccess && n_off > 0 && off_host) {
-        e = cudaMallocAsync(&d_off, (size_t)n_off * 8, s);
+        e = temp((size_t)n_off * 8, s, &d_off);
         if (e == cudaSuccess) {
             Launch L("k_rebase64", s);
             launch_pdl(k_rebase64, blocks(n_off), 256, 0, s, off + r0, n_off, e_lo, d_off);

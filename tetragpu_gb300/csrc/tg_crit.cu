@@ -274,7 +274,7 @@ k_crit_adj(const int64_t *__restrict__ off, const int *__restrict__ ent, const i
     if (heavy == 2 && s_n > kAdjCap) {  // a row longer than kMaxDeg lies in this window
         if (threadIdx.x == 0) {
             atomicOr(&st->flags, ST_HEAVY_DEG);
-            atomicMin(&st->bad_vertex, s_vlo);
+            note_lowest(&st->bad_vertex, s_vlo);
         }
         return;
     }
@@ -294,7 +294,7 @@ k_crit_adj(const int64_t *__restrict__ off, const int *__restrict__ ent, const i
         if (d > kMaxDeg) {
             if (heavy == 2) {
                 atomicOr(&st->flags, ST_HEAVY_DEG);
-                atomicMin(&st->bad_vertex, i);
+                note_lowest(&st->bad_vertex, i);
             }
             continue;
         }

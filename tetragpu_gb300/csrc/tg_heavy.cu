@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(64) k_heavy(HeavyStars h)
                 }
             if (n_et > 0xffff || n_ef > 0xffff) {
                 atomicOr(&p.st->flags, ST_STAR_OVERFLOW);
-                atomicMin(&p.st->bad_vertex, v);
+                note_lowest(&p.st->bad_vertex, v);
             }
             set_bit(p.eflag, slot);
             const unsigned g = atomicAdd(p.n_rec, 1u);
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(64) k_heavy(HeavyStars h)
             }
             if (cnt > 2) {
                 atomicOr(&p.st->flags, ST_NONMANIFOLD_FACE);
-                atomicMin(&p.st->bad_cell, c);
+                note_lowest(&p.st->bad_cell, c);
             }
         }
     }

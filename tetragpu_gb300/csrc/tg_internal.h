@@ -12,11 +12,11 @@
 namespace tg {
 
 // Device-side status word, written by kernels with atomics, read back by the
-// host at the synchronisation points of tg_extract.
+// host at the synchronisation points of tg_extract.  All zeros: clean.
 struct DevStatus {
     unsigned int flags;
-    int bad_cell;      // lowest offending cell (atomicMin), INT_MAX if none
-    int bad_vertex;    // lowest offending vertex (atomicMin), INT_MAX if none
+    int bad_cell;      // INT_MAX - the lowest offending cell (note_lowest), 0 if none
+    int bad_vertex;    // the same of vertices
     int max_star;      // largest number of cells around a vertex
     int max_deg;       // largest number of neighbours of a vertex
     int pad[3];
@@ -86,6 +86,8 @@ void scan_ws_begin(ScanWorkspace &ws, cudaStream_t s, unsigned long long **cur,
 void scan_ws_end(ScanWorkspace &ws, cudaStream_t s);
 
 #ifdef __CUDACC__
+__device__ __forceinline__ void note_lowest(int *at, int i) { atomicMax(at, 0x7fffffff - i); }
+
 // Single-pass scan step (decoupled look-back, Merrill and Garland), called by
 // one whole warp: publish tile `tile`'s sum in w[tile] (sum << 2 | 1), add
 // the published sums of the tiles before it, 32 at a time (lane i reads the
@@ -140,7 +142,6 @@ struct Sizes {
     int64_t V, T;
 };
 
-void launch_reset_status(DevStatus *st, cudaStream_t s);
 // Status word and up to 8 sizes (int64, or int32 sign-extended) stored by a
 // kernel into device-mapped pinned host memory (no copy engine involved)
 struct PublishArgs {
@@ -344,6 +345,8 @@ void launch_crit_classify(const LinkGraph &g, const void *field, int field_type,
 
 // the message tg_last_error_string returns on this thread
 void set_last_error(const char *msg);
+// a temporary from the library's own pool (freed with cudaFreeAsync)
+tg_status take_temp(size_t bytes, cudaStream_t s, void **out);
 // Cell segments of a mesh (the meshes of a batch, tg_batch.cu): seg_c_host
 // holds n + 1 cell starts; each extraction then fills n + 1 first edge ids
 // followed by n + 1 first face ids (device, read by mesh_segment_ids).

@@ -93,7 +93,7 @@ k_canon(const int32_t *tv, int64_t T, int V, int4 *tvs, int *deg_t, int4 *occ, D
         if ((unsigned)a >= (unsigned)V || (unsigned)b >= (unsigned)V ||
             (unsigned)d >= (unsigned)V || (unsigned)e >= (unsigned)V) {
             atomicOr(&st->flags, ST_BAD_ID);
-            atomicMin(&st->bad_cell, (int)c);
+            note_lowest(&st->bad_cell, (int)c);
             tvs[c] = make_int4(-1, -1, -1, -1);
         } else {
             TG_CSWAP(a, b);
@@ -103,7 +103,7 @@ k_canon(const int32_t *tv, int64_t T, int V, int4 *tvs, int *deg_t, int4 *occ, D
             TG_CSWAP(b, d);
             if (a == b || b == d || d == e) {
                 atomicOr(&st->flags, ST_DUP_VERTEX);
-                atomicMin(&st->bad_cell, (int)c);
+                note_lowest(&st->bad_cell, (int)c);
                 tvs[c] = make_int4(-1, -1, -1, -1);
             } else {
                 tvs[c] = make_int4(a, b, d, e);
@@ -560,16 +560,6 @@ k_pad_rows(const int64_t *__restrict__ off, const int *__restrict__ ent, int64_t
     if (k == 0 && counts) counts[r] = (unsigned)n;
 }
 
-__global__ void k_reset_status(DevStatus *st)
-{
-    griddep_wait();
-    st->flags = 0;
-    st->bad_cell = INT_MAX;
-    st->bad_vertex = INT_MAX;
-    st->max_star = 0;
-    st->max_deg = 0;
-}
-
 inline unsigned blocks_for(int64_t n, int threads)
 {
     return (unsigned)((n + threads - 1) / threads);
@@ -625,8 +615,8 @@ __global__ void k_publish(PublishArgs a)
         a.h_sz[i] = a.wide[i] ? *(const int64_t *)a.src[i] : (int64_t) * (const int32_t *)a.src[i];
     __threadfence_system();
     a.st->flags = 0;
-    a.st->bad_cell = INT_MAX;
-    a.st->bad_vertex = INT_MAX;
+    a.st->bad_cell = 0;
+    a.st->bad_vertex = 0;
     a.st->max_star = 0;
     a.st->max_deg = 0;
 }
@@ -635,12 +625,6 @@ void launch_publish(const PublishArgs &a, cudaStream_t s)
 {
     Launch L("k_publish", s);
     launch_pdl(k_publish, 1, 32, 0, s, a);
-}
-
-void launch_reset_status(DevStatus *st, cudaStream_t s)
-{
-    Launch L("k_reset_status", s);
-    launch_pdl(k_reset_status, 1, 1, 0, s, st);
 }
 
 void launch_canon(const int32_t *tv_in, int64_t T, int64_t V, int4 *tvs, int32_t *deg_t,

@@ -291,7 +291,7 @@ __device__ __forceinline__ void star_vertex(const StarPass &p, RecBuf<H> &S, int
                 }
                 if (here) {
                     atomicOr(&p.st->flags, ST_NONMANIFOLD_FACE);
-                    atomicMin(&p.st->bad_cell, c[h]);
+                    note_lowest(&p.st->bad_cell, c[h]);
                 }
             }
         }
