@@ -474,41 +474,176 @@ k_ee_fill(const int2 *__restrict__ ev, int64_t E, const int64_t *__restrict__ ei
 }
 
 // Vertex-sharing TT: the union of the VT rows of the cell's four vertices,
-// minus the cell itself, by a four-way merge of sorted rows.
+// minus the cell itself, by a four-way merge of sorted rows, a cell to a lane.
+// A merge reads a word or two per entry it writes; out of and into global
+// memory each of them is a cache line of its own for every lane (8,000 of the
+// load / store pipe's cycles a warp, which bounded the pass).  So a warp first
+// copies its cells' rows into shared memory, a row once (a table of the
+// vertices: 32 cells of a grid name some 28), an INT_MAX after each, and the
+// filling pass collects the warp's rows of TT, which are contiguous, there and
+// writes them out as whole lines.  Cells whose rows do not fit (vertices in
+// very many cells) merge in global memory.  On 40^3 cubes, a tenth coned, ids
+// permuted (0.42 M cells, 70 entries each): 145 us for the two passes (400
+// merging in global memory throughout), bounded by the shared-memory merges
+// (load / store pipe 67 % busy counting; filling, four blocks to an SM by what
+// they collect).
+constexpr int kTtWarps = 2;
+constexpr int kTtLists = 1536;    // words of rows a warp keeps
+constexpr int kTtTable = 256;     // twice the vertices 32 cells can name
+constexpr int kTtOut = 2560;      // entries of TT it collects (70 a cell in a grid)
+struct TtStage {
+    int list[kTtLists];
+    int key[kTtTable], off[kTtTable];
+    unsigned char row[kTtTable / 2];   // the table's slots in use
+    int n;
+};
+// the cell's merge in global memory
 template <bool FILL>
-__global__ void __launch_bounds__(256)
+__device__ __noinline__ void tt_merge_global(const int4 w, int c, const int64_t *__restrict__ vt_off,
+                                             const int *__restrict__ vt, int *cnt, int *out)
+{
+    int64_t pos[4], stop[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        pos[k] = vt_off[get4(w, k)];
+        stop[k] = vt_off[get4(w, k) + 1];
+    }
+    int n = 0;
+    while (true) {
+        int m = INT_MAX;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (pos[k] < stop[k]) m = min(m, vt[pos[k]]);
+        if (m == INT_MAX) break;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (pos[k] < stop[k] && vt[pos[k]] == m) pos[k]++;
+        if (m != c) {
+            if (FILL) out[n] = m;
+            n++;
+        }
+    }
+    if (!FILL) *cnt = n;
+}
+
+template <bool FILL>
+__global__ void __launch_bounds__(32 * kTtWarps)
 k_tt_vertex(const int4 *__restrict__ tvs, int64_t T, const int64_t *__restrict__ vt_off,
             const int *__restrict__ vt, int *__restrict__ cnt, const int64_t *__restrict__ tt_off,
             int *__restrict__ tt)
 {
     griddep_wait();
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= T) return;
-    const int4 w = tvs[c];
-    int64_t pos[4], end[4];
+    __shared__ TtStage s_stage[kTtWarps];
+    __shared__ __align__(16) int s_out[FILL ? kTtWarps : 1][FILL ? kTtOut : 4];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int64_t c0 = ((int64_t)blockIdx.x * kTtWarps + wp) * 32;
+    if (c0 >= T) return;   // warp-uniform
+    TtStage &S = s_stage[wp];
+    const int64_t c = c0 + lane;
+    for (int i = lane; i < kTtTable; i += 32) S.key[i] = -1;
+    if (lane == 0) S.n = 0;
+    __syncwarp();
+    int4 w = make_int4(0, 0, 0, 0);
+    int slot[4] = {0, 0, 0, 0};
+    if (c < T) {
+        w = tvs[c];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int v = get4(w, k);
+            unsigned h = ((unsigned)v * 0x9E3779B1u) >> 24;
+            for (int probe = 0; probe < kTtTable; probe++) {   // never full
+                const int old = atomicCAS(&S.key[h], -1, v);
+                if (old == -1) S.row[atomicAdd(&S.n, 1)] = (unsigned char)h;
+                if (old == -1 || old == v) break;
+                h = (h + 1) & (kTtTable - 1);
+            }
+            slot[k] = (int)h;
+        }
+    }
+    int64_t o0 = 0, o = 0;
+    bool fits = true;
+    if (FILL) {
+        o0 = tt_off[c0];
+        o = tt_off[min(c, T)];
+        fits = tt_off[min(c0 + 32, T)] - o0 + 4 <= kTtOut;
+    }
+    __syncwarp();
+    // the rows, a lane each, then eight lanes to each of four to copy them
+    const int rows = S.n;
+    int total = 0;
+    for (int r0 = 0; r0 < rows && fits; r0 += 32) {
+        int64_t src = 0;
+        int len = 0;
+        if (r0 + lane < rows) {
+            const int v = S.key[S.row[r0 + lane]];
+            src = vt_off[v];
+            len = (int)min(vt_off[v + 1] - src, (int64_t)kTtLists);
+        }
+        const int words = r0 + lane < rows ? len + 1 : 0;
+        int end = words;
+#pragma unroll
+        for (int q = 1; q < 32; q <<= 1) {
+            const int y = __shfl_up_sync(kFull, end, q);
+            if (lane >= q) end += y;
+        }
+        const int at = total + end - words;
+        total += __shfl_sync(kFull, end, 31);
+        fits = total <= kTtLists;   // warp-uniform
+        if (!fits) break;
+        if (words) {
+            S.off[S.row[r0 + lane]] = at;
+            S.list[at + len] = INT_MAX;
+        }
+        for (int j = 0; j < min(rows - r0, 32); j += 4) {
+            const int q = j + (lane >> 3);
+            const int64_t r = __shfl_sync(kFull, src, q);
+            const int n = __shfl_sync(kFull, len, q), to = __shfl_sync(kFull, at, q);
+            for (int i = lane & 7; i < n; i += 8) S.list[to + i] = __ldg(vt + r + i);
+        }
+    }
+    if (!fits) {   // warp-uniform
+        if (c < T)
+            tt_merge_global<FILL>(w, (int)c, vt_off, vt, FILL ? nullptr : cnt + c, FILL ? tt + o : nullptr);
+        return;
+    }
+    __syncwarp();
+    int p[4], h[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        const int v = get4(w, k);
-        pos[k] = vt_off[v];
-        end[k] = vt_off[v + 1];
+        p[k] = c < T ? S.off[slot[k]] : 0;
+        h[k] = c < T ? S.list[p[k]] : INT_MAX;
     }
+    const int shift = (int)(o0 & 3);   // word i collected is word i of the line o0 is in
+    int *out = FILL ? s_out[wp] + shift + (int)(o - o0) : nullptr;
     int n = 0;
-    int *out = FILL ? tt + tt_off[c] : nullptr;
     while (true) {
-        int m = INT_MAX;
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-            if (pos[k] < end[k]) m = min(m, vt[pos[k]]);
+        const int m = min(min(h[0], h[1]), min(h[2], h[3]));
         if (m == INT_MAX) break;
 #pragma unroll
         for (int k = 0; k < 4; k++)
-            if (pos[k] < end[k] && vt[pos[k]] == m) pos[k]++;
+            if (h[k] == m) h[k] = S.list[++p[k]];
         if (m != (int)c) {
             if (FILL) out[n] = m;
             n++;
         }
     }
-    if (!FILL) cnt[c] = n;
+    if (!FILL) {
+        if (c < T) cnt[c] = n;
+        return;
+    }
+    __syncwarp();
+    const int stop = __reduce_max_sync(kFull, c < T ? shift + (int)(o - o0) + n : 0);
+    int *line = tt + (o0 - shift);
+    for (int i = 4 * lane; i < stop; i += 128) {
+        const int4 q = *reinterpret_cast<const int4 *>(s_out[wp] + i);
+        if (i >= shift && i + 4 <= stop) {
+            *reinterpret_cast<int4 *>(line + i) = q;
+        } else {
+#pragma unroll
+            for (int t = 0; t < 4; t++)
+                if (i + t >= shift && i + t < stop) line[i + t] = get4(q, t);
+        }
+    }
 }
 
 // int32 -> int64 (the reference's vtkIdType) copy
@@ -685,7 +820,7 @@ void launch_tt_vertex_count(const int4 *tvs, int64_t T, const int64_t *vt_off, c
     if (T == 0) return;
     {
         Launch L("k_tt_vertex", s);
-        launch_pdl(k_tt_vertex<false>, blocks_for(T, 256), 256, 0, s, tvs, T, vt_off, vt, cnt, nullptr, nullptr);
+        launch_pdl(k_tt_vertex<false>, blocks_for(T, 32 * kTtWarps), 32 * kTtWarps, 0, s, tvs, T, vt_off, vt, cnt, nullptr, nullptr);
     }
 }
 
@@ -695,7 +830,7 @@ void launch_tt_vertex_fill(const int4 *tvs, int64_t T, const int64_t *vt_off, co
     if (T == 0) return;
     {
         Launch L("k_tt_vertex", s);
-        launch_pdl(k_tt_vertex<true>, blocks_for(T, 256), 256, 0, s, tvs, T, vt_off, vt, nullptr, tt_off, tt);
+        launch_pdl(k_tt_vertex<true>, blocks_for(T, 32 * kTtWarps), 32 * kTtWarps, 0, s, tvs, T, vt_off, vt, nullptr, tt_off, tt);
     }
 }
 
