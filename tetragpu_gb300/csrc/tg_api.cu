@@ -402,11 +402,14 @@ struct tg_mesh {
     int64_t n_wide = 0;         // light stars of more than 31 cells (64-bit masks)
     int max_deg = 0;            // largest degree above kMaxDeg seen by the extraction, else 0
     bool wide_deg = false;      // a vertex has more than kNarrowDeg neighbours
-    // the link adjacency of critical points (LinkGraph; adj null: not built)
-    BlockRef lg;
+    // VV by position (LinkGraph; off null: not built) and the link adjacency of
+    // critical points on it (adj null: not built)
+    BlockRef lg_rows, lg_masks;
     int64_t *lg_off = nullptr;
     int32_t *lg_ent = nullptr;
     void *lg_adj = nullptr;
+    std::mutex lg_mu;                // while a call looks for them or builds them
+    cudaEvent_t lg_done = nullptr;   // after the build of either outside an extraction
     DevStatus *st = nullptr;    // device
     DevStatus *st_host = nullptr;
     int64_t *sz_host = nullptr; // pinned slots for sizes read back at sync points
@@ -501,7 +504,8 @@ void set_csr(tg_mesh *m, int r, int64_t *off, int32_t *ent, int64_t rows, int64_
 
 void free_link_graph(tg_mesh *m)
 {
-    m->lg.reset();
+    m->lg_rows.reset();
+    m->lg_masks.reset();
     m->lg_off = nullptr;
     m->lg_ent = nullptr;
     m->lg_adj = nullptr;
@@ -515,36 +519,68 @@ LinkGraph link_graph(const tg_mesh *m, int64_t nvv)
     return {m->V, link_entries(m, nvv), m->lg_off, m->lg_ent, m->vorder, m->vpos, m->lg_adj, m->wide_deg};
 }
 
+// A call may use on one stream what an earlier call built on another.  (Under
+// capture work outside of it cannot be waited for: the caller has then.)
+tg_status link_built(tg_mesh *m, cudaStream_t s)
+{
+    if (!m->lg_done) CK(cudaEventCreateWithFlags(&m->lg_done, cudaEventDisableTiming));
+    CK(cudaEventRecord(m->lg_done, s));
+    return TG_OK;
+}
+
+tg_status link_wait(const tg_mesh *m, cudaStream_t s)
+{
+    if (m->lg_done && !capturing(s)) CK(cudaStreamWaitEvent(s, m->lg_done, 0));
+    return TG_OK;
+}
+
 // The link adjacency of critical points: VV renumbered into the star
-// processing order and its masks, kept on the mesh.  alloc makes every buffer,
-// the temporaries too, on the extraction's own stream (before a fork, so that
-// a side stream may use them); build launches.
+// processing order (what of it is missing) and its masks (unless only the rows
+// are wanted), kept on the mesh.  alloc makes every buffer, the temporaries
+// too, on the extraction's own stream (before a fork, so that a side stream may
+// use them); build launches.
 struct LinkBuild {
-    int32_t *len, *win;
-    tg_status alloc(tg_mesh *m, int64_t nvv, Temps &tmp, cudaStream_t s)
+    int32_t *len = nullptr, *win = nullptr;
+    bool rows = false, masks = false;
+    tg_status alloc(tg_mesh *m, int64_t nvv, bool with_masks, Temps &tmp, cudaStream_t s)
     {
         const int64_t n = link_entries(m, nvv);
-        Plan t, g;
-        t.add(&len, m->V);
-        t.add(&win, window_count(n, crit_window()) + 1);
+        rows = !m->lg_off;
+        masks = with_masks && !m->lg_adj;
+        Plan t, r, k;
+        if (rows) {
+            t.add(&len, m->V);
+            r.add(&m->lg_off, m->V + 1);
+            r.add(&m->lg_ent, n);
+        }
+        char *adj = nullptr;
+        if (masks) {
+            t.add(&win, window_count(n, crit_window()) + 1);
+            k.add(&adj, n * (m->wide_deg ? 8 : 4));
+        }
         TRY(tmp.add(t));
-        char *adj;
-        g.add(&m->lg_off, m->V + 1);
-        g.add(&m->lg_ent, n);
-        g.add(&adj, n * (m->wide_deg ? 8 : 4));
-        TRY(take_block(g, m, s, &m->lg));
-        m->lg_adj = adj;
+        BlockRef held;
+        TRY(take_block(k, m, s, &held));
+        TRY(take_block(r, m, s, &m->lg_rows));   // the last that can fail
+        if (masks) {
+            m->lg_masks = held;
+            m->lg_adj = adj;
+        }
         return TG_OK;
     }
     void build(tg_mesh *m, const int64_t *vv_off, const int32_t *vv, int64_t nvv, cudaStream_t s)
     {
         const LinkGraph g = link_graph(m, nvv);
-        launch_vv_lengths_in_order(vv_off, m->vorder, m->V, len, s);
-        ScanJob job{len, m->lg_off, m->V, SCAN_COUNT_PAD8, nullptr};
-        scan_batch(&job, 1, m->scan, m->st, s);
-        launch_window_starts(m->lg_off, m->V, g.n_ent, crit_window(), win, s);
-        launch_rows_in_order(vv_off, vv, m->vorder, m->vpos, m->V, m->lg_off, m->lg_ent, s);
-        launch_crit_adj(g, win, m->st, m->max_deg ? 1 : 0, s);
+        if (rows) {
+            launch_vv_lengths_in_order(vv_off, m->vorder, m->V, len, s);
+            ScanJob job{len, m->lg_off, m->V, SCAN_COUNT_PAD8, nullptr};
+            scan_batch(&job, 1, m->scan, m->st, s);
+            launch_rows_in_order(vv_off, vv, m->vorder, m->vpos, m->V, m->lg_off, m->lg_ent, s);
+        }
+        if (masks) {
+            launch_window_starts(m->lg_off, m->V, g.n_ent, crit_window(), win, s);
+            launch_crit_adj(g, win, m->st, m->max_deg ? 1 : 0, s);
+        }
     }
 };
 
@@ -737,7 +773,7 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         // beside EE (each reads only what the passes before it wrote)
         const bool prep_adj = (opts & TG_OPT_LINK_ADJACENCY) && (mask & TG_VV);
         LinkBuild lb;
-        if (prep_adj) TRY(lb.alloc(m, nvv, tmp, s));
+        if (prep_adj) TRY(lb.alloc(m, nvv, true, tmp, s));
         if (te || fe || tt || ff_off || ff || et || ef || prep_adj) {
             const cudaStream_t s2 = side.fork();
             ep.te = te; ep.et_off = et_off; ep.ef_off = ef_off; ep.et = et; ep.ef = ef; ep.tf = tf;
@@ -805,15 +841,20 @@ tg_status tg::critical_points_rows(tg_mesh *m, int64_t v0, int64_t nv, const voi
     m->last_stream = s;
     if (!m->rel[TG_REL_VV].ready) TRY(tg_extract(m, TG_VV, 0, s));
     const Rel &vv = m->rel[TG_REL_VV];
+    std::unique_lock<std::mutex> lk(m->lg_mu);
     if (!m->lg_adj) {
         // VV rows longer than the adjacency masks take the heavy path of the
         // classification, so no status read-back here
-        free_link_graph(m);
         Temps adj_tmp(s);
         LinkBuild lb;
-        TRY(lb.alloc(m, vv.entries, adj_tmp, s));
+        TRY(link_wait(m, s));
+        TRY(lb.alloc(m, vv.entries, true, adj_tmp, s));
         lb.build(m, vv.off, vv.ent, vv.entries, s);
+        if (!capturing(s)) TRY(link_built(m, s));
+    } else {
+        TRY(link_wait(m, s));
     }
+    lk.unlock();
     Temps tmp(s);
     const size_t esz = field_type == TG_FIELD_F64 ? 8 : 4;
     const void *f = field;
@@ -898,6 +939,7 @@ tg_status tg_mesh_destroy(tg_mesh *m)
     }
     cudaStreamSynchronize(s);  // no copy into the pinned slots is still in flight
     if (m->scan.done) cudaEventDestroy(m->scan.done);
+    if (m->lg_done) cudaEventDestroy(m->lg_done);
     g_pinned.put(m->st_host);
     g_pinned.put(m->sz_host);
     cudaSetDevice(cur);
@@ -1286,14 +1328,41 @@ int64_t tg_mesh_device_bytes(const tg_mesh *m)
         if (x.off) b += (x.rows + 1) * 8;
     }
     b += m->V * 8;
-    if (m->lg_adj)
-        b += link_entries(m, m->rel[TG_REL_VV].entries) * (m->wide_deg ? 12 : 8) + (m->V + 1) * 8;
+    const int64_t n = link_entries(m, m->rel[TG_REL_VV].entries);
+    if (m->lg_off) b += n * 4 + (m->V + 1) * 8;
+    if (m->lg_adj) b += n * (m->wide_deg ? 8 : 4);
     return b;
 }
 
 }  // extern "C"
 
 // ---------------------------------------------------------------------------
+// internal: VV by position (tg_consumers.cu)
+bool tg::capturing(cudaStream_t s)
+{
+    cudaStreamCaptureStatus c;
+    if (cudaStreamIsCapturing(s, &c) == cudaSuccess) return c != cudaStreamCaptureStatusNone;
+    (void)cudaGetLastError();   // the legacy stream, while another is capturing
+    return true;
+}
+
+tg_status tg::link_rows(tg_mesh *m, bool build, cudaStream_t s, LinkGraph *out)
+{
+    const Rel &vv = m->rel[TG_REL_VV];
+    std::lock_guard<std::mutex> lk(m->lg_mu);
+    if (m->lg_off) {
+        TRY(link_wait(m, s));
+    } else if (build) {
+        Temps tmp(s);
+        LinkBuild lb;
+        TRY(lb.alloc(m, vv.entries, false, tmp, s));
+        lb.build(m, vv.off, vv.ent, vv.entries, s);
+        TRY(link_built(m, s));
+    }
+    *out = link_graph(m, vv.entries);
+    return TG_OK;
+}
+
 // internal: temporaries and segments (tg_batch.cu)
 tg_status tg::take_temp(size_t bytes, cudaStream_t s, void **out) { return take(bytes, s, out, true); }
 

@@ -581,6 +581,15 @@ void classify(const LinkGraph &g, const F *field, F *ordered, int64_t v0, int64_
 }
 }  // namespace
 
+void launch_field_in_order(const float *field, const int32_t *order, int64_t V, float *out,
+                           cudaStream_t s)
+{
+    if (V == 0) return;
+    Launch L("k_field_in_order", s);
+    launch_pdl(k_field_in_order<float>, (unsigned)((V + 255) / 256), 256, 0, s, field, order, nullptr,
+               (int64_t)0, V, out);
+}
+
 bool classify_orders_field(int64_t nv) { return nv >= kOrderField; }
 
 void launch_crit_classify(const LinkGraph &g, const void *field, int field_type, void *ordered,

@@ -345,6 +345,14 @@ void launch_crit_classify(const LinkGraph &g, const void *field, int field_type,
 
 // the message tg_last_error_string returns on this thread
 void set_last_error(const char *msg);
+// the mesh's VV by position (off null when it has none yet and build is not
+// set), VV being extracted
+tg_status link_rows(tg_mesh *m, bool build, cudaStream_t s, LinkGraph *out);
+// work on the stream is being recorded, not run
+bool capturing(cudaStream_t s);
+// field values of every vertex by position
+void launch_field_in_order(const float *field, const int32_t *order, int64_t V, float *out,
+                           cudaStream_t s);
 // a temporary from the library's own pool (freed with cudaFreeAsync)
 tg_status take_temp(size_t bytes, cudaStream_t s, void **out);
 // Cell segments of a mesh (the meshes of a batch, tg_batch.cu): seg_c_host
