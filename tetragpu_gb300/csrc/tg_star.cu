@@ -809,7 +809,12 @@ k_inc_sort(const int64_t *__restrict__ off, int64_t V, const int2 *__restrict__ 
 // ET / EF / EE offsets: exclusive sums of the row lengths in edge-id order, in
 // one pass (a block takes the next tile in start order, sums it, adds the
 // tiles before it by look-back, and writes its offsets).  EV of the tile's
-// edges beside it.
+// edges beside it, while the look-back waits.  Two neighbouring edges to a lane
+// (one 32-byte record load, 16-byte stores), rows of 64 to a warp, so that a
+// request carries whole lines; ET and EF lengths are summed in the halves of
+// one word.  172 us at 128^3 cubes (208 with eight consecutive edges to a
+// thread, whose 128 bytes were lines of their own); its 0.9 GB take 135 at the
+// copy rate.
 constexpr int kEdgeThreads = 256;
 constexpr int kEdgeItems = TG_EDGE_ITEMS;             // edges per thread
 constexpr int kEdgeTile = kEdgeItems * kEdgeThreads;  // edges per tile
@@ -827,64 +832,16 @@ struct EdgeOffsets {
     int2 *ev;
 };
 
-template <int NT>
-__device__ __forceinline__ void block_scan3(long long x[3], long long excl[3], long long tot[3])
-{
-    static_assert(NT % 32 == 0 && NT <= 1024, "block of whole warps");
-    __shared__ long long sm[3][NT / 32 + 1];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-        long long incl = x[q];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const long long y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        if (lane == 31) sm[q][warp] = incl;
-        excl[q] = incl - x[q];
-    }
-    __syncthreads();
-    if (warp == 0) {
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-            const long long w = lane < NT / 32 ? sm[q][lane] : 0;
-            long long wi = w;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const long long y = __shfl_up_sync(0xffffffffu, wi, o);
-                if (lane >= o) wi += y;
-            }
-            if (lane < NT / 32) sm[q][lane] = wi - w;
-            if (lane == NT / 32 - 1) sm[q][NT / 32] = wi;
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-        excl[q] += sm[q][warp];
-        tot[q] = sm[q][NT / 32];
-    }
-    __syncthreads();
-}
-
-// len(k): the length of the thread's k-th row
-template <typename Fn>
-__device__ __forceinline__ void store_offsets(int64_t *out, int64_t k0, int64_t E, long long run, Fn len)
+// two offsets, 16 bytes (k is even)
+__device__ __forceinline__ void store_offsets(int64_t *out, int64_t k, int64_t E, long long first,
+                                              unsigned len)
 {
     if (!out) return;
-#pragma unroll
-    for (int k = 0; k < kEdgeItems; k += 2) {
-        const long long next = run + len(k);
-        if (k0 + k + 1 < E)   // two offsets, 16 bytes (k0 is even)
-            *reinterpret_cast<longlong2 *>(out + k0 + k) = make_longlong2(run, next);
-        else if (k0 + k < E)
-            out[k0 + k] = run;
-        run = next + len(k + 1);
-    }
+    if (k + 1 < E) *reinterpret_cast<longlong2 *>(out + k) = make_longlong2(first, first + len);
+    else if (k < E) out[k] = first;
 }
 
-__global__ void __launch_bounds__(kEdgeThreads) k_edge_offsets(EdgeOffsets p)
+__global__ void __launch_bounds__(kEdgeThreads, 6) k_edge_offsets(EdgeOffsets p)
 {
     griddep_wait();
     {
@@ -906,42 +863,103 @@ __global__ void __launch_bounds__(kEdgeThreads) k_edge_offsets(EdgeOffsets p)
         return;
     }
     if (tile >= p.n_tiles) return;
-    const int64_t k0 = tile * kEdgeTile + (int64_t)threadIdx.x * kEdgeItems;
-    uint2 len[kEdgeItems];   // {ET | EF << 16, EE}
-    long long x[3] = {0, 0, 0};
+    // rows of 64 edges a warp, two to a lane: records, offsets and EV move as
+    // whole lines
+    constexpr int kRows = kEdgeItems / 2, kWarps = kEdgeThreads / 32;
+    __shared__ unsigned long long s_tef[kWarps];
+    __shared__ long long s_ee[kWarps];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int64_t k0 = tile * kEdgeTile + wp * (32 * kEdgeItems) + 2 * lane;
+    unsigned slot[kRows][2], x[kRows], ex[kRows];   // x, ex: lengths of the first of the two
+    unsigned long long tef[kRows], run_tef = 0;   // sums of ET (low half) and EF lengths: below 2^27 each
+    long long ee[kRows], run_ee = 0;
 #pragma unroll
-    for (int k = 0; k < kEdgeItems; k++) {
-        len[k] = k0 + k < p.E ? __ldg(reinterpret_cast<const uint2 *>(p.edge + k0 + k) + 1)
-                              : make_uint2(0u, 0u);
-        x[0] += len[k].x & 0xffffu;
-        x[1] += len[k].x >> 16;
-        x[2] += len[k].y;
+    for (int r = 0; r < kRows; r++) {
+        const int64_t k = k0 + 64 * r;
+        unsigned w[8] = {};
+        if (k + 1 < p.E) {
+            load8(reinterpret_cast<const unsigned *>(p.edge + k), w);
+        } else if (k < p.E) {
+            const uint4 q = __ldg(p.edge + k);
+            w[0] = q.x;
+            w[2] = q.z;
+            w[3] = q.w;
+        }
+        slot[r][0] = w[0];
+        slot[r][1] = w[4];
+        x[r] = w[2];
+        ex[r] = w[3];
+        tef[r] = (unsigned long long)((w[2] & 0xffffu) + (w[6] & 0xffffu)) |
+                 (unsigned long long)((w[2] >> 16) + (w[6] >> 16)) << 32;
+        ee[r] = (long long)w[3] + w[7];
+        const unsigned long long a0 = tef[r];
+        const long long b0 = ee[r];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long a = __shfl_up_sync(0xffffffffu, tef[r], o);
+            const long long b = __shfl_up_sync(0xffffffffu, ee[r], o);
+            if (lane >= o) {
+                tef[r] += a;
+                ee[r] += b;
+            }
+        }
+        const unsigned long long a = __shfl_sync(0xffffffffu, tef[r], 31);
+        const long long b = __shfl_sync(0xffffffffu, ee[r], 31);
+        tef[r] += run_tef - a0;
+        ee[r] += run_ee - b0;
+        run_tef += a;
+        run_ee += b;
     }
-    long long excl[3], tot[3];
-    block_scan3<kEdgeThreads>(x, excl, tot);
-    if (threadIdx.x < 96) {   // one look-back per sum, warps 0-2 at once
-        const int q = threadIdx.x >> 5;
-        const long long t = q == 0 ? tot[0] : (q == 1 ? tot[1] : tot[2]);
-        const long long pre = look_back(p.tiles + q * p.n_tiles, tile, t, p.err);
-        if ((threadIdx.x & 31) == 0) s_pre[q] = pre;
+    if (lane == 0) {
+        s_tef[wp] = run_tef;
+        s_ee[wp] = run_ee;
     }
     __syncthreads();
-    store_offsets(p.et_off, k0, p.E, s_pre[0] + excl[0], [&](int k) { return len[k].x & 0xffffu; });
-    store_offsets(p.ef_off, k0, p.E, s_pre[1] + excl[1], [&](int k) { return len[k].x >> 16; });
-    store_offsets(p.ee_off, k0, p.E, s_pre[2] + excl[2], [&](int k) { return len[k].y; });
-    if (tile == p.n_tiles - 1 && threadIdx.x == 0) {
-        if (p.et_off) p.et_off[p.E] = s_pre[0] + tot[0];
-        if (p.ef_off) p.ef_off[p.E] = s_pre[1] + tot[1];
-        if (p.ee_off) p.ee_off[p.E] = s_pre[2] + tot[2];
-    }
-    if (!p.ev) return;
-#pragma unroll 4
-    for (int k = 0; k < kEdgeItems; k++) {
-        const int64_t id = tile * kEdgeTile + k * kEdgeThreads + threadIdx.x;
-        if (id < p.E) {
-            const EdgeEnds e = edge_ends(p.tvs, __ldg(reinterpret_cast<const unsigned *>(p.edge + id)));
-            p.ev[id] = make_int2(e.v, e.u);
+    unsigned long long pre_tef = 0, tot_tef = 0;
+    long long pre_ee = 0, tot_ee = 0;
+#pragma unroll
+    for (int i = 0; i < kWarps; i++) {
+        if (i == wp) {
+            pre_tef = tot_tef;
+            pre_ee = tot_ee;
         }
+        tot_tef += s_tef[i];
+        tot_ee += s_ee[i];
+    }
+    if (wp < 3) {   // one look-back per sum, warps 0-2 at once
+        const long long t = wp == 0 ? (long long)(tot_tef & 0xffffffffu)
+                                    : (wp == 1 ? (long long)(tot_tef >> 32) : tot_ee);
+        const long long pre = look_back(p.tiles + wp * p.n_tiles, tile, t, p.err);
+        if (lane == 0) s_pre[wp] = pre;
+    }
+    if (p.ev) {   // while they look
+#pragma unroll
+        for (int r = 0; r < kRows; r++) {
+            const int64_t k = k0 + 64 * r;
+            if (k >= p.E) continue;
+            const EdgeEnds e = edge_ends(p.tvs, slot[r][0]);
+            if (k + 1 < p.E) {
+                const EdgeEnds f = edge_ends(p.tvs, slot[r][1]);
+                *reinterpret_cast<int4 *>(p.ev + k) = make_int4(e.v, e.u, f.v, f.u);
+            } else {
+                p.ev[k] = make_int2(e.v, e.u);
+            }
+        }
+    }
+    __syncthreads();
+    const long long et0 = s_pre[0] + (long long)(pre_tef & 0xffffffffu);
+    const long long ef0 = s_pre[1] + (long long)(pre_tef >> 32), ee0 = s_pre[2] + pre_ee;
+#pragma unroll
+    for (int r = 0; r < kRows; r++) {
+        const int64_t k = k0 + 64 * r;
+        store_offsets(p.et_off, k, p.E, et0 + (long long)(tef[r] & 0xffffffffu), x[r] & 0xffffu);
+        store_offsets(p.ef_off, k, p.E, ef0 + (long long)(tef[r] >> 32), x[r] >> 16);
+        store_offsets(p.ee_off, k, p.E, ee0 + ee[r], ex[r]);
+    }
+    if (tile == p.n_tiles - 1 && threadIdx.x == 0) {
+        if (p.et_off) p.et_off[p.E] = s_pre[0] + (long long)(tot_tef & 0xffffffffu);
+        if (p.ef_off) p.ef_off[p.E] = s_pre[1] + (long long)(tot_tef >> 32);
+        if (p.ee_off) p.ee_off[p.E] = s_pre[2] + tot_ee;
     }
 }
 

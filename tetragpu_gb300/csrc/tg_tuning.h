@@ -24,7 +24,7 @@
 #define TG_VTS_THREADS 128   // threads per VT-sort block
 #endif
 #ifndef TG_EDGE_ITEMS
-#define TG_EDGE_ITEMS 8   // edges per thread of the edge-offset pass
+#define TG_EDGE_ITEMS 4   // edges per thread of the edge-offset pass
 #endif
 #ifndef TG_ADJ_WIN
 #define TG_ADJ_WIN 256   // VV entries per window of the link adjacency

@@ -48,7 +48,7 @@ CANDIDATES = [
     ("adj_threads_256", {"TG_ADJ_THREADS": 256}),
     ("vt_sort_threads_64", {"TG_VTS_THREADS": 64}),
     ("vt_sort_threads_256", {"TG_VTS_THREADS": 256}),
-    ("edge_items_16", {"TG_EDGE_ITEMS": 16}),
+    ("edge_items_8", {"TG_EDGE_ITEMS": 8}),
 ]
 # tet-count buckets of the batch's meshes: [lo, hi)
 BUCKETS = [(2000, 20000), (20000, 100000), (100000, 400001)]
