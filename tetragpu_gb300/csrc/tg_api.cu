@@ -985,7 +985,7 @@ static tg_status mesh_create_impl(const int32_t *tv, int64_t T, int64_t V, int o
     const int64_t nwk = (4 * T + 31) / 32;
     int32_t *deg_t, *heavy_cnt;
     uint32_t *vflag;
-    int4 *occ;
+    VtOrder vo{};
     uint2 *vrank;
     int64_t *vkey;
     {
@@ -995,15 +995,17 @@ static tg_status mesh_create_impl(const int32_t *tv, int64_t T, int64_t V, int o
         t.add(&vflag, nwk);
         t.add(&heavy_cnt, 4);
         const size_t zero = t.bytes;
-        t.add(&occ, T);
+        t.add(&vo.place, T);
+        t.add(&vo.head, canon_tiles(T));
+        t.add(&vo.verts, canon_tiles(T) * canon_pairs());
         t.add(&vrank, nwk + 1);
         t.add(&vkey, V);
         TRY(tmp.add(t, zero));
     }
-    launch_canon(src, T, V, m->tvs, deg_t, occ, m->st, s);
+    launch_canon(src, T, V, m->tvs, deg_t, vo, m->st, s);
     ScanJob job{deg_t, vt_off, V, SCAN_COUNT_I32, nullptr};
     scan_batch(&job, 1, m->scan, m->st, s);
-    launch_vt_fill(m->tvs, T, vt_off, occ, vt, s);
+    launch_vt_fill(T, vt_off, vo, vt, s);
     // VT row sort, which also marks each vertex's star-order key; then the
     // star processing order
     launch_vt_sort(vt_off, vt, V, 4 * T, m->tvs, vflag, vkey, heavy_cnt, m->heavy_off, s);

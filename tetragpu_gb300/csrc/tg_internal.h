@@ -165,12 +165,19 @@ struct NarrowJobs {
 void launch_narrow_multi(const NarrowJobs &j, cudaStream_t s);
 void launch_pad_rows(const int64_t *off, const int32_t *ent, int64_t rows, int width,
                      int64_t *out, uint32_t *counts, cudaStream_t s);
-// sort each TV row, validate ids, count cells per vertex; occ[c] = the
-// cell's place in each of its vertices' (unsorted) VT rows
+// What k_canon leaves of the (cell, vertex) pairs of each 32 cells for
+// k_vt_fill: their order by vertex
+struct VtOrder {
+    uint32_t *place;   // [T] the cell's four places in it, 8 bits each (all ones: rejected)
+    uint4 *head;       // [tiles] a bit per place that begins a vertex
+    int2 *verts;       // [tiles x canon_pairs] {vertex, place in its VT row less its place here}
+};
+int64_t canon_tiles(int64_t T);
+int64_t canon_pairs();
+// sort each TV row, validate ids, count cells per vertex
 void launch_canon(const int32_t *tv_in, int64_t T, int64_t V, int4 *tvs, int32_t *deg_t,
-                  int4 *occ, DevStatus *st, cudaStream_t s);
-void launch_vt_fill(const int4 *tvs, int64_t T, const int64_t *vt_off, const int4 *occ,
-                    int32_t *vt, cudaStream_t s);
+                  const VtOrder &vo, DevStatus *st, cudaStream_t s);
+void launch_vt_fill(int64_t T, const int64_t *vt_off, const VtOrder &vo, int32_t *vt, cudaStream_t s);
 // Windows of win_size entries over a CSR: win[w] = first row starting at or
 // after entry win_size * w (w = 0 .. window_count), win[window_count] = rows.
 int64_t window_count(int64_t n_entries, int win_size);

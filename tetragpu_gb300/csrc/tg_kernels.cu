@@ -58,26 +58,40 @@ __device__ __forceinline__ void cswap(int &x, int &y)
 // ---------------------------------------------------------------------------
 // k_canon
 // ---------------------------------------------------------------------------
-// A block's 1024 (cell, slot) pairs name far fewer distinct vertices on
-// meshes whose cells come in spatial order (a run of cubes shares its
-// corners): the block counts them in a shared-memory hash (vertex -> count;
-// each pair's place is its local rank there) and makes one global atomic per
-// distinct vertex, whose return value is the block's base in that vertex's
-// VT row.
-constexpr int kCanonHash = 2048;   // twice the block's pairs: never full
+// A warp's 128 (cell, slot) pairs name far fewer distinct vertices on meshes
+// whose cells come in spatial order (a run of cubes shares its corners): some
+// 26.  The pairs of a vertex agree on one of them (each writes its number where
+// the vertex hashes to and reads back whose stayed; a vertex that finds another
+// there tries again elsewhere), count themselves at it, and that one makes one
+// global atomic, whose return value is the warp's base in the vertex's VT row.
+// The warp leaves its pairs' order by vertex: a pair's place in it, a bit per
+// place that begins a vertex, and each vertex with its base less that place, so
+// that k_vt_fill writes a vertex's cells of the warp together.  210 us at 128^3 cubes,
+// vertex ids permuted (318 with a table of the block's 1024 pairs and barriers:
+// a compare-and-swap and an add a pair, of which lanes naming the same vertex
+// wait for each other); bound by the shared-memory pipe (83 %).  Whole warps
+// that agree by match instructions first took as long as the table.
+constexpr int kCanonThreads = 256, kCanonWarps = kCanonThreads / 32;
+constexpr int kCanonPairs = 128;   // of a warp
+constexpr int kCanonTable = 512;
+struct CanonStage {
+    int key[kCanonPairs];                // pair 32 k + lane: slot k of the lane's cell
+    int cnt[kCanonPairs];                // at the pair that stands for a vertex
+    unsigned char table[kCanonTable];
+    unsigned char pair[kCanonPairs];     // of each vertex, and its first place
+    unsigned char start[kCanonPairs + 4];
+};
 
-__global__ void __launch_bounds__(256)
-k_canon(const int32_t *tv, int64_t T, int V, int4 *tvs, int *deg_t, int4 *occ, DevStatus *st,
+__global__ void __launch_bounds__(kCanonThreads, 6)
+k_canon(const int32_t *tv, int64_t T, int V, int4 *tvs, int *deg_t, VtOrder vo, DevStatus *st,
         int aligned)
 {
     griddep_wait();
-    __shared__ int hkey[kCanonHash], hcnt[kCanonHash];
-    for (int i = threadIdx.x; i < kCanonHash; i += blockDim.x) {
-        hkey[i] = -1;
-        hcnt[i] = 0;
-    }
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    int q[4];
+    __shared__ CanonStage s_stage[kCanonWarps];
+    const int lane = threadIdx.x & 31;
+    CanonStage &S = s_stage[threadIdx.x >> 5];
+    const int64_t c = (int64_t)blockIdx.x * kCanonThreads + threadIdx.x;
+    int q[4] = {-1, -1, -1, -1};
     bool ok = false;
     if (c < T) {
         int a, b, d, e;
@@ -112,55 +126,136 @@ k_canon(const int32_t *tv, int64_t T, int V, int4 *tvs, int *deg_t, int4 *occ, D
             }
         }
     }
-    __syncthreads();
-    int hs[4], rk[4];
-    if (ok) {
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        S.key[32 * k + lane] = q[k];
+        S.cnt[32 * k + lane] = 0;
+    }
+    // rep[k]: the pair that stands for the vertex (a rejected cell's -1s are one
+    // more).  A vertex's pairs look in the same place each time, and one vertex
+    // at each place looked at stays: at most kCanonPairs rounds
+    int rep[4];
+    bool todo[4] = {true, true, true, true};
+    unsigned mul = 0x9E3779B1u;
+    for (int round = 0; round < kCanonPairs; round++, mul += 0x85EBCA6Eu) {
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (todo[k]) S.table[((unsigned)q[k] * mul) >> 23] = (unsigned char)(32 * k + lane);
+        __syncwarp();
+        int r[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) r[k] = S.table[((unsigned)q[k] * mul) >> 23] & (kCanonPairs - 1);
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            unsigned h = ((unsigned)q[k] * 0x9E3779B1u) >> 21;   // 11 bits
-            hs[k] = 0;
-            rk[k] = 0;
-            for (int probe = 0; probe < kCanonHash; probe++) {
-                const int old = atomicCAS(&hkey[h], -1, q[k]);
-                if (old == -1 || old == q[k]) {
-                    hs[k] = (int)h;
-                    rk[k] = atomicAdd(&hcnt[h], 1);
-                    break;
-                }
-                h = (h + 1) & (kCanonHash - 1);
-            }
+            const bool found = S.key[r[k]] == q[k];
+            rep[k] = todo[k] ? r[k] : rep[k];
+            todo[k] = todo[k] && !found;
         }
+        if (!__any_sync(kFull, todo[0] || todo[1] || todo[2] || todo[3])) break;
     }
-    __syncthreads();
-    // the count so far is the block's place in each vertex's VT row (rows
-    // are sorted afterwards)
-    for (int i = threadIdx.x; i < kCanonHash; i += blockDim.x) {
-        const int n = hcnt[i];
-        if (n) hcnt[i] = atomicAdd(deg_t + hkey[i], n);
+    int rk[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) rk[k] = atomicAdd(&S.cnt[rep[k]], 1);
+    __syncwarp();
+    // the places of this lane's vertices: vertices and pairs of the lanes
+    // before it, in the halves of a word
+    int n[4];
+    unsigned own = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int m = S.cnt[32 * k + lane];
+        n[k] = ok && rep[k] == 32 * k + lane ? m : 0;
+        own += n[k] ? (unsigned)n[k] << 16 | 1u : 0u;
     }
-    __syncthreads();
-    if (ok)
-        occ[c] = make_int4(hcnt[hs[0]] + rk[0], hcnt[hs[1]] + rk[1], hcnt[hs[2]] + rk[2],
-                           hcnt[hs[3]] + rk[3]);
+    unsigned at = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(kFull, at, o);
+        if (lane >= o) at += y;
+    }
+    const unsigned all = __shfl_sync(kFull, at, 31);
+    at -= own;
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (n[k]) {
+            S.pair[at & 0xffffu] = (unsigned char)(32 * k + lane);
+            S.start[at & 0xffffu] = (unsigned char)(at >> 16);
+            S.cnt[32 * k + lane] = (int)(at >> 16);
+            at += (unsigned)n[k] << 16 | 1u;
+        }
+    const int verts = (int)(all & 0xffffu);
+    if (lane == 0) S.start[verts] = (unsigned char)(all >> 16);
+    __syncwarp();
+    // the count so far of cells at a vertex is the warp's base in its VT row
+    // (rows are sorted afterwards)
+    const int64_t tile = c >> 5;
+    unsigned head[4] = {0, 0, 0, 0};
+    for (int i = lane; i < verts; i += 32) {
+        const int v = S.key[S.pair[i]], place = S.start[i];
+        vo.verts[tile * kCanonPairs + i] =
+            make_int2(v, atomicAdd(deg_t + v, S.start[i + 1] - place) - place);
+        const unsigned bit = 1u << (place & 31);
+#pragma unroll
+        for (int w = 0; w < 4; w++) head[w] |= place >> 5 == w ? bit : 0u;
+    }
+#pragma unroll
+    for (int w = 0; w < 4; w++) head[w] = __reduce_or_sync(kFull, head[w]);
+    if (c >= T) return;
+    if (lane == 0) vo.head[tile] = make_uint4(head[0], head[1], head[2], head[3]);
+    unsigned place = ~0u;   // rejected
+    if (ok) {
+        place = 0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) place |= (unsigned)(S.cnt[rep[k]] + rk[k]) << (8 * k);
+    }
+    vo.place[c] = place;
 }
 
 // ---------------------------------------------------------------------------
 // k_vt_fill
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
-k_vt_fill(const int4 *__restrict__ tvs, int64_t T, const int64_t *__restrict__ vt_off,
-          const int4 *__restrict__ occ, int *__restrict__ vt)
+// The cells of a k_canon warp to their vertices' VT rows, in the warp's order
+// by vertex: 32 words are some ten runs, not 32 words of their own.  229 us at 128^3 cubes,
+// vertex ids permuted (275 with a store and an offset's gather a pair), bound by
+// its gathers' and stores' latency; loading the vertices before their number is
+// known, 264.
+__global__ void __launch_bounds__(kCanonThreads)
+k_vt_fill(int64_t T, const int64_t *__restrict__ vt_off, const VtOrder vo, int *__restrict__ vt)
 {
     griddep_wait();
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= T) return;
-    const int4 w = tvs[c];
-    if (w.x < 0) return;  // rejected by k_canon
-    const int4 o = occ[c];
-    vt[vt_off[w.x] + o.x] = (int)c;
-    vt[vt_off[w.y] + o.y] = (int)c;
-    vt[vt_off[w.z] + o.z] = (int)c;
-    vt[vt_off[w.w] + o.w] = (int)c;
+    __shared__ long long s_to[kCanonWarps][kCanonPairs];   // of a vertex: the warp's part of its
+                                                           // row, less its place
+    __shared__ unsigned char s_cell[kCanonWarps][kCanonPairs];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int64_t c = (int64_t)blockIdx.x * kCanonThreads + threadIdx.x, tile = c >> 5;
+    if (32 * tile >= T) return;   // warp-uniform
+    const unsigned place = c < T ? vo.place[c] : ~0u;
+    const uint4 h = __ldg(vo.head + tile);
+    const int2 *verts = vo.verts + tile * kCanonPairs;
+    const int n = __popc(h.x) + __popc(h.y) + __popc(h.z) + __popc(h.w);
+    for (int i = lane; i < n; i += 32) {
+        const int2 v = __ldg(verts + i);
+        s_to[wp][i] = vt_off[v.x] + v.y;
+    }
+    const bool ok = place != ~0u;
+    if (ok) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) s_cell[wp][place >> (8 * k) & 0xffu] = (unsigned char)lane;
+    }
+    const int pairs = 4 * __popc(__ballot_sync(kFull, ok));
+    __syncwarp();
+    int before = -1;
+#pragma unroll
+    for (int w = 0; w < 4; w++) {
+        const unsigned bits = w == 0 ? h.x : (w == 1 ? h.y : (w == 2 ? h.z : h.w));
+        const int at = 32 * w + lane;
+        const int k = before + __popc(bits & (0xffffffffu >> (31 - lane)));
+        if (at < pairs) vt[s_to[wp][k] + at] = (int)(32 * tile) + s_cell[wp][at];
+        before += __popc(bits);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -762,24 +857,27 @@ void launch_publish(const PublishArgs &a, cudaStream_t s)
     launch_pdl(k_publish, 1, 32, 0, s, a);
 }
 
+int64_t canon_tiles(int64_t T) { return (T + 31) / 32; }
+int64_t canon_pairs() { return kCanonPairs; }
+
 void launch_canon(const int32_t *tv_in, int64_t T, int64_t V, int4 *tvs, int32_t *deg_t,
-                  int4 *occ, DevStatus *st, cudaStream_t s)
+                  const VtOrder &vo, DevStatus *st, cudaStream_t s)
 {
     if (T == 0) return;
     const int aligned = ((uintptr_t)tv_in & 15) == 0;
     {
         Launch L("k_canon", s);
-        launch_pdl(k_canon, blocks_for(T, 256), 256, 0, s, tv_in, T, (int)V, tvs, deg_t, occ, st, aligned);
+        launch_pdl(k_canon, blocks_for(T, kCanonThreads), kCanonThreads, 0, s, tv_in, T, (int)V, tvs,
+                   deg_t, vo, st, aligned);
     }
 }
 
-void launch_vt_fill(const int4 *tvs, int64_t T, const int64_t *vt_off, const int4 *occ, int32_t *vt,
-                    cudaStream_t s)
+void launch_vt_fill(int64_t T, const int64_t *vt_off, const VtOrder &vo, int32_t *vt, cudaStream_t s)
 {
     if (T == 0) return;
     {
         Launch L("k_vt_fill", s);
-        launch_pdl(k_vt_fill, blocks_for(T, 256), 256, 0, s, tvs, T, vt_off, occ, vt);
+        launch_pdl(k_vt_fill, blocks_for(T, kCanonThreads), kCanonThreads, 0, s, T, vt_off, vo, vt);
     }
 }
 
