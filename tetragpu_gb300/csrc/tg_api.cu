@@ -756,7 +756,7 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         ep.rec = sp.rec; ep.place = sp.place; ep.rec_hi = sp.rec_hi; ep.pairs = hv.pairs;
         ep.vt_off = vt_off; ep.vt = vt; ep.tvs = m->tvs;
         ep.erank = need_edge ? erank : nullptr;
-        ep.fflag = fflag; ep.fbnd = fbnd; ep.vbnd = sp.vbnd;
+        ep.frank = frank; ep.fbnd = fbnd; ep.vbnd = sp.vbnd;
         ep.vv_off = vv_off; ep.inc = inc; ep.vv = vv;
         ep.count_ef = (mask & TG_EF) != 0;
         launch_edge_ids(ep, s);
@@ -776,7 +776,7 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         if (prep_adj) TRY(lb.alloc(m, nvv, true, tmp, s));
         if (te || fe || tt || ff_off || ff || et || ef || prep_adj) {
             const cudaStream_t s2 = side.fork();
-            ep.te = te; ep.et_off = et_off; ep.ef_off = ef_off; ep.et = et; ep.ef = ef; ep.tf = tf;
+            ep.te = te; ep.et_off = et_off; ep.ef_off = ef_off; ep.et = et; ep.ef = ef;
             if (te || et || ef) launch_edge_rows(ep, s2);
             if (tt || ff_off) launch_cell_tt(T, F, tf, ft, brank, tt_off, tt, ff_off, s2);
             if (fe || ff) launch_face_fill(ft, tf, te, brank, F, fe, ff_off, ff, s2);

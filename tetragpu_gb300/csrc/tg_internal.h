@@ -257,7 +257,8 @@ struct EdgePass {
     const int4 *tvs;
     const uint2 *erank;        // {bits, prefix} per 32 edge occurrences; null when no ids are
                                // wanted (neither inc nor edge)
-    const uint32_t *fflag, *fbnd;
+    const uint2 *frank;        // {bits, prefix} per 32 face occurrences; read for ef
+    const uint32_t *fbnd;
     const uint8_t *vbnd;
     const int64_t *vv_off;
     // ids
@@ -270,7 +271,6 @@ struct EdgePass {
     int32_t *te;               // [6T]
     const int64_t *et_off, *ef_off;
     int32_t *et, *ef;
-    const int32_t *tf;         // read for ef
 };
 void launch_edge_ids(const EdgePass &p, cudaStream_t s);
 void launch_edge_rows(const EdgePass &p, cudaStream_t s);

@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(kStarThreads) k_star_wide(StarPass p)
 // faces have consecutive ids: their FT and FV rows pass through shared memory
 // and go out as whole lines.
 constexpr int kCellThreads = 256;
-__global__ void __launch_bounds__(kCellThreads)
+__global__ void __launch_bounds__(kCellThreads, 6)
 k_cell_faces(int64_t T, const int4 *__restrict__ tvs, const uint2 *__restrict__ frank,
              const int4 *__restrict__ fnext, int *__restrict__ tf, int2 *__restrict__ ft,
              int *__restrict__ fv)
@@ -534,8 +534,9 @@ __global__ void __launch_bounds__(256) k_edge_ids(EdgePass p)
 //
 // EF: an edge's faces at a cell are the columns omitting one of the other two
 // slots.  A face's cells all hold the edge, so a row is the faces at the cells
-// where they are first met (fflag), ascending: ids are ranks of first
-// occurrences (4 * cell + column).
+// where they are first met, ascending: ids are ranks of first occurrences (4 *
+// cell + column), so one word pair of frank gives both which faces these are
+// and their ids (78 us at 64^3 cubes; with TF read for the ids, 91).
 constexpr int kRowsThreads = 128;
 constexpr int kRowsTake = 16;                // cells an edge lists at a time
 constexpr int kRowsCap = 32 * kRowsTake;
@@ -571,10 +572,11 @@ __global__ void __launch_bounds__(kRowsThreads) k_edge_rows(EdgePass p)
                     if (p.te) p.te[6LL * c + pair_slot(s, t)] = (int)id;
                     if (p.et) p.et[et + k] = c;
                     if (p.ef) {
-                        const unsigned out = (__ldg(p.fflag + (c >> 3)) >> (4 * (c & 7))) & 0xfu &
-                                             ~((8u >> s) | (8u >> t));
+                        const uint2 rk = __ldg(p.frank + (c >> 3));
+                        const int sh = 4 * (c & 7);
+                        const unsigned out = (rk.x >> sh) & 0xfu & ~((8u >> s) | (8u >> t));
                         for (unsigned o = out; o; o &= o - 1)
-                            p.ef[k_ef++] = __ldg(p.tf + 4LL * c + mctz(o));
+                            p.ef[k_ef++] = (int)rk.y + __popc(rk.x & ((1u << (sh + mctz(o))) - 1u));
                     }
                 }
                 m = 0ull;
@@ -626,21 +628,17 @@ __global__ void __launch_bounds__(kRowsThreads) k_edge_rows(EdgePass p)
             }
             if (p.ef) {
                 const int t1 = s == 0 ? (t == 1 ? 2 : 1) : 0, t2 = 6 - s - t - t1;
-                int4 f = make_int4(0, 0, 0, 0);
-                unsigned nib = 0u;
-                if (act) {
-                    f = __ldg(reinterpret_cast<const int4 *>(p.tf) + c);
-                    nib = __ldg(p.fflag + (c >> 3)) >> (4 * (c & 7));
-                }
+                const uint2 rk = act ? __ldg(p.frank + (c >> 3)) : make_uint2(0u, 0u);
                 // columns 3 - t2 < 3 - t1
-                const bool first_a = (nib >> (3 - t2)) & 1u, first_b = (nib >> (3 - t1)) & 1u;
+                const int qa = 4 * (c & 7) + 3 - t2, qb = 4 * (c & 7) + 3 - t1;
+                const bool first_a = (rk.x >> qa) & 1u, first_b = (rk.x >> qb) & 1u;
                 const unsigned ba = __ballot_sync(kAll, first_a), bb = __ballot_sync(kAll, first_b);
                 // the entries of this edge before this one in the list's window
                 const int o = __shfl_sync(kAll, off, l) - i0;
                 const unsigned below = ((1u << lane) - 1u) & (o > 0 ? ~0u << o : ~0u);
                 int k = __shfl_sync(kAll, ef, l) + __popc(ba & below) + __popc(bb & below);
-                if (first_a) p.ef[k++] = get4(f, 3 - t2);
-                if (first_b) p.ef[k] = get4(f, 3 - t1);
+                if (first_a) p.ef[k++] = (int)rk.y + __popc(rk.x & ((1u << qa) - 1u));
+                if (first_b) p.ef[k] = (int)rk.y + __popc(rk.x & ((1u << qb) - 1u));
                 // this lane's own edge: past the entries written for it now
                 const int lo = max(off - i0, 0), hi = min(end - i0, 32);
                 if (lo < hi) {
