@@ -369,7 +369,9 @@ k_face_fill(const int *__restrict__ ft, const int *__restrict__ tf, const int *_
 // to an edge instead, whose entries went out in 16-byte pieces, sent 11
 // requests to L2 an edge (0.8 a clock and SM, what gets through; now 4) and 33
 // warp instructions (19): 92 -> 64 us at 64^3, 135 -> 93 us beside other kernels
-// on the 64^3 coned mesh, whose rows pass 16.
+// on the 64^3 coned mesh, whose rows pass 16.  Without bank conflicts of rows of
+// one length (rows below 16) and with eleven blocks of these to an SM: 545 -> 533
+// us at 128^3 beside other kernels.
 constexpr int kEeThreads = 128;
 constexpr int kEeWarps = kEeThreads / 32;
 // words that a warp's rows come to, of ends of at most N edges
@@ -426,9 +428,24 @@ __device__ __forceinline__ void ee_merge_lanes(const unsigned (&a)[16], const un
     const int shift = (int)(o0 & 3);   // word i of the stage is word i of the line o0 is in
     const int at = shift + (int)(o - o0);
     // sorted: an entry above e follows both copies of e
+    if constexpr (N == 16) {
+        // two by two, the upper half of the lanes the second one first: short
+        // rows are often of one even length, which puts lanes l and l + 16 on
+        // one bank (the longer ones' lengths vary: no gain there, 20 us lost on
+        // the 64^3 coned mesh)
+        const int late = lane >> 4;
+        unsigned *row = stage + at + late;
 #pragma unroll
-    for (int i = 0; i < 2 * N; i++)
-        if (i < n + 2 && x[i] != e) stage[at + (x[i] > e ? i - 2 : i)] = x[i];
+        for (int i = 0; i < 2 * N - 2; i += 2) {
+            const unsigned u = x[i] >= e ? x[i + 2] : x[i], w = x[i + 1] >= e ? x[i + 3] : x[i + 1];
+            if (i + late < n) row[i] = late ? w : u;
+            if (i + 1 - late < n) row[i + 1 - 2 * late] = late ? u : w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 2 * N; i++)
+            if (i < n + 2 && x[i] != e) stage[at + (x[i] > e ? i - 2 : i)] = x[i];
+    }
     __syncwarp();
     const int end = __reduce_max_sync(kFull, n >= 0 ? at + n : 0);
     int *line = ee + (o0 - shift);
@@ -516,7 +533,7 @@ __device__ __noinline__ void ee_merge_warp(const unsigned *__restrict__ ra, cons
 // ~0 at the end (so that a row's sixteenth word tells whether it goes on).
 // ROWS: 16 or 24 when every row is shorter than that (fewer registers), else 0.
 template <int ROWS>
-__global__ void __launch_bounds__(kEeThreads, ROWS == 16 ? 9 : 5)
+__global__ void __launch_bounds__(kEeThreads, ROWS == 16 ? 11 : 5)
 k_ee_fill(const int2 *__restrict__ ev, int64_t E, const int64_t *__restrict__ eid_off,
           const unsigned *__restrict__ eid, const int64_t *__restrict__ ee_off, int *__restrict__ ee)
 {
