@@ -10,6 +10,12 @@
 // it, so every wait ends; it is bounded all the same: after kLookbackPolls
 // polls the block records ST_SCAN_STALLED in the mesh status (reported at the
 // next status read-back) and goes on.
+//
+// A warp takes rows of 64 elements, two neighbours to a lane, so that its loads
+// and stores are whole lines: the four scans of an extraction of all relations
+// at 128^3 cubes take 105 us (140 with eight consecutive elements to a thread,
+// 128 with four elements a thread and six blocks to an SM); what is left is the
+// look-back's latency.
 #include "tg_internal.h"
 
 namespace tg {
@@ -32,10 +38,11 @@ struct ScanParams {
     int n_jobs;
 };
 
-__device__ __forceinline__ int64_t load_value(const ScanJob &j, int64_t i, int &largest)
+// the value of element i, whose words are x and (in2) y
+__device__ __forceinline__ int64_t value(const ScanJob &j, unsigned word, unsigned word2, int &largest)
 {
-    if (j.kind == SCAN_POPC_RANK) return (int64_t)__popc(__ldg((const uint32_t *)j.in + i));
-    const int x = __ldg((const int32_t *)j.in + i) + (j.in2 ? __ldg(j.in2 + i) : 0);
+    if (j.kind == SCAN_POPC_RANK) return (int64_t)__popc(word);
+    const int x = (int)(word + word2);
     if (j.kind == SCAN_COUNT_I32) return x;
     if (j.kind == SCAN_COUNT_PAD8) return pad8(x);
     if (j.kind == SCAN_EID_WORDS) return eid_words(x);
@@ -43,45 +50,28 @@ __device__ __forceinline__ int64_t load_value(const ScanJob &j, int64_t i, int &
     return (int64_t)x * x;
 }
 
-__device__ __forceinline__ void store_value(const ScanJob &j, int64_t i, int64_t v)
+// elements i and i + 1 (i even), those past the end 0
+__device__ __forceinline__ uint2 load_two(const void *in, int64_t i, int64_t n)
 {
-    if (j.kind != SCAN_POPC_RANK) ((int64_t *)j.out)[i] = v;
-    else ((uint2 *)j.out)[i] = make_uint2(i < j.n ? __ldg((const uint32_t *)j.in + i) : 0u,
-                                          (unsigned)v);
+    if (i + 1 < n) return __ldg(reinterpret_cast<const uint2 *>((const unsigned *)in + i));
+    return make_uint2(i < n ? __ldg((const unsigned *)in + i) : 0u, 0u);
 }
 
-// Block-wide exclusive scan of one int64 per thread; returns the block total.
-template <int NT>
-__device__ __forceinline__ int64_t block_exclusive_scan(int64_t x, int64_t &excl, int64_t *sm)
+// the sums before elements i and i + 1, as they are stored (i even; element n
+// is the closing one, stored by itself)
+__device__ __forceinline__ void store_two(const ScanJob &j, int64_t i, uint2 w, int64_t a, int64_t b)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int64_t incl = x;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        int64_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    if (lane == 31) sm[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        int64_t w = (lane < NT / 32) ? sm[lane] : 0;
-        int64_t wi = w;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            int64_t y = __shfl_up_sync(0xffffffffu, wi, o);
-            if (lane >= o) wi += y;
-        }
-        if (lane < NT / 32) sm[lane] = wi - w;  // exclusive warp offsets
-        if (lane == NT / 32 - 1) sm[NT / 32] = wi;
-    }
-    __syncthreads();
-    excl = sm[warp] + incl - x;
-    int64_t total = sm[NT / 32];
-    __syncthreads();
-    return total;
+    if (i >= j.n) return;
+    longlong2 v = make_longlong2(a, b);
+    if (j.kind == SCAN_POPC_RANK)   // {bits, prefix}
+        v = make_longlong2((long long)((unsigned long long)a << 32 | w.x),
+                           (long long)((unsigned long long)b << 32 | w.y));
+    int64_t *out = (int64_t *)j.out + i;
+    if (i + 1 < j.n) *reinterpret_cast<longlong2 *>(out) = v;
+    else *out = v.x;
 }
 
-__global__ void __launch_bounds__(kThreads) k_scan(ScanParams p)
+__global__ void __launch_bounds__(kThreads, 5) k_scan(ScanParams p)
 {
     griddep_wait();
     const int jb = blockIdx.y;
@@ -94,44 +84,64 @@ __global__ void __launch_bounds__(kThreads) k_scan(ScanParams p)
         const int64_t t0 = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
         for (int64_t i = t0; i < p.next_words; i += nthreads) p.next[i] = 0ull;
     }
-    __shared__ int64_t sm[kThreads / 32 + 1];
-    __shared__ int64_t s_tile, s_prefix;
+    __shared__ int64_t s_warp[kThreads / 32], s_tile, s_prefix;
     if (threadIdx.x == 0) s_tile = (int64_t)atomicAdd(w + ntiles, 1ull);   // the ticket
     __syncthreads();
     const int64_t tile = s_tile;
     if (ntiles == 0) {   // an empty array: its total alone
-        if (tile == 0 && threadIdx.x == 0) store_value(j, 0, 0);
+        if (tile == 0 && threadIdx.x == 0) *(int64_t *)j.out = 0;
         return;
     }
     if (tile >= ntiles) return;   // a surplus block of a shorter array
-    const int64_t base = tile * kTile + (int64_t)threadIdx.x * kItems;
-    int64_t v[kItems];
-    int64_t s = 0;
+    // rows of 64 elements to a warp, two neighbours to a lane
+    constexpr int kRows = kItems / 2;
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int64_t k0 = tile * kTile + wp * (32 * kItems) + 2 * lane;
+    uint2 word[kRows];
+    int64_t before[kRows], first[kRows], run = 0;
     int largest = 0;
 #pragma unroll
-    for (int k = 0; k < kItems; k++) {
-        v[k] = (base + k < j.n) ? load_value(j, base + k, largest) : 0;
-        s += v[k];
+    for (int r = 0; r < kRows; r++) word[r] = load_two(j.in, k0 + 64 * r, j.n);
+#pragma unroll
+    for (int r = 0; r < kRows; r++) {
+        const uint2 more = j.in2 ? load_two(j.in2, k0 + 64 * r, j.n) : make_uint2(0u, 0u);
+        const bool b0 = k0 + 64 * r < j.n, b1 = k0 + 64 * r + 1 < j.n;
+        first[r] = b0 ? value(j, word[r].x, more.x, largest) : 0;
+        const int64_t two = first[r] + (b1 ? value(j, word[r].y, more.y, largest) : 0);
+        int64_t x = two;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        before[r] = run + x - two;
+        run += __shfl_sync(0xffffffffu, x, 31);
     }
     if (j.kind == SCAN_DEG_SQUARE) {   // block-uniform
         largest = __reduce_max_sync(0xffffffffu, largest);
-        if ((threadIdx.x & 31) == 0 && largest > *(volatile int *)p.max_deg)
-            atomicMax(p.max_deg, largest);
+        if (lane == 0 && largest > *(volatile int *)p.max_deg) atomicMax(p.max_deg, largest);
     }
-    int64_t excl;
-    const int64_t total = block_exclusive_scan<kThreads>(s, excl, sm);
-    if (threadIdx.x < 32) {   // warp 0
+    if (lane == 0) s_warp[wp] = run;
+    __syncthreads();
+    int64_t total = 0, warps = 0;
+#pragma unroll
+    for (int i = 0; i < kThreads / 32; i++) {
+        if (i == wp) warps = total;
+        total += s_warp[i];
+    }
+    if (wp == 0) {
         const int64_t pre = look_back(w, tile, total, p.err);
-        if (threadIdx.x == 0) s_prefix = pre;
+        if (lane == 0) s_prefix = pre;
     }
     __syncthreads();
-    int64_t run = s_prefix + excl;
+    const int64_t base = s_prefix + warps;
 #pragma unroll
-    for (int k = 0; k < kItems; k++) {
-        if (base + k < j.n) store_value(j, base + k, run);
-        run += v[k];
+    for (int r = 0; r < kRows; r++)
+        store_two(j, k0 + 64 * r, word[r], base + before[r], base + before[r] + first[r]);
+    if (tile == ntiles - 1 && threadIdx.x == 0) {
+        const int64_t all = s_prefix + total;
+        ((int64_t *)j.out)[j.n] = j.kind == SCAN_POPC_RANK ? all << 32 : all;
     }
-    if (tile == ntiles - 1 && threadIdx.x == 0) store_value(j, j.n, s_prefix + total);
 }
 
 }  // namespace
