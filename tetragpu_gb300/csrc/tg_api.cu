@@ -540,7 +540,7 @@ tg_status link_wait(const tg_mesh *m, cudaStream_t s)
 // too, on the extraction's own stream (before a fork, so that a side stream may
 // use them); build launches.
 struct LinkBuild {
-    int32_t *len = nullptr, *win = nullptr;
+    int32_t *win = nullptr;
     bool rows = false, masks = false;
     tg_status alloc(tg_mesh *m, int64_t nvv, bool with_masks, Temps &tmp, cudaStream_t s)
     {
@@ -549,7 +549,6 @@ struct LinkBuild {
         masks = with_masks && !m->lg_adj;
         Plan t, r, k;
         if (rows) {
-            t.add(&len, m->V);
             r.add(&m->lg_off, m->V + 1);
             r.add(&m->lg_ent, n);
         }
@@ -572,13 +571,14 @@ struct LinkBuild {
     {
         const LinkGraph g = link_graph(m, nvv);
         if (rows) {
-            launch_vv_lengths_in_order(vv_off, m->vorder, m->V, len, s);
-            ScanJob job{len, m->lg_off, m->V, SCAN_COUNT_PAD8, nullptr};
+            ScanJob job{vv_off, m->lg_off, m->V, SCAN_ROW_PAD8, m->vorder};
             scan_batch(&job, 1, m->scan, m->st, s);
-            launch_rows_in_order(vv_off, vv, m->vorder, m->vpos, m->V, m->lg_off, m->lg_ent, s);
+            launch_rows_in_order(vv_off, vv, m->vorder, m->vpos, m->V, m->lg_off, m->lg_ent, win,
+                                 masks ? window_count(g.n_ent, crit_window()) : 0, s);
         }
         if (masks) {
-            launch_window_starts(m->lg_off, m->V, g.n_ent, crit_window(), win, s);
+            if (!rows || m->V == 0)   // else beside the rows
+                launch_window_starts(m->lg_off, m->V, g.n_ent, crit_window(), win, s);
             launch_crit_adj(g, win, m->st, m->max_deg ? 1 : 0, s);
         }
     }

@@ -43,7 +43,8 @@ constexpr int kOrderRows = 4;
 __global__ void __launch_bounds__(kOrderThreads, 9)
 k_rows_in_order(const int64_t *__restrict__ vv_off, const int *__restrict__ vv,
                 const int *__restrict__ order, const int *__restrict__ vpos, int64_t V,
-                const int64_t *__restrict__ off, int *__restrict__ ent)
+                const int64_t *__restrict__ off, int *__restrict__ ent, int *__restrict__ win,
+                int64_t n_win)
 {
     griddep_wait();
     __shared__ int row[kOrderCap + kOrderThreads];
@@ -61,6 +62,16 @@ k_rows_in_order(const int64_t *__restrict__ vv_off, const int *__restrict__ vv,
         const int v = __ldg(order + i);
         src = __ldg(vv_off + v);
         d = (int)(__ldg(vv_off + v + 1) - src);
+    }
+    if (win) {
+        // as k_window_starts: the windows that start in or right after row i,
+        // and those past the last entry
+        for (int64_t w = off[V] / kAdjWin + 1 + i; w <= n_win; w += (int64_t)gridDim.x * kOrderThreads)
+            win[w] = (int)V;
+        if (i == 0) win[0] = 0;
+        if (i < V)
+            for (int64_t w = b / kAdjWin + 1; w <= off[i + 1] / kAdjWin && w <= n_win; w++)
+                win[w] = (int)i + 1;
     }
     if (n > kOrderCap) {   // block-uniform: in place
         for (int k = 0; k < d; k++) ent[b + k] = __ldg(vpos + __ldg(vv + src + k));
@@ -102,17 +113,6 @@ k_rows_in_order(const int64_t *__restrict__ vv_off, const int *__restrict__ vv,
 }
 
 // row lengths of VV in that order
-__global__ void __launch_bounds__(256)
-k_vv_lengths_in_order(const int64_t *__restrict__ vv_off, const int *__restrict__ order, int64_t V,
-                      int *__restrict__ len)
-{
-    griddep_wait();
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= V) return;
-    const int v = order[i];
-    len[i] = (int)(vv_off[v + 1] - vv_off[v]);
-}
-
 // ---------------------------------------------------------------------------
 // Link adjacency: for every entry (v, u), bit j of the mask is set when v's
 // j-th neighbour is also a neighbour of u.  The common neighbours of v and u
@@ -510,21 +510,13 @@ k_crit_classify(const int64_t *__restrict__ off, const int *__restrict__ ent,
 int crit_window() { return kAdjWin; }
 
 void launch_rows_in_order(const int64_t *vv_off, const int32_t *vv, const int32_t *order,
-                          const int32_t *vpos, int64_t V, const int64_t *off, int32_t *ent,
-                          cudaStream_t s)
+                          const int32_t *vpos, int64_t V, const int64_t *off, int32_t *ent, int32_t *win,
+                          int64_t n_win, cudaStream_t s)
 {
     if (V == 0) return;
     Launch L("k_rows_in_order", s);
     launch_pdl(k_rows_in_order, (unsigned)((V + kOrderThreads - 1) / kOrderThreads), kOrderThreads, 0, s,
-               vv_off, vv, order, vpos, V, off, ent);
-}
-
-void launch_vv_lengths_in_order(const int64_t *vv_off, const int32_t *order, int64_t V, int32_t *len,
-                                cudaStream_t s)
-{
-    if (V == 0) return;
-    Launch L("k_vv_lengths_in_order", s);
-    launch_pdl(k_vv_lengths_in_order, (unsigned)((V + 255) / 256), 256, 0, s, vv_off, order, V, len);
+               vv_off, vv, order, vpos, V, off, ent, win, n_win);
 }
 
 void launch_crit_adj(const LinkGraph &g, const int32_t *win, DevStatus *st, int heavy, cudaStream_t s)

@@ -49,7 +49,8 @@ enum ScanKind : int {
     SCAN_COUNT_I32 = 0,  // in: int32 counts (+ in2's when given), out: int64 offsets [n + 1]
     SCAN_POPC_RANK = 1,  // in: uint32 bit words, out: uint2 {word, popcount prefix} [n + 1],
                          //     out[n] = {0, total}: rank of bit p = one 8-byte load
-    SCAN_COUNT_PAD8 = 3, // SCAN_COUNT_I32 of the counts rounded up to multiples of eight
+    SCAN_ROW_PAD8 = 3,   // in: int64 CSR offsets; SCAN_COUNT_I32 of the lengths of rows in2[i],
+                         //     rounded up to multiples of eight
     SCAN_EID_WORDS = 4,  // SCAN_COUNT_I32 of eid_words of the counts
     SCAN_DEG_SQUARE = 2  // in: int32 x (+ in2's), out: int64 prefix of x*x [n + 1]; the largest
                          //     x goes to the status word's max_deg
@@ -331,11 +332,10 @@ struct LinkGraph {
     bool wide;                     // a row holds more than 32 entries (always so without order)
 };
 // VV's row lengths by position, and (off their prefix) its rows
-void launch_vv_lengths_in_order(const int64_t *vv_off, const int32_t *order, int64_t V, int32_t *len,
-                                cudaStream_t s);
+// (win, unless null: the rows' window starts, n_win + 1 of them)
 void launch_rows_in_order(const int64_t *vv_off, const int32_t *vv, const int32_t *order,
-                          const int32_t *vpos, int64_t V, const int64_t *off, int32_t *ent,
-                          cudaStream_t s);
+                          const int32_t *vpos, int64_t V, const int64_t *off, int32_t *ent, int32_t *win,
+                          int64_t n_win, cudaStream_t s);
 // the masks; win: window table of off (launch_window_starts, crit_window())
 int crit_window();
 // heavy: 0 no row longer than kMaxDeg, 1 such rows get the heavy path

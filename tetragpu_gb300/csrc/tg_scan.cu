@@ -44,7 +44,7 @@ __device__ __forceinline__ int64_t value(const ScanJob &j, unsigned word, unsign
     if (j.kind == SCAN_POPC_RANK) return (int64_t)__popc(word);
     const int x = (int)(word + word2);
     if (j.kind == SCAN_COUNT_I32) return x;
-    if (j.kind == SCAN_COUNT_PAD8) return pad8(x);
+    if (j.kind == SCAN_ROW_PAD8) return pad8(x);
     if (j.kind == SCAN_EID_WORDS) return eid_words(x);
     largest = max(largest, x);
     return (int64_t)x * x;
@@ -55,6 +55,17 @@ __device__ __forceinline__ uint2 load_two(const void *in, int64_t i, int64_t n)
 {
     if (i + 1 < n) return __ldg(reinterpret_cast<const uint2 *>((const unsigned *)in + i));
     return make_uint2(i < n ? __ldg((const unsigned *)in + i) : 0u, 0u);
+}
+
+// SCAN_ROW_PAD8: the lengths of rows in2[i] and in2[i + 1] of the CSR offsets
+__device__ __forceinline__ uint2 load_rows(const ScanJob &j, int64_t i)
+{
+    const int64_t *off = (const int64_t *)j.in;
+    const uint2 r = load_two(j.in2, i, j.n);
+    uint2 len = make_uint2(0u, 0u);
+    if (i < j.n) len.x = (unsigned)(__ldg(off + r.x + 1) - __ldg(off + r.x));
+    if (i + 1 < j.n) len.y = (unsigned)(__ldg(off + r.y + 1) - __ldg(off + r.y));
+    return len;
 }
 
 // the sums before elements i and i + 1, as they are stored (i even; element n
@@ -101,10 +112,11 @@ __global__ void __launch_bounds__(kThreads, 5) k_scan(ScanParams p)
     int64_t before[kRows], first[kRows], run = 0;
     int largest = 0;
 #pragma unroll
-    for (int r = 0; r < kRows; r++) word[r] = load_two(j.in, k0 + 64 * r, j.n);
+    for (int r = 0; r < kRows; r++)
+        word[r] = j.kind == SCAN_ROW_PAD8 ? load_rows(j, k0 + 64 * r) : load_two(j.in, k0 + 64 * r, j.n);
 #pragma unroll
     for (int r = 0; r < kRows; r++) {
-        const uint2 more = j.in2 ? load_two(j.in2, k0 + 64 * r, j.n) : make_uint2(0u, 0u);
+        const uint2 more = j.in2 && j.kind != SCAN_ROW_PAD8 ? load_two(j.in2, k0 + 64 * r, j.n) : make_uint2(0u, 0u);
         const bool b0 = k0 + 64 * r < j.n, b1 = k0 + 64 * r + 1 < j.n;
         first[r] = b0 ? value(j, word[r].x, more.x, largest) : 0;
         const int64_t two = first[r] + (b1 ? value(j, word[r].y, more.y, largest) : 0);
