@@ -71,3 +71,20 @@ def test_edge_rows_of_given_lengths(gpu_lib, oracle, k):
     tv = np.concatenate([ring + j * (k + 2) for j in range(5)])
     n = 5 * (k + 2)
     _check(gpu_lib, oracle, rng.permutation(n)[tv].astype(np.int32), n)
+
+
+@pytest.mark.parametrize("names", [["EV", "TE"], ["EV", "ET"], ["EV", "EF"], ["EV", "TE", "FV"],
+                                   ["EV", "EF", "EE"], ["EF", "VV"]])
+def test_ev_beside_rows(gpu_lib, oracle, names):
+    # EV by the pass that writes rows, or before it where EE reads it; EF
+    # without TF; a last warp of one edge to thirty-one
+    for dims, coned, hub in (((1, 1, 1), 0.0, 0), ((3, 2, 1), 0.0, 0), ((5, 4, 3), 0.5, 70)):
+        m = meshgen.kuhn_mesh(dims, coned, seed=7)
+        n = m.n_verts
+        fan = [[n, n + 1 + i, n + 2 + i, n + hub + 2] for i in range(hub)]
+        tv = np.concatenate([m.tv, np.array(fan, np.int32).reshape(-1, 4)]).astype(np.int32)
+        n += hub + 3 if hub else 0
+        ref = oracle.extract(oracle.canonicalize(tv, n), n)
+        with gpu_lib.Mesh(tv, n) as g:
+            g.extract(names)
+            assert_relations_equal({r: g.relation(r) for r in names}, ref, names)

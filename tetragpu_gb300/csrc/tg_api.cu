@@ -606,7 +606,7 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         int64_t *vv_off;
         // FE is read off each face's first cell (k_face_fill), which the
         // face's FT row and the cell's TF row tell; EF off TF
-        const bool need_tf = (mask & (TG_TF | TG_FE | TG_FF | TG_EF)) || want_tt_face;
+        const bool need_tf = (mask & (TG_TF | TG_FE | TG_FF)) || want_tt_face;
         const bool need_ft = (mask & (TG_FT | TG_FE | TG_FF)) || want_tt_face;
         const bool need_te = mask & (TG_TE | TG_FE);
         const bool need_ev = mask & (TG_EV | TG_EE);
@@ -761,8 +761,10 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         ep.count_ef = (mask & TG_EF) != 0;
         launch_edge_ids(ep, s);
         if (tf || ft || fv) launch_cell_faces(T, m->tvs, frank, sp.fnext, tf, ft, fv, s);
-        if (et_off || ef_off || ee_off || ev)
-            launch_edge_offsets(ep, et_off, ef_off, ee_off, ev, m->scan, m->st, s);
+        // EV by the first pass over the edges by id; EE reads it
+        const bool ev_with_rows = ev && !want_ee && (te || et || ef);
+        if (et_off || ef_off || ee_off || (ev && !ev_with_rows))
+            launch_edge_offsets(ep, et_off, ef_off, ee_off, ev_with_rows ? nullptr : ev, m->scan, m->st, s);
         if (inc) launch_inc_sort(vv_off, V, inc, vv, eid_off, eid, s);
         else launch_vv_sort(vv_off, V, nvv, vv, s);
         set_csr(m, TG_REL_VV, vv_off, vv, V, nvv, hold_vv_off, hold_vv);
@@ -776,6 +778,7 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         if (prep_adj) TRY(lb.alloc(m, nvv, true, tmp, s));
         if (te || fe || tt || ff_off || ff || et || ef || prep_adj) {
             const cudaStream_t s2 = side.fork();
+            ep.ev = ev_with_rows ? ev : nullptr;
             ep.te = te; ep.et_off = et_off; ep.ef_off = ef_off; ep.et = et; ep.ef = ef;
             if (te || et || ef) launch_edge_rows(ep, s2);
             if (tt || ff_off) launch_cell_tt(T, F, tf, ft, brank, tt_off, tt, ff_off, s2);

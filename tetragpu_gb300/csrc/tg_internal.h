@@ -269,6 +269,7 @@ struct EdgePass {
     uint32_t *edge_hi;         // [E] rec_hi by id (with rec_hi)
     int count_ef;              // whether the EF lengths are wanted
     // rows (each or null), of the edges by id
+    int32_t *ev;               // [2E]
     int32_t *te;               // [6T]
     const int64_t *et_off, *ef_off;
     int32_t *et, *ef;

@@ -524,11 +524,13 @@ __global__ void __launch_bounds__(256) k_edge_ids(EdgePass p)
     if (W && D > kNarrowStar) p.edge_hi[id] = hi;
 }
 
-// k_edge_rows: TE at each cell of an edge, ET and EF rows.  A warp takes 32
-// consecutive edges and spreads their cells over its lanes (a list in shared
-// memory), so that the cells gathered and the entries written by one
-// instruction belong to a few neighbouring edges and share cache lines: what
-// bounds the pass is the number of lines its instructions touch (about 0.8 a
+// k_edge_rows: TE at each cell of an edge, ET and EF rows, and EV when nothing
+// before it needs it (without ET, EF or EE k_edge_offsets has nothing else to
+// do: 60 us at 96^3 cubes).  A warp takes 32 consecutive edges and spreads their
+// cells over its lanes (a list in shared memory), so that the cells gathered
+// and the entries written by one instruction belong to a few neighbouring
+// edges and share cache lines: what bounds the pass is the number of lines its
+// instructions touch (about 0.8 a
 // clock and SM get through to L2).  A thread per edge touched 20 lines an
 // edge; records in the star pass's order 13, their ET and EF rows lying apart.
 //
@@ -556,6 +558,7 @@ __global__ void __launch_bounds__(kRowsThreads) k_edge_rows(EdgePass p)
         const EdgeEnds e = edge_ends(p.tvs, rec.x);
         v = e.v;
         u = e.u;
+        if (p.ev) reinterpret_cast<int2 *>(p.ev)[id] = make_int2(v, u);
         rs = (int)__ldg(p.vt_off + v);
         if (p.et) et = (int)__ldg(p.et_off + id);
         if (p.ef) ef = (int)__ldg(p.ef_off + id);
