@@ -60,8 +60,11 @@ __device__ __forceinline__ int mctz(unsigned long long m) { return __ffsll((long
 // of 32 to 64 cells) and, of that cell's vertices, those above v: the
 // candidates.  The warp takes its smallest candidate u (one warp reduction);
 // a ballot of the lanes whose cell holds u is the edge's mask, and its lowest
-// bit the lane of the first occurrence.  A vertex costs one such round of a
-// dozen instructions per edge it owns (seven on average in a grid) and nothing
+// bit the lane of the first occurrence.  A cell's vertices are sorted, so a
+// lane only ever compares its first remaining candidate, and one that has been
+// taken leaves the front as the next ones move up.  A vertex costs one such
+// round of a dozen instructions per edge it owns (seven on average in a grid)
+// and nothing
 // is shared between warps but the record buffer; the block-wide hash of
 // (vertex, neighbour) pairs this replaces spent 600 warp instructions a vertex
 // on table inserts, work lists and barriers, and a second pass over it 840
@@ -71,6 +74,11 @@ __device__ __forceinline__ int mctz(unsigned long long m) { return __ffsll((long
 // go out with a lane each once the warp is through (or has no room for
 // another vertex): first-occurrence flags, places in the high ends' incident
 // rows, records.  No warp waits for another.
+//
+// Bound by the integer pipe (118 of its instructions a vertex; 166 with three
+// candidates compared each round and each face's cells counted in full): 700 ->
+// 668 us at 128^3 cubes (DRAM: 1.6 GB), 306 -> 252 at 96^3, 118 -> 95 on the
+// 64^3 coned mesh.
 constexpr int kStarThreads = TG_STAR_THREADS;
 constexpr int kStarPer = TG_STAR_PER;     // most vertices per warp, in sequence
 constexpr int kRecCap = TG_STAR_WIN;      // edges a warp keeps
@@ -164,12 +172,10 @@ __device__ __forceinline__ void or_if(bool yes, uint32_t *at, unsigned x)
                  "l"(at), "r"(x)
                  : "memory");
 }
-__device__ __forceinline__ void store_shared_if(bool yes, unsigned at, const uint2 &x)
+// the same words by the whole warp
+__device__ __forceinline__ void store_shared(unsigned at, const uint2 &x)
 {
-    asm volatile("{ .reg .pred q; setp.ne.s32 q, %0, 0; @q st.shared.v2.u32 [%1], {%2, %3}; }" ::"r"(
-                     (int)yes),
-                 "r"(at), "r"(x.x), "r"(x.y)
-                 : "memory");
+    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at), "r"(x.x), "r"(x.y) : "memory");
 }
 
 // One vertex; H: cells per lane.  n: edges the warp holds, with room for any
@@ -179,57 +185,56 @@ __device__ __forceinline__ void star_vertex(const StarPass &p, RecBuf<H> &S, int
                                             const int (&c)[H], const int4 (&w)[H], int &n)
 {
     using M = typename std::conditional<H == 1, unsigned, unsigned long long>::type;
-    // d: the candidates in slots 1..3 (slot 0 is never above another vertex
-    // of its cell); one that has been looked at turns into its mask, marked by
-    // the top bit (a candidate is below 2^31, and so is a narrow star's mask:
-    // at most kNarrowStar cells); with two cells a lane the marks and the
-    // masks are apart
+    // d: a cell's vertices above v, ascending (the slots after v's), looked at
+    // from the first on; one that has been looked at leaves for the end as its
+    // mask, marked by the top bit (a vertex is below 2^31, and so is a narrow
+    // star's mask: at most kNarrowStar cells); with two cells a lane the marks
+    // and the masks are apart.  In the end they stand for slots 1 to 3 (slot 0
+    // is never above another vertex of its cell), empty where not above v
     constexpr unsigned kDone = 0x80000000u;
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     unsigned d[H][3];
     M m[H][3];
 #pragma unroll
     for (int h = 0; h < H; h++) {
-        d[h][0] = w[h].y > v ? (unsigned)w[h].y : kDone;
-        d[h][1] = w[h].z > v ? (unsigned)w[h].z : kDone;
-        d[h][2] = w[h].w > v ? (unsigned)w[h].w : kDone;
+        const bool above1 = w[h].y > v, above2 = w[h].z > v, above3 = w[h].w > v;
+        d[h][0] = above1 ? (unsigned)w[h].y : (above2 ? (unsigned)w[h].z : (above3 ? (unsigned)w[h].w : kDone));
+        d[h][1] = above1 ? (unsigned)w[h].z : (above2 ? (unsigned)w[h].w : kDone);
+        d[h][2] = above1 ? (unsigned)w[h].w : kDone;
         m[h][0] = m[h][1] = m[h][2] = 0;
     }
-    const int n0 = n;
-    unsigned out = (unsigned)__cvta_generic_to_shared(S.e[wp] + n);
+    const unsigned out0 = (unsigned)__cvta_generic_to_shared(S.e[wp] + n);
+    unsigned out = out0;
     while (true) {
-        unsigned cn = min(d[0][0], min(d[0][1], d[0][2]));
-        if constexpr (H == 2) cn = min(cn, min(d[1][0], min(d[1][1], d[1][2])));
+        unsigned cn = d[0][0];
+        if constexpr (H == 2) cn = min(cn, d[1][0]);
         const unsigned u = __reduce_min_sync(kAll, cn);
         if (u >= kDone) break;
         M mu = 0;
-        bool hit[H][3];
+        bool hit[H];
 #pragma unroll
         for (int h = 0; h < H; h++) {
-            hit[h][0] = (unsigned)w[h].y == u;
-            hit[h][1] = (unsigned)w[h].z == u;
-            hit[h][2] = (unsigned)w[h].w == u;
-            const unsigned b = __ballot_sync(kAll, hit[h][0] || hit[h][1] || hit[h][2]);
-            mu |= (M)b << (32 * h);
+            hit[h] = d[h][0] == u;
+            mu |= (M)__ballot_sync(kAll, hit[h]) << (32 * h);
         }
 #pragma unroll
-        for (int h = 0; h < H; h++)
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                if constexpr (H == 1) {
-                    d[h][k] = hit[h][k] ? (unsigned)mu | kDone : d[h][k];
-                } else {
-                    d[h][k] = hit[h][k] ? kDone : d[h][k];
-                    m[h][k] = hit[h][k] ? mu : m[h][k];
-                }
+        for (int h = 0; h < H; h++) {
+            d[h][0] = hit[h] ? d[h][1] : d[h][0];
+            d[h][1] = hit[h] ? d[h][2] : d[h][1];
+            d[h][2] = hit[h] ? (H == 1 ? (unsigned)mu | kDone : kDone) : d[h][2];
+            if constexpr (H == 2) {
+                m[h][0] = hit[h] ? m[h][1] : m[h][0];
+                m[h][1] = hit[h] ? m[h][2] : m[h][1];
+                m[h][2] = hit[h] ? mu : m[h][2];
             }
-        store_shared_if(lane == 0, out, make_uint2((unsigned)mu, u));
-        if constexpr (H == 2)
-            if (lane == 0) S.hi[wp][n] = (unsigned)(mu >> 32);
+        }
+        store_shared(out, make_uint2((unsigned)mu, u));
+        if constexpr (H == 2) S.hi[wp][n + (int)((out - out0) / sizeof(uint2))] = (unsigned)(mu >> 32);
         out += sizeof(uint2);
-        n++;
     }
-    store_if(lane == 0, p.deg_own + v, n - n0);
+    const int own = (int)((out - out0) / sizeof(uint2));
+    store_if(lane == 0, p.deg_own + v, own);
+    n += own;
 
     // faces whose lowest vertex is v: two of the candidates, the third left
     // out (v in slot 0: slot 1, 2 or 3; v in slot 1: slot 0; the masks of
@@ -240,56 +245,49 @@ __device__ __forceinline__ void star_vertex(const StarPass &p, RecBuf<H> &S, int
 #pragma unroll
             for (int k = 0; k < 3; k++) m[0][k] = d[0][k] & ~kDone;
         }
-        const M bit = (M)1 << (lane + 32 * h);
+        // this lane's position, and those up to it
+        const M bit = (M)1 << (lane + 32 * h), upto = bit | (bit - 1);
         const int sh = 4 * (c[h] & 7);
         // the column of the face omitting slot o is 3 - o
         const int col0 = w[h].x == v ? 2 : 3;
-        unsigned firsts = 0u, alone = 0u;
-        M more = 0;
+        auto face = [&](int k) {
+            return k == 0 ? m[h][1] & m[h][2] : (k == 1 ? m[h][0] & m[h][2] : m[h][0] & m[h][1]);
+        };
+        auto cells = [](M f) { return sizeof(M) == 8 ? __popcll((unsigned long long)f) : __popc((unsigned)f); };
+        unsigned firsts = 0u;
+        bool odd = false;   // a face of other than two cells is first met here
         int *next = F ? p.fnext + 4LL * c[h] : nullptr;
         int *next0 = F ? next + col0 : nullptr;
 #pragma unroll
         for (int k = 0; k < 3; k++) {
-            const M f = k == 0 ? m[h][1] & m[h][2] : (k == 1 ? m[h][0] & m[h][2] : m[h][0] & m[h][1]);
-            const M rest = f & (f - 1);
-            const bool is_first = (f ^ rest) == bit;
-            const unsigned mark = k == 0 ? 1u << col0 : 1u << (2 - k);
-            firsts |= is_first ? mark : 0u;
-            alone |= is_first && !rest ? mark : 0u;
-            more |= rest & (rest - 1);
+            const M f = face(k);
+            const bool is_first = (f & upto) == bit;
+            firsts |= is_first ? (k == 0 ? 1u << col0 : 1u << (2 - k)) : 0u;
+            odd = odd || (is_first && cells(f) != 2);
             if constexpr (F) {
-                const int s2 = last_bit(rest);
+                const int s2 = last_bit(f);
                 int c2 = __shfl_sync(kAll, c[0], s2);
                 if constexpr (H == 2) {
                     const int c2b = __shfl_sync(kAll, c[1], s2);
                     c2 = s2 >= 32 ? c2b : c2;
                 }
-                store_if(is_first, k == 0 ? next0 : next + (2 - k), rest ? c2 : -1);
+                store_if(is_first, k == 0 ? next0 : next + (2 - k), c2);
             }
         }
         or_if(firsts != 0u, p.fflag + (c[h] >> 3), firsts << sh);
-        if (__any_sync(kAll, alone || more)) {   // boundary faces, faces of too many cells
-            if (alone) {
-                atomicOr(p.fbnd + (c[h] >> 3), alone << sh);
+        if (__any_sync(kAll, odd) && odd) {   // boundary faces, faces of too many cells
 #pragma unroll
-                for (int col = 0; col < 4; col++)
-                    if ((alone >> col) & 1u) {
-                        p.vbnd[col == 3 ? w[h].y : w[h].x] = 1;
-                        p.vbnd[col >= 2 ? w[h].z : w[h].y] = 1;
-                        p.vbnd[col >= 1 ? w[h].w : w[h].z] = 1;
-                    }
-            }
-            if (more) {
-                // reported by the face's first cell
-                bool here = false;
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    const M f = k == 0 ? m[h][1] & m[h][2]
-                                       : (k == 1 ? m[h][0] & m[h][2] : m[h][0] & m[h][1]);
-                    const M rest = f & (f - 1);
-                    here |= (f ^ rest) == bit && (rest & (rest - 1)) != 0;
-                }
-                if (here) {
+            for (int k = 0; k < 3; k++) {
+                const M f = face(k);
+                if ((f & upto) != bit) continue;
+                if (cells(f) == 1) {
+                    const int col = k == 0 ? col0 : 2 - k;
+                    if (F) next[col] = -1;
+                    atomicOr(p.fbnd + (c[h] >> 3), 1u << (sh + col));
+                    p.vbnd[col == 3 ? w[h].y : w[h].x] = 1;
+                    p.vbnd[col >= 2 ? w[h].z : w[h].y] = 1;
+                    p.vbnd[col >= 1 ? w[h].w : w[h].z] = 1;
+                } else if (cells(f) > 2) {   // reported by the face's first cell
                     atomicOr(&p.st->flags, ST_NONMANIFOLD_FACE);
                     note_lowest(&p.st->bad_cell, c[h]);
                 }
