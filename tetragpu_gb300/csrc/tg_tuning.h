@@ -15,7 +15,9 @@
 #define TG_STAR_THREADS 128   // threads per star-pass block
 #endif
 #ifndef TG_STAR_PER
-#define TG_STAR_PER 16   // most vertices per warp of the star pass
+#define TG_STAR_PER 18   // most vertices per warp of the star pass: 126 edges of a grid's seven
+                         // a vertex, four full rounds of lanes (664 us at 128^3 cubes; 694
+                         // with 16, 727 with 14; 24 and more go out early, 696)
 #endif
 #ifndef TG_STAR_MINB
 #define TG_STAR_MINB 10   // resident blocks per SM asked of the star pass
