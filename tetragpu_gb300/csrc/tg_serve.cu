@@ -40,7 +40,7 @@ constexpr int64_t kEstBytesPerVert = 128;
 int64_t estimate(int64_t T, int64_t V) { return kEstBytesPerCell * T + kEstBytesPerVert * V; }
 
 struct Group {                        // a resident batch
-    tg_batch *b = nullptr;
+    tg_batch *b = nullptr;            // null once it is evicted or dropped
     int64_t bytes = 0;
     int64_t live = 0;                 // members not released
     int busy = 0;                     // requests using it now
@@ -52,7 +52,7 @@ struct MeshRec {
     int64_t id = 0;
     std::vector<int32_t> tv;          // host copy, 4 * T
     int64_t T = 0, V = 0;
-    std::shared_ptr<Group> g;         // resident batch, or null (pending / evicted)
+    std::shared_ptr<Group> g;         // its batch (resident while g->b), or null (pending)
     int64_t idx = 0;                  // member index in g
     bool pending = true;              // its first batch has not finished
     bool failed = false;              // its first batch rejected it
@@ -118,22 +118,23 @@ void note_used(tg_server *S)
 }
 
 // Free idle resident batches, least recently used first, until `need` bytes
-// are released or none is idle.  Called with S->mu held.
+// are released or none is idle.  Called with S->mu held, so a batch costs one
+// look at the resident ones and none at the meshes: theirs see by the batch
+// that it is gone.  (With every mesh looked at, 2,000 evictions among 10,000
+// meshes held the lock for a third of a second.)
 void evict_idle(tg_server *S, int64_t need)
 {
-    std::vector<std::shared_ptr<Group>> idle;
-    for (auto &g : S->groups)
-        if (g->busy == 0) idle.push_back(g);
-    std::sort(idle.begin(), idle.end(),
-              [](const std::shared_ptr<Group> &a, const std::shared_ptr<Group> &b) {
-                  return a->last_use < b->last_use;
-              });
     int64_t freed = 0;
-    for (auto &g : idle) {
-        if (freed >= need) break;
-        for (auto &kv : S->meshes)
-            if (kv.second->g == g) kv.second->g.reset();
-        S->groups.erase(std::find(S->groups.begin(), S->groups.end(), g));
+    while (freed < need) {
+        size_t k = S->groups.size();
+        for (size_t i = 0; i < S->groups.size(); i++)
+            if (S->groups[i]->busy == 0 &&
+                (k == S->groups.size() || S->groups[i]->last_use < S->groups[k]->last_use))
+                k = i;
+        if (k == S->groups.size()) break;
+        const std::shared_ptr<Group> g = S->groups[k];
+        S->groups[k] = S->groups.back();
+        S->groups.pop_back();
         S->graveyard.push_back(g->b);
         g->b = nullptr;
         S->used -= g->bytes;
@@ -382,7 +383,7 @@ tg_status acquire(tg_server *S, int64_t mesh_id, cudaStream_t s, std::shared_ptr
         // (or finished): wait for it rather than building the mesh twice
         S->cv_done.wait(lk, [&] { return !m->pending; });
         if (m->failed) return sfail(TG_ERR_INVALID_MESH, "the mesh was rejected");
-        if (m->g) {
+        if (m->g && m->g->b) {
             take();
             return TG_OK;
         }
@@ -390,7 +391,7 @@ tg_status acquire(tg_server *S, int64_t mesh_id, cudaStream_t s, std::shared_ptr
     std::lock_guard<std::mutex> bl(m->build_mu);
     {
         std::lock_guard<std::mutex> lk(S->mu);
-        if (m->g) {  // rebuilt by another request meanwhile
+        if (m->g && m->g->b) {  // rebuilt by another request meanwhile
             take();
             return TG_OK;
         }
