@@ -112,7 +112,6 @@ k_rows_in_order(const int64_t *__restrict__ vv_off, const int *__restrict__ vv,
     }
 }
 
-// row lengths of VV in that order
 // ---------------------------------------------------------------------------
 // Link adjacency: for every entry (v, u), bit j of the mask is set when v's
 // j-th neighbour is also a neighbour of u.  The common neighbours of v and u

@@ -16,13 +16,13 @@
 //
 // Kernels, in pipeline order (one thread per cell/face/edge unless noted):
 //   k_canon        sort TV rows, validate ids, count cells per vertex
-//   k_vt_fill      scatter cells into VT rows (atomic cursors)
-//   k_vt_sort, k_star, k_cell_faces, k_edge_ids, k_edge_offsets, k_vv_sort,
-//   k_edge_rows    the star pass and what follows it (tg_star.cu)
+//   k_vt_fill      cells into VT rows, those of 32 cells vertex by vertex
+//   k_vt_sort, k_star, k_cell_faces, k_edge_ids, k_edge_offsets, k_inc_sort,
+//   k_vv_sort, k_edge_rows    the star pass and what follows it (tg_star.cu)
 //   k_cell_tt      face-sharing TT
 //   k_face_fill    FE (from TE of a face's first cell), FF
 //   k_ee_fill      EE
-//   k_tt_vertex_*  vertex-sharing TT
+//   k_tt_vertex    vertex-sharing TT
 #include <algorithm>
 #include <climits>
 
@@ -362,9 +362,9 @@ k_face_fill(const int *__restrict__ ft, const int *__restrict__ tf, const int *_
 // and b without the edge itself, which is in both (they share nothing else).
 // A warp takes 32 consecutive edges, a lane each: both rows are loaded into
 // registers eight entries at a time (padded to whole sectors with ~0), a's
-// ascending and b's descending around ~0s form one bitonic sequence, and one bitonic merge in registers sorts it.  The warp's
-// rows are contiguous in EE: they pass through shared memory and go out as
-// whole lines.  Bound by the load / store pipe (80%; a lane's two rows are lines
+// ascending and b's descending around ~0s form one bitonic sequence, and one
+// bitonic merge in registers sorts it.  The warp's rows are contiguous in EE:
+// they pass through shared memory and go out as whole lines.  Bound by the load / store pipe (80%; a lane's two rows are lines
 // of their own, the entries reach shared memory a word at a time).  Four lanes
 // to an edge instead, whose entries went out in 16-byte pieces, sent 11
 // requests to L2 an edge (0.8 a clock and SM, what gets through; now 4) and 33

@@ -3,8 +3,9 @@
     python -m tetragpu_gb300.tune [--apply] [--steps K]
 
 The tile constants of the kernels (the star pass's block size and vertices
-per warp, block sizes of the row sorts and the link adjacency, edges per thread of the edge-offset pass) are compile-time constants.  For every candidate setting
-(the default and one change at a time from it) this builds a variant of
+per warp, block sizes of the row sorts and the link adjacency, edges per thread
+of the edge-offset pass) are compile-time constants.  For every candidate
+setting (the default and one change at a time from it) this builds a variant of
 libtetragpu.so with -D overrides under tetragpu_gb300/_build/variants/, loads
 it, and times the batched pipeline (tg_batch create + all 13 relations with
 the link adjacency + critical points + destroy; CUDA events, L2 flushed
@@ -40,10 +41,10 @@ TUNING_H = os.path.join(PKG, "csrc", "tg_tuning.h")
 # over the defaults there) and one change at a time from it
 CANDIDATES = [
     ("default", {}),
-    ("star_per_2", {"TG_STAR_PER": 2}),
-    ("star_per_8", {"TG_STAR_PER": 8, "TG_STAR_WIN": 512}),
-    ("star_threads_256", {"TG_STAR_THREADS": 256, "TG_STAR_WIN": 512, "TG_STAR_MINB": 6}),
-    ("star_minb_10", {"TG_STAR_MINB": 10}),
+    ("star_per_16", {"TG_STAR_PER": 16}),
+    ("star_per_22", {"TG_STAR_PER": 22}),
+    ("star_threads_256", {"TG_STAR_THREADS": 256, "TG_STAR_MINB": 5}),
+    ("star_minb_8", {"TG_STAR_MINB": 8}),
     ("adj_threads_64", {"TG_ADJ_THREADS": 64}),
     ("adj_threads_256", {"TG_ADJ_THREADS": 256}),
     ("vt_sort_threads_64", {"TG_VTS_THREADS": 64}),
