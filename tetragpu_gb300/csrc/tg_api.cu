@@ -410,6 +410,7 @@ struct tg_mesh {
     void *lg_adj = nullptr;
     std::mutex lg_mu;                // while a call looks for them or builds them
     cudaEvent_t lg_done = nullptr;   // after the build of either outside an extraction
+    bool lg_pending = false;         // which has not been seen to be over
     DevStatus *st = nullptr;    // device
     DevStatus *st_host = nullptr;
     int64_t *sz_host = nullptr; // pinned slots for sizes read back at sync points
@@ -524,13 +525,20 @@ LinkGraph link_graph(const tg_mesh *m, int64_t nvv)
 tg_status link_built(tg_mesh *m, cudaStream_t s)
 {
     if (!m->lg_done) CK(cudaEventCreateWithFlags(&m->lg_done, cudaEventDisableTiming));
+    m->lg_pending = true;
     CK(cudaEventRecord(m->lg_done, s));
     return TG_OK;
 }
 
-tg_status link_wait(const tg_mesh *m, cudaStream_t s)
+tg_status link_wait(tg_mesh *m, cudaStream_t s)
 {
-    if (m->lg_done && !capturing(s)) CK(cudaStreamWaitEvent(s, m->lg_done, 0));
+    if (!m->lg_pending || capturing(s)) return TG_OK;
+    if (cudaEventQuery(m->lg_done) == cudaSuccess) {
+        m->lg_pending = false;
+        return TG_OK;
+    }
+    (void)cudaGetLastError();   // not yet
+    CK(cudaStreamWaitEvent(s, m->lg_done, 0));
     return TG_OK;
 }
 

@@ -529,9 +529,9 @@ __global__ void __launch_bounds__(256) k_edge_ids(EdgePass p)
 // for TE and EV at 96^3 against a word and a byte), so that the cells gathered
 // and the entries written by one instruction belong to a few neighbouring
 // edges and share cache lines: what bounds the pass is the number of lines its
-// instructions touch (about 0.8 a
-// clock and SM get through to L2).  A thread per edge touched 20 lines an
-// edge; records in the star pass's order 13, their ET and EF rows lying apart.
+// instructions touch (about 0.8 a clock and SM get through to L2).  A thread per
+// edge touched 20 lines an edge; records in the star pass's order 13, their ET
+// and EF rows lying apart.
 //
 // EF: an edge's faces at a cell are the columns omitting one of the other two
 // slots.  A face's cells all hold the edge, so a row is the faces at the cells
