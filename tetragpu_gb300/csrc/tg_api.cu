@@ -406,7 +406,7 @@ struct tg_mesh {
     // critical points on it (adj null: not built)
     BlockRef lg_rows, lg_masks;
     int64_t *lg_off = nullptr;
-    int32_t *lg_ent = nullptr;
+    int32_t *lg_ent = nullptr, *lg_ids = nullptr;
     void *lg_adj = nullptr;
     std::mutex lg_mu;                // while a call looks for them or builds them
     cudaEvent_t lg_done = nullptr;   // after the build of either outside an extraction
@@ -509,6 +509,7 @@ void free_link_graph(tg_mesh *m)
     m->lg_masks.reset();
     m->lg_off = nullptr;
     m->lg_ent = nullptr;
+    m->lg_ids = nullptr;
     m->lg_adj = nullptr;
 }
 
@@ -517,7 +518,8 @@ int64_t link_entries(const tg_mesh *m, int64_t nvv) { return nvv + 7 * m->V; }
 
 LinkGraph link_graph(const tg_mesh *m, int64_t nvv)
 {
-    return {m->V, link_entries(m, nvv), m->lg_off, m->lg_ent, m->vorder, m->vpos, m->lg_adj, m->wide_deg};
+    return {m->V, link_entries(m, nvv), m->lg_off, m->lg_ent, m->vorder, m->vpos, m->lg_adj, m->wide_deg,
+            m->lg_ids};
 }
 
 // A call may use on one stream what an earlier call built on another.  (Under
@@ -559,6 +561,7 @@ struct LinkBuild {
         if (rows) {
             r.add(&m->lg_off, m->V + 1);
             r.add(&m->lg_ent, n);
+            if (m->V < kOrderField) r.add(&m->lg_ids, n);
         }
         char *adj = nullptr;
         if (masks) {
@@ -581,7 +584,7 @@ struct LinkBuild {
         if (rows) {
             ScanJob job{vv_off, m->lg_off, m->V, SCAN_ROW_PAD8, m->vorder};
             scan_batch(&job, 1, m->scan, m->st, s);
-            launch_rows_in_order(vv_off, vv, m->vorder, m->vpos, m->V, m->lg_off, m->lg_ent, win,
+            launch_rows_in_order(vv_off, vv, m->vorder, m->vpos, m->V, m->lg_off, m->lg_ent, m->lg_ids, win,
                                  masks ? window_count(g.n_ent, crit_window()) : 0, s);
         }
         if (masks) {
@@ -1342,7 +1345,7 @@ int64_t tg_mesh_device_bytes(const tg_mesh *m)
     }
     b += m->V * 8;
     const int64_t n = link_entries(m, m->rel[TG_REL_VV].entries);
-    if (m->lg_off) b += n * 4 + (m->V + 1) * 8;
+    if (m->lg_off) b += n * (m->lg_ids ? 8 : 4) + (m->V + 1) * 8;
     if (m->lg_adj) b += n * (m->wide_deg ? 8 : 4);
     return b;
 }

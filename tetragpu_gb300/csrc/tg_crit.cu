@@ -43,8 +43,8 @@ constexpr int kOrderRows = 4;
 __global__ void __launch_bounds__(kOrderThreads, 9)
 k_rows_in_order(const int64_t *__restrict__ vv_off, const int *__restrict__ vv,
                 const int *__restrict__ order, const int *__restrict__ vpos, int64_t V,
-                const int64_t *__restrict__ off, int *__restrict__ ent, int *__restrict__ win,
-                int64_t n_win)
+                const int64_t *__restrict__ off, int *__restrict__ ent, int *__restrict__ ids,
+                int *__restrict__ win, int64_t n_win)
 {
     griddep_wait();
     __shared__ int row[kOrderCap + kOrderThreads];
@@ -77,6 +77,9 @@ k_rows_in_order(const int64_t *__restrict__ vv_off, const int *__restrict__ vv,
         for (int k = 0; k < d; k++) ent[b + k] = __ldg(vpos + __ldg(vv + src + k));
         for (int k = d; k < pad8(d); k++) ent[b + k] = -1;
         sort_rows_warp(ent + b, d);
+        __syncwarp();   // a row may have been written by the whole warp
+        if (ids)
+            for (int k = 0; k < pad8(d); k++) ids[b + k] = ent[b + k] < 0 ? -1 : __ldg(order + ent[b + k]);
         return;
     }
     s_src[threadIdx.x] = src;
@@ -108,7 +111,11 @@ k_rows_in_order(const int64_t *__restrict__ vv_off, const int *__restrict__ vv,
     __syncthreads();
     for (int q = threadIdx.x >> 4; q < kOrderThreads; q += kStep) {
         const int at = s_at[q], full = pad8(s_len[q]);
-        for (int k = lane; k < full; k += 16) ent[base + at + k] = row[at + q + k];
+        for (int k = lane; k < full; k += 16) {
+            const int x = row[at + q + k];
+            ent[base + at + k] = x;
+            if (ids) ids[base + at + k] = x < 0 ? -1 : __ldg(order + x);
+        }
     }
 }
 
@@ -403,13 +410,13 @@ k_crit_adj(const int64_t *__restrict__ off, const int *__restrict__ ent, const i
 
 // ---------------------------------------------------------------------------
 constexpr int kClassifyThreads = 128;
-// From this many vertices on the field is put in processing order first (a
+// From kOrderField vertices on the field is put in processing order first (a
 // launch and a buffer: 3 us), so that a block's field gathers lie together;
 // below, they hit L1 and L2 anyway.  A call by id and in order: 9.3 and 11.4 us
 // at 4,913 vertices, 11.2 and 11.4 us at 118k, 15.0 and 13.0 us at 185k, 180
 // and 105 us at 2.1M.
-constexpr int64_t kOrderField = 1 << 17;
-
+// The rows of smaller meshes are kept as vertices too, one gather of a chain
+// of four fewer: 21.0 -> 20.3 us a call on 16^3 coned cubes.
 // a field's values by position: of every vertex (vpos null: a thread per
 // position), or of the vertices from v0 on (a thread per vertex)
 template <typename F>
@@ -433,14 +440,15 @@ k_field_in_order(const F *__restrict__ field_v0, const int *__restrict__ order,
 // A thread per vertex: positions 0 .. nv - 1 (vpos null), or the positions of
 // the vertices v0 .. v0 + nv - 1 (a vertex range that holds every neighbour of
 // its vertices: a whole mesh of a batch).  order: the vertex at each position
-// (null: positions are ids), for ties and output.  field: values by position,
-// or (BY_ID) by vertex from v0.
+// (null: positions are ids), for output; to_id: the vertex of an entry (null:
+// entries are vertices), for ties and by id.  field: values by position, or
+// (BY_ID) by vertex from v0.
 template <typename F, typename M, bool PAD, bool BY_ID>
 __global__ void __launch_bounds__(kClassifyThreads)
 k_crit_classify(const int64_t *__restrict__ off, const int *__restrict__ ent,
                 const M *__restrict__ adj, const F *__restrict__ field,
-                const int *__restrict__ order, const int *__restrict__ vpos, int64_t v0, int64_t nv,
-                unsigned *__restrict__ classes3_v0)
+                const int *__restrict__ order, const int *__restrict__ to_id,
+                const int *__restrict__ vpos, int64_t v0, int64_t nv, unsigned *__restrict__ classes3_v0)
 {
     griddep_wait();
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -462,9 +470,10 @@ k_crit_classify(const int64_t *__restrict__ off, const int *__restrict__ ent,
         auto look = [&](int k, int u) {
             if (u < 0) return;   // padding
             all |= (M)1 << k;
-            const F fu = __ldg(field + (BY_ID && order ? __ldg(order + u) : u));
+            const int id = BY_ID && to_id ? __ldg(to_id + u) : u;
+            const F fu = __ldg(field + id);
             bool is_lower = fu < fv;
-            if (fu == fv) is_lower = (order ? __ldg(order + u) : u) < (int)v;
+            if (fu == fv) is_lower = (!BY_ID && to_id ? __ldg(to_id + u) : id) < (int)v;
             lower |= (M)is_lower << k;
         };
         if constexpr (PAD) {
@@ -512,13 +521,13 @@ k_crit_classify(const int64_t *__restrict__ off, const int *__restrict__ ent,
 int crit_window() { return kAdjWin; }
 
 void launch_rows_in_order(const int64_t *vv_off, const int32_t *vv, const int32_t *order,
-                          const int32_t *vpos, int64_t V, const int64_t *off, int32_t *ent, int32_t *win,
-                          int64_t n_win, cudaStream_t s)
+                          const int32_t *vpos, int64_t V, const int64_t *off, int32_t *ent, int32_t *ids,
+                          int32_t *win, int64_t n_win, cudaStream_t s)
 {
     if (V == 0) return;
     Launch L("k_rows_in_order", s);
     launch_pdl(k_rows_in_order, (unsigned)((V + kOrderThreads - 1) / kOrderThreads), kOrderThreads, 0, s,
-               vv_off, vv, order, vpos, V, off, ent, win, n_win);
+               vv_off, vv, order, vpos, V, off, ent, ids, win, n_win);
 }
 
 void launch_crit_adj(const LinkGraph &g, const int32_t *win, DevStatus *st, int heavy, cudaStream_t s)
@@ -544,17 +553,20 @@ void classify(const LinkGraph &g, const F *field, const int32_t *vpos, int64_t v
 {
     const unsigned grid = (unsigned)((nv + kClassifyThreads - 1) / kClassifyThreads);
     Launch L("k_crit_classify", s);
+    // by id, over the rows as vertices where there are such
+    const int32_t *ent = BY_ID && g.ids ? g.ids : g.ent;
+    const int32_t *to_id = BY_ID && g.ids ? nullptr : g.order;
     if (!g.order)
         launch_pdl(k_crit_classify<F, unsigned long long, false, BY_ID>, grid, kClassifyThreads, 0, s,
-                   g.off, g.ent, (const unsigned long long *)g.adj, field, g.order, vpos, v0, nv,
+                   g.off, ent, (const unsigned long long *)g.adj, field, g.order, to_id, vpos, v0, nv,
                    classes3);
     else if (g.wide)
         launch_pdl(k_crit_classify<F, unsigned long long, true, BY_ID>, grid, kClassifyThreads, 0, s,
-                   g.off, g.ent, (const unsigned long long *)g.adj, field, g.order, vpos, v0, nv,
+                   g.off, ent, (const unsigned long long *)g.adj, field, g.order, to_id, vpos, v0, nv,
                    classes3);
     else
-        launch_pdl(k_crit_classify<F, unsigned, true, BY_ID>, grid, kClassifyThreads, 0, s, g.off, g.ent,
-                   (const unsigned *)g.adj, field, g.order, vpos, v0, nv, classes3);
+        launch_pdl(k_crit_classify<F, unsigned, true, BY_ID>, grid, kClassifyThreads, 0, s, g.off, ent,
+                   (const unsigned *)g.adj, field, g.order, to_id, vpos, v0, nv, classes3);
 }
 
 template <typename F>

@@ -331,12 +331,17 @@ struct LinkGraph {
     const int32_t *order, *vpos;   // vertex at each position, and back; both null or neither
     void *adj;                     // a mask per entry: 64-bit when wide, else 32-bit
     bool wide;                     // a row holds more than 32 entries (always so without order)
+    const int32_t *ids;            // the rows as vertices (small meshes), or null
 };
+// From this many vertices on a field is put in processing order for its
+// classification; the rows of smaller meshes are there as vertices too
+constexpr int64_t kOrderField = 1 << 17;
 // VV's row lengths by position, and (off their prefix) its rows
-// (win, unless null: the rows' window starts, n_win + 1 of them)
+// (ids, unless null: the rows as vertices; win, unless null: the rows' window
+// starts, n_win + 1 of them)
 void launch_rows_in_order(const int64_t *vv_off, const int32_t *vv, const int32_t *order,
-                          const int32_t *vpos, int64_t V, const int64_t *off, int32_t *ent, int32_t *win,
-                          int64_t n_win, cudaStream_t s);
+                          const int32_t *vpos, int64_t V, const int64_t *off, int32_t *ent, int32_t *ids,
+                          int32_t *win, int64_t n_win, cudaStream_t s);
 // the masks; win: window table of off (launch_window_starts, crit_window())
 int crit_window();
 // heavy: 0 no row longer than kMaxDeg, 1 such rows get the heavy path
