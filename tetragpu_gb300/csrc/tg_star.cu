@@ -551,6 +551,10 @@ __global__ void __launch_bounds__(kRowsThreads) k_edge_rows(EdgePass p)
     const int64_t id = (int64_t)blockIdx.x * kRowsThreads + threadIdx.x;
     if ((id & ~(int64_t)31) >= p.E) return;   // warp-uniform
     int v = 0, u = 0, rs = 0, et = 0, ef = 0;
+    // EF has up to 12T entries, past 2^31: the warp's rows from an int64 start,
+    // a lane's within them (below 32 * 2^16)
+    const int64_t ef0 = p.ef ? __ldg(p.ef_off + (id & ~(int64_t)31)) : 0;
+    int *const ef_out = p.ef + ef0;
     unsigned long long m = 0ull;
     if (id < p.E) {
         const uint2 rec = __ldg(reinterpret_cast<const uint2 *>(p.edge + id));
@@ -560,7 +564,7 @@ __global__ void __launch_bounds__(kRowsThreads) k_edge_rows(EdgePass p)
         if (p.ev) reinterpret_cast<int2 *>(p.ev)[id] = make_int2(v, u);
         rs = (int)__ldg(p.vt_off + v);
         if (p.et) et = (int)__ldg(p.et_off + id);
-        if (p.ef) ef = (int)__ldg(p.ef_off + id);
+        if (p.ef) ef = (int)(__ldg(p.ef_off + id) - ef0);
         m = rec.y;
         if constexpr (W) {
             const int D = (int)(__ldg(p.vt_off + v + 1) - rs);
@@ -578,7 +582,7 @@ __global__ void __launch_bounds__(kRowsThreads) k_edge_rows(EdgePass p)
                         const int sh = 4 * (c & 7);
                         const unsigned out = (rk.x >> sh) & 0xfu & ~((8u >> s) | (8u >> t));
                         for (unsigned o = out; o; o &= o - 1)
-                            p.ef[k_ef++] = (int)rk.y + __popc(rk.x & ((1u << (sh + mctz(o))) - 1u));
+                            ef_out[k_ef++] = (int)rk.y + __popc(rk.x & ((1u << (sh + mctz(o))) - 1u));
                     }
                 }
                 m = 0ull;
@@ -634,8 +638,8 @@ __global__ void __launch_bounds__(kRowsThreads) k_edge_rows(EdgePass p)
                 const int o = __shfl_sync(kAll, off, l) - i0;
                 const unsigned below = ((1u << lane) - 1u) & (o > 0 ? ~0u << o : ~0u);
                 int k = __shfl_sync(kAll, ef, l) + __popc(ba & below) + __popc(bb & below);
-                if (first_a) p.ef[k++] = (int)rk.y + __popc(rk.x & ((1u << qa) - 1u));
-                if (first_b) p.ef[k] = (int)rk.y + __popc(rk.x & ((1u << qb) - 1u));
+                if (first_a) ef_out[k++] = (int)rk.y + __popc(rk.x & ((1u << qa) - 1u));
+                if (first_b) ef_out[k] = (int)rk.y + __popc(rk.x & ((1u << qb) - 1u));
                 // this lane's own edge: past the entries written for it now
                 const int lo = max(off - i0, 0), hi = min(end - i0, 32);
                 if (lo < hi) {
