@@ -380,7 +380,9 @@ void tg::set_last_error(const char *msg) { g_err = msg; }
 
 struct tg_mesh {
     int device = 0;
-    cudaStream_t last_stream = nullptr;  // stream of the last call, used to free asynchronously
+    // stream of the last call, which frees are ordered on (smoothing and
+    // classification of one mesh may come from several threads)
+    std::atomic<cudaStream_t> last_stream{nullptr};
     int64_t V = 0, T = 0, E = -1, F = -1;
     void *base = nullptr;       // one allocation: everything from here to VT, the scan workspace
                                 // and the status word
@@ -411,6 +413,7 @@ struct tg_mesh {
     std::mutex lg_mu;                // while a call looks for them or builds them
     cudaEvent_t lg_done = nullptr;   // after the build of either outside an extraction
     bool lg_pending = false;         // which has not been seen to be over
+    cudaEvent_t lg_used = nullptr;   // after the last smoothing over the rows
     DevStatus *st = nullptr;    // device
     DevStatus *st_host = nullptr;
     int64_t *sz_host = nullptr; // pinned slots for sizes read back at sync points
@@ -420,7 +423,7 @@ namespace {
 
 Block::~Block()
 {
-    if (p) cudaFreeAsync(p, m->last_stream);
+    if (p) cudaFreeAsync(p, m->last_stream.load(std::memory_order_relaxed));
 }
 
 // Read the status word plus up to 8 device scalars (int64 if `wide[i]`,
@@ -501,6 +504,16 @@ void set_csr(tg_mesh *m, int r, int64_t *off, int32_t *ent, int64_t rows, int64_
     x.hold_ent = hold_ent;
     x.ready = true;
     x.opts = opts;
+}
+
+// The link graph is built, and smoothed over, on the caller's stream, which
+// need not be the one the mesh's memory goes back on: what frees it, or the VV
+// it is built from, waits for both first.
+void await_link_graph(tg_mesh *m)
+{
+    const cudaStream_t s = m->last_stream.load(std::memory_order_relaxed);
+    if (m->lg_pending) cudaStreamWaitEvent(s, m->lg_done, 0);
+    if (m->lg_used) cudaStreamWaitEvent(s, m->lg_used, 0);
 }
 
 void free_link_graph(tg_mesh *m)
@@ -778,6 +791,7 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
             launch_edge_offsets(ep, et_off, ef_off, ee_off, ev_with_rows ? nullptr : ev, m->scan, m->st, s);
         if (inc) launch_inc_sort(vv_off, V, inc, vv, eid_off, eid, s);
         else launch_vv_sort(vv_off, V, nvv, vv, s);
+        await_link_graph(m);
         set_csr(m, TG_REL_VV, vv_off, vv, V, nvv, hold_vv_off, hold_vv);
         free_link_graph(m);
 
@@ -941,7 +955,8 @@ tg_status tg_mesh_destroy(tg_mesh *m)
     cudaSetDevice(m->device);
     // stream-ordered frees on the stream the mesh was last used on, then one
     // wait for that stream (no device-wide synchronisation)
-    cudaStream_t s = m->last_stream;
+    const cudaStream_t s = m->last_stream.load(std::memory_order_relaxed);
+    await_link_graph(m);
     for (auto &r : m->rel) r = Rel();
     free_link_graph(m);
     if (m->seg_c) cudaFreeAsync(m->seg_c, s);
@@ -954,6 +969,7 @@ tg_status tg_mesh_destroy(tg_mesh *m)
     cudaStreamSynchronize(s);  // no copy into the pinned slots is still in flight
     if (m->scan.done) cudaEventDestroy(m->scan.done);
     if (m->lg_done) cudaEventDestroy(m->lg_done);
+    if (m->lg_used) cudaEventDestroy(m->lg_used);
     g_pinned.put(m->st_host);
     g_pinned.put(m->sz_host);
     cudaSetDevice(cur);
@@ -1378,6 +1394,16 @@ tg_status tg::link_rows(tg_mesh *m, bool build, cudaStream_t s, LinkGraph *out)
     *out = link_graph(m, vv.entries);
     return TG_OK;
 }
+
+tg_status tg::link_rows_used(tg_mesh *m, cudaStream_t s)
+{
+    std::lock_guard<std::mutex> lk(m->lg_mu);
+    if (!m->lg_used) CK(cudaEventCreateWithFlags(&m->lg_used, cudaEventDisableTiming));
+    CK(cudaEventRecord(m->lg_used, s));
+    return TG_OK;
+}
+
+void tg::note_stream(tg_mesh *m, cudaStream_t s) { m->last_stream.store(s, std::memory_order_relaxed); }
 
 // internal: temporaries and segments (tg_batch.cu)
 tg_status tg::take_temp(size_t bytes, cudaStream_t s, void **out) { return take(bytes, s, out, true); }

@@ -361,6 +361,11 @@ void set_last_error(const char *msg);
 // the mesh's VV by position (off null when it has none yet and build is not
 // set), VV being extracted
 tg_status link_rows(tg_mesh *m, bool build, cudaStream_t s, LinkGraph *out);
+// after the last work on the stream that reads those rows
+tg_status link_rows_used(tg_mesh *m, cudaStream_t s);
+// the mesh's memory is used on the stream (the mesh's frees are ordered on the
+// last one)
+void note_stream(tg_mesh *m, cudaStream_t s);
 // work on the stream is being recorded, not run
 bool capturing(cudaStream_t s);
 // field values of every vertex by position
