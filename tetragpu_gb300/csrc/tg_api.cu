@@ -317,8 +317,9 @@ struct Plan {
     }
 };
 
-// from the pool of kept memory (temp false) or of temporaries
-tg_status take(size_t bytes, cudaStream_t s, void **out, bool temp = false)
+// from the pool of kept memory (temp false) or of temporaries; need false: the
+// caller can do without, so the call waits for nothing
+tg_status take(size_t bytes, cudaStream_t s, void **out, bool temp = false, bool need = true)
 {
     bytes = std::max<size_t>(bytes, 256);
     int dev = 0;
@@ -326,7 +327,7 @@ tg_status take(size_t bytes, cudaStream_t s, void **out, bool temp = false)
     const Pools *p = device_pools(dev);
     cudaError_t e = p ? cudaMallocFromPoolAsync(out, bytes, temp ? p->temp : p->keep, s)
                       : cudaMallocAsync(out, bytes, s);
-    if (e == cudaErrorMemoryAllocation && p) {
+    if (e == cudaErrorMemoryAllocation && p && need && !capturing(s)) {
         (void)cudaGetLastError();
         // what was freed on this stream counts once the stream is through
         cudaStreamSynchronize(s);
@@ -337,11 +338,11 @@ tg_status take(size_t bytes, cudaStream_t s, void **out, bool temp = false)
 }
 
 // a plan's arrays in a block
-tg_status take_block(const Plan &plan, const tg_mesh *m, cudaStream_t s, BlockRef *out)
+tg_status take_block(const Plan &plan, const tg_mesh *m, cudaStream_t s, BlockRef *out, bool need = true)
 {
     if (plan.n == 0) return TG_OK;
     void *q = nullptr;
-    TRY(take(plan.bytes, s, &q));
+    TRY(take(plan.bytes, s, &q, false, need));
     *out = std::make_shared<Block>(q, m);
     plan.place(q);
     return TG_OK;
@@ -358,12 +359,12 @@ struct Temps {
         for (int i = 0; i < n; i++) cudaFreeAsync(p[i], s);
     }
     // a plan's arrays; the first zero_bytes zeroed
-    tg_status add(const Plan &plan, size_t zero_bytes = 0)
+    tg_status add(const Plan &plan, size_t zero_bytes = 0, bool need = true)
     {
         if (plan.n == 0) return TG_OK;
         if (n >= 8) return fail(TG_ERR_UNSUPPORTED, "too many temporaries in one stage");
         void *q = nullptr;
-        TRY(take(plan.bytes, s, &q, true));
+        TRY(take(plan.bytes, s, &q, true, need));
         p[n++] = q;
         if (zero_bytes) {
             const cudaError_t e = cudaMemsetAsync(q, 0, zero_bytes, s);
@@ -377,6 +378,14 @@ struct Temps {
 }  // namespace
 
 void tg::set_last_error(const char *msg) { g_err = msg; }
+
+// VV by position (LinkGraph; off null: not there) and the link adjacency of
+// critical points on it (adj null: not there)
+struct LinkArrays {
+    int64_t *off = nullptr;
+    int32_t *ent = nullptr, *ids = nullptr;
+    char *adj = nullptr;
+};
 
 struct tg_mesh {
     int device = 0;
@@ -404,12 +413,8 @@ struct tg_mesh {
     int64_t n_wide = 0;         // light stars of more than 31 cells (64-bit masks)
     int max_deg = 0;            // largest degree above kMaxDeg seen by the extraction, else 0
     bool wide_deg = false;      // a vertex has more than kNarrowDeg neighbours
-    // VV by position (LinkGraph; off null: not built) and the link adjacency of
-    // critical points on it (adj null: not built)
+    LinkArrays lg;
     BlockRef lg_rows, lg_masks;
-    int64_t *lg_off = nullptr;
-    int32_t *lg_ent = nullptr, *lg_ids = nullptr;
-    void *lg_adj = nullptr;
     std::mutex lg_mu;                // while a call looks for them or builds them
     cudaEvent_t lg_done = nullptr;   // after the build of either outside an extraction
     bool lg_pending = false;         // which has not been seen to be over
@@ -520,19 +525,15 @@ void free_link_graph(tg_mesh *m)
 {
     m->lg_rows.reset();
     m->lg_masks.reset();
-    m->lg_off = nullptr;
-    m->lg_ent = nullptr;
-    m->lg_ids = nullptr;
-    m->lg_adj = nullptr;
+    m->lg = LinkArrays();
 }
 
 // entries of the link graph, at most: its rows are padded to multiples of eight
 int64_t link_entries(const tg_mesh *m, int64_t nvv) { return nvv + 7 * m->V; }
 
-LinkGraph link_graph(const tg_mesh *m, int64_t nvv)
+LinkGraph link_graph(const tg_mesh *m, const LinkArrays &a, int64_t nvv)
 {
-    return {m->V, link_entries(m, nvv), m->lg_off, m->lg_ent, m->vorder, m->vpos, m->lg_adj, m->wide_deg,
-            m->lg_ids};
+    return {m->V, link_entries(m, nvv), a.off, a.ent, m->vorder, m->vpos, a.adj, m->wide_deg, a.ids};
 }
 
 // A call may use on one stream what an earlier call built on another.  (Under
@@ -563,46 +564,61 @@ tg_status link_wait(tg_mesh *m, cudaStream_t s)
 // too, on the extraction's own stream (before a fork, so that a side stream may
 // use them); build launches.
 struct LinkBuild {
+    LinkArrays a;
     int32_t *win = nullptr;
     bool rows = false, masks = false;
-    tg_status alloc(tg_mesh *m, int64_t nvv, bool with_masks, Temps &tmp, cudaStream_t s)
+    ScanWorkspace own;   // recorded only
+    // recorded: the calls are being recorded into a graph, which owns what it
+    // allocates and may run later, often or never: nothing stays on the mesh,
+    // and the scan has a workspace of its own (the mesh's alternates between two
+    // buffers from call to call)
+    tg_status alloc(tg_mesh *m, int64_t nvv, bool with_masks, Temps &tmp, cudaStream_t s,
+                    bool recorded = false, bool need = true)
     {
         const int64_t n = link_entries(m, nvv);
-        rows = !m->lg_off;
-        masks = with_masks && !m->lg_adj;
-        Plan t, r, k;
-        if (rows) {
-            r.add(&m->lg_off, m->V + 1);
-            r.add(&m->lg_ent, n);
-            if (m->V < kOrderField) r.add(&m->lg_ids, n);
+        a = m->lg;
+        rows = !a.off;
+        masks = with_masks && !a.adj;
+        Plan t, keep_rows, keep_masks;
+        Plan &r = recorded ? t : keep_rows, &k = recorded ? t : keep_masks;
+        size_t zero = 0;
+        if (recorded && rows) {
+            own.job_words = scan_job_words(m->V);
+            t.add(&own.buf, 2 * kMaxScanJobs * own.job_words);
+            zero = t.bytes;
         }
-        char *adj = nullptr;
+        if (rows) {
+            r.add(&a.off, m->V + 1);
+            r.add(&a.ent, n);
+            if (m->V < kOrderField) r.add(&a.ids, n);
+        }
         if (masks) {
             t.add(&win, window_count(n, crit_window()) + 1);
-            k.add(&adj, n * (m->wide_deg ? 8 : 4));
+            k.add(&a.adj, n * (m->wide_deg ? 8 : 4));
         }
-        TRY(tmp.add(t));
-        BlockRef held;
-        TRY(take_block(k, m, s, &held));
-        TRY(take_block(r, m, s, &m->lg_rows));   // the last that can fail
-        if (masks) {
-            m->lg_masks = held;
-            m->lg_adj = adj;
+        BlockRef held_rows, held_masks;
+        TRY(tmp.add(t, zero, need));
+        TRY(take_block(keep_masks, m, s, &held_masks, need));
+        TRY(take_block(keep_rows, m, s, &held_rows, need));
+        if (!recorded) {
+            if (held_rows) m->lg_rows = held_rows;
+            if (held_masks) m->lg_masks = held_masks;
+            m->lg = a;
         }
         return TG_OK;
     }
     void build(tg_mesh *m, const int64_t *vv_off, const int32_t *vv, int64_t nvv, cudaStream_t s)
     {
-        const LinkGraph g = link_graph(m, nvv);
+        const LinkGraph g = link_graph(m, a, nvv);
         if (rows) {
-            ScanJob job{vv_off, m->lg_off, m->V, SCAN_ROW_PAD8, m->vorder};
-            scan_batch(&job, 1, m->scan, m->st, s);
-            launch_rows_in_order(vv_off, vv, m->vorder, m->vpos, m->V, m->lg_off, m->lg_ent, m->lg_ids, win,
+            ScanJob job{vv_off, a.off, m->V, SCAN_ROW_PAD8, m->vorder};
+            scan_batch(&job, 1, own.buf ? own : m->scan, m->st, s);
+            launch_rows_in_order(vv_off, vv, m->vorder, m->vpos, m->V, a.off, a.ent, a.ids, win,
                                  masks ? window_count(g.n_ent, crit_window()) : 0, s);
         }
         if (masks) {
             if (!rows || m->V == 0)   // else beside the rows
-                launch_window_starts(m->lg_off, m->V, g.n_ent, crit_window(), win, s);
+                launch_window_starts(a.off, m->V, g.n_ent, crit_window(), win, s);
             launch_crit_adj(g, win, m->st, m->max_deg ? 1 : 0, s);
         }
     }
@@ -869,21 +885,22 @@ tg_status tg::critical_points_rows(tg_mesh *m, int64_t v0, int64_t nv, const voi
     m->last_stream = s;
     if (!m->rel[TG_REL_VV].ready) TRY(tg_extract(m, TG_VV, 0, s));
     const Rel &vv = m->rel[TG_REL_VV];
+    Temps adj_tmp(s), tmp(s);
     std::unique_lock<std::mutex> lk(m->lg_mu);
-    if (!m->lg_adj) {
+    LinkArrays lg = m->lg;
+    TRY(link_wait(m, s));
+    if (!lg.adj) {
         // VV rows longer than the adjacency masks take the heavy path of the
         // classification, so no status read-back here
-        Temps adj_tmp(s);
+        const bool recorded = capturing(s);
         LinkBuild lb;
-        TRY(link_wait(m, s));
-        TRY(lb.alloc(m, vv.entries, true, adj_tmp, s));
+        TRY(lb.alloc(m, vv.entries, true, adj_tmp, s, recorded));
         lb.build(m, vv.off, vv.ent, vv.entries, s);
-        if (!capturing(s)) TRY(link_built(m, s));
-    } else {
-        TRY(link_wait(m, s));
+        if (!recorded) TRY(link_built(m, s));
+        lg = lb.a;
     }
     lk.unlock();
-    Temps tmp(s);
+    const LinkGraph g = link_graph(m, lg, vv.entries);
     const size_t esz = field_type == TG_FIELD_F64 ? 8 : 4;
     const void *f = field;
     uint32_t *out = classes_out;
@@ -910,7 +927,7 @@ tg_status tg::critical_points_rows(tg_mesh *m, int64_t v0, int64_t nv, const voi
         CK(cudaMemcpyAsync(d_field, field, nv * esz, cudaMemcpyHostToDevice, s));
         f = d_field;
     }
-    launch_crit_classify(link_graph(m, vv.entries), f, field_type, ordered, v0, nv, out, s);
+    launch_crit_classify(g, f, field_type, ordered, v0, nv, out, s);
     if (m->max_deg)
         launch_crit_heavy(vv.off, vv.ent, v0, nv, max_listed, f, field_type, out, list, n_list,
                           scratch, s);
@@ -1361,8 +1378,8 @@ int64_t tg_mesh_device_bytes(const tg_mesh *m)
     }
     b += m->V * 8;
     const int64_t n = link_entries(m, m->rel[TG_REL_VV].entries);
-    if (m->lg_off) b += n * (m->lg_ids ? 8 : 4) + (m->V + 1) * 8;
-    if (m->lg_adj) b += n * (m->wide_deg ? 8 : 4);
+    if (m->lg.off) b += n * (m->lg.ids ? 8 : 4) + (m->V + 1) * 8;
+    if (m->lg.adj) b += n * (m->wide_deg ? 8 : 4);
     return b;
 }
 
@@ -1382,7 +1399,7 @@ tg_status tg::link_rows(tg_mesh *m, bool build, cudaStream_t s, LinkGraph *out)
 {
     const Rel &vv = m->rel[TG_REL_VV];
     std::lock_guard<std::mutex> lk(m->lg_mu);
-    if (m->lg_off) {
+    if (m->lg.off) {
         TRY(link_wait(m, s));
     } else if (build) {
         Temps tmp(s);
@@ -1391,7 +1408,7 @@ tg_status tg::link_rows(tg_mesh *m, bool build, cudaStream_t s, LinkGraph *out)
         lb.build(m, vv.off, vv.ent, vv.entries, s);
         TRY(link_built(m, s));
     }
-    *out = link_graph(m, vv.entries);
+    *out = link_graph(m, m->lg, vv.entries);
     return TG_OK;
 }
 

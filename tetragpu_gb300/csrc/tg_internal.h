@@ -67,7 +67,7 @@ constexpr int kMaxScanJobs = 8;
 // workspace of two buffers of kMaxScanJobs * job_words words (zeroed once when
 // made): a scan uses one buffer and zeroes the other for the next scan, so no
 // scan needs a memset.  A scan issued on another stream than the last one
-// waits for the last one first (event `done`).  A stalled scan sets
+// waits for the last one first (event `done`; null: used on one stream only).  A stalled scan sets
 // ST_SCAN_STALLED in st.
 struct ScanWorkspace {
     unsigned long long *buf = nullptr;   // 2 * kMaxScanJobs * job_words words

@@ -199,7 +199,7 @@ void scan_ws_begin(ScanWorkspace &ws, cudaStream_t s, unsigned long long **cur,
 
 void scan_ws_end(ScanWorkspace &ws, cudaStream_t s)
 {
-    cudaEventRecord(ws.done, s);
+    if (ws.done) cudaEventRecord(ws.done, s);
     ws.last = s;
     ws.used = true;
     ws.cur ^= 1;
