@@ -920,8 +920,19 @@ tg_status tg::critical_points_rows(tg_mesh *m, int64_t v0, int64_t nv, const voi
         }
         if (!field_on_device) t.add(&d_field, nv * (int64_t)esz);
         if (!out_on_device) t.add(&out, 3 * nv);
-        if (classify_orders_field(nv)) t.add(&ordered, m->V * (int64_t)esz);
         TRY(tmp.add(t, zero));
+    }
+    // the field in processing order is worth a buffer, not an error: without
+    // the memory, or recorded (no allocations in the graph), by vertex
+    Temps opt(s);
+    if (classify_orders_field(nv) && !capturing(s)) {
+        Plan o;
+        o.add(&ordered, m->V * (int64_t)esz);
+        const std::string before = g_err;
+        if (opt.add(o, 0, false) != TG_OK) {
+            ordered = nullptr;
+            g_err = before;
+        }
     }
     if (!field_on_device) {
         CK(cudaMemcpyAsync(d_field, field, nv * esz, cudaMemcpyHostToDevice, s));
@@ -1404,7 +1415,12 @@ tg_status tg::link_rows(tg_mesh *m, bool build, cudaStream_t s, LinkGraph *out)
     } else if (build) {
         Temps tmp(s);
         LinkBuild lb;
-        TRY(lb.alloc(m, vv.entries, false, tmp, s));
+        const std::string before = g_err;
+        if (lb.alloc(m, vv.entries, false, tmp, s, false, false) != TG_OK) {
+            g_err = before;
+            *out = LinkGraph{};
+            return TG_OK;   // without the memory: none
+        }
         lb.build(m, vv.off, vv.ent, vv.entries, s);
         TRY(link_built(m, s));
     }

@@ -350,8 +350,8 @@ int crit_window();
 void launch_crit_adj(const LinkGraph &g, const int32_t *win, DevStatus *st, int heavy, cudaStream_t s);
 // classify the vertices [v0, v0 + nv) (all of them, or a range that holds
 // every neighbour of its vertices): field and classes3 hold nv values / rows
-// from v0; ordered: scratch for V field values if classify_orders_field(nv)
-// (never without an order), else null
+// from v0; ordered: scratch for V field values, worth having if
+// classify_orders_field(nv) (never without an order), or null
 bool classify_orders_field(int64_t nv);
 void launch_crit_classify(const LinkGraph &g, const void *field, int field_type, void *ordered,
                           int64_t v0, int64_t nv, uint32_t *classes3, cudaStream_t s);
@@ -359,7 +359,7 @@ void launch_crit_classify(const LinkGraph &g, const void *field, int field_type,
 // the message tg_last_error_string returns on this thread
 void set_last_error(const char *msg);
 // the mesh's VV by position (off null when it has none yet and build is not
-// set), VV being extracted
+// set, or there is no memory for it), VV being extracted
 tg_status link_rows(tg_mesh *m, bool build, cudaStream_t s, LinkGraph *out);
 // after the last work on the stream that reads those rows
 tg_status link_rows_used(tg_mesh *m, cudaStream_t s);
