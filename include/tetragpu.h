@@ -243,7 +243,10 @@ tg_status tg_get_device_mesh(const tg_mesh *mesh, tg_device_mesh *out);
  * steps replacing f[v] by the mean of f[v] and its neighbours' values.  in,
  * out and scratch (needed when iterations > 1) are device arrays of n_verts
  * floats, in may not alias out or scratch; extracts VV if needed.
- * Stream-ordered. */
+ * Stream-ordered.  The values repeat bit for bit for one TV, field and number
+ * of steps.  On large meshes a call that is recorded into a graph, or that
+ * finds no memory for VV in another order, adds the neighbours up in the order
+ * of VV instead: the same values to rounding. */
 tg_status tg_smooth_field(tg_mesh *mesh, const float *in, float *out, int iterations,
                           float *scratch, void *stream);
 

@@ -1040,23 +1040,26 @@ static tg_status mesh_create_impl(const int32_t *tv, int64_t T, int64_t V, int o
     }
     CK(cudaEventCreateWithFlags(&m->scan.done, cudaEventDisableTiming));
     Temps tmp(s);
-    const int64_t nwk = (4 * T + 31) / 32;
+    const int64_t nwk = (4 * T + 31) / 32, nwh = (V + 31) / 32;
     int32_t *deg_t, *heavy_cnt;
-    uint32_t *vflag;
+    uint32_t *vflag, *hflag;
     VtOrder vo{};
-    uint2 *vrank;
+    uint2 *vrank, *hrank;
     int64_t *vkey;
     {
-        // the per-vertex cell counts and the first-cell bitmap are zeroed
+        // the per-vertex cell counts and the bitmaps of first cells and of
+        // heavy vertices are zeroed
         Plan t;
         t.add(&deg_t, V);
         t.add(&vflag, nwk);
+        t.add(&hflag, nwh);
         t.add(&heavy_cnt, 4);
         const size_t zero = t.bytes;
         t.add(&vo.place, T);
         t.add(&vo.head, canon_tiles(T));
         t.add(&vo.verts, canon_tiles(T) * canon_pairs());
         t.add(&vrank, nwk + 1);
+        t.add(&hrank, nwh + 1);
         t.add(&vkey, V);
         TRY(tmp.add(t, zero));
     }
@@ -1066,10 +1069,11 @@ static tg_status mesh_create_impl(const int32_t *tv, int64_t T, int64_t V, int o
     launch_vt_fill(T, vt_off, vo, vt, s);
     // VT row sort, which also marks each vertex's star-order key; then the
     // star processing order
-    launch_vt_sort(vt_off, vt, V, 4 * T, m->tvs, vflag, vkey, heavy_cnt, m->heavy_off, s);
-    ScanJob jf{vflag, vrank, nwk, SCAN_POPC_RANK, nullptr};
-    scan_batch(&jf, 1, m->scan, m->st, s);
-    launch_vorder_place(vt_off, V, vkey, vrank, nwk, heavy_cnt, m->vorder, m->vpos, s);
+    launch_vt_sort(vt_off, vt, V, 4 * T, m->tvs, vflag, vkey, hflag, heavy_cnt, s);
+    const ScanJob jf[2] = {{vflag, vrank, nwk, SCAN_POPC_RANK, nullptr},
+                           {hflag, hrank, nwh, SCAN_POPC_RANK, nullptr}};
+    scan_batch(jf, 2, m->scan, m->st, s);
+    launch_vorder_place(vt_off, V, vkey, vrank, nwk, hrank, heavy_cnt, m->heavy_off, m->vorder, m->vpos, s);
     CK(cudaGetLastError());
     set_csr(m, TG_REL_VT, vt_off, vt, V, 4 * T, nullptr, nullptr);
     // vertices with light stars, heavy ones, the heavy stars' entries and
@@ -1406,13 +1410,13 @@ bool tg::capturing(cudaStream_t s)
     return true;
 }
 
-tg_status tg::link_rows(tg_mesh *m, bool build, cudaStream_t s, LinkGraph *out)
+tg_status tg::link_rows(tg_mesh *m, cudaStream_t s, LinkGraph *out)
 {
     const Rel &vv = m->rel[TG_REL_VV];
     std::lock_guard<std::mutex> lk(m->lg_mu);
     if (m->lg.off) {
         TRY(link_wait(m, s));
-    } else if (build) {
+    } else {
         Temps tmp(s);
         LinkBuild lb;
         const std::string before = g_err;

@@ -63,8 +63,9 @@ k_smooth_ordered(const int64_t *__restrict__ off, const int *__restrict__ ent, i
 // 64^3, 433 against 604 on 128^3, but 74 against 72 on 48^3 (0.12 M), where
 // both kinds of step are bound by their launches.
 constexpr int64_t kOrderVerts = 1 << 17;
-constexpr int kOrderSteps = 2;        // when the mesh has those rows already
-constexpr int kOrderBuildSteps = 5;   // when they are to be made
+// The vertices and steps alone decide, so that a call gives the same bits
+// whether or not the mesh has those rows already.
+constexpr int kOrderSteps = 5;
 
 }  // namespace
 }  // namespace tg
@@ -140,7 +141,7 @@ extern "C" tg_status tg_smooth_field(tg_mesh *mesh, const float *in, float *out,
     if (m.n_verts >= kOrderVerts && iterations >= kOrderSteps && !recorded) {
         LinkGraph g{};
         // without the memory for them: by id
-        if (link_rows(mesh, iterations >= kOrderBuildSteps, s, &g) == TG_OK && g.off) {
+        if (link_rows(mesh, s, &g) == TG_OK && g.off) {
             // steps alternate between the two buffers so that the last one
             // reads scratch
             float *src = iterations % 2 ? scratch : out, *dst = iterations % 2 ? out : scratch;

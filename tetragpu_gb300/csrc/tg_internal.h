@@ -187,12 +187,10 @@ void launch_window_starts(const int64_t *off, int64_t rows, int64_t n_entries, i
 // sort every VT row (tg_star.cu).  Also marks each vertex's star-order key
 // 4 * (lowest cell) + (slot in it) in vflag (4T bits, zeroed by the caller)
 // and stores it in vkey[v]; rows with no cells are left alone.  A vertex of
-// more than kMaxStar cells takes no key: it is counted in heavy_cnt[0] (vkey
-// -1 - index) with its entries in heavy_cnt[1], where they start in
-// heavy_off[index].  heavy_cnt[2] counts the wide light stars.
+// more than kMaxStar cells takes no key: its bit is set in hflag (V bits,
+// zeroed).  heavy_cnt[2] counts the wide light stars.
 void launch_vt_sort(const int64_t *vt_off, int32_t *vt, int64_t V, int64_t nvt, const int4 *tvs,
-                    uint32_t *vflag, int64_t *vkey, int32_t *heavy_cnt, int32_t *heavy_off,
-                    cudaStream_t s);
+                    uint32_t *vflag, int64_t *vkey, uint32_t *hflag, int32_t *heavy_cnt, cudaStream_t s);
 // sort VV rows in place
 void launch_vv_sort(const int64_t *vv_off, int64_t V, int64_t nvv, int32_t *vv, cudaStream_t s);
 // VV rows and incident-edge rows from inc (EdgePass), sorted; the latter at
@@ -200,11 +198,14 @@ void launch_vv_sort(const int64_t *vv_off, int64_t V, int64_t nvv, int32_t *vv, 
 void launch_inc_sort(const int64_t *vv_off, int64_t V, const int2 *inc, int32_t *vv,
                      const int64_t *eid_off, uint32_t *eid, cudaStream_t s);
 // Star processing order (vertices by first cell): vorder[pos] = vertex, pos =
-// rank of its key; vpos the way back (heavy vertices after the light ones,
-// vertices without cells last, counted in heavy_cnt[3])
-void launch_vorder_place(const int64_t *vt_off, int64_t V, const int64_t *vkey,
-                         const uint2 *vrank, int64_t nwk, int32_t *heavy_cnt, int32_t *vorder,
-                         int32_t *vpos, cudaStream_t s);
+// rank of its key; vpos the way back (heavy vertices after the light ones, by
+// id, vertices without cells last).  vrank, hrank: ranks of vflag and hflag.
+// heavy_off[i]: where the i-th heavy vertex's entries start among theirs.
+// heavy_cnt[0], [1], [3]: heavy vertices, their entries, vertices without cells
+// (zeroed by the caller).
+void launch_vorder_place(const int64_t *vt_off, int64_t V, const int64_t *vkey, const uint2 *vrank,
+                         int64_t nwk, const uint2 *hrank, int32_t *heavy_cnt, int32_t *heavy_off,
+                         int32_t *vorder, int32_t *vpos, cudaStream_t s);
 
 // Star pass (tg_star.cu): the edges and faces of the light vertices.
 struct StarPass {
@@ -358,9 +359,9 @@ void launch_crit_classify(const LinkGraph &g, const void *field, int field_type,
 
 // the message tg_last_error_string returns on this thread
 void set_last_error(const char *msg);
-// the mesh's VV by position (off null when it has none yet and build is not
-// set, or there is no memory for it), VV being extracted
-tg_status link_rows(tg_mesh *m, bool build, cudaStream_t s, LinkGraph *out);
+// the mesh's VV by position, made if it has none yet (off null when there is no
+// memory for it), VV being extracted
+tg_status link_rows(tg_mesh *m, cudaStream_t s, LinkGraph *out);
 // after the last work on the stream that reads those rows
 tg_status link_rows_used(tg_mesh *m, cudaStream_t s);
 // the mesh's memory is used on the stream (the mesh's frees are ordered on the

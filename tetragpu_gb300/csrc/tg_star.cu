@@ -657,17 +657,15 @@ __global__ void __launch_bounds__(kRowsThreads) k_edge_rows(EdgePass p)
 // Star processing order (see k_vorder_place): vertex v with first cell c in
 // slot k has key 4c + k; its bit in vflag marks it, its rank is v's position.
 // A vertex whose star holds more than kMaxStar cells is heavy: it takes no
-// key and is numbered among the heavy vertices instead (vkey = -1 - index),
-// which follow every other vertex with cells in the processing order, so
-// that the star pass stops where they begin (tg_heavy.cu processes them).
+// key, but a bit among the heavy vertices (hflag), which follow every other
+// vertex with cells in the processing order, by id, so that the star pass
+// stops where they begin (tg_heavy.cu processes them).
 __device__ __forceinline__ void mark_first(const int4 *__restrict__ tvs, uint32_t *vflag,
-                                           int64_t *vkey, int *heavy_cnt, int *heavy_off, int v,
-                                           int c, int D)
+                                           int64_t *vkey, uint32_t *hflag, int v, int c, int D)
 {
-    if (D > kMaxStar) {   // heavy_cnt[0]: heavy vertices, [1]: their star entries
-        const int k = atomicAdd(heavy_cnt, 1);
-        vkey[v] = -1 - (long long)k;
-        heavy_off[k] = atomicAdd(heavy_cnt + 1, D);   // its share of the heavy scratch
+    if (D > kMaxStar) {
+        vkey[v] = -1;
+        atomicOr(hflag + (v >> 5), 1u << (v & 31));
         return;
     }
     const int4 w = __ldg(tvs + c);
@@ -729,14 +727,14 @@ __device__ __forceinline__ void sort_block_rows(RowStage &S, const int64_t *__re
 __global__ void __launch_bounds__(kVtsThreads)
 k_vt_sort(const int64_t *__restrict__ vt_off, int64_t V, int64_t total, int *__restrict__ vt,
           const int4 *__restrict__ tvs, uint32_t *__restrict__ vflag, int64_t *__restrict__ vkey,
-          int *__restrict__ heavy_cnt, int *__restrict__ heavy_off)
+          uint32_t *__restrict__ hflag, int *__restrict__ heavy_cnt)
 {
     griddep_wait();
     __shared__ RowStage S;
     int wide = 0;
     sort_block_rows(S, vt_off, V, total, vt, [&](int v, int c, int D) {
         wide = D > kNarrowStar && D <= kMaxStar;
-        mark_first(tvs, vflag, vkey, heavy_cnt, heavy_off, v, c, D);
+        mark_first(tvs, vflag, vkey, hflag, v, c, D);
     });
     // heavy_cnt[2]: light stars of more than kNarrowStar cells
     wide = __syncthreads_count(wide);
@@ -991,17 +989,19 @@ k_window_starts(const int64_t *__restrict__ off, int64_t V, int64_t n_win, int w
 // they write are completed by blocks running at the same time.
 // k_vt_sort marks each vertex's key 4 * first cell + slot in a bitmap over
 // the 4T cell slots; the key's rank is the vertex's position.  Heavy vertices
-// (vkey < 0) follow at n_light + their index; vertices without cells come
-// last.
+// (vkey < 0) follow at n_light + their rank among the heavy ones; vertices
+// without cells come last, in any order (no row of any relation names them).
 __global__ void __launch_bounds__(256)
 k_vorder_place(const int64_t *__restrict__ vt_off, int64_t V, const int64_t *__restrict__ vkey,
-               const uint2 *__restrict__ vrank, int64_t nwk, int *__restrict__ heavy_cnt,
-               int *__restrict__ vorder, int *__restrict__ vpos)
+               const uint2 *__restrict__ vrank, int64_t nwk, const uint2 *__restrict__ hrank,
+               int *__restrict__ heavy_cnt, int *__restrict__ heavy_off, int *__restrict__ vorder,
+               int *__restrict__ vpos)
 {
     griddep_wait();
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= V) return;
-    const int64_t n_light = (int64_t)__ldg(&vrank[nwk].y);
+    const int64_t n_light = (int64_t)__ldg(&vrank[nwk].y), n_heavy = (int64_t)__ldg(&hrank[(V + 31) / 32].y);
+    if (v == 0) heavy_cnt[0] = (int)n_heavy;
     int64_t pos;
     if (vt_off[v + 1] == vt_off[v]) {
         const unsigned together = __activemask();
@@ -1009,11 +1009,14 @@ k_vorder_place(const int64_t *__restrict__ vt_off, int64_t V, const int64_t *__r
         int at = 0;
         if (lane == leader) at = atomicAdd(heavy_cnt + 3, __popc(together));
         at = __shfl_sync(together, at, leader) + __popc(together & ((1u << lane) - 1u));
-        pos = n_light + heavy_cnt[0] + at;
+        pos = n_light + n_heavy + at;
     } else {
         const long long key = vkey[v];
         if (key < 0) {
-            pos = n_light + (-1 - key);
+            const int k = rank_of(hrank, v);
+            pos = n_light + k;
+            // its share of the heavy scratch
+            heavy_off[k] = atomicAdd(heavy_cnt + 1, (int)(vt_off[v + 1] - vt_off[v]));
         } else {
             const uint2 r = __ldg(vrank + (key >> 5));
             pos = (int64_t)r.y + __popc(r.x & ((1u << (key & 31)) - 1u));
@@ -1126,13 +1129,12 @@ void launch_edge_rows(const EdgePass &p, cudaStream_t s)
 }
 
 void launch_vt_sort(const int64_t *vt_off, int32_t *vt, int64_t V, int64_t nvt, const int4 *tvs,
-                    uint32_t *vflag, int64_t *vkey, int32_t *heavy_cnt, int32_t *heavy_off,
-                    cudaStream_t s)
+                    uint32_t *vflag, int64_t *vkey, uint32_t *hflag, int32_t *heavy_cnt, cudaStream_t s)
 {
     if (V == 0) return;
     Launch L("k_vt_sort", s);
     launch_pdl(k_vt_sort, (unsigned)((V + kVtsThreads - 1) / kVtsThreads), kVtsThreads, 0, s, vt_off,
-               V, nvt, vt, tvs, vflag, vkey, heavy_cnt, heavy_off);
+               V, nvt, vt, tvs, vflag, vkey, hflag, heavy_cnt);
 }
 
 void launch_vv_sort(const int64_t *vv_off, int64_t V, int64_t nvv, int32_t *vv, cudaStream_t s)
@@ -1152,14 +1154,14 @@ void launch_inc_sort(const int64_t *vv_off, int64_t V, const int2 *inc, int32_t 
                inc, vv, eid_off, reinterpret_cast<int *>(eid));
 }
 
-void launch_vorder_place(const int64_t *vt_off, int64_t V, const int64_t *vkey,
-                         const uint2 *vrank, int64_t nwk, int32_t *heavy_cnt, int32_t *vorder,
-                         int32_t *vpos, cudaStream_t s)
+void launch_vorder_place(const int64_t *vt_off, int64_t V, const int64_t *vkey, const uint2 *vrank,
+                         int64_t nwk, const uint2 *hrank, int32_t *heavy_cnt, int32_t *heavy_off,
+                         int32_t *vorder, int32_t *vpos, cudaStream_t s)
 {
     if (V == 0) return;
     Launch L("k_vorder_place", s);
     launch_pdl(k_vorder_place, (unsigned)((V + 255) / 256), 256, 0, s, vt_off, V, vkey, vrank, nwk,
-               heavy_cnt, vorder, vpos);
+               hrank, heavy_cnt, heavy_off, vorder, vpos);
 }
 
 void launch_seg_ranks(const int64_t *seg_c, int64_t n, const uint2 *erank, const uint2 *frank,
