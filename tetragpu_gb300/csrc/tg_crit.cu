@@ -12,9 +12,11 @@
 //
 // The graph both kernels work on is VV renumbered into the star processing
 // order (vertices by first cell): rows of neighbour positions, ascending, row
-// after row in that order.  Vertex ids need not carry locality; positions do,
-// so the neighbours' rows and field values a block gathers lie together.  (The
-// no-allocation entry point has no such order: there positions are ids.)
+// after row in that order.  Vertex ids need not carry locality; positions
+// mostly do, so the neighbours' rows and field values a block gathers lie
+// together.  Where ids keep neighbours together as well as positions do,
+// positions are ids.  (So they are for the no-allocation entry point, which
+// works on VV as it is.)
 //
 //   k_rows_in_order  VV -> the renumbered rows
 //   k_crit_adj       field-independent: for every entry (v, u), the bitmask
@@ -56,10 +58,11 @@ k_rows_in_order(const int64_t *__restrict__ vv_off, const int *__restrict__ vv,
     const int64_t base = off[i0];
     const int64_t n = off[i1] - base;
     const int64_t b = off[min(i, i1)];
+    auto place = [&](int u) { return vpos ? __ldg(vpos + u) : u; };
     long long src = 0;
     int d = 0;
     if (i < V) {
-        const int v = __ldg(order + i);
+        const int v = order ? __ldg(order + i) : (int)i;
         src = __ldg(vv_off + v);
         d = (int)(__ldg(vv_off + v + 1) - src);
     }
@@ -74,9 +77,9 @@ k_rows_in_order(const int64_t *__restrict__ vv_off, const int *__restrict__ vv,
                 win[w] = (int)i + 1;
     }
     if (n > kOrderCap) {   // block-uniform: in place
-        for (int k = 0; k < d; k++) ent[b + k] = __ldg(vpos + __ldg(vv + src + k));
+        for (int k = 0; k < d; k++) ent[b + k] = place(__ldg(vv + src + k));
         for (int k = d; k < pad8(d); k++) ent[b + k] = -1;
-        sort_rows_warp(ent + b, d);
+        if (vpos) sort_rows_warp(ent + b, d);
         __syncwarp();   // a row may have been written by the whole warp
         if (ids)
             for (int k = 0; k < pad8(d); k++) ids[b + k] = ent[b + k] < 0 ? -1 : __ldg(order + ent[b + k]);
@@ -97,18 +100,20 @@ k_rows_in_order(const int64_t *__restrict__ vv_off, const int *__restrict__ vv,
         }
 #pragma unroll
         for (int t = 0; t < kOrderRows; t++)
-            if (u[t] >= 0) u[t] = __ldg(vpos + u[t]);
+            if (u[t] >= 0) u[t] = place(u[t]);
 #pragma unroll
         for (int t = 0; t < kOrderRows; t++) {
             const int q = r + kStep * t, at = s_at[q] + q, len = s_len[q], full = pad8(len);
             if (lane < full) row[at + lane] = u[t];
             for (int k = lane + 16; k < full; k += 16)
-                row[at + k] = k < len ? __ldg(vpos + __ldg(vv + s_src[q] + k)) : -1;
+                row[at + k] = k < len ? place(__ldg(vv + s_src[q] + k)) : -1;
         }
     }
     __syncthreads();
-    sort_rows_warp(row + (int)(b - base) + threadIdx.x, d);
-    __syncthreads();
+    if (vpos) {   // (VV's rows are ascending)
+        sort_rows_warp(row + (int)(b - base) + threadIdx.x, d);
+        __syncthreads();
+    }
     for (int q = threadIdx.x >> 4; q < kOrderThreads; q += kStep) {
         const int at = s_at[q], full = pad8(s_len[q]);
         for (int k = lane; k < full; k += 16) {
@@ -437,9 +442,10 @@ k_field_in_order(const F *__restrict__ field_v0, const int *__restrict__ order,
 // Every neighbour is visited exactly once, so a vertex costs deg iterations
 // whatever the link's shape (no data-dependent find loops).
 //
-// A thread per vertex: positions 0 .. nv - 1 (vpos null), or the positions of
-// the vertices v0 .. v0 + nv - 1 (a vertex range that holds every neighbour of
-// its vertices: a whole mesh of a batch).  order: the vertex at each position
+// A thread per vertex: positions v0 .. v0 + nv - 1 (vpos null: all of them, or
+// positions are ids), or the positions of the vertices v0 .. v0 + nv - 1 (a
+// vertex range that holds every neighbour of its vertices: a whole mesh of a
+// batch).  order: the vertex at each position
 // (null: positions are ids), for output; to_id: the vertex of an entry (null:
 // entries are vertices), for ties and by id.  field: values by position, or
 // (BY_ID) by vertex from v0.
@@ -453,8 +459,8 @@ k_crit_classify(const int64_t *__restrict__ off, const int *__restrict__ ent,
     griddep_wait();
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nv) return;
-    const int64_t i = vpos ? vpos[v0 + t] : t;
-    const int64_t v = vpos ? v0 + t : (order ? order[t] : t);
+    const int64_t i = vpos ? vpos[v0 + t] : v0 + t;
+    const int64_t v = vpos || !order ? v0 + t : order[t];
     unsigned *classes3 = classes3_v0 - 3 * v0;
     const int64_t b = off[i];
     const int n = (int)(off[i + 1] - b);
@@ -535,7 +541,7 @@ void launch_crit_adj(const LinkGraph &g, const int32_t *win, DevStatus *st, int 
     if (g.V == 0) return;
     Launch L("k_crit_adj", s);
     const unsigned grid = (unsigned)window_count(g.n_ent, kAdjWin);
-    if (!g.order)   // plain VV: 64-bit masks
+    if (!g.padded)   // plain VV: 64-bit masks
         launch_pdl(k_crit_adj<unsigned long long, false>, grid, kAdjThreads, 0, s, g.off, g.ent, win,
                    (unsigned long long *)g.adj, st, heavy);
     else if (g.wide)
@@ -556,7 +562,7 @@ void classify(const LinkGraph &g, const F *field, const int32_t *vpos, int64_t v
     // by id, over the rows as vertices where there are such
     const int32_t *ent = BY_ID && g.ids ? g.ids : g.ent;
     const int32_t *to_id = BY_ID && g.ids ? nullptr : g.order;
-    if (!g.order)
+    if (!g.padded)
         launch_pdl(k_crit_classify<F, unsigned long long, false, BY_ID>, grid, kClassifyThreads, 0, s,
                    g.off, ent, (const unsigned long long *)g.adj, field, g.order, to_id, vpos, v0, nv,
                    classes3);

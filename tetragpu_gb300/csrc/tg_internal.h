@@ -49,8 +49,8 @@ enum ScanKind : int {
     SCAN_COUNT_I32 = 0,  // in: int32 counts (+ in2's when given), out: int64 offsets [n + 1]
     SCAN_POPC_RANK = 1,  // in: uint32 bit words, out: uint2 {word, popcount prefix} [n + 1],
                          //     out[n] = {0, total}: rank of bit p = one 8-byte load
-    SCAN_ROW_PAD8 = 3,   // in: int64 CSR offsets; SCAN_COUNT_I32 of the lengths of rows in2[i],
-                         //     rounded up to multiples of eight
+    SCAN_ROW_PAD8 = 3,   // in: int64 CSR offsets; SCAN_COUNT_I32 of the lengths of rows in2[i]
+                         //     (null: i), rounded up to multiples of eight
     SCAN_EID_WORDS = 4,  // SCAN_COUNT_I32 of eid_words of the counts
     SCAN_DEG_SQUARE = 2  // in: int32 x (+ in2's), out: int64 prefix of x*x [n + 1]; the largest
                          //     x goes to the status word's max_deg
@@ -206,6 +206,11 @@ void launch_inc_sort(const int64_t *vv_off, int64_t V, const int2 *inc, int32_t 
 void launch_vorder_place(const int64_t *vt_off, int64_t V, const int64_t *vkey, const uint2 *vrank,
                          int64_t nwk, const uint2 *hrank, int32_t *heavy_cnt, int32_t *heavy_off,
                          int32_t *vorder, int32_t *vpos, cudaStream_t s);
+// Whether positions or ids keep neighbours together: the lines of 32 vertices
+// that a run of 32 cells names, by id added to lines[0] and by position to
+// lines[1], over kOrderTiles runs spread over the mesh (fewer cells: none).
+constexpr int kOrderTiles = 256;
+void launch_order_lines(int64_t T, const int4 *tvs, const int32_t *vpos, int32_t *lines, cudaStream_t s);
 
 // Star pass (tg_star.cu): the edges and faces of the light vertices.
 struct StarPass {
@@ -323,23 +328,24 @@ void launch_crit_heavy(const int64_t *vv_off, const int32_t *vv, int64_t v0, int
 
 // critical points (tg_crit.cu)
 // The graph of the link adjacency: VV's rows by position, each vertex named by
-// its position in `order`, entries ascending and padded with -1 to a multiple
-// of eight; or (order null) VV itself, unpadded, positions being ids
+// its position in `order` (null: its id), entries ascending and padded with -1
+// to a multiple of eight; or (not padded) VV itself
 struct LinkGraph {
     int64_t V, n_ent;              // n_ent: at least the entries, padding included
     const int64_t *off;
     const int32_t *ent;
     const int32_t *order, *vpos;   // vertex at each position, and back; both null or neither
     void *adj;                     // a mask per entry: 64-bit when wide, else 32-bit
-    bool wide;                     // a row holds more than 32 entries (always so without order)
+    bool wide;                     // a row holds more than 32 entries (always so if not padded)
+    bool padded;
     const int32_t *ids;            // the rows as vertices (small meshes), or null
 };
 // From this many vertices on a field is put in processing order for its
 // classification; the rows of smaller meshes are there as vertices too
 constexpr int64_t kOrderField = 1 << 17;
 // VV's row lengths by position, and (off their prefix) its rows
-// (ids, unless null: the rows as vertices; win, unless null: the rows' window
-// starts, n_win + 1 of them)
+// (order and vpos null: in the order of ids; ids, unless null: the rows as
+// vertices; win, unless null: the rows' window starts, n_win + 1 of them)
 void launch_rows_in_order(const int64_t *vv_off, const int32_t *vv, const int32_t *order,
                           const int32_t *vpos, int64_t V, const int64_t *off, int32_t *ent, int32_t *ids,
                           int32_t *win, int64_t n_win, cudaStream_t s);
@@ -360,7 +366,7 @@ void launch_crit_classify(const LinkGraph &g, const void *field, int field_type,
 // the message tg_last_error_string returns on this thread
 void set_last_error(const char *msg);
 // the mesh's VV by position, made if it has none yet (off null when there is no
-// memory for it), VV being extracted
+// memory for it or positions are ids), VV being extracted
 tg_status link_rows(tg_mesh *m, cudaStream_t s, LinkGraph *out);
 // after the last work on the stream that reads those rows
 tg_status link_rows_used(tg_mesh *m, cudaStream_t s);

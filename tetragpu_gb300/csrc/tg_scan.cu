@@ -57,11 +57,12 @@ __device__ __forceinline__ uint2 load_two(const void *in, int64_t i, int64_t n)
     return make_uint2(i < n ? __ldg((const unsigned *)in + i) : 0u, 0u);
 }
 
-// SCAN_ROW_PAD8: the lengths of rows in2[i] and in2[i + 1] of the CSR offsets
+// SCAN_ROW_PAD8: the lengths of rows in2[i] and in2[i + 1] of the CSR offsets (in2
+// null: rows i and i + 1)
 __device__ __forceinline__ uint2 load_rows(const ScanJob &j, int64_t i)
 {
     const int64_t *off = (const int64_t *)j.in;
-    const uint2 r = load_two(j.in2, i, j.n);
+    const uint2 r = j.in2 ? load_two(j.in2, i, j.n) : make_uint2((unsigned)i, (unsigned)i + 1u);
     uint2 len = make_uint2(0u, 0u);
     if (i < j.n) len.x = (unsigned)(__ldg(off + r.x + 1) - __ldg(off + r.x));
     if (i + 1 < j.n) len.y = (unsigned)(__ldg(off + r.y + 1) - __ldg(off + r.y));
