@@ -535,7 +535,8 @@ int64_t link_entries(const tg_mesh *m, int64_t nvv) { return nvv + 7 * m->V; }
 LinkGraph link_graph(const tg_mesh *m, const LinkArrays &a, int64_t nvv)
 {
     return {m->V, link_entries(m, nvv), a.off, a.ent, m->lg_by_id ? nullptr : m->vorder,
-            m->lg_by_id ? nullptr : m->vpos, a.adj, m->wide_deg, true, a.ids};
+            m->lg_by_id ? nullptr : m->vpos, a.adj, m->wide_deg, true, a.ids,
+            m->n_light, m->n_heavy};
 }
 
 // A call may use on one stream what an earlier call built on another.  (Under

@@ -26,6 +26,7 @@
 //                    of each kind counted by a bitmask search over the
 //                    adjacency masks of same-kind neighbours.
 // A second field on the same mesh reuses the first two.
+#include <algorithm>
 #include <climits>
 
 #include "tg_internal.h"
@@ -436,11 +437,40 @@ k_field_in_order(const F *__restrict__ field_v0, const int *__restrict__ order,
     else out[i] = __ldg(field_v0 + order[i]);
 }
 
+// u == v for many u.  Doubles by their bits: the FP64 pipe, which takes the other
+// comparison, bounds the classification of float64 fields.
+template <typename F>
+struct EqualTo {
+    F v;
+    unsigned long long care = ~0ull, bits = 0ull;
+    __device__ __forceinline__ explicit EqualTo(F x) : v(x)
+    {
+        if constexpr (sizeof(F) == 8) {
+            bits = (unsigned long long)__double_as_longlong(x);
+            if (bits << 1 == 0ull) {   // both zeros
+                care = ~0ull >> 1;
+                bits = 0ull;
+            } else if (bits << 1 > 0xffe0000000000000ull) {   // NaN: nothing
+                care = 0ull;
+            }
+        }
+    }
+    __device__ __forceinline__ bool operator()(F u) const
+    {
+        if constexpr (sizeof(F) == 8) return ((unsigned long long)__double_as_longlong(u) & care) == bits;
+        else return u == v;
+    }
+};
+
 // Components of the lower and upper link subgraphs by bitmask search: a
-// component grows from its lowest unvisited member, each member reached
-// once adding its same-kind neighbours (its adjacency mask) to the frontier.
-// Every neighbour is visited exactly once, so a vertex costs deg iterations
-// whatever the link's shape (no data-dependent find loops).
+// component grows from its lowest unreached member, each member reached
+// once adding its same-kind neighbours (its adjacency mask) to the frontier,
+// until none is left to reach: at most deg turns whatever the link's shape.  One
+// loop over the members of all components: with a loop per component the lanes
+// of a warp wait for each other at the end of each (86 -> 74 us at 128^3 cubes).
+// The heavy stars' rows, a mesh's longest, are neighbours in star order: they
+// take the last lane of a warp each, of the first warps (hn of them, from
+// position h0 on), and the rows of those lanes the places of the heavy ones.
 //
 // A thread per vertex: positions v0 .. v0 + nv - 1 (vpos null: all of them, or
 // positions are ids), or the positions of the vertices v0 .. v0 + nv - 1 (a
@@ -454,11 +484,14 @@ __global__ void __launch_bounds__(kClassifyThreads)
 k_crit_classify(const int64_t *__restrict__ off, const int *__restrict__ ent,
                 const M *__restrict__ adj, const F *__restrict__ field,
                 const int *__restrict__ order, const int *__restrict__ to_id,
-                const int *__restrict__ vpos, int64_t v0, int64_t nv, unsigned *__restrict__ classes3_v0)
+                const int *__restrict__ vpos, int64_t v0, int64_t nv, int64_t h0, int64_t hn,
+                unsigned *__restrict__ classes3_v0)
 {
     griddep_wait();
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nv) return;
+    if ((t & 31) == 31 && (t >> 5) < hn) t = h0 + (t >> 5);
+    else if (t >= h0 && t < h0 + hn) t = 32 * (t - h0) + 31;
     const int64_t i = vpos ? vpos[v0 + t] : v0 + t;
     const int64_t v = vpos || !order ? v0 + t : order[t];
     unsigned *classes3 = classes3_v0 - 3 * v0;
@@ -472,41 +505,58 @@ k_crit_classify(const int64_t *__restrict__ off, const int *__restrict__ ent,
     {
         if constexpr (BY_ID) field -= v0;
         const F fv = field[BY_ID ? v : i];
-        M lower = 0, all = 0;
-        auto look = [&](int k, int u) {
-            if (u < 0) return;   // padding
-            all |= (M)1 << k;
-            const int id = BY_ID && to_id ? __ldg(to_id + u) : u;
-            const F fu = __ldg(field + id);
-            bool is_lower = fu < fv;
-            if (fu == fv) is_lower = (!BY_ID && to_id ? __ldg(to_id + u) : id) < (int)v;
-            lower |= (M)is_lower << k;
-        };
-        if constexpr (PAD) {
-            for (int k = 0; k < n; k += 8) {
-                unsigned u[8];
+        const EqualTo<F> equal(fv);
+        M lower = 0, all = 0, same = 0;   // same: ties, decided by id afterwards
+        // eight entries at a time without a branch, so that their values are on
+        // the way together; a missing entry (padding) looks at the vertex itself
+        for (int k = 0; k < n; k += 8) {
+            unsigned u[8];
+            if constexpr (PAD) {
                 load8(reinterpret_cast<const unsigned *>(ent + b + k), u);
+            } else {
 #pragma unroll
-                for (int t = 0; t < 8; t++) look(k + t, (int)u[t]);
+                for (int q = 0; q < 8; q++) u[q] = k + q < n ? (unsigned)__ldg(ent + b + k + q) : ~0u;
             }
-        } else {
-            for (int k = 0; k < n; k++) look(k, __ldg(ent + b + k));
+            unsigned some = 0u, less = 0u, tie = 0u;
+            F fu[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const int x = (int)u[q];
+                if constexpr (BY_ID) {
+                    const int id = to_id && x >= 0 ? __ldg(to_id + x) : x;
+                    fu[q] = __ldg(field + (x >= 0 ? id : (int)v));
+                } else {
+                    fu[q] = __ldg(field + (x >= 0 ? x : (int)i));
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                some |= (int)u[q] >= 0 ? 1u << q : 0u;
+                less |= fu[q] < fv ? 1u << q : 0u;
+                tie |= equal(fu[q]) ? 1u << q : 0u;
+            }
+            all |= (M)some << k;
+            lower |= (M)less << k;
+            same |= (M)(tie & some) << k;
         }
-        M rem = all;
+        for (; same; same &= same - 1) {
+            const int u = __ldg(ent + b + first(same));
+            if ((to_id ? __ldg(to_id + u) : u) < (int)v) lower |= same & (0 - same);
+        }
+        M rem = all, frontier = 0, kind = 0;   // rem: not reached yet
         while (rem) {
-            const int s = first(rem);
-            const bool is_lo = (lower >> s) & 1;
-            const M kind = is_lo ? lower : (all & ~lower);
-            M comp = (M)1 << s, frontier = comp;
-            while (frontier) {
-                const int j = first(frontier);
-                frontier &= frontier - 1;
-                const M nb = __ldg(adj + b + j) & kind & ~comp;
-                comp |= nb;
-                frontier |= nb;
+            if (!frontier) {   // the next component
+                frontier = rem & (0 - rem);
+                rem ^= frontier;
+                const bool is_lo = (lower & frontier) != 0;
+                kind = is_lo ? lower : ~lower;
+                if (is_lo) lo++; else up++;
             }
-            rem &= ~comp;
-            if (is_lo) lo++; else up++;
+            const int j = first(frontier);
+            frontier &= frontier - 1;
+            const M nb = __ldg(adj + b + j) & kind & rem;
+            rem ^= nb;
+            frontier |= nb;
         }
     }
     unsigned code;
@@ -562,17 +612,20 @@ void classify(const LinkGraph &g, const F *field, const int32_t *vpos, int64_t v
     // by id, over the rows as vertices where there are such
     const int32_t *ent = BY_ID && g.ids ? g.ids : g.ent;
     const int32_t *to_id = BY_ID && g.ids ? nullptr : g.order;
+    // (positions are ids, or a range by vertex: those rows lie anywhere)
+    const int64_t h0 = g.heavy0, hn = g.order && !vpos ? std::min(g.n_heavy, g.heavy0 / 32) : 0;
     if (!g.padded)
         launch_pdl(k_crit_classify<F, unsigned long long, false, BY_ID>, grid, kClassifyThreads, 0, s,
                    g.off, ent, (const unsigned long long *)g.adj, field, g.order, to_id, vpos, v0, nv,
-                   classes3);
+                   h0, hn, classes3);
     else if (g.wide)
         launch_pdl(k_crit_classify<F, unsigned long long, true, BY_ID>, grid, kClassifyThreads, 0, s,
                    g.off, ent, (const unsigned long long *)g.adj, field, g.order, to_id, vpos, v0, nv,
-                   classes3);
+                   h0, hn, classes3);
     else
         launch_pdl(k_crit_classify<F, unsigned, true, BY_ID>, grid, kClassifyThreads, 0, s, g.off, ent,
-                   (const unsigned *)g.adj, field, g.order, to_id, vpos, v0, nv, classes3);
+                   (const unsigned *)g.adj, field, g.order, to_id, vpos, v0, nv, h0, hn,
+                   classes3);
 }
 
 template <typename F>

@@ -339,6 +339,7 @@ struct LinkGraph {
     bool wide;                     // a row holds more than 32 entries (always so if not padded)
     bool padded;
     const int32_t *ids;            // the rows as vertices (small meshes), or null
+    int64_t heavy0, n_heavy;       // positions of the heavy stars (with an order)
 };
 // From this many vertices on a field is put in processing order for its
 // classification; the rows of smaller meshes are there as vertices too

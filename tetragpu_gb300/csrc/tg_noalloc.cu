@@ -108,7 +108,7 @@ extern "C" tg_status tg_critical_points_noalloc(const int64_t *vv_off, const int
     if (e != cudaSuccess) return fail(TG_ERR_CUDA, "clearing the status word", e);
     tg::launch_window_starts(vv_off, n_verts, n_vv_entries, tg::crit_window(), (int32_t *)win, s);
     // (no processing order to renumber VV into: positions are ids)
-    const tg::LinkGraph g{n_verts, n_vv_entries, vv_off, vv, nullptr, nullptr, adj, true, false, nullptr};
+    const tg::LinkGraph g{n_verts, n_vv_entries, vv_off, vv, nullptr, nullptr, adj, true, false, nullptr, 0, 0};
     tg::launch_crit_adj(g, (const int32_t *)win, (tg::DevStatus *)status, 2, s);
     tg::launch_crit_classify(g, field, field_type, nullptr, 0, n_verts, classes_out, s);
     e = cudaGetLastError();
