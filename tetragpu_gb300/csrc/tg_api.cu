@@ -850,24 +850,31 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
     }
 
     if ((mask & TG_TT) && tt_vertex) {
-        int32_t *cnt, *tt;
+        int32_t *cnt, *tt, *far = nullptr, *n_far = nullptr;
         int64_t *tt_off;
         BlockRef hold_off, hold_ent;
         Plan t, o;
+        size_t zero = 0;
+        if (const int64_t n = tt_far_tiles(T)) {
+            t.add(&n_far, 1);
+            zero = t.bytes;
+            t.add(&far, n);
+        }
         t.add(&cnt, T);
         o.add(&tt_off, T + 1);
-        TRY(tmp.add(t));
+        TRY(tmp.add(t, zero));
         TRY(take_block(o, m, s, &hold_off));
-        launch_tt_vertex_count(m->tvs, T, vt_off, vt, cnt, s);
+        launch_tt_vertex_count(m->tvs, T, vt_off, vt, far, n_far, cnt, s);
         ScanJob job{cnt, tt_off, T, SCAN_COUNT_I32, nullptr};
         scan_batch(&job, 1, m->scan, m->st, s);
-        const void *src[1] = {tt_off + T};
-        const bool w8[1] = {true};
-        TRY(sync_read(m, s, 1, src, w8));
+        const void *src[2] = {tt_off + T, n_far};
+        const bool w8[2] = {true, false};
+        TRY(sync_read(m, s, far ? 2 : 1, src, w8));
+        const int64_t listed = far ? m->sz_host[1] : 0;
         Plan e;
         e.add(&tt, m->sz_host[0]);
         TRY(take_block(e, m, s, &hold_ent));
-        launch_tt_vertex_fill(m->tvs, T, vt_off, vt, tt_off, tt, s);
+        launch_tt_vertex_fill(m->tvs, T, vt_off, vt, far, n_far, listed, tt_off, tt, s);
         set_csr(m, TG_REL_TT, tt_off, tt, T, m->sz_host[0], hold_off, hold_ent,
                 TG_OPT_TT_VERTEX_SHARING);
     }

@@ -22,7 +22,7 @@
 //   k_cell_tt      face-sharing TT
 //   k_face_fill    FE (from TE of a face's first cell), FF
 //   k_ee_fill      EE
-//   k_tt_vertex    vertex-sharing TT
+//   k_tt_vertex, k_tt_vertex_far   vertex-sharing TT
 #include <algorithm>
 #include <climits>
 
@@ -593,8 +593,12 @@ k_ee_fill(const int2 *__restrict__ ev, int64_t E, const int64_t *__restrict__ ei
 // copies its cells' rows into shared memory, a row once (a table of the
 // vertices: 32 cells of a grid name some 28), an INT_MAX after each, and the
 // filling pass collects the warp's rows of TT, which are contiguous, there and
-// writes them out as whole lines.  Cells whose rows do not fit (vertices in
-// very many cells) merge in global memory.  On 40^3 cubes, a tenth coned, ids
+// writes them out as whole lines; where those do not fit, each lane stores its
+// own row as it merges.  Warps whose VT rows do not fit (cells in no order,
+// vertices in very many cells) leave their cells to k_tt_vertex_far, which
+// merges in global memory with a full SM of warps and the rows' heads in
+// registers (64^3 cubes, cells scattered: 0.81 ms a pass; 5.6 here, with the
+// twelve warps an SM that the stage leaves).  On 40^3 cubes, a tenth coned, ids
 // permuted (0.42 M cells, 70 entries each): 145 us for the two passes (400
 // merging in global memory throughout), bounded by the shared-memory merges
 // (load / store pipe 67 % busy counting; filling, four blocks to an SM by what
@@ -611,25 +615,23 @@ struct TtStage {
 };
 // the cell's merge in global memory
 template <bool FILL>
-__device__ __noinline__ void tt_merge_global(const int4 w, int c, const int64_t *__restrict__ vt_off,
+__device__ __forceinline__ void tt_merge_far(const int4 w, int c, const int64_t *__restrict__ vt_off,
                                              const int *__restrict__ vt, int *cnt, int *out)
 {
-    int64_t pos[4], stop[4];
+    int pos[4], stop[4], h[4];   // VT has 4T entries: below 2^31
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        pos[k] = vt_off[get4(w, k)];
-        stop[k] = vt_off[get4(w, k) + 1];
+        pos[k] = (int)vt_off[get4(w, k)];
+        stop[k] = (int)vt_off[get4(w, k) + 1];
+        h[k] = pos[k] < stop[k] ? vt[pos[k]] : INT_MAX;
     }
     int n = 0;
     while (true) {
-        int m = INT_MAX;
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-            if (pos[k] < stop[k]) m = min(m, vt[pos[k]]);
+        const int m = min(min(h[0], h[1]), min(h[2], h[3]));
         if (m == INT_MAX) break;
 #pragma unroll
         for (int k = 0; k < 4; k++)
-            if (pos[k] < stop[k] && vt[pos[k]] == m) pos[k]++;
+            if (h[k] == m) h[k] = ++pos[k] < stop[k] ? vt[pos[k]] : INT_MAX;
         if (m != c) {
             if (FILL) out[n] = m;
             n++;
@@ -637,12 +639,38 @@ __device__ __noinline__ void tt_merge_global(const int4 w, int c, const int64_t 
     }
     if (!FILL) *cnt = n;
 }
+template <bool FILL>
+__device__ __noinline__ void tt_merge_global(const int4 w, int c, const int64_t *__restrict__ vt_off,
+                                             const int *__restrict__ vt, int *cnt, int *out)
+{
+    tt_merge_far<FILL>(w, c, vt_off, vt, cnt, out);
+}
 
+// a warp per 32 cells that k_tt_vertex listed
+template <bool FILL>
+__global__ void __launch_bounds__(256)
+k_tt_vertex_far(const int4 *__restrict__ tvs, int64_t T, const int64_t *__restrict__ vt_off,
+                const int *__restrict__ vt, const int *__restrict__ far, const int *__restrict__ n_far,
+                int *__restrict__ cnt, const int64_t *__restrict__ tt_off, int *__restrict__ tt)
+{
+    griddep_wait();
+    const int n = *n_far;
+    for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n;
+         i += (int64_t)gridDim.x * (blockDim.x >> 5)) {
+        const int64_t c = 32LL * far[i] + (threadIdx.x & 31);
+        if (c < T)
+            tt_merge_far<FILL>(tvs[c], (int)c, vt_off, vt, FILL ? nullptr : cnt + c,
+                               FILL ? tt + tt_off[c] : nullptr);
+    }
+}
+
+// far, n_far: where the warps whose rows do not fit are listed; far null: they
+// merge in global memory themselves (n_far null) or are left out
 template <bool FILL>
 __global__ void __launch_bounds__(32 * kTtWarps)
 k_tt_vertex(const int4 *__restrict__ tvs, int64_t T, const int64_t *__restrict__ vt_off,
-            const int *__restrict__ vt, int *__restrict__ cnt, const int64_t *__restrict__ tt_off,
-            int *__restrict__ tt)
+            const int *__restrict__ vt, int *__restrict__ far, int *__restrict__ n_far, int *__restrict__ cnt,
+            const int64_t *__restrict__ tt_off, int *__restrict__ tt)
 {
     griddep_wait();
     __shared__ TtStage s_stage[kTtWarps];
@@ -673,15 +701,24 @@ k_tt_vertex(const int4 *__restrict__ tvs, int64_t T, const int64_t *__restrict__
         }
     }
     int64_t o0 = 0, o = 0;
-    bool fits = true;
+    bool collect = false;   // the warp's rows of TT fit what it collects
     if (FILL) {
         o0 = tt_off[c0];
         o = tt_off[min(c, T)];
-        fits = tt_off[min(c0 + 32, T)] - o0 + 4 <= kTtOut;
+        collect = tt_off[min(c0 + 32, T)] - o0 + 4 <= kTtOut;
     }
     __syncwarp();
-    // the rows, a lane each, then eight lanes to each of four to copy them
     const int rows = S.n;
+    bool fits = true;
+    if (rows > 32) {   // before any is copied
+        int words = 0;
+        for (int r = lane; r < rows; r += 32) {
+            const int v = S.key[S.row[r]];
+            words += 1 + (int)min(vt_off[v + 1] - vt_off[v], (int64_t)kTtLists);
+        }
+        fits = __reduce_add_sync(kFull, words) <= kTtLists;
+    }
+    // the rows, a lane each, then eight lanes to each of four to copy them
     int total = 0;
     for (int r0 = 0; r0 < rows && fits; r0 += 32) {
         int64_t src = 0;
@@ -714,8 +751,11 @@ k_tt_vertex(const int4 *__restrict__ tvs, int64_t T, const int64_t *__restrict__
         }
     }
     if (!fits) {   // warp-uniform
-        if (c < T)
+        if (far) {
+            if (lane == 0) far[atomicAdd(n_far, 1)] = (int)(c0 >> 5);
+        } else if (!n_far && c < T) {
             tt_merge_global<FILL>(w, (int)c, vt_off, vt, FILL ? nullptr : cnt + c, FILL ? tt + o : nullptr);
+        }
         return;
     }
     __syncwarp();
@@ -726,23 +766,30 @@ k_tt_vertex(const int4 *__restrict__ tvs, int64_t T, const int64_t *__restrict__
         h[k] = c < T ? S.list[p[k]] : INT_MAX;
     }
     const int shift = (int)(o0 & 3);   // word i collected is word i of the line o0 is in
-    int *out = FILL ? s_out[wp] + shift + (int)(o - o0) : nullptr;
     int n = 0;
-    while (true) {
-        const int m = min(min(h[0], h[1]), min(h[2], h[3]));
-        if (m == INT_MAX) break;
+    auto merge = [&](int *out) {
+        while (true) {
+            const int m = min(min(h[0], h[1]), min(h[2], h[3]));
+            if (m == INT_MAX) break;
 #pragma unroll
-        for (int k = 0; k < 4; k++)
-            if (h[k] == m) h[k] = S.list[++p[k]];
-        if (m != (int)c) {
-            if (FILL) out[n] = m;
-            n++;
+            for (int k = 0; k < 4; k++)
+                if (h[k] == m) h[k] = S.list[++p[k]];
+            if (m != (int)c) {
+                if (FILL) out[n] = m;
+                n++;
+            }
         }
-    }
+    };
     if (!FILL) {
+        merge(nullptr);
         if (c < T) cnt[c] = n;
         return;
     }
+    if (!collect) {   // warp-uniform
+        merge(tt + o);
+        return;
+    }
+    merge(s_out[wp] + shift + (int)(o - o0));
     __syncwarp();
     const int stop = __reduce_max_sync(kFull, c < T ? shift + (int)(o - o0) + n : 0);
     int *line = tt + (o0 - shift);
@@ -929,23 +976,41 @@ void launch_ee_fill(const int32_t *ev, int64_t E, const int64_t *eid_off, const 
                eid, ee_off, ee);
 }
 
+// Below kTtFar cells every warp is on the GPU at once whichever kernel has it: no
+// list.
+constexpr int64_t kTtFar = 1 << 16;
+int64_t tt_far_tiles(int64_t T) { return T >= kTtFar ? (T + 31) / 32 : 0; }
+
 void launch_tt_vertex_count(const int4 *tvs, int64_t T, const int64_t *vt_off, const int32_t *vt,
-                            int32_t *cnt, cudaStream_t s)
+                            int32_t *far, int32_t *n_far, int32_t *cnt, cudaStream_t s)
 {
     if (T == 0) return;
     {
         Launch L("k_tt_vertex", s);
-        launch_pdl(k_tt_vertex<false>, blocks_for(T, 32 * kTtWarps), 32 * kTtWarps, 0, s, tvs, T, vt_off, vt, cnt, nullptr, nullptr);
+        launch_pdl(k_tt_vertex<false>, blocks_for(T, 32 * kTtWarps), 32 * kTtWarps, 0, s, tvs, T, vt_off, vt,
+                   far, n_far, cnt, nullptr, nullptr);
+    }
+    if (far) {   // (how many there are is known on the device)
+        Launch L("k_tt_vertex_far", s);
+        launch_pdl(k_tt_vertex_far<false>, (unsigned)std::min<int64_t>((T + 255) / 256, 152 * 8), 256, 0, s,
+                   tvs, T, vt_off, vt, (const int *)far, (const int *)n_far, cnt, nullptr, nullptr);
     }
 }
 
 void launch_tt_vertex_fill(const int4 *tvs, int64_t T, const int64_t *vt_off, const int32_t *vt,
-                           const int64_t *tt_off, int32_t *tt, cudaStream_t s)
+                           const int32_t *far, int32_t *n_far, int64_t listed, const int64_t *tt_off,
+                           int32_t *tt, cudaStream_t s)
 {
     if (T == 0) return;
-    {
+    if (listed < (T + 31) / 32) {
         Launch L("k_tt_vertex", s);
-        launch_pdl(k_tt_vertex<true>, blocks_for(T, 32 * kTtWarps), 32 * kTtWarps, 0, s, tvs, T, vt_off, vt, nullptr, tt_off, tt);
+        launch_pdl(k_tt_vertex<true>, blocks_for(T, 32 * kTtWarps), 32 * kTtWarps, 0, s, tvs, T, vt_off, vt,
+                   nullptr, n_far, nullptr, tt_off, tt);
+    }
+    if (listed > 0) {
+        Launch L("k_tt_vertex_far", s);
+        launch_pdl(k_tt_vertex_far<true>, blocks_for(32 * listed, 256), 256, 0, s, tvs, T, vt_off, vt, far,
+                   (const int *)n_far, nullptr, tt_off, tt);
     }
 }
 
