@@ -112,6 +112,7 @@ tg_status cuda_fail(cudaError_t e, const char *what, int line)
     } while (0)
 
 constexpr int64_t kMaxCells = 357913941LL;  // 6 * cells must fit in 31 bits
+constexpr int64_t kFewRecords = 1 << 20;    // cells from which room for edge records is tight
 
 // Where memory comes from: the device's default stream-ordered pool for what a
 // mesh keeps, a pool of the library's own for temporaries.  Out of one pool, a
@@ -329,10 +330,17 @@ tg_status take(size_t bytes, cudaStream_t s, void **out, bool temp = false, bool
                       : cudaMallocAsync(out, bytes, s);
     if (e == cudaErrorMemoryAllocation && p && need && !capturing(s)) {
         (void)cudaGetLastError();
-        // what was freed on this stream counts once the stream is through
+        // what was freed on this stream counts once the stream is through; what
+        // lies idle in either pool goes back to the device
         cudaStreamSynchronize(s);
-        cudaMemPoolTrimTo(temp ? p->keep : p->temp, 0);
+        cudaMemPoolTrimTo(p->keep, 0);
+        cudaMemPoolTrimTo(p->temp, 0);
         e = cudaMallocFromPoolAsync(out, bytes, temp ? p->temp : p->keep, s);
+        if (e == cudaErrorMemoryAllocation) {
+            // blocks freed on streams that are still running serve their pool only
+            (void)cudaGetLastError();
+            e = cudaMallocFromPoolAsync(out, bytes, temp ? p->keep : p->temp, s);
+        }
     }
     return e == cudaSuccess ? TG_OK : cuda_fail(e, "cudaMallocFromPoolAsync", __LINE__);
 }
@@ -358,6 +366,8 @@ struct Temps {
     {
         for (int i = 0; i < n; i++) cudaFreeAsync(p[i], s);
     }
+    // the last plan's arrays go back
+    void drop() { cudaFreeAsync(p[--n], s); }
     // a plan's arrays; the first zero_bytes zeroed
     tg_status add(const Plan &plan, size_t zero_bytes = 0, bool need = true)
     {
@@ -644,7 +654,6 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         // the status is clean: the read-back that ended the last call reset it
         // ---- star pass: first occurrences, edge records, neighbour counts ----
         const int64_t nwe = (6 * T + 31) / 32, nwf = (4 * T + 31) / 32;
-        uint32_t *eflag, *fflag, *fbnd;
         uint2 *erank, *frank, *brank;
         int64_t *vv_off;
         // FE is read off each face's first cell (k_face_fill), which the
@@ -659,33 +668,6 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         StarPass sp{};
         HeavyStars hv{};
         int64_t *deg_sq, *eid_off = nullptr;
-        {
-            // the bitmaps the star pass sets bits in, the neighbour counts
-            // and the record counter are zeroed
-            Plan t;
-            t.add(&eflag, nwe);
-            t.add(&fflag, nwf);
-            t.add(&fbnd, nwf);
-            t.add(&sp.deg_own, V);
-            t.add(&sp.deg_in, V);
-            t.add(&sp.vbnd, V);
-            t.add(&sp.n_rec, 2);
-            const size_t zero = t.bytes;
-            t.add(&erank, nwe + 1);
-            t.add(&frank, nwf + 1);
-            t.add(&brank, nwf + 1);
-            t.add(&deg_sq, V + 1);   // prefix of deg^2: its total sizes EE (sum deg^2 - 2E)
-            if (want_ee) t.add(&eid_off, V + 1);   // EE's incident-edge rows are padded
-            // at most six edges a cell (their number is read back below)
-            t.add(&sp.rec, 6 * T);
-            t.add(&sp.place, 6 * T);
-            if (m->n_wide > 0 || m->n_heavy > 0) t.add(&sp.rec_hi, 6 * T);
-            if (m->n_wide > 0) t.add(&sp.wide, m->n_wide);
-            if (m->n_heavy > 0) t.add(&hv.pairs, 3 * m->heavy_entries);
-            if (need_tf || need_ft) t.add(&sp.fnext, 4 * T);
-            TRY(tmp.add(t, zero));
-            sp.n_wide = sp.n_rec + 1;
-        }
         BlockRef hold_vv_off, hold_vv, hold_tt, hold;
         {
             Plan o;
@@ -697,35 +679,62 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         sp.vt_off = vt_off;
         sp.vt = vt;
         sp.tvs = m->tvs;
-        sp.eflag = eflag;
-        sp.fflag = fflag;
-        sp.fbnd = fbnd;
         sp.st = m->st;
-        launch_star(sp, s);
-        launch_star_wide(sp, m->n_wide, s);
-        if (m->n_heavy > 0) {
-            hv.star = sp;
-            hv.n_heavy = m->n_heavy;
-            hv.heavy_off = m->heavy_off;
-            launch_heavy(hv, s);
-        }
-        ScanJob jobs[6] = {{sp.deg_own, vv_off, V, SCAN_COUNT_I32, sp.deg_in},
-                           {eflag, erank, nwe, SCAN_POPC_RANK, nullptr},
-                           {fflag, frank, nwf, SCAN_POPC_RANK, nullptr},
-                           {fbnd, brank, nwf, SCAN_POPC_RANK, nullptr},
-                           {sp.deg_own, deg_sq, V, SCAN_DEG_SQUARE, sp.deg_in},
-                           {sp.deg_own, eid_off, V, SCAN_EID_WORDS, sp.deg_in}};
-        scan_batch(jobs, want_ee ? 6 : 5, m->scan, m->st, s);
+        // room for records: a mesh has at most six edges a cell (cells that share
+        // nothing), nearly all have below 1.7; a large mesh that turns out to
+        // have more than two goes through the pass again.  16 to 20 bytes each: all
+        // of six would be 0.8 GB more at 128^3 cubes
+        for (sp.rec_cap = T >= kFewRecords ? 2 * T : 6 * T;; sp.rec_cap = 6 * T) {
+            // the bitmaps the star pass sets bits in, the neighbour counts
+            // and the record counter are zeroed
+            Plan t;
+            t.add(&sp.eflag, nwe);
+            t.add(&sp.fflag, nwf);
+            t.add(&sp.fbnd, nwf);
+            t.add(&sp.deg_own, V);
+            t.add(&sp.deg_in, V);
+            t.add(&sp.vbnd, V);
+            t.add(&sp.n_rec, 2);
+            const size_t zero = t.bytes;
+            t.add(&erank, nwe + 1);
+            t.add(&frank, nwf + 1);
+            t.add(&brank, nwf + 1);
+            t.add(&deg_sq, V + 1);   // prefix of deg^2: its total sizes EE (sum deg^2 - 2E)
+            if (want_ee) t.add(&eid_off, V + 1);   // EE's incident-edge rows are padded
+            t.add(&sp.rec, sp.rec_cap);
+            t.add(&sp.place, sp.rec_cap);
+            if (m->n_wide > 0 || m->n_heavy > 0) t.add(&sp.rec_hi, sp.rec_cap);
+            if (m->n_wide > 0) t.add(&sp.wide, m->n_wide);
+            if (m->n_heavy > 0) t.add(&hv.pairs, 3 * m->heavy_entries);
+            if (need_tf || need_ft) t.add(&sp.fnext, 4 * T);
+            TRY(tmp.add(t, zero));
+            sp.n_wide = sp.n_rec + 1;
+            launch_star(sp, s);
+            launch_star_wide(sp, m->n_wide, s);
+            if (m->n_heavy > 0) {
+                hv.star = sp;
+                hv.n_heavy = m->n_heavy;
+                hv.heavy_off = m->heavy_off;
+                launch_heavy(hv, s);
+            }
+            ScanJob jobs[6] = {{sp.deg_own, vv_off, V, SCAN_COUNT_I32, sp.deg_in},
+                               {sp.eflag, erank, nwe, SCAN_POPC_RANK, nullptr},
+                               {sp.fflag, frank, nwf, SCAN_POPC_RANK, nullptr},
+                               {sp.fbnd, brank, nwf, SCAN_POPC_RANK, nullptr},
+                               {sp.deg_own, deg_sq, V, SCAN_DEG_SQUARE, sp.deg_in},
+                               {sp.deg_own, eid_off, V, SCAN_EID_WORDS, sp.deg_in}};
+            scan_batch(jobs, want_ee ? 6 : 5, m->scan, m->st, s);
 
-        // ---- the one synchronisation: edge, face, neighbour and boundary
-        // counts size every output from here on ----
-        {
-            const void *src[5] = {vv_off + V, &erank[nwe].y, &frank[nwf].y, &brank[nwf].y,
-                                  deg_sq + V};
-            const bool w8[5] = {true, false, false, false, true};
-            TRY(sync_read(m, s, 5, src, w8));
+            // ---- the one synchronisation: edge, face, neighbour and boundary
+            // counts size every output from here on ----
+            const void *src[6] = {vv_off + V, &erank[nwe].y, &frank[nwf].y, &brank[nwf].y,
+                                  deg_sq + V, eid_off + V};
+            const bool w8[6] = {true, false, false, false, true, true};
+            TRY(sync_read(m, s, want_ee ? 6 : 5, src, w8));
+            if (m->st_host->flags) return check_flags(m);
+            if (m->sz_host[1] <= sp.rec_cap) break;
+            tmp.drop();
         }
-        if (m->st_host->flags) return check_flags(m);
         m->max_deg = m->st_host->max_deg > kMaxDeg ? m->st_host->max_deg : 0;
         m->wide_deg = m->st_host->max_deg > kNarrowDeg;
         const int largest_deg = m->st_host->max_deg;
@@ -755,7 +764,7 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
             Plan t, o, ovv, ott;
             ovv.add(&vv, nvv);
             if (want_ee) {
-                t.add(&eid, nvv + 16 * V);   // eid_words of each row at most
+                t.add(&eid, m->sz_host[5]);
                 t.add(&inc, nvv);
             }
             if (need_edge) t.add(&ep.edge, E);
@@ -799,7 +808,7 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         ep.rec = sp.rec; ep.place = sp.place; ep.rec_hi = sp.rec_hi; ep.pairs = hv.pairs;
         ep.vt_off = vt_off; ep.vt = vt; ep.tvs = m->tvs;
         ep.erank = need_edge ? erank : nullptr;
-        ep.frank = frank; ep.fbnd = fbnd; ep.vbnd = sp.vbnd;
+        ep.frank = frank; ep.fbnd = sp.fbnd; ep.vbnd = sp.vbnd;
         ep.vv_off = vv_off; ep.inc = inc; ep.vv = vv;
         ep.count_ef = (mask & TG_EF) != 0;
         launch_edge_ids(ep, s);

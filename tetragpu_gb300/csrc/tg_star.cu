@@ -137,6 +137,7 @@ __device__ __forceinline__ void put_edges(const StarPass &p, const RecBuf<H> &S,
         const unsigned slot = (unsigned)(6 * c + pair_slot(sv, su));
         atomicOr(p.eflag + (slot >> 5), 1u << (slot & 31));
         const int64_t g = (int64_t)base + i;
+        if (g >= p.rec_cap) continue;
         p.rec[g] = make_uint2(slot, e.x);
         p.place[g] = make_uint2(place, in);
         if constexpr (H == 2) p.rec_hi[g] = hi;
