@@ -320,14 +320,15 @@ struct Plan {
 
 // from the pool of kept memory (temp false) or of temporaries; need false: the
 // caller can do without, so the call waits for nothing
-tg_status take(size_t bytes, cudaStream_t s, void **out, bool temp = false, bool need = true)
+cudaError_t take_cuda(size_t bytes, cudaStream_t s, void **out, bool temp, bool need)
 {
     bytes = std::max<size_t>(bytes, 256);
     int dev = 0;
-    CK(cudaGetDevice(&dev));
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
     const Pools *p = device_pools(dev);
-    cudaError_t e = p ? cudaMallocFromPoolAsync(out, bytes, temp ? p->temp : p->keep, s)
-                      : cudaMallocAsync(out, bytes, s);
+    e = p ? cudaMallocFromPoolAsync(out, bytes, temp ? p->temp : p->keep, s)
+          : cudaMallocAsync(out, bytes, s);
     if (e == cudaErrorMemoryAllocation && p && need && !capturing(s)) {
         (void)cudaGetLastError();
         // what was freed on this stream counts once the stream is through; what
@@ -342,6 +343,11 @@ tg_status take(size_t bytes, cudaStream_t s, void **out, bool temp = false, bool
             e = cudaMallocFromPoolAsync(out, bytes, temp ? p->keep : p->temp, s);
         }
     }
+    return e;
+}
+tg_status take(size_t bytes, cudaStream_t s, void **out, bool temp = false, bool need = true)
+{
+    const cudaError_t e = take_cuda(bytes, s, out, temp, need);
     return e == cudaSuccess ? TG_OK : cuda_fail(e, "cudaMallocFromPoolAsync", __LINE__);
 }
 
@@ -1471,7 +1477,10 @@ tg_status tg::link_rows_used(tg_mesh *m, cudaStream_t s)
 void tg::note_stream(tg_mesh *m, cudaStream_t s) { m->last_stream.store(s, std::memory_order_relaxed); }
 
 // internal: temporaries and segments (tg_batch.cu)
-tg_status tg::take_temp(size_t bytes, cudaStream_t s, void **out) { return take(bytes, s, out, true); }
+cudaError_t tg::take_temp(size_t bytes, cudaStream_t s, void **out)
+{
+    return take_cuda(bytes, s, out, true, true);
+}
 
 tg_status tg::mesh_set_segments(tg_mesh *m, const int64_t *seg_c_host, int64_t n, cudaStream_t s)
 {

@@ -91,7 +91,7 @@ tg_status bfail(tg_status code, const char *msg)
 template <class T>
 cudaError_t temp(size_t bytes, cudaStream_t s, T **out)
 {
-    return take_temp(bytes, s, (void **)out) == TG_OK ? cudaSuccess : cudaErrorMemoryAllocation;
+    return take_temp(bytes, s, (void **)out);
 }
 
 #define TRY_B(call)                                                                 \

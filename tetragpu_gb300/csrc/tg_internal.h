@@ -386,7 +386,7 @@ bool capturing(cudaStream_t s);
 void launch_field_in_order(const float *field, const int32_t *order, int64_t V, float *out,
                            cudaStream_t s);
 // a temporary from the library's own pool (freed with cudaFreeAsync)
-tg_status take_temp(size_t bytes, cudaStream_t s, void **out);
+cudaError_t take_temp(size_t bytes, cudaStream_t s, void **out);
 // Cell segments of a mesh (the meshes of a batch, tg_batch.cu): seg_c_host
 // holds n + 1 cell starts; each extraction then fills n + 1 first edge ids
 // followed by n + 1 first face ids (device, read by mesh_segment_ids).
