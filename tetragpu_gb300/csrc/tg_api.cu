@@ -17,6 +17,7 @@
 #include <cstring>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -357,7 +358,12 @@ tg_status take_block(const Plan &plan, const tg_mesh *m, cudaStream_t s, BlockRe
     if (plan.n == 0) return TG_OK;
     void *q = nullptr;
     TRY(take(plan.bytes, s, &q, false, need));
-    *out = std::make_shared<Block>(q, m);
+    try {
+        *out = std::make_shared<Block>(q, m);
+    } catch (const std::bad_alloc &) {
+        cudaFreeAsync(q, s);
+        return fail(TG_ERR_OUT_OF_MEMORY, "host memory");
+    }
     plan.place(q);
     return TG_OK;
 }
