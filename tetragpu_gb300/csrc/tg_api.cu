@@ -473,10 +473,10 @@ tg_status sync_read(tg_mesh *m, cudaStream_t s, int n, const void *const *src, c
     return TG_OK;
 }
 
-tg_status check_flags(const tg_mesh *m, unsigned mask_ok = 0)
+tg_status check_flags(const tg_mesh *m)
 {
     const DevStatus &h = *m->st_host;
-    const unsigned f = h.flags & ~mask_ok;
+    const unsigned f = h.flags;
     if (!f) return TG_OK;
     auto lowest = [](int noted) { return INT_MAX - noted; };
     if (f & ST_BAD_ID)
@@ -487,16 +487,6 @@ tg_status check_flags(const tg_mesh *m, unsigned mask_ok = 0)
     if (f & ST_NONMANIFOLD_FACE)
         return fail(TG_ERR_INVALID_MESH, "a face of cell %d lies in more than two cells",
                     lowest(h.bad_cell));
-    if (f & ST_HEAVY_STAR)
-        return fail(TG_ERR_UNSUPPORTED,
-                    "vertex %d lies in more than %d cells (largest star this build handles)",
-                    lowest(h.bad_vertex), kMaxStar);
-    if (f & ST_HEAVY_DEG)
-        return fail(TG_ERR_UNSUPPORTED,
-                    "a vertex has %d neighbours (more than %d, the largest this build handles)",
-                    h.max_deg, kMaxDeg);
-    if (f & ST_HASH_FULL)
-        return fail(TG_ERR_UNSUPPORTED, "vertex %d: neighbour table overflow", lowest(h.bad_vertex));
     if (f & ST_STAR_OVERFLOW)
         return fail(TG_ERR_UNSUPPORTED, "vertex %d: neighbour summary overflow", lowest(h.bad_vertex));
     if (f & ST_SCAN_STALLED)

@@ -17,19 +17,16 @@ struct DevStatus {
     unsigned int flags;
     int bad_cell;      // INT_MAX - the lowest offending cell (note_lowest), 0 if none
     int bad_vertex;    // the same of vertices
-    int max_star;      // largest number of cells around a vertex
     int max_deg;       // largest number of neighbours of a vertex
-    int pad[3];
+    int pad[4];
 };
 
 enum StatusFlag : unsigned int {
     ST_BAD_ID = 1u,            // vertex id outside [0, n_verts)
     ST_DUP_VERTEX = 2u,        // a cell repeats a vertex
-    ST_HEAVY_STAR = 4u,        // a vertex lies in more cells than the star kernels hold
-    ST_STAR_OVERFLOW = 8u,     // more neighbours than the summary slot holds
+    ST_STAR_OVERFLOW = 8u,     // an edge lies in more cells than the row lengths hold
     ST_NONMANIFOLD_FACE = 16u, // a face lies in more than two cells
-    ST_HASH_FULL = 32u,        // per-vertex neighbour table overflowed
-    ST_HEAVY_DEG = 64u,        // a vertex has more neighbours than the kernels hold
+    ST_HEAVY_DEG = 64u,        // a vertex has more neighbours than the link masks hold (tg_noalloc.cu)
     ST_SCAN_STALLED = 128u     // a scan tile gave up waiting for the tiles before it
 };
 
@@ -139,10 +136,6 @@ __device__ __forceinline__ long long look_back(unsigned long long *w, long long 
 #endif
 
 // ---- pipeline kernels (tg_kernels.cu) ----
-struct Sizes {
-    int64_t V, T;
-};
-
 // Status word and up to 8 sizes (int64, or int32 sign-extended) stored by a
 // kernel into device-mapped pinned host memory (no copy engine involved)
 struct PublishArgs {

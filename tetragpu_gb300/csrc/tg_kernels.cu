@@ -911,7 +911,6 @@ __global__ void k_publish(PublishArgs a)
     a.st->flags = 0;
     a.st->bad_cell = 0;
     a.st->bad_vertex = 0;
-    a.st->max_star = 0;
     a.st->max_deg = 0;
 }
 
