@@ -1095,7 +1095,8 @@ static tg_status mesh_create_impl(const int32_t *tv, int64_t T, int64_t V, int o
                            {hflag, hrank, nwh, SCAN_POPC_RANK, nullptr}};
     scan_batch(jf, 2, m->scan, m->st, s);
     launch_vorder_place(vt_off, V, vkey, vrank, nwk, hrank, heavy_cnt, m->heavy_off, m->vorder, m->vpos, s);
-    if (V >= kOrderField) launch_order_lines(T, m->tvs, m->vpos, heavy_cnt + 4, s);
+    if (V >= kOrderField)
+        launch_order_lines(V, vt_off, vt, m->tvs, m->vorder, m->vpos, heavy_cnt + 4, s);
     CK(cudaGetLastError());
     set_csr(m, TG_REL_VT, vt_off, vt, V, 4 * T, nullptr, nullptr);
     // vertices with light stars, heavy ones, the heavy stars' entries and
@@ -1107,13 +1108,13 @@ static tg_status mesh_create_impl(const int32_t *tv, int64_t T, int64_t V, int o
     m->n_heavy = T ? m->sz_host[1] : 0;
     m->heavy_entries = T ? m->sz_host[2] : 0;
     m->n_wide = T ? m->sz_host[3] : 0;
-    // VV in star order pays where that keeps a run of cells on well fewer lines
-    // than ids do: 0.15 to 0.25 of them where cells lie together and ids do not,
-    // 0.5 on a Delaunay mesh in no special order, 0.8 to 1.5 where ids are in
-    // order or cells are not.  A field on 64^3 cubes, cells scattered and ids in
-    // order: 21 us by id, 30 by position; a float64 field on 128^3, both in
-    // order: 130 and 143.  The count is a launch: 4 us of 100 to 200 at 64^3
-    m->lg_by_id = 4 * m->sz_host[5] > 3 * m->sz_host[4];
+    // VV in star order pays where that keeps a run of vertices' neighbours on well
+    // fewer lines than ids do.  By id and by position on 64^3 cubes: 14 and 14
+    // with both in order, 274 and 14 with ids permuted, 14 and 155 with cells
+    // scattered, 274 and 155 with both; on a Delaunay mesh of random points 292
+    // and 88.  A field on 64^3, cells scattered and ids in order: 18 us by id, 30
+    // by position.  The count is a launch: 4 us of 100 to 200 at 64^3
+    m->lg_by_id = 2 * m->sz_host[5] > m->sz_host[4];
     return check_flags(m);
 }
 

@@ -200,10 +200,11 @@ void launch_vorder_place(const int64_t *vt_off, int64_t V, const int64_t *vkey, 
                          int64_t nwk, const uint2 *hrank, int32_t *heavy_cnt, int32_t *heavy_off,
                          int32_t *vorder, int32_t *vpos, cudaStream_t s);
 // Whether positions or ids keep neighbours together: the lines of 32 vertices
-// that a run of 32 cells names, by id added to lines[0] and by position to
-// lines[1], over kOrderTiles runs spread over the mesh (fewer cells: none).
-constexpr int kOrderTiles = 256;
-void launch_order_lines(int64_t T, const int4 *tvs, const int32_t *vpos, int32_t *lines, cudaStream_t s);
+// that the cells of kOrderRuns runs of 32 vertices name, by id added to lines[0]
+// and by position to lines[1] (fewer vertices: nothing).
+constexpr int kOrderRuns = 128;
+void launch_order_lines(int64_t V, const int64_t *vt_off, const int32_t *vt, const int4 *tvs,
+                        const int32_t *vorder, const int32_t *vpos, int32_t *lines, cudaStream_t s);
 
 // Star pass (tg_star.cu): the edges and faces of the light vertices.
 struct StarPass {

@@ -1027,40 +1027,47 @@ k_vorder_place(const int64_t *__restrict__ vt_off, int64_t V, const int64_t *__r
     vpos[v] = (int)pos;
 }
 
-// A warp per run of 32 cells: how many lines of 32 vertices (32 words of a
-// field) its cells name, by id and by position; counted as the bits set in a
-// bitmap that the lines hash to (at most 128 in 4,096: 1.5% meet another).
+// How far apart neighbours lie by id and by position: the lines of 32 vertices
+// (32 words of a field) that the cells of 32 consecutive vertices name, a warp
+// per run of them and four cells a vertex; counted as the bits set in a bitmap
+// that the lines hash to.
 constexpr int kLinesWarps = 4;
 __global__ void __launch_bounds__(32 * kLinesWarps)
-k_order_lines(int64_t T, const int4 *__restrict__ tvs, const int *__restrict__ vpos, int *__restrict__ lines)
+k_order_lines(int64_t V, const int64_t *__restrict__ vt_off, const int *__restrict__ vt,
+              const int4 *__restrict__ tvs, const int *__restrict__ vorder, const int *__restrict__ vpos,
+              int *__restrict__ lines)
 {
     griddep_wait();
-    __shared__ unsigned s_bits[kLinesWarps][2][128];
+    __shared__ unsigned s_bits[kLinesWarps][128];
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     const int i = blockIdx.x * kLinesWarps + wp;
-    const int4 w = __ldg(tvs + 32 * (T / 32 * i / kOrderTiles) + lane);
+    const bool by_pos = i & 1;
+    const int64_t at = 32 * (V / 32 * (i >> 1) / kOrderRuns) + lane;
 #pragma unroll
-    for (int k = 0; k < 8; k++) s_bits[wp][k >> 2][32 * (k & 3) + lane] = 0u;
-    int p[4];   // (a rejected cell holds -1s; the mesh is not used then)
-#pragma unroll
-    for (int k = 0; k < 4; k++) p[k] = get4(w, k) < 0 ? 0 : __ldg(vpos + get4(w, k));
+    for (int k = 0; k < 4; k++) s_bits[wp][32 * k + lane] = 0u;
     __syncwarp();
+    const int64_t v = by_pos ? vorder[at] : at;
+    const int64_t b = vt_off[v];
+    const int D = (int)(vt_off[v + 1] - b);
+    if (D > 0) {
+        int4 w[4];
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const unsigned a = (unsigned)(get4(w, k) >> 5) * 0x9E3779B1u >> 20;
-        const unsigned b = (unsigned)(p[k] >> 5) * 0x9E3779B1u >> 20;
-        atomicOr(&s_bits[wp][0][a >> 5], 1u << (a & 31));
-        atomicOr(&s_bits[wp][1][b >> 5], 1u << (b & 31));
+        for (int k = 0; k < 4; k++) w[k] = __ldg(tvs + __ldg(vt + b + (int64_t)D * k / 4));
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                const int u = get4(w[k], t), x = by_pos ? __ldg(vpos + u) : u;
+                const unsigned h = (unsigned)(x >> 5) * 0x9E3779B1u >> 20;
+                atomicOr(&s_bits[wp][h >> 5], 1u << (h & 31));
+            }
     }
     __syncwarp();
+    int n = 0;
 #pragma unroll
-    for (int q = 0; q < 2; q++) {
-        int n = 0;
-#pragma unroll
-        for (int k = 0; k < 4; k++) n += __popc(s_bits[wp][q][32 * k + lane]);
-        n = __reduce_add_sync(kAll, n);
-        if (lane == 0) atomicAdd(lines + q, n);
-    }
+    for (int k = 0; k < 4; k++) n += __popc(s_bits[wp][32 * k + lane]);
+    n = __reduce_add_sync(kAll, n);
+    if (lane == 0) atomicAdd(lines + by_pos, n);
 }
 
 // First edge and face id of each segment of cells (a mesh of a batch):
@@ -1201,12 +1208,14 @@ void launch_vorder_place(const int64_t *vt_off, int64_t V, const int64_t *vkey, 
                hrank, heavy_cnt, heavy_off, vorder, vpos);
 }
 
-void launch_order_lines(int64_t T, const int4 *tvs, const int32_t *vpos, int32_t *lines, cudaStream_t s)
+void launch_order_lines(int64_t V, const int64_t *vt_off, const int32_t *vt, const int4 *tvs,
+                        const int32_t *vorder, const int32_t *vpos, int32_t *lines, cudaStream_t s)
 {
-    if (T / 32 < kOrderTiles) return;
+    if (V / 32 < kOrderRuns) return;
     Launch L("k_order_lines", s);
-    static_assert(kOrderTiles % kLinesWarps == 0, "whole blocks");
-    launch_pdl(k_order_lines, kOrderTiles / kLinesWarps, 32 * kLinesWarps, 0, s, T, tvs, vpos, lines);
+    static_assert(2 * kOrderRuns % kLinesWarps == 0, "whole blocks");
+    launch_pdl(k_order_lines, 2 * kOrderRuns / kLinesWarps, 32 * kLinesWarps, 0, s, V, vt_off, vt, tvs, vorder,
+               vpos, lines);
 }
 
 void launch_seg_ranks(const int64_t *seg_c, int64_t n, const uint2 *erank, const uint2 *frank,
