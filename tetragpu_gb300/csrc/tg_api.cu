@@ -683,10 +683,12 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         sp.tvs = m->tvs;
         sp.st = m->st;
         // room for records: a mesh has at most six edges a cell (cells that share
-        // nothing), nearly all have below 1.7; a large mesh that turns out to
-        // have more than two goes through the pass again.  16 to 20 bytes each: all
-        // of six would be 0.8 GB more at 128^3 cubes
-        for (sp.rec_cap = T >= kFewRecords ? 2 * T : 6 * T;; sp.rec_cap = 6 * T) {
+        // nothing).  Cells glued into manifolds have about T + 2V at most: E = V +
+        // T + half the boundary faces less the Euler characteristic, and a closed
+        // surface has two faces a vertex.  A large mesh that has more goes through
+        // the pass again.  16 to 20 bytes each: all of six would be 0.9 GB more at
+        // 128^3 cubes
+        for (sp.rec_cap = T >= kFewRecords ? std::min(6 * T, T + 2 * V) : 6 * T;; sp.rec_cap = 6 * T) {
             // the bitmaps the star pass sets bits in, the neighbour counts
             // and the record counter are zeroed
             Plan t;
