@@ -435,6 +435,7 @@ struct tg_mesh {
     int64_t n_wide = 0;         // light stars of more than 31 cells (64-bit masks)
     int max_deg = 0;            // largest degree above kMaxDeg seen by the extraction, else 0
     bool wide_deg = false;      // a vertex has more than kNarrowDeg neighbours
+    bool lg_plain = false;       // short rows: the link graph is VV as it is
     bool lg_by_id = false;       // ids keep neighbours as close as positions: positions are ids there
     LinkArrays lg;
     BlockRef lg_rows, lg_masks;
@@ -542,13 +543,13 @@ void free_link_graph(tg_mesh *m)
 }
 
 // entries of the link graph, at most: its rows are padded to multiples of eight
-int64_t link_entries(const tg_mesh *m, int64_t nvv) { return nvv + 7 * m->V; }
+int64_t link_entries(const tg_mesh *m, int64_t nvv) { return m->lg_plain ? nvv : nvv + 7 * m->V; }
 
 LinkGraph link_graph(const tg_mesh *m, const LinkArrays &a, int64_t nvv)
 {
-    return {m->V, link_entries(m, nvv), a.off, a.ent, m->lg_by_id ? nullptr : m->vorder,
-            m->lg_by_id ? nullptr : m->vpos, a.adj, m->wide_deg, true, a.ids,
-            m->n_light, m->n_heavy};
+    const bool by_id = m->lg_by_id || m->lg_plain;
+    return {m->V, link_entries(m, nvv), a.off, a.ent, by_id ? nullptr : m->vorder, by_id ? nullptr : m->vpos,
+            a.adj, m->wide_deg || m->lg_plain, !m->lg_plain, a.ids, m->n_light, m->n_heavy};
 }
 
 // A call may use on one stream what an earlier call built on another.  (Under
@@ -592,6 +593,10 @@ struct LinkBuild {
     {
         const int64_t n = link_entries(m, nvv);
         a = m->lg;
+        if (m->lg_plain && !a.off) {
+            a.off = m->rel[TG_REL_VV].off;
+            a.ent = m->rel[TG_REL_VV].ent;
+        }
         rows = !a.off;
         masks = with_masks && !a.adj;
         Plan t, keep_rows, keep_masks;
@@ -609,7 +614,7 @@ struct LinkBuild {
         }
         if (masks) {
             t.add(&win, window_count(n, crit_window()) + 1);
-            k.add(&a.adj, n * (m->wide_deg ? 8 : 4));
+            k.add(&a.adj, n * (m->wide_deg || m->lg_plain ? 8 : 4));
         }
         BlockRef held_rows, held_masks;
         TRY(tmp.add(t, zero, need));
@@ -741,6 +746,10 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         }
         m->max_deg = m->st_host->max_deg > kMaxDeg ? m->st_host->max_deg : 0;
         m->wide_deg = m->st_host->max_deg > kNarrowDeg;
+        // rows of four entries or fewer on average would be half padding: 1.5M
+        // cells that share nothing, VV and classification 1.90 ms padded, 1.39 as
+        // it is
+        m->lg_plain = m->sz_host[0] <= 4 * (m->n_light + m->n_heavy);
         const int largest_deg = m->st_host->max_deg;
         const int64_t nvv = m->sz_host[0];
         const int64_t E = m->sz_host[1], F = m->sz_host[2];
@@ -868,7 +877,7 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         BlockRef hold_off, hold_ent;
         Plan t, o;
         size_t zero = 0;
-        if (const int64_t n = tt_far_tiles(T)) {
+        if (const int64_t n = tt_far_tiles(T, V)) {
             t.add(&n_far, 1);
             zero = t.bytes;
             t.add(&far, n);
@@ -877,7 +886,7 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         o.add(&tt_off, T + 1);
         TRY(tmp.add(t, zero));
         TRY(take_block(o, m, s, &hold_off));
-        launch_tt_vertex_count(m->tvs, T, vt_off, vt, far, n_far, cnt, s);
+        launch_tt_vertex_count(m->tvs, T, V, vt_off, vt, far, n_far, cnt, s);
         ScanJob job{cnt, tt_off, T, SCAN_COUNT_I32, nullptr};
         scan_batch(&job, 1, m->scan, m->st, s);
         const void *src[2] = {tt_off + T, n_far};
@@ -887,7 +896,7 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         Plan e;
         e.add(&tt, m->sz_host[0]);
         TRY(take_block(e, m, s, &hold_ent));
-        launch_tt_vertex_fill(m->tvs, T, vt_off, vt, far, n_far, listed, tt_off, tt, s);
+        launch_tt_vertex_fill(m->tvs, T, V, vt_off, vt, far, n_far, listed, tt_off, tt, s);
         set_csr(m, TG_REL_TT, tt_off, tt, T, m->sz_host[0], hold_off, hold_ent,
                 TG_OPT_TT_VERTEX_SHARING);
     }
@@ -1425,8 +1434,8 @@ int64_t tg_mesh_device_bytes(const tg_mesh *m)
     }
     b += m->V * 8;
     const int64_t n = link_entries(m, m->rel[TG_REL_VV].entries);
-    if (m->lg.off) b += n * (m->lg.ids ? 8 : 4) + (m->V + 1) * 8;
-    if (m->lg.adj) b += n * (m->wide_deg ? 8 : 4);
+    if (m->lg.off && !m->lg_plain) b += n * (m->lg.ids ? 8 : 4) + (m->V + 1) * 8;
+    if (m->lg.adj) b += n * (m->wide_deg || m->lg_plain ? 8 : 4);
     return b;
 }
 
@@ -1445,7 +1454,7 @@ bool tg::capturing(cudaStream_t s)
 tg_status tg::link_rows(tg_mesh *m, cudaStream_t s, LinkGraph *out)
 {
     *out = LinkGraph{};
-    if (m->lg_by_id) return TG_OK;
+    if (m->lg_by_id || m->lg_plain) return TG_OK;
     const Rel &vv = m->rel[TG_REL_VV];
     std::lock_guard<std::mutex> lk(m->lg_mu);
     if (m->lg.off) {

@@ -295,13 +295,13 @@ void launch_face_fill(const int32_t *ft, const int32_t *tf, const int32_t *te, c
 // max_deg the longest
 void launch_ee_fill(const int32_t *ev, int64_t E, const int64_t *eid_off, const uint32_t *eid,
                     const int64_t *ee_off, int32_t *ee, int max_deg, cudaStream_t s);
-// Vertex-sharing TT.  far (tt_far_tiles(T) entries, null for none), n_far (zeroed
+// Vertex-sharing TT.  far (tt_far_tiles entries, null for none), n_far (zeroed
 // by the caller, null with far): the runs of 32 cells listed by the count for the
 // kernel that merges in global memory; listed: their number, for the fill.
-int64_t tt_far_tiles(int64_t T);
-void launch_tt_vertex_count(const int4 *tvs, int64_t T, const int64_t *vt_off, const int32_t *vt,
+int64_t tt_far_tiles(int64_t T, int64_t V);
+void launch_tt_vertex_count(const int4 *tvs, int64_t T, int64_t V, const int64_t *vt_off, const int32_t *vt,
                             int32_t *far, int32_t *n_far, int32_t *cnt, cudaStream_t s);
-void launch_tt_vertex_fill(const int4 *tvs, int64_t T, const int64_t *vt_off, const int32_t *vt,
+void launch_tt_vertex_fill(const int4 *tvs, int64_t T, int64_t V, const int64_t *vt_off, const int32_t *vt,
                            const int32_t *far, int32_t *n_far, int64_t listed, const int64_t *tt_off,
                            int32_t *tt, cudaStream_t s);
 

@@ -646,7 +646,7 @@ __device__ __noinline__ void tt_merge_global(const int4 w, int c, const int64_t 
     tt_merge_far<FILL>(w, c, vt_off, vt, cnt, out);
 }
 
-// a warp per 32 cells that k_tt_vertex listed
+// a warp per 32 cells that k_tt_vertex listed (far null: of all cells)
 template <bool FILL>
 __global__ void __launch_bounds__(256)
 k_tt_vertex_far(const int4 *__restrict__ tvs, int64_t T, const int64_t *__restrict__ vt_off,
@@ -654,10 +654,10 @@ k_tt_vertex_far(const int4 *__restrict__ tvs, int64_t T, const int64_t *__restri
                 int *__restrict__ cnt, const int64_t *__restrict__ tt_off, int *__restrict__ tt)
 {
     griddep_wait();
-    const int n = *n_far;
+    const int64_t n = far ? *n_far : (T + 31) / 32;
     for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n;
          i += (int64_t)gridDim.x * (blockDim.x >> 5)) {
-        const int64_t c = 32LL * far[i] + (threadIdx.x & 31);
+        const int64_t c = 32 * (far ? far[i] : i) + (threadIdx.x & 31);
         if (c < T)
             tt_merge_far<FILL>(tvs[c], (int)c, vt_off, vt, FILL ? nullptr : cnt + c,
                                FILL ? tt + tt_off[c] : nullptr);
@@ -976,14 +976,23 @@ void launch_ee_fill(const int32_t *ev, int64_t E, const int64_t *eid_off, const 
 }
 
 // Below kTtFar cells every warp is on the GPU at once whichever kernel has it: no
-// list.
+// list.  With two vertices a cell or more (cells that share little) rows are a
+// word or two, and staging them costs more than merging them: k_tt_vertex_far for
+// all (1.5M cells that share nothing: 23 us a pass against 249).
 constexpr int64_t kTtFar = 1 << 16;
-int64_t tt_far_tiles(int64_t T) { return T >= kTtFar ? (T + 31) / 32 : 0; }
+static bool tt_short_rows(int64_t T, int64_t V) { return V >= 2 * T; }
+int64_t tt_far_tiles(int64_t T, int64_t V) { return T >= kTtFar && !tt_short_rows(T, V) ? (T + 31) / 32 : 0; }
 
-void launch_tt_vertex_count(const int4 *tvs, int64_t T, const int64_t *vt_off, const int32_t *vt,
+void launch_tt_vertex_count(const int4 *tvs, int64_t T, int64_t V, const int64_t *vt_off, const int32_t *vt,
                             int32_t *far, int32_t *n_far, int32_t *cnt, cudaStream_t s)
 {
     if (T == 0) return;
+    if (tt_short_rows(T, V)) {
+        Launch L("k_tt_vertex_far", s);
+        launch_pdl(k_tt_vertex_far<false>, blocks_for(T, 256), 256, 0, s, tvs, T, vt_off, vt, nullptr, nullptr,
+                   cnt, nullptr, nullptr);
+        return;
+    }
     {
         Launch L("k_tt_vertex", s);
         launch_pdl(k_tt_vertex<false>, blocks_for(T, 32 * kTtWarps), 32 * kTtWarps, 0, s, tvs, T, vt_off, vt,
@@ -996,11 +1005,17 @@ void launch_tt_vertex_count(const int4 *tvs, int64_t T, const int64_t *vt_off, c
     }
 }
 
-void launch_tt_vertex_fill(const int4 *tvs, int64_t T, const int64_t *vt_off, const int32_t *vt,
+void launch_tt_vertex_fill(const int4 *tvs, int64_t T, int64_t V, const int64_t *vt_off, const int32_t *vt,
                            const int32_t *far, int32_t *n_far, int64_t listed, const int64_t *tt_off,
                            int32_t *tt, cudaStream_t s)
 {
     if (T == 0) return;
+    if (tt_short_rows(T, V)) {
+        Launch L("k_tt_vertex_far", s);
+        launch_pdl(k_tt_vertex_far<true>, blocks_for(T, 256), 256, 0, s, tvs, T, vt_off, vt, nullptr, nullptr,
+                   nullptr, tt_off, tt);
+        return;
+    }
     if (listed < (T + 31) / 32) {
         Launch L("k_tt_vertex", s);
         launch_pdl(k_tt_vertex<true>, blocks_for(T, 32 * kTtWarps), 32 * kTtWarps, 0, s, tvs, T, vt_off, vt,

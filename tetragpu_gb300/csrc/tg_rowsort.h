@@ -106,8 +106,10 @@ __device__ __forceinline__ void sort_rows_warp(int *row, int n)
         sort_row_net<32>(row, m);
     else if (__any_sync(kAll, m > 16))
         sort_row_net<24>(row, m);
-    else
+    else if (__any_sync(kAll, m > 8))
         sort_row_net<16>(row, m);
+    else if (__any_sync(kAll, m > 1))   // (rows of cells that share little)
+        sort_row_net<8>(row, m);
     for (unsigned mid = __ballot_sync(kAll, n > 32 && n <= 64); mid; mid &= mid - 1) {
         const int src = __ffs(mid) - 1;
         int *r = (int *)__shfl_sync(kAll, (unsigned long long)row, src);

@@ -297,8 +297,92 @@ __device__ __forceinline__ void star_vertex(const StarPass &p, RecBuf<H> &S, int
     }
 }
 
+// Stars of one or two cells (D; 0: none), a lane each: every edge and face by
+// itself, compared with the other cell.  All 32 lanes call it.
+__device__ __forceinline__ bool holds(const int4 &w, int x)
+{
+    return w.x == x || w.y == x || w.z == x || w.w == x;
+}
+constexpr int kFewCells = 2;
+constexpr int kFewLanes = 4;   // in a warp from which on this is less work than a round each
+template <bool F>
+__device__ __forceinline__ void few_cells(const StarPass &p, int v, int rs, int D)
+{
+    const int lane = threadIdx.x & 31;
+    int c[2];
+    int4 w[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        c[q] = q < D ? __ldg(p.vt + rs + q) : -1;
+        w[q] = load_cell(p.tvs, c[q]);
+    }
+    unsigned first = 0u;   // bit 4 q + t: the edge to slot t of cell q, first met there
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            const int u = get4(w[q], t);
+            if (q < D && u > v && !(q == 1 && holds(w[0], u))) first |= 1u << (4 * q + t);
+        }
+    const int own = __popc(first);
+    int end = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(kAll, end, o);
+        if (lane >= o) end += y;
+    }
+    unsigned base = 0u;
+    if (lane == 31) base = atomicAdd(p.n_rec, (unsigned)end);
+    const int64_t g0 = (int64_t)__shfl_sync(kAll, base, 31) + end - own;
+    if (D == 0) return;
+    p.deg_own[v] = own;
+    unsigned place = 0u;
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        const int sv = (w[q].x < v) + (w[q].y < v) + (w[q].z < v);
+#pragma unroll
+        for (int t = 1; t < 4; t++) {   // (slot 0 is never above another vertex of its cell)
+            if (!(first >> (4 * q + t) & 1u)) continue;
+            const int u = get4(w[q], t);
+            const unsigned in = (unsigned)atomicAdd(p.deg_in + u, 1);
+            const unsigned slot = (unsigned)(6 * c[q] + pair_slot(sv, t));
+            atomicOr(p.eflag + (slot >> 5), 1u << (slot & 31));
+            const int64_t g = g0 + place;
+            if (g < p.rec_cap) {
+                p.rec[g] = make_uint2(slot, q == 1 ? 2u : (D == 2 && holds(w[1], u) ? 3u : 1u));
+                p.place[g] = make_uint2(place, in);
+            }
+            place++;
+        }
+        if (q >= D || sv > 1) continue;
+        // faces whose lowest vertex is v: v in slot 0 (all but the one that omits
+        // it) or in slot 1 (the one that omits slot 0)
+        unsigned firsts = 0u, alone = 0u;
+#pragma unroll
+        for (int o = 0; o < 4; o++) {
+            if ((sv == 0) == (o == 0)) continue;
+            const int x = o == 0 || o == 1 ? w[q].z : w[q].y, y = o == 3 ? w[q].z : w[q].w;
+            const bool both = D == 2 && holds(w[1 - q], x) && holds(w[1 - q], y);
+            if (q == 1 && both) continue;   // first met in the other cell
+            firsts |= 8u >> o;
+            if (!both) alone |= 8u >> o;
+            if (F) p.fnext[4LL * c[q] + 3 - o] = both ? c[1 - q] : -1;
+            if (!both) {
+                p.vbnd[v] = 1;
+                p.vbnd[x] = 1;
+                p.vbnd[y] = 1;
+            }
+        }
+        const int sh = 4 * (c[q] & 7);
+        atomicOr(p.fflag + (c[q] >> 3), firsts << sh);
+        if (alone) atomicOr(p.fbnd + (c[q] >> 3), alone << sh);
+    }
+}
+
 // The light vertices of at most kNarrowStar cells; the others go on a list
-// (about in processing order) that k_star_wide takes.
+// (about in processing order) that k_star_wide takes.  Stars of one or two cells
+// go lane by lane where a warp has several: on 1.5M cells that share nothing a
+// warp's round for each takes 1,100 us, this 530.
 template <bool F>
 __global__ void __launch_bounds__(kStarThreads, TG_STAR_MINB) k_star(StarPass p, int per)
 {
@@ -313,6 +397,12 @@ __global__ void __launch_bounds__(kStarThreads, TG_STAR_MINB) k_star(StarPass p,
         lrs = (int)p.vt_off[lv];
         lD = (int)(p.vt_off[lv + 1] - lrs);
         if (lD > kNarrowStar) p.wide[atomicAdd(p.n_wide, 1u)] = lv;
+    }
+    const bool few = lD > 0 && lD <= kFewCells;
+    if (__popc(__ballot_sync(kAll, few)) >= kFewLanes) {
+        few_cells<F>(p, lv, lrs, few ? lD : 0);
+        if (few) lD = 0;
+        if (!__any_sync(kAll, lD > 0)) return;
     }
     auto load_entry = [&](int k) {   // this lane's cell of the k-th vertex (the first 32)
         const int rs = __shfl_sync(kAll, lrs, k & 31), D = __shfl_sync(kAll, lD, k & 31);
@@ -330,7 +420,8 @@ __global__ void __launch_bounds__(kStarThreads, TG_STAR_MINB) k_star(StarPass p,
         if (v < 0) break;
         const int4 w1 = load_cell(p.tvs, c1);
         const int c2 = load_entry(k + 2);
-        if (__shfl_sync(kAll, lD, k) <= kNarrowStar) {
+        const int D = __shfl_sync(kAll, lD, k);
+        if (D > 0 && D <= kNarrowStar) {
             if (n > kRecCap - 3 * kNarrowStar) {   // out with the edges of the vertices before this
                 put_edges<1>(p, S, n, lv, lrs, start);
                 n = 0;
@@ -341,7 +432,7 @@ __global__ void __launch_bounds__(kStarThreads, TG_STAR_MINB) k_star(StarPass p,
             const int4 w[1] = {w0};
             star_vertex<1, F>(p, S, v, c, w, n);
         } else if (lane == k) {
-            start = n;   // no edges here
+            start = n;   // no edges here (a wide star, or done)
         }
         c0 = c1;
         w0 = w1;
