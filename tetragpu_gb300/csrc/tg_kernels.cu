@@ -393,9 +393,10 @@ __device__ __forceinline__ void bitonic_merge(unsigned (&x)[P])
 }
 
 // One edge a lane, rows of at most N entries; a lane's n words of EE (from o;
-// the lanes' rows follow one another) through `stage`.  P: the power of two at
-// or above 2 N; a, b: the rows' first 16 words.
-template <int N, int P>
+// the lanes' rows follow one another) through `stage`, or (APART: some lanes have
+// no part in it) each lane's own stored by itself.  P: the power of two at or
+// above 2 N; a, b: the rows' first 16 words.
+template <int N, int P, bool APART = false>
 __device__ __forceinline__ void ee_merge_lanes(const unsigned (&a)[16], const unsigned (&b)[16],
                                                const unsigned *__restrict__ ra,
                                                const unsigned *__restrict__ rb, unsigned e, int64_t o,
@@ -423,6 +424,12 @@ __device__ __forceinline__ void ee_merge_lanes(const unsigned (&a)[16], const un
         }
     }
     bitonic_merge<P>(x);
+    if constexpr (APART) {
+#pragma unroll
+        for (int i = 0; i < 2 * N; i++)
+            if (i < n + 2 && x[i] != e) ee[o + (x[i] > e ? i - 2 : i)] = (int)x[i];
+        return;
+    }
     const int lane = threadIdx.x & 31;
     const int64_t o0 = __shfl_sync(kFull, o, 0);
     const int shift = (int)(o0 & 3);   // word i of the stage is word i of the line o0 is in
@@ -463,10 +470,11 @@ __device__ __forceinline__ void ee_merge_lanes(const unsigned (&a)[16], const un
 }
 
 // An edge by the whole warp: the same merge over 32 * R positions (lane l holds
-// positions l + 32 r), for rows of at most 16 R entries.
+// positions l + 32 r), for rows of at most 16 R entries; wa, wb: the rows' words,
+// padding included, n: the entries written.
 template <int R>
-__device__ __forceinline__ void ee_merge_warp_r(const unsigned *__restrict__ ra, int na,
-                                                const unsigned *__restrict__ rb, int nb, unsigned e,
+__device__ __forceinline__ void ee_merge_warp_r(const unsigned *__restrict__ ra, int wa,
+                                                const unsigned *__restrict__ rb, int wb, int n, unsigned e,
                                                 int *__restrict__ out, int lane)
 {
     constexpr int P = 32 * R;
@@ -475,7 +483,7 @@ __device__ __forceinline__ void ee_merge_warp_r(const unsigned *__restrict__ ra,
     for (int r = 0; r < R; r++) {
         const int p = lane + 32 * r;
         const int j = P - 1 - p;
-        x[r] = p < P / 2 ? (p < na ? __ldg(ra + p) : ~0u) : (j < nb ? __ldg(rb + j) : ~0u);
+        x[r] = p < P / 2 ? (p < wa ? __ldg(ra + p) : ~0u) : (j < wb ? __ldg(rb + j) : ~0u);
     }
     // strides >= 32: between registers
 #pragma unroll
@@ -502,32 +510,9 @@ __device__ __forceinline__ void ee_merge_warp_r(const unsigned *__restrict__ ra,
 #pragma unroll
     for (int r = 0; r < R; r++) {
         const int p = lane + 32 * r;
-        if (p < na + nb && x[r] != e) out[p - (x[r] > e ? 2 : 0)] = (int)x[r];
+        if (p < n + 2 && x[r] != e) out[p - (x[r] > e ? 2 : 0)] = (int)x[r];
     }
 }
-// entries of a row (at most kMaxDeg; kMaxDeg + 1: more, the heavy path's)
-__device__ __forceinline__ int ee_row_length(const unsigned *__restrict__ row, int lane)
-{
-    int n = 0;
-    while (n <= kMaxDeg) {
-        // words n .. n + 15, then eight at a time: the row goes on while the
-        // last word is an entry
-        const int w = n == 0 ? 16 : 8;
-        const unsigned ends = __ballot_sync(kFull, lane < w && __ldg(row + n + (lane < w ? lane : 0)) == ~0u);
-        if (ends) return min(n + __ffs((int)ends) - 1, kMaxDeg + 1);
-        n += w;
-    }
-    return kMaxDeg + 1;
-}
-__device__ __noinline__ void ee_merge_warp(const unsigned *__restrict__ ra, const unsigned *__restrict__ rb,
-                                           unsigned e, int *__restrict__ out, int lane)
-{
-    const int na = ee_row_length(ra, lane), nb = ee_row_length(rb, lane), m = max(na, nb);
-    if (m > kMaxDeg) return;   // k_ee_heavy's
-    if (m <= 32) ee_merge_warp_r<2>(ra, na, rb, nb, e, out, lane);
-    else ee_merge_warp_r<4>(ra, na, rb, nb, e, out, lane);
-}
-
 // eid: each vertex's incident edges, ascending, from word eid_off[v] on, padded
 // with ~0 to 16 words, or beyond those to a multiple of eight that leaves a
 // ~0 at the end (so that a row's sixteenth word tells whether it goes on).
@@ -576,12 +561,28 @@ k_ee_fill(const int2 *__restrict__ ev, int64_t E, const int64_t *__restrict__ ei
         return;
     }
     if constexpr (ROWS != 0) return;
-    // by the whole warp
-    const int cnt = E - e0 < 32 ? (int)(E - e0) : 32;
-    for (int j = 0; j < cnt; j++) {
+    // the others a lane each all the same, those by the whole warp (but for rows
+    // of more than kMaxDeg entries: k_ee_heavy's)
+    ee_merge_lanes<24, 64, true>(a, b, ra, rb, (unsigned)e, o, longer ? -2 : n, nullptr, ee);
+    int wa = 0, wb = 0;
+    if (longer) {
+        const int2 ab = __ldg(ev + e);
+        wa = (int)(__ldg(eid_off + ab.x + 1) - (ra - eid));
+        wb = (int)(__ldg(eid_off + ab.y + 1) - (rb - eid));
+        // a row of kMaxDeg entries has the words of the few after it
+        constexpr int kLast = (kMaxDeg + 8) & ~7;
+        if (wa > kLast || wb > kLast || (wa == kLast && __ldg(ra + kMaxDeg) != ~0u) ||
+            (wb == kLast && __ldg(rb + kMaxDeg) != ~0u))
+            longer = false;
+    }
+    for (unsigned by_warp = __ballot_sync(kFull, longer); by_warp; by_warp &= by_warp - 1) {
+        const int j = __ffs((int)by_warp) - 1;
         const unsigned *pa = (const unsigned *)__shfl_sync(kFull, (unsigned long long)ra, j);
         const unsigned *pb = (const unsigned *)__shfl_sync(kFull, (unsigned long long)rb, j);
-        ee_merge_warp(pa, pb, (unsigned)(e0 + j), ee + __shfl_sync(kFull, o, j), lane);
+        const int ja = __shfl_sync(kFull, wa, j), jb = __shfl_sync(kFull, wb, j), jn = __shfl_sync(kFull, n, j);
+        int *out = ee + __shfl_sync(kFull, o, j);
+        if (max(ja, jb) <= 32) ee_merge_warp_r<2>(pa, ja, pb, jb, jn, (unsigned)(e0 + j), out, lane);
+        else ee_merge_warp_r<4>(pa, ja, pb, jb, jn, (unsigned)(e0 + j), out, lane);
     }
 }
 
