@@ -1482,7 +1482,13 @@ tg_status tg::link_rows_used(tg_mesh *m, cudaStream_t s)
     return TG_OK;
 }
 
-void tg::note_stream(tg_mesh *m, cudaStream_t s) { m->last_stream.store(s, std::memory_order_relaxed); }
+void tg::note_stream(tg_mesh *m, cudaStream_t s)
+{
+    // (asking whether a stream is being recorded takes a microsecond, a tenth of a
+    // short call)
+    if (m->last_stream.load(std::memory_order_relaxed) == s || capturing(s)) return;
+    m->last_stream.store(s, std::memory_order_relaxed);
+}
 
 // internal: temporaries and segments (tg_batch.cu)
 cudaError_t tg::take_temp(size_t bytes, cudaStream_t s, void **out)

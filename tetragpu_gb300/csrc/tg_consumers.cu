@@ -126,8 +126,7 @@ extern "C" tg_status tg_smooth_field(tg_mesh *mesh, const float *in, float *out,
     cudaStream_t s = (cudaStream_t)stream;
     tg_status st = tg_extract(mesh, TG_VV, 0, stream);   // no-op when VV is resident
     if (st != TG_OK) return st;
-    const bool recorded = capturing(s);
-    if (!recorded) note_stream(mesh, s);   // (with VV resident the extraction did nothing)
+    note_stream(mesh, s);   // (with VV resident the extraction did nothing)
     tg_device_mesh m;
     tg_get_device_mesh(mesh, &m);
     const unsigned grid = (unsigned)std::max<int64_t>((m.n_verts + 255) / 256, 1);
@@ -141,7 +140,7 @@ extern "C" tg_status tg_smooth_field(tg_mesh *mesh, const float *in, float *out,
         return TG_OK;
     }
     // (under capture the steps are recorded by id: nothing is made then)
-    if (m.n_verts >= kOrderVerts && iterations >= kOrderSteps && !recorded) {
+    if (m.n_verts >= kOrderVerts && iterations >= kOrderSteps && !capturing(s)) {
         LinkGraph g{};
         // without the memory for them: by id
         if (link_rows(mesh, s, &g) == TG_OK && g.off) {

@@ -372,7 +372,7 @@ tg_status link_rows(tg_mesh *m, cudaStream_t s, LinkGraph *out);
 // after the last work on the stream that reads those rows
 tg_status link_rows_used(tg_mesh *m, cudaStream_t s);
 // the mesh's memory is used on the stream (the mesh's frees are ordered on the
-// last one)
+// last one; not if the work is being recorded)
 void note_stream(tg_mesh *m, cudaStream_t s);
 // work on the stream is being recorded, not run
 bool capturing(cudaStream_t s);
