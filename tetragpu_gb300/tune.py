@@ -12,9 +12,10 @@ the link adjacency + critical points + destroy; CUDA events, L2 flushed
 before every step) on each size bucket of the uneven 512-mesh batch (its
 meshes grouped by tet count, each bucket run as a batch of its own) and on
 the whole batch.  It records every time in tetragpu_gb300/tuning.json
-together with the best setting of each bucket and the setting it selects:
-the one with the smallest total over the buckets, with its margin to each
-bucket's best.  --apply merges the selected change into the TUNED block of
+together with the best setting of each bucket and the setting it selects,
+with its margin to each bucket's best: the one with the smallest total over the
+buckets if it leads the default by more than LEAD_PCT there and trails it by no
+more in any bucket, else the default.  --apply merges the selected change into the TUNED block of
 csrc/tg_tuning.h (the settings the default build compiles in).
 
 The batch runs as one disjoint-union mesh, so every kernel launches once per
@@ -51,6 +52,8 @@ CANDIDATES = [
     ("vt_sort_threads_256", {"TG_VTS_THREADS": 256}),
     ("edge_items_8", {"TG_EDGE_ITEMS": 8}),
 ]
+# two sweeps of one build differ by up to this much: a smaller lead is none
+LEAD_PCT = 1.0
 # tet-count buckets of the batch's meshes: [lo, hi)
 BUCKETS = [(2000, 20000), (20000, 100000), (100000, 400001)]
 
@@ -123,6 +126,19 @@ def write_header(defines: dict, path: str = TUNING_H):
         fh.write(head + "// BEGIN TUNED\n" + body + "// END TUNED\n" + tail)
 
 
+def select(results: dict, buckets) -> str:
+    """The setting to compile in (results: ms per batch, by setting)."""
+    def total(name):
+        return sum(results[name][i] for i in buckets)
+    best = min(results, key=total)
+    base, lead = results.get("default"), 1.0 + LEAD_PCT / 100.0
+    if base is None:
+        return best
+    if total(best) * lead >= total("default") or any(results[best][i] > base[i] * lead for i in buckets):
+        return "default"
+    return best
+
+
 def main(argv=None):
     ap = argparse.ArgumentParser(description=__doc__.split("\n\n")[0])
     ap.add_argument("--steps", type=int, default=5)
@@ -151,7 +167,7 @@ def main(argv=None):
     labels = [b[0] for b in batches]
     bucket_idx = [i for i, lab in enumerate(labels) if lab != "all"]
     best = {labels[i]: min(results, key=lambda n: results[n][i]) for i in range(len(labels))}
-    selected = min(results, key=lambda n: sum(results[n][i] for i in bucket_idx))
+    selected = select(results, bucket_idx)
     margin = {labels[i]: round(100.0 * (results[selected][i] / results[best[labels[i]]][i] - 1.0), 2)
               for i in range(len(labels))}
     rec = {
