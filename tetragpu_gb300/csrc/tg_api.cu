@@ -693,7 +693,8 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
         // surface has two faces a vertex.  A large mesh that has more goes through
         // the pass again.  16 to 20 bytes each: all of six would be 0.9 GB more at
         // 128^3 cubes
-        for (sp.rec_cap = T >= kFewRecords ? std::min(6 * T, T + 2 * V) : 6 * T;; sp.rec_cap = 6 * T) {
+        for (int64_t room = T >= kFewRecords ? std::min(6 * T, T + 2 * V) : 6 * T;; room = 6 * T) {
+            sp.rec_last = (unsigned)std::max<int64_t>(room, 1) - 1;
             // the bitmaps the star pass sets bits in, the neighbour counts
             // and the record counter are zeroed
             Plan t;
@@ -710,9 +711,9 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
             t.add(&brank, nwf + 1);
             t.add(&deg_sq, V + 1);   // prefix of deg^2: its total sizes EE (sum deg^2 - 2E)
             if (want_ee) t.add(&eid_off, V + 1);   // EE's incident-edge rows are padded
-            t.add(&sp.rec, sp.rec_cap);
-            t.add(&sp.place, sp.rec_cap);
-            if (m->n_wide > 0 || m->n_heavy > 0) t.add(&sp.rec_hi, sp.rec_cap);
+            t.add(&sp.rec, room);
+            t.add(&sp.place, room);
+            if (m->n_wide > 0 || m->n_heavy > 0) t.add(&sp.rec_hi, room);
             if (m->n_wide > 0) t.add(&sp.wide, m->n_wide);
             if (m->n_heavy > 0) t.add(&hv.pairs, 3 * m->heavy_entries);
             if (need_tf || need_ft) t.add(&sp.fnext, 4 * T);
@@ -741,7 +742,7 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
             const bool w8[6] = {true, false, false, false, true, true};
             TRY(sync_read(m, s, want_ee ? 6 : 5, src, w8));
             if (m->st_host->flags) return check_flags(m);
-            if (m->sz_host[1] <= sp.rec_cap) break;
+            if (m->sz_host[1] <= room) break;
             tmp.drop();
         }
         m->max_deg = m->st_host->max_deg > kMaxDeg ? m->st_host->max_deg : 0;

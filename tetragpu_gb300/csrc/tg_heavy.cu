@@ -174,13 +174,10 @@ __global__ void __launch_bounds__(64) k_heavy(HeavyStars h)
                 note_lowest(&p.st->bad_vertex, v);
             }
             set_bit(p.eflag, slot);
-            const unsigned g = atomicAdd(p.n_rec, 1u);
-            const uint2 place = make_uint2((unsigned)n_own++, (unsigned)atomicAdd(p.deg_in + u, 1));
-            if (g < p.rec_cap) {
-                p.rec[g] = make_uint2((unsigned)slot, (unsigned)(pair0 + s0));
-                p.place[g] = place;
-                p.rec_hi[g] = (unsigned)n_et;
-            }
+            const unsigned g = min(atomicAdd(p.n_rec, 1u), p.rec_last);
+            p.rec[g] = make_uint2((unsigned)slot, (unsigned)(pair0 + s0));
+            p.place[g] = make_uint2((unsigned)n_own++, (unsigned)atomicAdd(p.deg_in + u, 1));
+            p.rec_hi[g] = (unsigned)n_et;
         }
         s0 = s1;
     }

@@ -221,8 +221,9 @@ struct StarPass {
                                // occurrence, or null
     int32_t *deg_own;          // [V] edges a vertex is the low end of (zeroed by the caller)
     int32_t *deg_in;           // [V] edges it is the high end of (zeroed by the caller)
-    // a record per edge, in no particular order; those past rec_cap are counted only:
-    int64_t rec_cap;
+    // a record per edge, in no particular order; those past the room are counted
+    // only (and written over the last)
+    unsigned rec_last;         // the room less one
     uint2 *rec;                // {first occurrence slot, star positions of the low end's star
                                // holding the edge (the low 32)}
     uint2 *place;              // {place among the low end's own edges, among the high end's others}
