@@ -631,7 +631,8 @@ __global__ void __launch_bounds__(256) k_edge_ids(EdgePass p)
 constexpr int kRowsThreads = 128;
 constexpr int kRowsTake = 16;                // cells an edge lists at a time
 constexpr int kRowsCap = 32 * kRowsTake;
-template <bool W>
+// EF: whether EF rows are wanted
+template <bool W, bool EF>
 __global__ void __launch_bounds__(kRowsThreads) k_edge_rows(EdgePass p)
 {
     griddep_wait();
@@ -643,7 +644,7 @@ __global__ void __launch_bounds__(kRowsThreads) k_edge_rows(EdgePass p)
     int v = 0, u = 0, rs = 0, et = 0, ef = 0;
     // EF has up to 12T entries, past 2^31: the warp's rows from an int64 start,
     // a lane's within them (below 32 * 2^16)
-    const int64_t ef0 = p.ef ? __ldg(p.ef_off + (id & ~(int64_t)31)) : 0;
+    const int64_t ef0 = EF ? __ldg(p.ef_off + (id & ~(int64_t)31)) : 0;
     int *const ef_out = p.ef + ef0;
     unsigned long long m = 0ull;
     if (id < p.E) {
@@ -654,7 +655,7 @@ __global__ void __launch_bounds__(kRowsThreads) k_edge_rows(EdgePass p)
         if (p.ev) reinterpret_cast<int2 *>(p.ev)[id] = make_int2(v, u);
         rs = (int)__ldg(p.vt_off + v);
         if (p.et) et = (int)__ldg(p.et_off + id);
-        if (p.ef) ef = (int)(__ldg(p.ef_off + id) - ef0);
+        if constexpr (EF) ef = (int)(__ldg(p.ef_off + id) - ef0);
         m = rec.y;
         if constexpr (W) {
             const int D = (int)(__ldg(p.vt_off + v + 1) - rs);
@@ -667,7 +668,7 @@ __global__ void __launch_bounds__(kRowsThreads) k_edge_rows(EdgePass p)
                     slots_of(__ldg(p.tvs + c), v, u, s, t);
                     if (p.te) p.te[6LL * c + pair_slot(s, t)] = (int)id;
                     if (p.et) p.et[et + k] = c;
-                    if (p.ef) {
+                    if constexpr (EF) {
                         const uint2 rk = __ldg(p.frank + (c >> 3));
                         const int sh = 4 * (c & 7);
                         const unsigned out = (rk.x >> sh) & 0xfu & ~((8u >> s) | (8u >> t));
@@ -717,7 +718,7 @@ __global__ void __launch_bounds__(kRowsThreads) k_edge_rows(EdgePass p)
                 const int b = __shfl_sync(kAll, etb, l);
                 if (act) p.et[b + i] = c;
             }
-            if (p.ef) {
+            if constexpr (EF) {
                 const int t1 = s == 0 ? (t == 1 ? 2 : 1) : 0, t2 = 6 - s - t - t1;
                 const uint2 rk = act ? __ldg(p.frank + (c >> 3)) : make_uint2(0u, 0u);
                 // columns 3 - t2 < 3 - t1
@@ -1256,9 +1257,9 @@ void launch_edge_rows(const EdgePass &p, cudaStream_t s)
     Launch L("k_edge_rows", s);
     const unsigned grid = (unsigned)((p.E + kRowsThreads - 1) / kRowsThreads);
     if (p.rec_hi)
-        launch_pdl(k_edge_rows<true>, grid, kRowsThreads, 0, s, p);
+        launch_pdl(p.ef ? k_edge_rows<true, true> : k_edge_rows<true, false>, grid, kRowsThreads, 0, s, p);
     else
-        launch_pdl(k_edge_rows<false>, grid, kRowsThreads, 0, s, p);
+        launch_pdl(p.ef ? k_edge_rows<false, true> : k_edge_rows<false, false>, grid, kRowsThreads, 0, s, p);
 }
 
 void launch_vt_sort(const int64_t *vt_off, int32_t *vt, int64_t V, int64_t nvt, const int4 *tvs,
