@@ -100,8 +100,8 @@ typedef struct tg_mesh tg_mesh;
 /* Library version string. */
 const char *tg_version(void);
 
-/* The tile parameters this build's kernels use (star-pass windows, block
- * sizes, lanes per edge; the values tetragpu_gb300/tune.py selects), as a
+/* The tile parameters this build's kernels use (vertices per star-pass warp,
+ * block sizes, edges per thread; tetragpu_gb300/tune.py measures others), as a
  * JSON object. */
 const char *tg_tuning_info(void);
 
@@ -378,7 +378,7 @@ tg_status tg_server_copy_relation(tg_server *server, int64_t mesh_id, int relati
 tg_status tg_server_release_mesh(tg_server *server, int64_t mesh_id);
 tg_status tg_server_get_stats(tg_server *server, tg_server_stats *out);
 
-/* Time every launch of one kernel (by name, e.g. "k_star_b") with CUDA
+/* Time every launch of one kernel (by name, e.g. "k_star") with CUDA
  * events recorded on the stream it is launched on; NULL or "" turns timing
  * off.  For measurement tools; the reference's analogue is its Timer class
  * (src/metrics.cpp).  Not thread-safe against concurrent extractions. */

@@ -62,3 +62,32 @@ def test_among_others(gpu_lib, oracle):
     tv = np.concatenate(tvs)
     _check(gpu_lib, oracle, tv, n, 1)
     _check(gpu_lib, oracle, tv[np.random.default_rng(3).permutation(len(tv))], n, 2)
+
+
+def test_with_heavy_vertices(gpu_lib, oracle):
+    """Short rows on average, but vertices of more than 64 neighbours too (and of
+    33 to 64), some of them in the same windows of the link masks."""
+    tvs, n = [], 0
+    for k in (80, 70, 40, 25, 66):     # fans around a vertex, rings around an edge
+        tvs.append(n + np.stack([0 * np.arange(k), *(3 * np.arange(k) + j for j in (1, 2, 3))], 1))
+        n += 3 * k + 1
+        i = np.arange(k)
+        tvs.append(np.stack([0 * i + n, 0 * i + n + 1, n + 2 + i, n + 2 + (i + 1) % k], 1))
+        n += k + 2
+    tv, n = _pairs(3000, 0, n)
+    tvs.append(tv)
+    _check(gpu_lib, oracle, np.concatenate(tvs), n, 3)
+
+
+def test_in_a_batch(gpu_lib, oracle):
+    rng = np.random.default_rng(4)
+    meshes = [_pairs(40 * i, shared, 0) for i, shared in ((1, 0), (30, 2), (3, 1), (50, 0))]
+    meshes = [(rng.permutation(n)[tv].astype(np.int32), n) for tv, n in meshes]
+    fields = [[rng.standard_normal(n).astype(d) for d in (np.float32, np.float64)] for _, n in meshes]
+    with gpu_lib.Server(n_slots=1) as srv:
+        sent = [srv.submit_mesh(tv, n, f[0]) for (tv, n), f in zip(meshes, fields)]
+        got = [[srv.wait(rid)[0], srv.wait(srv.submit_field(mid, f[1]))[0]] for (rid, mid), f in zip(sent, fields)]
+    for (tv, n), f, g in zip(meshes, fields, got):
+        tvs = oracle.canonicalize(tv, n)
+        for k in range(2):
+            assert np.array_equal(g[k], oracle.critical_points(tvs, n, f[k]))

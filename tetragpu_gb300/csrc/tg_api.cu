@@ -5,7 +5,7 @@
 // with an unlimited release threshold, so repeated extractions reuse blocks
 // instead of returning them to the driver; a stage's arrays come out of one
 // allocation each for what stays and what does not (some forty calls a step
-// before: 357 -> 308 us at 24,576 cells, 24 requests to the server 5.6 -> 3.2
+// before: 357 -> 308 us at 24,576 cells, 24 requests to the server 5.6 -> 4.8
 // ms).  tg_extract synchronises the stream at two points, to learn the
 // edge/face/neighbour counts and then the CSR totals that size the outputs;
 // everything between those points is asynchronous on the caller's stream.

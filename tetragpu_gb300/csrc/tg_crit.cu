@@ -37,9 +37,11 @@ namespace {
 
 // ---------------------------------------------------------------------------
 // Rows into processing order, each padded with -1 to whole 32-byte sectors (so
-// that a thread loads eight entries at once): sixteen lanes copy a row, four rows' loads in flight; a thread sorts it (a
-// word between the rows in shared memory: 16-word rows would all begin in two
-// banks).
+// that a thread loads eight entries at once): sixteen lanes copy a row, four rows'
+// loads in flight; a thread sorts it (a word between the rows in shared memory:
+// 16-word rows would all begin in two banks).  Nine blocks to an SM spill 32 bytes
+// a thread, eight none: 79 and 76 us at 96^3 cubes, 37.6 and 38.9 on the 64^3
+// coned mesh.
 constexpr int kOrderThreads = 128;
 constexpr int kOrderCap = 24 * kOrderThreads;
 constexpr int kOrderRows = 4;
@@ -417,13 +419,15 @@ k_crit_adj(const int64_t *__restrict__ off, const int *__restrict__ ent, const i
 // ---------------------------------------------------------------------------
 constexpr int kClassifyThreads = 128;
 // From kOrderField vertices on the field is put in processing order first (a
-// launch and a buffer: 3 us), so that a block's field gathers lie together;
-// below, they hit L1 and L2 anyway.  A call by id and in order: 9.3 and 11.4 us
-// at 4,913 vertices, 11.2 and 11.4 us at 118k, 15.0 and 13.0 us at 185k, 180
-// and 105 us at 2.1M.
+// launch and a buffer: 3 to 4 us), so that a block's field gathers lie together;
+// below, they hit L1 and L2 anyway.  A call by id and in order, grids with ids
+// permuted: 11.6 and 16.3 us at 4,913 vertices, 16.0 and 17.2 at 118k, 18.6 and
+// 18.5 at 185k, 24.0 and 21.8 at 275k, 143 and 95 at 2.1M (float64 17.7 and 20.2,
+// 19.9 and 22.5, 27.0 and 26.7, 152 and 119 from 118k on).
 // The rows of smaller meshes are kept as vertices too, one gather of a chain
-// of four fewer: 21.0 -> 20.3 us a call on 16^3 coned cubes.
-// a field's values by position: of every vertex (vpos null: a thread per
+// of four fewer.
+//
+// A field's values by position: of every vertex (vpos null: a thread per
 // position), or of the vertices from v0 on (a thread per vertex)
 template <typename F>
 __global__ void __launch_bounds__(256)

@@ -370,8 +370,10 @@ k_face_fill(const int *__restrict__ ft, const int *__restrict__ tf, const int *_
 // requests to L2 an edge (0.8 a clock and SM, what gets through; now 4) and 33
 // warp instructions (19): 92 -> 64 us at 64^3, 135 -> 93 us beside other kernels
 // on the 64^3 coned mesh, whose rows pass 16.  Without bank conflicts of rows of
-// one length (rows below 16) and with eleven blocks of these to an SM: 545 -> 533
-// us at 128^3 beside other kernels.
+// one length (rows below 16) and with eleven blocks of these to an SM (20 bytes of
+// spills a thread): 545 -> 533 us at 128^3 beside other kernels.  A warp with
+// longer ends: the short rows a lane each, stored as they are, the others by the
+// whole warp (all of them so: 294 us instead of 152 on 200,000 Delaunay vertices).
 constexpr int kEeThreads = 128;
 constexpr int kEeWarps = kEeThreads / 32;
 // words that a warp's rows come to, of ends of at most N edges

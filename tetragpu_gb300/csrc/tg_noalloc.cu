@@ -1,7 +1,7 @@
 // tg_noalloc.cu -- critical-point classification that allocates no memory.
 //
-// tg_critical_points builds the link adjacency of every vertex (one 64-bit
-// mask per VV entry) in memory it allocates and caches on the mesh.  Some
+// tg_critical_points builds the link adjacency of every vertex (a mask per
+// entry of its copy of VV) in memory it allocates and caches on the mesh.  Some
 // callers cannot allocate device memory when they classify: a host
 // application that hands this library a fixed device-memory budget at
 // start-up and accounts for every byte afterwards, or a real-time loop whose
@@ -9,7 +9,7 @@
 // it runs.  tg_critical_points_noalloc serves them: the caller passes VV
 // (device CSR), the field and the output, and the adjacency lives in
 // file-scope device arrays of fixed size, TG_NOALLOC_MAX_VV_ENTRIES masks
-// (64 MiB) plus their window table (128 KiB), which every GPU that loads
+// (64 MiB of 64-bit ones) plus their window table (128 KiB), which every GPU that loads
 // this library holds until the process exits.  The call reads the kernels'
 // status word back and waits for its stream to do so.
 #include <climits>

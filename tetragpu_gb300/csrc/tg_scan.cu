@@ -14,8 +14,9 @@
 // A warp takes rows of 64 elements, two neighbours to a lane, so that its loads
 // and stores are whole lines: the four scans of an extraction of all relations
 // at 128^3 cubes take 105 us (140 with eight consecutive elements to a thread,
-// 128 with four elements a thread and six blocks to an SM); what is left is the
-// look-back's latency.
+// 128 with four elements a thread and six blocks to an SM; 114 without the bound
+// of five blocks, which spills 4 bytes a thread); what is left is the look-back's
+// latency.
 #include "tg_internal.h"
 
 namespace tg {

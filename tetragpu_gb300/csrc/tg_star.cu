@@ -843,7 +843,8 @@ k_vv_sort(const int64_t *__restrict__ off, int64_t V, int64_t total, int *__rest
 
 // VV and incident-edge rows from inc (the same rows, {neighbour, edge id}
 // pairs), each sorted by itself; the incident-edge rows padded with ~0 to
-// eid_words at eid_off
+// eid_words at eid_off.  Nine blocks to an SM spill 32 bytes a thread: 64 us at
+// 96^3 cubes, 66 with eight and no spills.
 constexpr int kIncCap = 20 * kVtsThreads;
 __global__ void __launch_bounds__(kVtsThreads, 9)
 k_inc_sort(const int64_t *__restrict__ off, int64_t V, const int2 *__restrict__ inc,
@@ -902,7 +903,8 @@ k_inc_sort(const int64_t *__restrict__ off, int64_t V, const int2 *__restrict__ 
 // request carries whole lines; ET and EF lengths are summed in the halves of
 // one word.  172 us at 128^3 cubes (208 with eight consecutive edges to a
 // thread, whose 128 bytes were lines of their own); its 0.9 GB take 135 at the
-// copy rate.
+// copy rate.  Six blocks to an SM spill 36 bytes a thread and are still ahead:
+// 190 us with four.
 constexpr int kEdgeThreads = 256;
 constexpr int kEdgeItems = TG_EDGE_ITEMS;             // edges per thread
 constexpr int kEdgeTile = kEdgeItems * kEdgeThreads;  // edges per tile
