@@ -63,6 +63,7 @@ k_smooth_ordered(const int64_t *__restrict__ off, const int *__restrict__ ent, i
 // 64^3, 433 against 604 on 128^3, but 74 against 72 on 48^3 (0.12 M), where
 // both kinds of step are bound by their launches.
 constexpr int64_t kOrderVerts = 1 << 17;
+static_assert(kOrderVerts >= kOrderField, "whether ids are as good is known from there on");
 // The vertices, the steps and the mesh's order alone decide, so that a call gives
 // the same bits whether or not the mesh has those rows already.  Meshes whose
 // link graph is in the order of ids stay by id (lg_by_id, tg_api.cu): ten steps
