@@ -129,8 +129,10 @@ tg_status tg_tv_narrow_i64(const int64_t *cells, int64_t n_cells, int64_t n_poin
 tg_status tg_mesh_create_i64(const int64_t *tv, int64_t n_cells, int64_t n_verts, void *stream,
                              tg_mesh **out);
 
-/* Frees the mesh's device memory, ordered on the stream of its last call and
- * waiting for that stream: destroy a mesh before the stream it last used. */
+/* Frees the mesh's device memory, ordered on the stream of its last call
+ * (tg_smooth_field is waited for on whatever streams it ran, and does not count
+ * as one) and waiting for that stream: destroy a mesh before the stream it last
+ * used. */
 tg_status tg_mesh_destroy(tg_mesh *mesh);
 
 /* Extract every relation whose bit is set (plus what they depend on) and keep

@@ -411,9 +411,12 @@ struct LinkArrays {
 
 struct tg_mesh {
     int device = 0;
-    // stream of the last call, which frees are ordered on (smoothing and
-    // classification of one mesh may come from several threads)
+    // stream of the last call, which frees are ordered on (classifications of
+    // one mesh may come from several threads)
     std::atomic<cudaStream_t> last_stream{nullptr};
+    // streams that smoothed over the mesh besides, with an event after that each
+    // (lg_mu)
+    std::vector<std::pair<cudaStream_t, cudaEvent_t>> readers;
     int64_t V = 0, T = 0, E = -1, F = -1;
     void *base = nullptr;       // one allocation: everything from here to VT, the scan workspace
                                 // and the status word
@@ -442,7 +445,6 @@ struct tg_mesh {
     std::mutex lg_mu;                // while a call looks for them or builds them
     cudaEvent_t lg_done = nullptr;   // after the build of either outside an extraction
     bool lg_pending = false;         // which has not been seen to be over
-    cudaEvent_t lg_used = nullptr;   // after the last smoothing over the rows
     DevStatus *st = nullptr;    // device
     DevStatus *st_host = nullptr;
     int64_t *sz_host = nullptr; // pinned slots for sizes read back at sync points
@@ -525,14 +527,15 @@ void set_csr(tg_mesh *m, int r, int64_t *off, int32_t *ent, int64_t rows, int64_
     x.opts = opts;
 }
 
-// The link graph is built, and smoothed over, on the caller's stream, which
-// need not be the one the mesh's memory goes back on: what frees it, or the VV
-// it is built from, waits for both first.
-void await_link_graph(tg_mesh *m)
+// The link graph is built, and VV and it are smoothed over, on the caller's
+// stream, which need not be the one the mesh's memory goes back on: what frees
+// any of them waits for all of that first.
+void await_readers(tg_mesh *m)
 {
     const cudaStream_t s = m->last_stream.load(std::memory_order_relaxed);
+    std::lock_guard<std::mutex> lk(m->lg_mu);
     if (m->lg_pending) cudaStreamWaitEvent(s, m->lg_done, 0);
-    if (m->lg_used) cudaStreamWaitEvent(s, m->lg_used, 0);
+    for (const auto &r : m->readers) cudaStreamWaitEvent(s, r.second, 0);
 }
 
 void free_link_graph(tg_mesh *m)
@@ -833,7 +836,7 @@ tg_status run_extract(tg_mesh *m, uint32_t mask, uint32_t opts, cudaStream_t s)
             launch_edge_offsets(ep, et_off, ef_off, ee_off, ev_with_rows ? nullptr : ev, m->scan, m->st, s);
         if (inc) launch_inc_sort(vv_off, V, inc, vv, eid_off, eid, s);
         else launch_vv_sort(vv_off, V, nvv, vv, s);
-        await_link_graph(m);
+        await_readers(m);
         set_csr(m, TG_REL_VV, vv_off, vv, V, nvv, hold_vv_off, hold_vv);
         free_link_graph(m);
 
@@ -1017,7 +1020,7 @@ tg_status tg_mesh_destroy(tg_mesh *m)
     // stream-ordered frees on the stream the mesh was last used on, then one
     // wait for that stream (no device-wide synchronisation)
     const cudaStream_t s = m->last_stream.load(std::memory_order_relaxed);
-    await_link_graph(m);
+    await_readers(m);
     for (auto &r : m->rel) r = Rel();
     free_link_graph(m);
     if (m->seg_c) cudaFreeAsync(m->seg_c, s);
@@ -1030,7 +1033,7 @@ tg_status tg_mesh_destroy(tg_mesh *m)
     cudaStreamSynchronize(s);  // no copy into the pinned slots is still in flight
     if (m->scan.done) cudaEventDestroy(m->scan.done);
     if (m->lg_done) cudaEventDestroy(m->lg_done);
-    if (m->lg_used) cudaEventDestroy(m->lg_used);
+    for (const auto &r : m->readers) cudaEventDestroy(r.second);
     g_pinned.put(m->st_host);
     g_pinned.put(m->sz_host);
     cudaSetDevice(cur);
@@ -1475,20 +1478,27 @@ tg_status tg::link_rows(tg_mesh *m, cudaStream_t s, LinkGraph *out)
     return TG_OK;
 }
 
-tg_status tg::link_rows_used(tg_mesh *m, cudaStream_t s)
+tg_status tg::note_reader(tg_mesh *m, cudaStream_t s, bool rows)
 {
+    // on the mesh's own stream what frees VV comes later anyway (the rows may be
+    // freed from another).  (Asking whether a stream is being recorded takes a
+    // microsecond, a tenth of a short call.)
+    if (!rows && (m->last_stream.load(std::memory_order_relaxed) == s || capturing(s))) return TG_OK;
     std::lock_guard<std::mutex> lk(m->lg_mu);
-    if (!m->lg_used) CK(cudaEventCreateWithFlags(&m->lg_used, cudaEventDisableTiming));
-    CK(cudaEventRecord(m->lg_used, s));
+    cudaEvent_t done = nullptr;
+    for (const auto &r : m->readers)
+        if (r.first == s) done = r.second;
+    if (!done) {
+        CK(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
+        try {
+            m->readers.push_back({s, done});
+        } catch (const std::bad_alloc &) {
+            cudaEventDestroy(done);
+            return fail(TG_ERR_OUT_OF_MEMORY, "host memory");
+        }
+    }
+    CK(cudaEventRecord(done, s));
     return TG_OK;
-}
-
-void tg::note_stream(tg_mesh *m, cudaStream_t s)
-{
-    // (asking whether a stream is being recorded takes a microsecond, a tenth of a
-    // short call)
-    if (m->last_stream.load(std::memory_order_relaxed) == s || capturing(s)) return;
-    m->last_stream.store(s, std::memory_order_relaxed);
 }
 
 // internal: temporaries and segments (tg_batch.cu)

@@ -127,7 +127,6 @@ extern "C" tg_status tg_smooth_field(tg_mesh *mesh, const float *in, float *out,
     cudaStream_t s = (cudaStream_t)stream;
     tg_status st = tg_extract(mesh, TG_VV, 0, stream);   // no-op when VV is resident
     if (st != TG_OK) return st;
-    note_stream(mesh, s);   // (with VV resident the extraction did nothing)
     tg_device_mesh m;
     tg_get_device_mesh(mesh, &m);
     const unsigned grid = (unsigned)std::max<int64_t>((m.n_verts + 255) / 256, 1);
@@ -161,7 +160,7 @@ extern "C" tg_status tg_smooth_field(tg_mesh *mesh, const float *in, float *out,
                 set_last_error(cudaGetErrorString(e));
                 return TG_ERR_CUDA;
             }
-            return link_rows_used(mesh, s);
+            return note_reader(mesh, s, true);
         }
     }
     // steps alternate between out and scratch so that the last one lands in out
@@ -179,5 +178,5 @@ extern "C" tg_status tg_smooth_field(tg_mesh *mesh, const float *in, float *out,
         set_last_error(cudaGetErrorString(e));
         return TG_ERR_CUDA;
     }
-    return TG_OK;
+    return note_reader(mesh, s, false);
 }

@@ -370,11 +370,9 @@ void set_last_error(const char *msg);
 // the mesh's VV by position, made if it has none yet (off null when there is no
 // memory for it or positions are ids), VV being extracted
 tg_status link_rows(tg_mesh *m, cudaStream_t s, LinkGraph *out);
-// after the last work on the stream that reads those rows
-tg_status link_rows_used(tg_mesh *m, cudaStream_t s);
-// the mesh's memory is used on the stream (the mesh's frees are ordered on the
-// last one; not if the work is being recorded)
-void note_stream(tg_mesh *m, cudaStream_t s);
+// the stream was given work that reads the mesh's VV or (rows) VV by position:
+// what frees them waits for it, whatever the mesh's last stream
+tg_status note_reader(tg_mesh *m, cudaStream_t s, bool rows);
 // work on the stream is being recorded, not run
 bool capturing(cudaStream_t s);
 // field values of every vertex by position
